@@ -49,6 +49,19 @@ def _fp16_scale(d: int, bits: int) -> float:
     return _fp16_scales[key]
 
 
+_proj_rot_cache: dict[tuple[int, int, int, str], torch.Tensor] = {}
+
+
+def _rotated_projection(d: int, m: int, rotation_seed: int, device) -> torch.Tensor:
+    """S @ R^T (m, d), float32, cached per (d, m, seed, device) like the matrices it is made of."""
+    key = (d, m, rotation_seed, str(device))
+    if key not in _proj_rot_cache:
+        s = generate_projection_matrix_host(d, m).astype("float64")
+        r = generate_rotation_matrix_host(d, rotation_seed).astype("float64")
+        _proj_rot_cache[key] = torch.from_numpy((s @ r.T).astype("float32")).to(device)
+    return _proj_rot_cache[key]
+
+
 class _Side:
     """Packed storage of one side (keys or values): codes, norms and the optional QJL sketch."""
 
@@ -77,10 +90,10 @@ class _Side:
         w_hi, w_lo = kernels.packed_widths(d, self.bits_hi, self.bits_lo)
 
         def grow(old, shape, dtype):
-            if old is None:   # e.g. a sketch that a reloaded state did not carry: zero = no correction
+            if old is None and used > 0:   # a sketch that a reloaded state did not carry: zero = no correction
                 return torch.zeros(shape, dtype=dtype, device=device)
             new = torch.empty(shape, dtype=dtype, device=device)
-            if used > 0:
+            if old is not None and used > 0:
                 new[:, :, :used] = old[:, :, :used]
             return new
 
@@ -152,9 +165,7 @@ class TurboQuantKVCache:
                                                  self._v.cent_hi, self._v.bits_hi, self._v.fp16_scale_hi)
         if self.qjl_correction:
             self._qjl_proj = get_projection_matrix(d, self.qjl_n_proj, device=device)
-            s = generate_projection_matrix_host(d, self.qjl_n_proj).astype("float64")
-            r = generate_rotation_matrix_host(d, self.rotation_seed).astype("float64")
-            self._qjl_proj_rot = torch.from_numpy((s @ r.T).astype("float32")).to(device)
+            self._qjl_proj_rot = _rotated_projection(d, self.qjl_n_proj, self.rotation_seed, device)
 
     @property
     def rotation(self):
@@ -284,51 +295,65 @@ class TurboQuantKVCache:
         return dict(proj_rot=self._qjl_proj_rot, cent_hi=side.cent_hi, cent_lo=side.cent_lo,
                     bits=side.qbits, gamma=side.qgamma)
 
-    def _drain_chunk(self, n: int) -> None:
-        """Compress and evict the first n recent tokens (cache.py:535-575).
-
-        The kernels read the buffer before the remaining tokens are shifted to the front (both
-        are ordered on the current stream), so the chunk is never overwritten first.
-        """
-        b, h, _, d = self.keys.shape
-        dev = self.keys.device
-        for side, buf in ((self._k, self.keys), (self._v, self.values)):
-            side.reserve(b, h, d, self._compressed_len + n, self._compressed_len, dev, self.qjl_correction)
-            kernels.quantize_pack(buf[:, :, :n], self._rotation, side.bnd_hi, side.bits_hi, side.bnd_lo, side.bits_lo,
-                                  out_hi=side.hi, out_lo=side.lo, out_norms=side.norms,
-                                  out_offset=self._compressed_len, qjl=self._qjl_args(side))
-        rem = self._fp16_len - n
-        # A long prefill leaves buffers sized for the whole prompt; once most of it is packed they are swapped for
-        # buffers of the size a fresh cache would get for what remains (batch 64 x 32K tokens: 17 GB per layer otherwise).
-        small_cap = max(rem, self.residual_window * 2) + 256
-        if self._fp16_capacity > 4 * small_cap:
-            nk = torch.zeros((b, h, small_cap, d), dtype=self.keys.dtype, device=dev)
-            nv = torch.zeros((b, h, small_cap, d), dtype=self.values.dtype, device=dev)
-            if rem > 0:
-                self._append(nk, nv, self.keys[:, :, n:self._fp16_len], self.values[:, :, n:self._fp16_len], 0)
-            self.keys, self.values, self._fp16_capacity = nk, nv, small_cap
-        elif rem > 0:
-            for buf in (self.keys, self.values):
-                tail = buf[:, :, n:self._fp16_len]
-                buf[:, :, :rem] = tail.clone() if n < rem else tail
-        self._fp16_len = rem
-        self._compressed_len += n
-
-    def _compress_old_tokens(self) -> None:
-        """Drain schedule (cache.py:497-533)."""
-        if self.keys is None:
-            return
+    def _due(self, length: int) -> int:
+        """How many of ``length`` recent tokens the schedule compresses now (cache.py:497-533).  The reference drains one chunk
+        per loop iteration while the buffer holds ``residual_window + chunk_size``; tokens are quantized independently, so
+        all those chunks go together with the same result."""
         if self.chunk_size <= 0:
-            if self._fp16_len <= self.residual_window * 2:
-                return
-            self._drain_chunk(self._fp16_len - self.residual_window)
-            return
-        # The reference drains one chunk per loop iteration while fp16_len >= residual_window + chunk_size; tokens
-        # are quantized independently, so all those chunks go to the GPU as one launch with the same result.
-        threshold = self.residual_window + self.chunk_size
-        if self._fp16_len >= threshold:
-            n_chunks = (self._fp16_len - self.residual_window) // self.chunk_size
-            self._drain_chunk(n_chunks * self.chunk_size)
+            return length - self.residual_window if length > self.residual_window * 2 else 0
+        if length < self.residual_window + self.chunk_size:
+            return 0
+        return (length - self.residual_window) // self.chunk_size * self.chunk_size
+
+    def _take(self, k_new, v_new) -> None:
+        """Append (B, H, T, D) new tokens to the recent-token buffer and compress what the schedule says (cache.py:497-575,
+        632-672).  Tokens that leave at once are quantized where they are - in the buffer or in the caller's tensors - and
+        never pass through the buffer: a long prompt costs one read of its rows, not a fill, a copy and a read back."""
+        b, h, t_new, d = k_new.shape
+        dev = k_new.device
+        have = 0 if self.keys is None else self._fp16_len
+        length = have + t_new
+        cap = self._fp16_capacity
+        if self.keys is None:
+            cap = max(t_new, self.residual_window * 2) + 256
+        elif length > cap:
+            cap = length + 256
+            if self.keys.dtype != k_new.dtype or self.values.dtype != v_new.dtype:      # a grown buffer has the newcomers' dtype
+                self.keys, self.values = self.keys.to(k_new.dtype), self.values.to(v_new.dtype)
+        if self.keys is not None and (self.keys.dtype != k_new.dtype or self.values.dtype != v_new.dtype):
+            k_new, v_new = k_new.to(self.keys.dtype), v_new.to(self.values.dtype)
+        n = self._due(length)
+        old = min(n, have)                     # of the n, those that sit in the buffer
+        if n > 0:
+            at = self._compressed_len
+            for side, buf, new in ((self._k, self.keys, k_new), (self._v, self.values, v_new)):
+                side.reserve(b, h, d, at + n, at, dev, self.qjl_correction)
+                for rows, where in ((buf[:, :, :old] if old else None, at), (new[:, :, :n - old] if n > old else None, at + old)):
+                    if rows is not None:
+                        kernels.quantize_pack(rows, self._rotation, side.bnd_hi, side.bits_hi, side.bnd_lo, side.bits_lo,
+                                              out_hi=side.hi, out_lo=side.lo, out_norms=side.norms, out_offset=where,
+                                              qjl=self._qjl_args(side))
+            # A long prefill would leave buffers sized for the whole prompt; they get the size a fresh cache would get for what
+            # remains instead (batch 64 x 32K tokens: 17 GB per layer otherwise).
+            small = max(length - n, self.residual_window * 2) + 256
+            if cap > 4 * small:
+                cap = small
+        kept = have - old
+        if self.keys is None or cap != self.keys.shape[2]:
+            nk, nv = torch.zeros((2, b, h, cap, d), dtype=k_new.dtype, device=dev) if k_new.dtype == v_new.dtype else (
+                torch.zeros((b, h, cap, d), dtype=t.dtype, device=dev) for t in (k_new, v_new))
+            if kept > 0:
+                self._append(nk, nv, self.keys[:, :, old:have], self.values[:, :, old:have], 0)
+            self.keys, self.values = nk, nv
+        elif old > 0 and kept > 0:             # the kept tokens move to the front (the kernels above have read the buffer by then)
+            for buf in (self.keys, self.values):
+                tail = buf[:, :, old:have]
+                buf[:, :, :kept] = tail.clone() if old < kept else tail
+        if n - old < t_new:
+            self._append(self.keys, self.values, k_new[:, :, n - old:], v_new[:, :, n - old:], kept)
+        self._fp16_capacity = cap
+        self._fp16_len = length - n
+        self._compressed_len += n
 
     def _route_sink(self, keys, values):
         """Peel the tokens that belong to the permanent sink off the head of the batch (cache.py:577-618)."""
@@ -342,24 +367,21 @@ class TurboQuantKVCache:
             b, h, _, d = keys.shape
             self.sink_keys = torch.zeros((b, h, self.fp16_sink_size, d), dtype=keys.dtype, device=keys.device)
             self.sink_values = torch.zeros((b, h, self.fp16_sink_size, d), dtype=values.dtype, device=values.device)
-        if n_sink == t_new:
-            self._append(self.sink_keys, self.sink_values, keys, values, self.offset)
-        else:
-            self.sink_keys[:, :, self.offset:self.offset + n_sink] = keys[:, :, :n_sink]
-            self.sink_values[:, :, self.offset:self.offset + n_sink] = values[:, :, :n_sink]
+        self._append(self.sink_keys, self.sink_values, keys[:, :, :n_sink], values[:, :, :n_sink], self.offset)
         self._sink_len = self.offset + n_sink
         return keys[:, :, n_sink:], values[:, :, n_sink:]
 
     @staticmethod
     def _append(k_buf, v_buf, k_new, v_new, row0: int) -> None:
         """k_buf[:, :, row0:row0+T] = k_new (same for values): one library launch when the layout allows it."""
-        t_new = k_new.shape[2]
+        b, h, t_new, d = k_new.shape
         _lib.require_cuda(k_buf, v_buf, k_new, v_new)
-        if (k_new.is_contiguous() and v_new.is_contiguous() and k_new.dtype == k_buf.dtype and v_new.dtype == v_buf.dtype
-                and k_buf.dtype == v_buf.dtype and (k_buf.shape[3] * k_buf.element_size()) % 16 == 0):
-            b, h, cap, d = k_buf.shape
+        lane = k_new.stride(1)
+        if (k_new.dtype == k_buf.dtype == v_new.dtype == v_buf.dtype and k_new.stride() == v_new.stride()
+                and k_new.stride(3) == 1 and k_new.stride(2) == d and (b == 1 or k_new.stride(0) == h * lane) and lane % d == 0
+                and (d * k_buf.element_size()) % 16 == 0 and (lane >= t_new * d or h == 1)):
             rc = _lib.launch(k_buf.device, "tq_append_tokens", k_new.data_ptr(), v_new.data_ptr(), k_buf.data_ptr(), v_buf.data_ptr(),
-                             b * h, t_new, d * k_buf.element_size(), t_new, cap, row0, _lib.stream_ptr(k_buf.device))
+                             b * h, t_new, d * k_buf.element_size(), max(lane // d, t_new), k_buf.shape[2], row0, _lib.stream_ptr(k_buf.device))
             if rc == 0:
                 return
             if rc != -2:                      # anything but "layout not supported" is an error
@@ -377,28 +399,9 @@ class TurboQuantKVCache:
         self._bind(dev)
         t_total = keys.shape[2]
         keys_rest, values_rest = self._route_sink(keys, values)
-        t_new = keys_rest.shape[2]
-        if t_new > 0:
-            if self.keys is None:
-                b, h, _, d = keys_rest.shape
-                cap = max(t_new, self.residual_window * 2) + 256
-                self._fp16_capacity = cap
-                self._fp16_len = 0
-                self.keys = torch.zeros((b, h, cap, d), dtype=keys_rest.dtype, device=dev)
-                self.values = torch.zeros((b, h, cap, d), dtype=values_rest.dtype, device=dev)
-            new_len = self._fp16_len + t_new
-            if new_len > self._fp16_capacity:
-                b, h, _, d = self.keys.shape
-                new_cap = new_len + 256
-                nk = torch.zeros((b, h, new_cap, d), dtype=keys_rest.dtype, device=dev)
-                nv = torch.zeros((b, h, new_cap, d), dtype=values_rest.dtype, device=dev)
-                nk[:, :, :self._fp16_len] = self.keys[:, :, :self._fp16_len]
-                nv[:, :, :self._fp16_len] = self.values[:, :, :self._fp16_len]
-                self.keys, self.values, self._fp16_capacity = nk, nv, new_cap
-            self._append(self.keys, self.values, keys_rest, values_rest, self._fp16_len)
-            self._fp16_len = new_len
+        if keys_rest.shape[2] > 0 or (self.keys is not None and self._due(self._fp16_len) > 0):
+            self._take(keys_rest, values_rest)
         self.offset += t_total
-        self._compress_old_tokens()
 
     # ---- dense output ------------------------------------------------------------------------------
     def _ensure_dense(self) -> None:
