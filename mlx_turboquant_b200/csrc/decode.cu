@@ -594,6 +594,7 @@ static int g_tune_splits = 0;          // > 0: fixed number of packed splits
 extern int g_tune_dequantize_tc;       // rowops.cu: 0 = dequantize always on the CUDA-core row kernel
 extern int g_tune_prefill_tc;          // prefill.cu: 0 = several-query-token attention always on the mma.sync kernel
 static int g_tune_pdl = 1;             // programmatic dependent launch between consecutive calls
+static int g_tune_lut = 1;             // 0: never take the lookup kernel for the other widths
 static int g_tune_stream = 1;          // 0: never take the streaming kernel
 static int g_tune_stream_min_run = 24; // fewest packed tiles per warp for which the streaming kernel is chosen over the table-lookup kernel (a third of it over the general kernel)
 static int g_tune_stream_max_parts = 40;  // most partials per lane with which it is chosen over the table-lookup kernel (64 over the general kernel)
@@ -761,11 +762,25 @@ int decode_prepare(const tq_decode_args* a, void* workspace, size_t workspace_by
         const int max_parts = direct ? std::min(g_tune_stream_max_parts, 64) : 64;
         stream = stp.range >= min_run && stp.npp + stp.nd <= max_parts && stream_supported(d, qjl);
     }
+    // everything else the lookup kernel's tables cover (two to four bits, their fractional splits).  The general kernel is one launch instead of three: with whole-byte tables
+    // (4-bit keys, 2-bit values) it is the faster one for few tiles (head_dim 64, 16 lanes x 218 tiles: 17 against 29 us;
+    // head_dim 128 with sketches, 72 lanes x 230 tiles: 63 against 35 us)
+    bool lut = !direct && !stream && g_tune_lut && !g_tune_force_general && a->c_lane_stride % 16 == 0 &&
+               aligned(a->k_hi, 16) && aligned(a->v_hi, 16) && aligned(a->k_norms, 16) && aligned(a->v_norms, 16) &&
+               (!a->k_bits_lo || aligned(a->k_lo, 16)) && (!a->v_bits_lo || aligned(a->v_lo, 16)) &&
+               (!qjl || (aligned(a->k_qjl_bits, 16) && aligned(a->v_qjl_bits, 16) && aligned(a->k_qjl_gamma, 16) && aligned(a->v_qjl_gamma, 16) && aligned(a->qjl_proj, 16))) &&
+               (a->sink_len == 0 || (aligned(a->sink_k, 16) && aligned(a->sink_v, 16))) && (!a->res_k || (aligned(a->res_k, 16) && aligned(a->res_v, 16)));
+    if (lut) {
+        stp = lut_plan(a->batch, a->n_q_heads, a->n_kv_heads, d, a->c_len, dense_len, sm_count());
+        const int64_t tiles = int64_t(a->batch) * a->n_kv_heads * ((a->c_len + TILE - 1) / TILE);
+        const bool bytes = a->k_bits_hi == 4 && !a->k_bits_lo && a->v_bits_hi == 2 && !a->v_bits_lo;
+        lut = stp.ok && !(a->c_len > 0 && bytes && tiles < 8000) && lut_supported(d, qjl, a->c_len > 0 ? a->k_bits_hi : 4, a->c_len > 0 ? a->k_bits_lo : 0, a->c_len > 0 ? a->v_bits_hi : 4, a->c_len > 0 ? a->v_bits_lo : 0);
+    }
     const SplitPlan sp = plan_splits(a->batch, a->n_q_heads, a->n_kv_heads, a->c_len, dense_len, sm_count(), direct);
     const WsLayout wl = ws_layout(a->batch, a->n_q_heads, a->n_kv_heads, d, sp);
     const size_t st_base = align_up(std::max(size_t(a->batch) * a->n_kv_heads * sp.hg * sizeof(int), COUNTER_AREA), 256);
-    if (stream && st_base + stp.q16_bytes + stp.part_bytes > workspace_bytes) stream = false;   // (a workspace sized for the other kernels only)
-    if (!stream && wl.total > workspace_bytes) return fail(TQ_ERR_INVALID, "tq_decode_attn: workspace %zu B < %zu B", workspace_bytes, wl.total);
+    if ((stream || lut) && st_base + stp.q16_bytes + stp.part_bytes > workspace_bytes) stream = lut = false;   // (a workspace sized for the other kernels only)
+    if (!stream && !lut && wl.total > workspace_bytes) return fail(TQ_ERR_INVALID, "tq_decode_attn: workspace %zu B < %zu B", workspace_bytes, wl.total);
     if (sp.n_ps + sp.n_ds > MAX_SPLITS) return fail(TQ_ERR_UNSUPPORTED, "tq_decode_attn: too many splits");
 
     DecodeParams p{};
@@ -813,7 +828,8 @@ int decode_prepare(const tq_decode_args* a, void* workspace, size_t workspace_by
     p.pdl = g_tune_pdl;
     p.words_ok = (a->c_len > 0 && aligned(a->k_hi, 4) && aligned(a->v_hi, 4)) ? 1 : 0;   // packed rows readable as 32-bit words
     p.tables = (direct || stream) ? a->tables : nullptr;
-    if (stream) {
+    if (stream || lut) {
+        p.st_lut = lut ? 1 : 0; p.st_fold = stp.fold;
         p.st_grid = stp.grid; p.st_npp = stp.npp; p.st_nd = stp.nd; p.st_dt = stp.dt; p.st_range = stp.range;
         p.st_q16 = reinterpret_cast<__half*>(ws + st_base);
         p.st_part = reinterpret_cast<float*>(ws + st_base + stp.q16_bytes);
@@ -830,7 +846,7 @@ int decode_launch(const DecodeParams& p0, bool direct, cudaStream_t s) {
         if (int rc = launch_gather_wait(p.await_ll, p.await_epochs, p.await_words, p.await_out, p.await_polls, s)) return rc;
         p.await_ll = nullptr;
     }
-    if (p.st_grid > 0) return launch_decode_stream(p, s);
+    if (p.st_grid > 0) return p.st_lut ? launch_decode_lut(p, s) : launch_decode_stream(p, s);
     if (direct) return launch_decode_direct(p, s);
     const bool qjl = p.qjl_proj != nullptr;
     if (p.D == 64) return qjl ? launch_decode<64, true>(p, s) : launch_decode<64, false>(p, s);
@@ -849,6 +865,7 @@ extern "C" int tq_set_tuning(const char* key, int value) {
     if (k == "decode_ctas_per_sm" && value >= 1 && value <= 8) g_tune_ctas_per_sm = value;
     else if (k == "decode_force_general" && (value == 0 || value == 1)) g_tune_force_general = value;
     else if (k == "decode_pdl" && (value == 0 || value == 1)) g_tune_pdl = value;
+    else if (k == "decode_lut" && (value == 0 || value == 1)) g_tune_lut = value;
     else if (k == "decode_stream" && (value == 0 || value == 1)) g_tune_stream = value;
     else if (k == "decode_stream_min_run" && value >= 1 && value <= (1 << 20)) g_tune_stream_min_run = value;
     else if (k == "decode_stream_max_parts" && value >= 1 && value <= 64) g_tune_stream_max_parts = value;
@@ -864,7 +881,7 @@ extern "C" int tq_decode_kernel_choice(const tq_decode_args* a) {
     DecodeParams p;
     bool direct = false;
     if (decode_prepare(a, a ? a->workspace : nullptr, a ? a->workspace_bytes : 0, &p, &direct)) return -1;
-    return p.st_grid > 0 ? 2 : direct ? 1 : 0;
+    return p.st_grid > 0 ? (p.st_lut ? 3 : 2) : direct ? 1 : 0;
 }
 
 extern "C" int tq_gather_wait(const unsigned long long* ll, const unsigned* epochs, int64_t n_words, void* out, void* stream) {
@@ -976,6 +993,11 @@ extern "C" size_t tq_decode_workspace_bytes(int batch, int n_q_heads, int n_kv_h
         const int hg = (n_q_heads / n_kv_heads + HPG - 1) / HPG;
         if (sp.npp + sp.nd <= 64)
             c = align_up(std::max(size_t(batch) * n_kv_heads * hg * sizeof(int), COUNTER_AREA), 256) + sp.q16_bytes + sp.part_bytes;
+    }
+    const StreamPlan lp = lut_plan(batch, n_q_heads, n_kv_heads, d, c_len, dense_len, sm_count());
+    if (lp.ok) {
+        const int hg = (n_q_heads / n_kv_heads + HPG - 1) / HPG;
+        c = std::max(c, align_up(std::max(size_t(batch) * n_kv_heads * hg * sizeof(int), COUNTER_AREA), 256) + lp.q16_bytes + lp.part_bytes);
     }
     return std::max(a, c);
 }

@@ -53,6 +53,7 @@ struct DecodeParams {
     // streaming kernel (decode_stream.cu): every warp of a persistent grid walks its own contiguous run of the packed
     // tiles of all cache lanes; partials per (lane, slot) and the prepared queries live in the workspace
     int st_grid;                       // CTAs of the persistent grid (0: another kernel runs)
+    int st_lut, st_fold;               // decode_lut.cu runs (decode_stream.cu otherwise); its CTAs fold their warps' partials
     int st_npp, st_nd, st_dt;          // packed-partial slots per lane; dense items per lane and tiles per dense item
     int64_t st_range;                  // packed tiles per warp
     __half* st_q16;                    // workspace: per query head [rotated | raw | sketch] scaled fp16 query
@@ -94,10 +95,14 @@ int direct_tables_build(int d, const float* rot, const float* k_cent, const floa
 int launch_decode_direct(const DecodeParams& p, cudaStream_t s);
 // decode_stream.cu: persistent kernel for 4-bit keys / 2-bit values at d = 96 / 128 (sign sketches optional) when the
 // packed tokens of all lanes amount to many tiles per warp.
-struct StreamPlan { int grid, npp, nd, dt; int64_t range; size_t q16_bytes, part_bytes; };
+struct StreamPlan { int grid, npp, nd, dt; int64_t range; size_t q16_bytes, part_bytes; int fold, ok; };
 bool stream_supported(int d, bool qjl);
 StreamPlan stream_plan(int batch, int n_q_heads, int n_kv_heads, int d, int64_t c_len, int64_t dense_len, int sms);
 int launch_decode_stream(const DecodeParams& p, cudaStream_t s);
+// decode_lut.cu: the same idea for every other width (2, 3, 4 bits, 4 | 3, 3 | 2) and head_dim 64 / 96 / 128 / 256.
+bool lut_supported(int d, bool qjl, int kb_hi, int kb_lo, int vb_hi, int vb_lo);
+StreamPlan lut_plan(int batch, int n_q_heads, int n_kv_heads, int d, int64_t c_len, int64_t dense_len, int sms);
+int launch_decode_lut(const DecodeParams& p, cudaStream_t s);
 int launch_gather_wait(const unsigned long long* ll, const unsigned* epochs, int64_t n_words, void* out, int max_polls, cudaStream_t s);
 int* decode_status_ptr();          // device address of the status word on the current device (null on error)
 int decode_status_host();          // code of the first bounded wait that ran out on this device (0 = none), -1 on error

@@ -1,0 +1,1066 @@
+// Decode attention for the widths and head dims without a kernel of their own: keys and values at 2, 3 or 4 bits or a
+// fractional split (4 | 3 or 3 | 2 bits), head_dim 64 / 96 / 128 / 256, with or without the QJL sign sketches.
+//
+// One persistent CTA per SM; the packed 16-token tiles of ALL cache lanes (sequence, KV head, head group) are dealt out as
+// one flat sequence, an equal contiguous run per warp (as decode_stream.cu does for 4-bit keys / 2-bit values).  Three
+// launches chained with programmatic dependent launch: lut_query_kernel (rotates the queries once, on mma.sync),
+// decode_lut_kernel, lut_merge_kernel (log-sum-exp merge, rotation back, normalisation).
+//
+// Operands.  What bounds a decode step at these widths is how packed codes become fp16 operand registers, so no code is
+// ever looked at on its own: one shared-memory lookup turns a PAIR of codes (4 bits: a byte; 3 bits: a six-bit field) or
+// four codes (2 bits: a byte) into one or two half2 registers, every lane reading its own copy of the table (no bank
+// conflicts).  Keys pair neighbouring coordinates of a token, as the A operand of S = K q^T wants them; values pair the
+// same coordinate of two tokens, as the A operand of O^T = V^T P^T wants them - the codes of two tokens are interleaved
+// with one three-input logic op per eight (bytes at 4 and 2 bits; alternate octal digits at 3 bits).  Per 16-token tile,
+// d = 128 and lane: 32 half2 a side = 32 lookups at 4 bits, 32 at 3 bits, 16 (of 64 bits) at 2 bits.
+//   (The general kernel of decode.cu takes codes one by one through a 16-entry table and shared-memory staging: 906 us per
+//   call for 4 sequences x 8 KV heads x 11,777 tokens at 3.5 / 3.5 bits.)
+//
+// Tiles reach a warp through its own ring of NS stages in shared memory (16-byte asynchronous copies, an mbarrier per
+// stage).  A lane reads the bits it owns of a row as aligned words and shifts them into place, so any row length works.
+//
+// Partials.  Long lanes (a CTA's tiles span at most two of them): the warps of a CTA fold their partials of a lane into
+// one before it leaves the SM, so that few lanes of many tiles do not flood the merge.  Short lanes: a warp writes a
+// partial per lane it touches.
+//
+// Every mbarrier wait is bounded; a wait that runs out records a status (tq_device_status), the warp drains the copies it
+// still has in flight (bounded again) and stops.
+#include <algorithm>
+#include <atomic>
+
+#include "decode_dev.cuh"
+
+namespace tq {
+namespace lut {
+
+constexpr int QM = 32;                         // sketch rows (one 32-bit sign word per token)
+constexpr float QJL_C = 1.2533141373155003f;   // sqrt(pi / 2), qjl.py:91-92
+constexpr uint32_t WAIT_LIMIT = 4u << 20;
+constexpr int ERR_RING = 109, ERR_LAYOUT = 110;
+constexpr int MAX_PARTS = 192;                 // partial slots per lane the merge handles
+
+// Code formats of a side: the bits of its coordinates, or of its two halves (hi * 10 + lo).
+enum Fmt { F2 = 2, F3 = 3, F4 = 4, F43 = 43, F32 = 32 };
+
+// Shared-window addresses are compile-time constants (they travel in the instructions): the dynamic allocation starts at
+// sbase <= LO_BASE.  Byte tables: slot e (256 B) holds the key entry of byte e (32 copies of a half2 at 4 bits, 16 of a pair
+// of half2 at 2 bits), then the value entry likewise; the six-bit tables have 64 entries of 128 B.
+constexpr uint32_t LO_BASE = 2048u;
+constexpr uint32_t TAB_B = LO_BASE, TAB_K3 = TAB_B + 65536u, TAB_V3 = TAB_K3 + 8192u, AREA0 = TAB_V3 + 8192u;
+
+template <int D, bool QJL> struct Plan {
+    static constexpr int NW = D == 256 ? 8 : 16, NT = NW * 32;                       // (d = 256: 128 accumulator / query registers per thread)
+    static constexpr uint32_t SC = (QJL ? 6u : 2u) * TILE * 4u;                      // scalars first: norms, sign words, residual norms
+    static constexpr uint32_t O_KN = 0, O_VN = 64, O_KB = 128, O_KG = 192, O_VB = 256, O_VG = 320;
+    static constexpr uint32_t STAGE = SC + 2u * TILE * D / 2;                        // 4-bit keys and values fill it
+    static constexpr int NC = (int(STAGE / 16) + 31) / 32;                           // 16-byte chunks per lane at most
+    static constexpr int NS = 3;
+    static constexpr uint32_t RING = NS * STAGE + 16u;                               // (+ a word that is read but not used past the last row)
+    static constexpr uint32_t DSTAGE = 2u * TILE * stage_ld<D>() * 2u;               // 16-bit keys + values of one uncompressed tile
+    static constexpr uint32_t PART = HPG * (D + QM + 4) * 4u;                        // one warp's partial of up to eight heads
+    static constexpr uint32_t A0 = RING > DSTAGE ? RING : DSTAGE;
+    static constexpr uint32_t AREA = ((A0 > PART ? A0 : PART) + 127u) / 128u * 128u;
+    static constexpr uint32_t SPILL = AREA0 + NW * AREA;                             // partial of the lane a warp leaves (one warp per CTA can)
+    static constexpr uint32_t BARS = SPILL + (PART + 127u) / 128u * 128u;
+    static constexpr uint32_t OWNER = BARS + 8u * NW * NS;                           // lane of each warp's partial, then of the spilled one
+    static constexpr uint32_t SMEM_END = OWNER + 4u * (NW + 1) + 60u;
+    static_assert(SMEM_END <= 227u * 1024u, "shared-memory plan");
+    static_assert(STAGE % 16 == 0 && AREA % 128 == 0, "copies need 16-byte alignment");
+};
+
+// Query heads in the workspace, halves: rotated (fp16) | raw, fp16 or the bf16 high part | bf16 low part | sketch
+__host__ __device__ constexpr int q_stride(int d) { return 3 * d + QM; }
+__host__ __device__ constexpr int part_stride(int d) { return d + QM + 4; }    // floats per head of a partial: values | sketch rows | max, sum, pad
+
+// ---- PTX wrappers ---------------------------------------------------------------------------------------
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+    for (uint32_t i = 0; i < WAIT_LIMIT; ++i)
+        if (mbar_try(bar, parity)) return true;
+    return false;
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Table lookups: the table's address is an immediate of the load.
+template <uint32_t OFF> __device__ __forceinline__ uint32_t tab32(uint32_t addr) {
+    uint32_t v;
+    asm("ld.shared.b32 %0, [%1 + %2];" : "=r"(v) : "r"(addr), "n"(OFF));
+    return v;
+}
+template <uint32_t OFF> __device__ __forceinline__ uint2 tab64(uint32_t addr) {
+    uint2 v;
+    asm("ld.shared.v2.b32 {%0,%1}, [%2 + %3];" : "=r"(v.x), "=r"(v.y) : "r"(addr), "n"(OFF));
+    return v;
+}
+// Ring reads: ordered after the wait that made the stage visible.
+template <uint32_t OFF> __device__ __forceinline__ uint32_t ring32o(uint32_t base) {
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1 + %2];" : "=r"(v) : "r"(base), "n"(OFF) : "memory");
+    return v;
+}
+template <uint32_t OFF> __device__ __forceinline__ float ring_f32o(uint32_t base) { return __uint_as_float(ring32o<OFF>(base)); }
+template <int LUT> __device__ __forceinline__ uint32_t lop3(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, %4;" : "=r"(d) : "r"(a), "r"(b), "r"(c), "n"(LUT));
+    return d;
+}
+// (a & m) | (b & ~m)
+__device__ __forceinline__ uint32_t pick(uint32_t a, uint32_t b, uint32_t m) { return lop3<0xE4>(a, b, m); }
+// half2 of two signs (+1 for a set bit) from bits 15 and 31
+__device__ __forceinline__ uint32_t sign_pair16(uint32_t x) { return lop3<0x6A>(x, 0x80008000u, 0xBC00BC00u); }
+
+// Token in MMA row / k slot s: slots 2a + e of a half hold tokens a + 4 e, so the four lanes of a thread group read value
+// rows of four consecutive tokens and the eight row groups key rows of eight consecutive tokens.
+__device__ __forceinline__ int tok_of_slot(int s) { return ((s & 7) >> 1) + 4 * (s & 1) + (s & 8); }
+
+// Compile-time loop: f(Ic<0>{}), f(Ic<1>{}), ...
+template <int I> struct Ic { static constexpr int v = I; };
+template <int N, int I = 0, typename F> __device__ __forceinline__ void each(F&& f) {
+    if constexpr (I < N) {
+        f(Ic<I>{});
+        each<N, I + 1>(f);
+    }
+}
+
+constexpr int gcd32(int x) { return x % 32 == 0 ? 32 : x % 16 == 0 ? 16 : x % 8 == 0 ? 8 : x % 4 == 0 ? 4 : x % 2 == 0 ? 2 : 1; }
+// BITS bits that start `sh` bits into the word at addr, as words; sh is a multiple of gcd(BITS, 32).
+template <int BITS> struct Bits {
+    static constexpr int NW = (BITS + 31) / 32;
+    static constexpr bool ALIGNED = BITS % 32 == 0;
+    static constexpr int NR = ALIGNED ? NW : (32 - gcd32(BITS) + BITS + 31) / 32;     // words that can hold a part of them
+    uint32_t w[NW];
+    __device__ __forceinline__ void read(uint32_t addr, uint32_t sh) {
+        uint32_t r[NR + 1];
+        each<NR>([&](auto ic) {
+            constexpr int i = decltype(ic)::v;
+            r[i] = ring32o<4 * i>(addr);
+        });
+        r[NR] = 0;
+#pragma unroll
+        for (int i = 0; i < NW; ++i) w[i] = ALIGNED ? r[i] : NR == 1 ? r[i] >> sh : __funnelshift_r(r[i], r[i + 1], sh);
+    }
+    // bits [p, ...) moved to bit `to`; callers mask
+    template <int P, int TO> __device__ __forceinline__ uint32_t at() const {
+        constexpr int base = P - TO;
+        if constexpr (base < 0) return w[0] << (-base);
+        else {
+            constexpr int i = base / 32, r = base % 32;
+            if constexpr (r == 0) return w[i];
+            else if constexpr (i + 1 < NW) return __funnelshift_r(w[i], w[i + 1], r);
+            else return w[i] >> r;
+        }
+    }
+};
+template <> struct Bits<64> {      // (aligned pairs of words)
+    static constexpr int NW = 2;
+    uint32_t w[2];
+    __device__ __forceinline__ void read(uint32_t addr, uint32_t) {
+        asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "r"(addr) : "memory");
+    }
+};
+template <> struct Bits<128> {
+    static constexpr int NW = 4;
+    uint32_t w[4];
+    __device__ __forceinline__ void read(uint32_t addr, uint32_t) {
+        asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr) : "memory");
+    }
+};
+
+template <> struct Bits<256> {
+    static constexpr int NW = 8;
+    uint32_t w[8];
+    __device__ __forceinline__ void read(uint32_t addr, uint32_t) {
+        asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr) : "memory");
+        asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4 + 16];" : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "r"(addr) : "memory");
+    }
+};
+
+// Per-lane constants: copy offsets inside an entry.
+struct Copies { uint32_t c4, c2; };            // 4 lane, 8 (lane & 15)
+constexpr uint32_t M3 = 63u << 7;              // six-bit field in entry position
+
+// Scores of NK k-steps: this lane's 4 NK coordinates (B bits each, `sh` bits into the word at `addr`) of token row g, and of
+// row g + 8, `row8` bytes further.  bq: the query fragments of these k-steps.
+template <int B, int NK>
+__device__ __forceinline__ void key_part(float (&s)[4], uint32_t addr, uint32_t row8, uint32_t sh, const uint32_t (*bq)[2], const Copies& c) {
+    Bits<4 * NK * B> a, b;
+    a.read(addr, sh);
+    b.read(addr + row8, sh);
+    each<NK>([&](auto ic) {
+        constexpr int ks = decltype(ic)::v;
+        uint32_t a0, a1, a2, a3;
+        if constexpr (B == 4) {
+            constexpr uint32_t s0 = 0x7604u | uint32_t((2 * ks) & 3) << 4, s1 = 0x7604u | uint32_t((2 * ks + 1) & 3) << 4;
+            const uint32_t wa = a.w[ks / 2], wb = b.w[ks / 2];
+            a0 = tab32<TAB_B>(__byte_perm(wa, c.c4, s0));
+            a1 = tab32<TAB_B>(__byte_perm(wb, c.c4, s0));
+            a2 = tab32<TAB_B>(__byte_perm(wa, c.c4, s1));
+            a3 = tab32<TAB_B>(__byte_perm(wb, c.c4, s1));
+        } else if constexpr (B == 3) {
+            a0 = tab32<TAB_K3>((a.template at<12 * ks, 7>() & M3) | c.c4);
+            a1 = tab32<TAB_K3>((b.template at<12 * ks, 7>() & M3) | c.c4);
+            a2 = tab32<TAB_K3>((a.template at<12 * ks + 6, 7>() & M3) | c.c4);
+            a3 = tab32<TAB_K3>((b.template at<12 * ks + 6, 7>() & M3) | c.c4);
+        } else {
+            constexpr uint32_t s0 = 0x7604u | uint32_t(ks & 3) << 4;
+            const uint2 x = tab64<TAB_B>(__byte_perm(a.w[ks / 4], c.c2, s0)), y = tab64<TAB_B>(__byte_perm(b.w[ks / 4], c.c2, s0));
+            a0 = x.x; a2 = x.y; a1 = y.x; a3 = y.y;
+        }
+        mma16816(s, a0, a1, a2, a3, bq[ks][0], bq[ks][1]);
+    });
+}
+
+// O^T += V^T P^T for MT m-tiles: this lane's 2 MT coordinates of tokens t, t + 4 (k slots 2t, 2t + 1) and t + 8, t + 12;
+// token rows `row4` bytes apart.
+template <int B, int MT>
+__device__ __forceinline__ void value_part(float (*o)[4], uint32_t addr, uint32_t row4, uint32_t sh, const uint32_t (&bp)[2], const Copies& c) {
+    Bits<2 * MT * B> va, vb, vc, vd;
+    va.read(addr, sh);
+    vb.read(addr + row4, sh);
+    vc.read(addr + 2 * row4, sh);
+    vd.read(addr + 3 * row4, sh);
+    if constexpr (B == 3) {
+        constexpr uint32_t even = 0x1C71C7u;                     // octal digits 0, 2, 4, 6
+        each<(MT + 3) / 4>([&](auto ic) {                        // groups of eight coordinates (24 bits)
+            constexpr int gq = decltype(ic)::v;
+            const uint32_t a = va.template at<24 * gq, 0>(), b = vb.template at<24 * gq, 0>(), cc = vc.template at<24 * gq, 0>(), d = vd.template at<24 * gq, 0>();
+            const uint32_t e0 = pick(a, b << 3, even), o0 = pick(a >> 3, b, even), e1 = pick(cc, d << 3, even), o1 = pick(cc >> 3, d, even);
+            each<4>([&](auto jc) {
+                constexpr int j = decltype(jc)::v, m = 4 * gq + j;
+                if constexpr (m < MT) {
+                    auto idx = [&](uint32_t x) -> uint32_t {
+                        if constexpr (j < 2) return ((x << (7 - 6 * j)) & M3) | c.c4;
+                        else return ((x >> (6 * j - 7)) & M3) | c.c4;
+                    };
+                    mma16816(o[m], tab32<TAB_V3>(idx(e0)), tab32<TAB_V3>(idx(o0)), tab32<TAB_V3>(idx(e1)), tab32<TAB_V3>(idx(o1)), bp[0], bp[1]);
+                }
+            });
+        });
+    } else {
+        constexpr uint32_t low = 0x0F0F0F0Fu;
+        each<Bits<2 * MT * B>::NW>([&](auto ic) {
+            constexpr int w = decltype(ic)::v;
+            const uint32_t z0 = pick(va.w[w], vb.w[w] << 4, low), z1 = pick(va.w[w] >> 4, vb.w[w], low);
+            const uint32_t y0 = pick(vc.w[w], vd.w[w] << 4, low), y1 = pick(vc.w[w] >> 4, vd.w[w], low);
+            each<4>([&](auto jc) {
+                constexpr int j = decltype(jc)::v;
+                constexpr uint32_t sel = 0x7604u | uint32_t(j) << 4;
+                if constexpr (B == 4) {                          // byte j of z0 / z1: coordinates 8 w + 2 j, + 1 of the two tokens
+                    constexpr int m = 4 * w + j;
+                    if constexpr (m < MT)
+                        mma16816(o[m], tab32<TAB_B + 128>(__byte_perm(z0, c.c4, sel)), tab32<TAB_B + 128>(__byte_perm(z1, c.c4, sel)),
+                                 tab32<TAB_B + 128>(__byte_perm(y0, c.c4, sel)), tab32<TAB_B + 128>(__byte_perm(y1, c.c4, sel)), bp[0], bp[1]);
+                } else {                                         // byte j of z0: coordinates 16 w + 4 j, + 1 of the two tokens; z1: + 2, + 3
+                    constexpr int m = 8 * w + 2 * j;
+                    if constexpr (m < MT) {
+                        const uint2 e = tab64<TAB_B + 128>(__byte_perm(z0, c.c2, sel)), f = tab64<TAB_B + 128>(__byte_perm(y0, c.c2, sel));
+                        mma16816(o[m], e.x, e.y, f.x, f.y, bp[0], bp[1]);
+                    }
+                    if constexpr (m + 1 < MT) {
+                        const uint2 e = tab64<TAB_B + 128>(__byte_perm(z1, c.c2, sel)), f = tab64<TAB_B + 128>(__byte_perm(y1, c.c2, sel));
+                        mma16816(o[m + 1], e.x, e.y, f.x, f.y, bp[0], bp[1]);
+                    }
+                }
+            });
+        });
+    }
+}
+
+// Softmax step on scores that already carry the key norms (and the sketch term); tokens past the end come in with score
+// -inf and norm 0.  pr: the four weights times the value scale.
+template <int D, int NZ>
+__device__ __forceinline__ void softmax_scores(float (&s)[4], float vn0, float vn1, float vx, WarpAcc<D, NZ>& st, float (&pr)[4]) {
+    const float mx0 = fmaxf(s[0], s[2]), mx1 = fmaxf(s[1], s[3]), vmax = fmaxf(fmaxf(vn0, vn1), vx);
+    if (__any_sync(0xffffffffu, mx0 > st.mt[0] || mx1 > st.mt[1] || vmax > st.vt)) softmax_refresh<D, NZ>(mx0, mx1, vmax, st);
+    const float p0 = ex2(s[0] - st.m[0]), p1 = ex2(s[1] - st.m[1]), p2 = ex2(s[2] - st.m[0]), p3 = ex2(s[3] - st.m[1]);
+    st.l[0] += p0 + p2;
+    st.l[1] += p1 + p3;
+    pr[0] = p0 * st.vsc; pr[1] = p1 * st.vsc; pr[2] = p2 * st.vsc; pr[3] = p3 * st.vsc;
+}
+
+__device__ __forceinline__ uint32_t pack_bf2(float lo, float hi) {
+    const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&b);
+}
+
+// Uncompressed tokens (sink, recent window, the token a step appends) of cache lane kvl, tiles [tile_lo, tile_hi), 16-bit
+// caches: a tile's rows come in with asynchronous copies and feed the MMAs in their own type.  bf16 rows take the
+// query and the weights as high + low bf16 parts (16 bits between them), so nothing is converted and any magnitude works.
+template <int D, bool BF16>
+__device__ __forceinline__ void dense_run(const DecodeParams& p, int64_t kvl, int tile_lo, int tile_hi, uint32_t stage, const __half* qraw, bool live_q,
+                                          WarpAcc<D, 0>& st, int lane) {
+    constexpr int LD = stage_ld<D>(), CPR = D / 8;                       // halves per staged row, 16-byte chunks per row
+    const int g = lane >> 2, t = lane & 3;
+    const int64_t n_tok = p.sink_len + p.res_len + (p.k_new ? 1 : 0);
+    uint32_t bh[D / 16][2], bl[BF16 ? D / 16 : 1][2];
+#pragma unroll
+    for (int ks = 0; ks < D / 16; ++ks)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int c = ks * 16 + 2 * t + 8 * u;
+            bh[ks][u] = live_q ? __ldcg(reinterpret_cast<const uint32_t*>(qraw + c)) : 0u;
+            if (BF16) bl[ks][u] = live_q ? __ldcg(reinterpret_cast<const uint32_t*>(qraw + D + c)) : 0u;
+        }
+    const uint32_t vstage = stage + TILE * LD * 2;
+    for (int tile = tile_lo; tile < tile_hi; ++tile) {
+        const int64_t tok0 = int64_t(tile) * TILE;
+        if (int64_t(tile) * TILE >= n_tok) break;
+#pragma unroll 4
+        for (int i = lane; i < TILE * CPR; i += 32) {
+            const int r = i / CPR, c = i - r * CPR;
+            const int64_t tok = tok0 + r, rr = tok - p.sink_len;
+            const bool in_sink = tok < p.sink_len, fresh = rr >= p.res_len;
+            const int64_t e = in_sink ? (kvl * p.sink_ls + tok) * D : fresh ? kvl * D : (kvl * p.res_ls + rr) * D;
+            const uint16_t* kb = static_cast<const uint16_t*>(in_sink ? p.sink_k : fresh ? p.k_new : p.res_k);
+            const uint16_t* vb = static_cast<const uint16_t*>(in_sink ? p.sink_v : fresh ? p.v_new : p.res_v);
+            const int n = tok < n_tok ? 16 : 0;                          // rows past the end are zero-filled
+            const uint16_t* ks = n ? kb + e + c * 8 : reinterpret_cast<const uint16_t*>(p.rot);
+            const uint16_t* vs = n ? vb + e + c * 8 : reinterpret_cast<const uint16_t*>(p.rot);
+            cp_async16(stage + (r * LD + c * 8) * 2, ks, n);
+            cp_async16(vstage + (r * LD + c * 8) * 2, vs, n);
+            // the warp that owns the new token's tile also stores the row at the end of the recent-token buffer (the caller's
+            // slice assignment, cache.py:632-672); head groups write the same bytes
+            if (n && fresh && !in_sink) {
+                const int64_t dst = (kvl * p.res_ls + p.res_len) * D + c * 8;
+                *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.res_k_w) + dst) = __ldg(reinterpret_cast<const uint4*>(ks));
+                *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.res_v_w) + dst) = __ldg(reinterpret_cast<const uint4*>(vs));
+            }
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncwarp();
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+        const uint32_t ka = stage + ((lane & 15) * LD + (lane >> 4) * 8) * 2;
+        auto ldsm = [](uint32_t (&r)[4], uint32_t addr) {
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+        };
+        auto ldsm_t = [](uint32_t (&r)[4], uint32_t addr) {
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+        };
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) {
+            uint32_t a[4];
+            ldsm(a, ka + ks * 32);
+            if (BF16) { mma_bf16(s, a, bh[ks][0], bh[ks][1]); mma_bf16(s, a, bl[ks][0], bl[ks][1]); }
+            else mma16816(s, a[0], a[1], a[2], a[3], bh[ks][0], bh[ks][1]);
+        }
+        const bool ok0 = tok0 + g < n_tok, ok1 = tok0 + g + 8 < n_tok;
+        s[0] = ok0 ? s[0] : -INFINITY; s[1] = ok0 ? s[1] : -INFINITY;
+        s[2] = ok1 ? s[2] : -INFINITY; s[3] = ok1 ? s[3] : -INFINITY;
+        float pr[4];
+        softmax_scores<D, 0>(s, 1.f, 1.f, 0.f, st, pr);                 // (value norms are 1)
+        uint32_t bp[2], bpl[2] = {0u, 0u};
+        if (BF16) {
+            const uint32_t h0 = pack_bf2(pr[0], pr[1]), h1 = pack_bf2(pr[2], pr[3]);
+            bp[0] = movm_t(h0); bp[1] = movm_t(h1);
+            bpl[0] = movm_t(pack_bf2(pr[0] - __uint_as_float(h0 << 16), pr[1] - __uint_as_float(h0 & 0xffff0000u)));
+            bpl[1] = movm_t(pack_bf2(pr[2] - __uint_as_float(h1 << 16), pr[3] - __uint_as_float(h1 & 0xffff0000u)));
+        } else {
+            bp[0] = movm_t(pack_h2(pr[0], pr[1])); bp[1] = movm_t(pack_h2(pr[2], pr[3]));
+        }
+        const uint32_t vaddr = vstage + (((lane & 7) + ((lane >> 4) & 1) * 8) * LD + ((lane >> 3) & 1) * 8) * 2;
+#pragma unroll
+        for (int mt = 0; mt < D / 16; ++mt) {
+            uint32_t a[4];
+            ldsm_t(a, vaddr + mt * 32);
+            if (BF16) { mma_bf16(st.o[mt], a, bp[0], bp[1]); mma_bf16(st.o[mt], a, bpl[0], bpl[1]); }
+            else mma16816(st.o[mt], a[0], a[1], a[2], a[3], bp[0], bp[1]);
+        }
+        __syncwarp();
+    }
+}
+
+// ---- launch 1: the queries ------------------------------------------------------------------------------
+// q_rot[h][j] = sum_k q[h][k] R[j][k] (rotation.py:81-110), u[h][p] = sum_k q[h][k] S[p][k] (qjl.py:70-94), both times
+// scale * log2(e), fp16; the raw query likewise (bf16 caches: high and low bf16 parts).  A warp owns 16 rows of R (or S) as
+// the A operand and eight query heads as the B operand; both are split into fp16 high and 2^-11 low parts (the product of
+// the low parts is below float32 resolution).  Grid (eight heads, groups of four warps' rows).
+template <int D>
+__global__ void __launch_bounds__(128) lut_query_kernel(DecodeParams p) {
+    constexpr int QS = q_stride(D), KS = D / 16;
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int slab = blockIdx.y * 4 + (threadIdx.x >> 5), n_slabs = KS + (p.qjl_proj ? 2 : 0);
+    const int64_t n_q = int64_t(p.B) * p.Hq, q0 = int64_t(blockIdx.x) * 8;
+    pdl_trigger();
+    auto split = [](float2 x, uint32_t& h, uint32_t& l) {
+        const __half2 a = __floats2half2_rn(x.x, x.y);
+        const float2 af = __half22float2(a);
+        h = *reinterpret_cast<const uint32_t*>(&a);
+        l = pack_h2((x.x - af.x) * 2048.f, (x.y - af.y) * 2048.f);
+    };
+    // this warp's rows of R (or S) as operand fragments: constants, so they are in registers before the wait
+    const bool sk = slab >= KS, live = slab < n_slabs;
+    const float* row = sk && live ? p.qjl_proj + int64_t(slab - KS) * 16 * D : p.rot + int64_t(min(slab, KS - 1)) * 16 * D;
+    uint32_t ah[KS][4], al[KS][4];
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            split(__ldg(reinterpret_cast<const float2*>(row + (g + (r & 1) * 8) * D + ks * 16 + 2 * t + (r >> 1) * 8)), ah[ks][r], al[ks][r]);
+    pdl_wait();
+    await_gather(p);   // (head-sharded decoding) the peers' heads of an earlier call have arrived
+    if (p.n_peers > 0 && blockIdx.y == 0) {           // this call's epoch of every group, for the merge launch
+        const int n_groups = p.B * p.Hkv * p.HG;
+        for (int i = blockIdx.x * 128 + threadIdx.x; i < n_groups; i += gridDim.x * 128) ++p.epochs[i];
+    }
+    const float f = p.scale * LOG2E;
+    float2 x[KS][2];                                  // head q0 + g: coordinates 16 ks + 2 t, + 1 and the same + 8
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            x[ks][u] = make_float2(0.f, 0.f);
+            if (q0 + g < n_q) {
+                const int64_t e = (q0 + g) * D + ks * 16 + 2 * t + 8 * u;
+                x[ks][u] = make_float2(load_as_f32(p.q, p.q_dtype, e) * f, load_as_f32(p.q, p.q_dtype, e + 1) * f);
+            }
+        }
+    float ym[4] = {0.f, 0.f, 0.f, 0.f}, yc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+        uint32_t bh[2], bl[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            split(x[ks][u], bh[u], bl[u]);
+            if (slab == 0 && q0 + g < n_q) {          // the raw query
+                const int64_t o = (q0 + g) * QS + D + ks * 16 + 2 * t + 8 * u;
+                if (p.dense_dtype == TQ_BF16) {
+                    const uint32_t h = pack_bf2(x[ks][u].x, x[ks][u].y);
+                    *reinterpret_cast<uint32_t*>(p.st_q16 + o) = h;
+                    *reinterpret_cast<uint32_t*>(p.st_q16 + o + D) = pack_bf2(x[ks][u].x - __uint_as_float(h << 16), x[ks][u].y - __uint_as_float(h & 0xffff0000u));
+                } else {
+                    *reinterpret_cast<uint32_t*>(p.st_q16 + o) = bh[u];
+                }
+            }
+        }
+        mma16816(ym, ah[ks][0], ah[ks][1], ah[ks][2], ah[ks][3], bh[0], bh[1]);
+        mma16816(yc, al[ks][0], al[ks][1], al[ks][2], al[ks][3], bh[0], bh[1]);
+        mma16816(yc, ah[ks][0], ah[ks][1], ah[ks][2], ah[ks][3], bl[0], bl[1]);
+    }
+    if (!live) return;
+    const int dst = sk ? 3 * D + (slab - KS) * 16 : slab * 16;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {              // rows g, g + 8 of the slab x heads 2t, 2t + 1
+        const int64_t h = q0 + 2 * t + (r & 1);
+        if (h < n_q) p.st_q16[h * QS + dst + g + (r >> 1) * 8] = __float2half_rn(ym[r] + yc[r] * (1.f / 2048.f));
+    }
+}
+
+// ---- launch 2: the persistent grid ----------------------------------------------------------------------
+__device__ __forceinline__ int fmt_of(int hi, int lo) { return lo ? hi * 10 + lo : hi; }
+
+template <int D, bool QJL>
+__global__ void __launch_bounds__(Plan<D, QJL>::NT, 1) decode_lut_kernel(DecodeParams p) {
+    using P = Plan<D, QJL>;
+    constexpr int NZ = QJL ? QM / 16 : 0, NS = P::NS, NW = P::NW, NT = P::NT, NC = P::NC;
+    constexpr int QS = q_stride(D), PS = part_stride(D);
+    extern __shared__ __align__(16) unsigned char smem[];
+    const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+    auto gp = [&](uint32_t addr) -> unsigned char* { return smem + (addr - sbase); };
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    if (sbase > LO_BASE || (sbase & 15u)) {            // cannot happen after the host-side probe; never run on a bad plan
+        if (tid == 0) atomicCAS(p.status, 0, ERR_LAYOUT);
+        return;
+    }
+    pdl_trigger();
+    const uint32_t bar0 = P::BARS + 8u * uint32_t(warp) * NS, my_area = AREA0 + uint32_t(warp) * P::AREA;
+    int* owner = reinterpret_cast<int*>(gp(P::OWNER));
+    if (lane == 0) {
+#pragma unroll
+        for (int s = 0; s < NS; ++s) mbar_init(bar0 + 8u * s, 32);      // every lane arrives when its copies into the stage have completed
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        owner[warp] = -1;
+        if (warp == 0) owner[NW] = -1;
+    }
+    const int kf = fmt_of(p.kb_hi, p.kb_lo), vf = fmt_of(p.vb_hi, p.vb_lo);
+    // ---------------- tables: constants only, before the wait for the previous launch ----------------
+    if (p.c_len > 0) {
+        auto cent = [&](const float* c, int i, float sc) -> uint32_t { return uint32_t(__half_as_ushort(__float2half_rn(__ldg(c + i) * sc))); };
+        const float* ck[2] = {p.kc_hi, p.kc_lo};
+        const float* cv[2] = {p.vc_hi, p.vc_lo};
+        const int kb[2] = {p.kb_hi, p.kb_lo}, vb[2] = {p.vb_hi, p.vb_lo};
+        for (int side = 0; side < 2; ++side) {
+            const float* const* cc = side ? cv : ck;
+            const int* bb = side ? vb : kb;
+            for (int part = 0; part < 2; ++part) {
+                const float* c = cc[part];
+                const int b = bb[part];
+                const float sc = side == 0 ? 1.f : part ? p.v_scale_lo : p.v_scale_hi;
+                if (b == 3) {
+                    for (int i = tid; i < 64 * 8; i += NT) {               // 64 entries of eight 16-byte pieces
+                        const int e = i >> 3;
+                        const uint32_t x = cent(c, e & 7, sc) | (cent(c, e >> 3, sc) << 16);
+                        *reinterpret_cast<uint4*>(gp((side ? TAB_V3 : TAB_K3) + uint32_t(i) * 16u)) = make_uint4(x, x, x, x);
+                    }
+                } else if (b == 4) {
+                    for (int i = tid; i < 256 * 8; i += NT) {
+                        const int e = i >> 3;
+                        const uint32_t x = cent(c, e & 15, sc) | (cent(c, e >> 4, sc) << 16);
+                        *reinterpret_cast<uint4*>(gp(TAB_B + uint32_t(e) * 256u + (side ? 128u : 0u) + uint32_t(i & 7) * 16u)) = make_uint4(x, x, x, x);
+                    }
+                } else if (b == 2) {
+                    for (int i = tid; i < 256 * 8; i += NT) {
+                        const int e = i >> 3;
+                        // keys: four coordinates in a row; values: low nibble = two coordinates of the first token, high nibble of the second
+                        const int i0 = e & 3, i1 = (e >> 2) & 3, i2 = (e >> 4) & 3, i3 = e >> 6;
+                        const uint32_t x = cent(c, i0, sc) | (cent(c, side ? i2 : i1, sc) << 16), y = cent(c, side ? i1 : i2, sc) | (cent(c, i3, sc) << 16);
+                        *reinterpret_cast<uint4*>(gp(TAB_B + uint32_t(e) * 256u + (side ? 128u : 0u) + uint32_t(i & 7) * 16u)) = make_uint4(x, y, x, y);
+                    }
+                }
+            }
+        }
+    }
+    __syncthreads();
+    pdl_wait();        // the prepared queries, the cache and the workspace are settled from here on
+    bool failed = false;
+
+    const int L = p.B * p.Hkv * p.HG;                          // cache lanes x head groups
+    const int n_tiles = int((p.c_len + TILE - 1) / TILE);      // packed tiles per lane
+    const int n_slots = p.st_npp + p.st_nd;                    // partial slots per lane
+    const int wg = blockIdx.x * NW + warp, n_warps = gridDim.x * NW;
+    const int c_len = int(p.c_len);
+    const bool fold = p.st_fold != 0;                          // the warps of the CTA fold their partials of a lane into one
+    const int64_t unit = fold ? p.st_range * NW : p.st_range;  // tiles behind one partial slot
+    auto heads_of = [&](int a) { return min(HPG, p.G - (a % p.HG) * HPG); };
+    auto qhead_of = [&](int a) -> int64_t {                    // first query head of lane a
+        const int kvl = a / p.HG, hg = a - kvl * p.HG, b = kvl / p.Hkv, hkv = kvl - b * p.Hkv;
+        return int64_t(b) * p.Hq + int64_t(hkv) * p.G + hg * HPG;
+    };
+
+    // ---------------- uncompressed tokens: items i in [i0, i1) of the L * nd (lane, run of dt tiles) pairs ----------------
+    if (p.st_nd > 0) {
+        const int64_t n_items = int64_t(L) * p.st_nd;
+        // dealt from the far end: with few items the warps that have none are the ones whose packed runs are full
+        const int wr = n_warps - 1 - wg;
+        const int i0 = int((int64_t(wr) * n_items + n_warps - 1) / n_warps), i1 = int((int64_t(wr + 1) * n_items + n_warps - 1) / n_warps);
+        for (int i = i0; i < i1; ++i) {
+            const int a = i / p.st_nd, part = i - a * p.st_nd, heads_here = heads_of(a);
+            const __half* qraw = p.st_q16 + (qhead_of(a) + min(g, heads_here - 1)) * QS + D;
+            WarpAcc<D, 0> sd;
+            sd.init();
+            if (p.dense_dtype == TQ_F16) {
+                dense_run<D, false>(p, a / p.HG, part * p.st_dt, (part + 1) * p.st_dt, my_area, qraw, g < heads_here, sd, lane);
+            } else if (p.dense_dtype == TQ_BF16) {
+                dense_run<D, true>(p, a / p.HG, part * p.st_dt, (part + 1) * p.st_dt, my_area, qraw, g < heads_here, sd, lane);
+            } else {
+                uint32_t bq[D / 16][2];
+#pragma unroll
+                for (int ks = 0; ks < D / 16; ++ks) {
+                    bq[ks][0] = g < heads_here ? __ldcg(reinterpret_cast<const uint32_t*>(qraw + ks * 16 + 2 * t)) : 0u;
+                    bq[ks][1] = g < heads_here ? __ldcg(reinterpret_cast<const uint32_t*>(qraw + ks * 16 + 2 * t + 8)) : 0u;
+                }
+                __half* Ks = reinterpret_cast<__half*>(gp(my_area));
+                dense_tiles<D, 1, 0>(p, a / p.HG, int64_t(part) * p.st_dt, int64_t(part + 1) * p.st_dt, Ks, Ks + TILE * stage_ld<D>(), bq, sd, 0, lane);
+            }
+            sd.finish();
+#pragma unroll
+            for (int off = 4; off < 32; off <<= 1) {
+                sd.l[0] += __shfl_xor_sync(0xffffffffu, sd.l[0], off);
+                sd.l[1] += __shfl_xor_sync(0xffffffffu, sd.l[1], off);
+            }
+            float* pp = p.st_part + (int64_t(a) * n_slots + p.st_npp + part) * p.slots * PS;
+            if (2 * t < heads_here) {
+                const bool two = 2 * t + 1 < heads_here;
+                float* h0 = pp + (2 * t) * PS;
+                float* h1 = h0 + PS;
+#pragma unroll
+                for (int mt = 0; mt < D / 16; ++mt) {           // rows are coordinates mt * 16 + g and + 8
+                    const int c = mt * 16 + g;
+                    h0[c] = sd.o[mt][0]; h0[c + 8] = sd.o[mt][2];
+                    if (two) { h1[c] = sd.o[mt][1]; h1[c + 8] = sd.o[mt][3]; }
+                }
+                if (g == 0) {
+                    h0[D + QM] = sd.m[0]; h0[D + QM + 1] = sd.l[0];
+                    if (two) { h1[D + QM] = sd.m[1]; h1[D + QM + 1] = sd.l[1]; }
+                }
+            }
+            __syncwarp();
+        }
+    }
+
+    // ---------------- packed tokens: flat tiles [T0, T1) of the L * n_tiles ----------------------------------
+    const int64_t total = int64_t(L) * n_tiles;
+    const int64_t T0 = min(int64_t(wg) * p.st_range, total), T1 = min(T0 + p.st_range, total);
+    const int n_my = int(T1 - T0);
+    if (n_my > 0) {
+        const int kwh = packed_bytes(p.kb_lo ? D / 2 : D, p.kb_hi), kwl = p.kb_lo ? packed_bytes(D / 2, p.kb_lo) : 0;
+        const int vwh = packed_bytes(p.vb_lo ? D / 2 : D, p.vb_hi), vwl = p.vb_lo ? packed_bytes(D / 2, p.vb_lo) : 0;
+        // A stage holds the tile's scalars, then its key rows (first part, second part) and value rows, back to back; lane l
+        // copies 16-byte chunks l, l + 32, ...  (16 rows of w bytes are w chunks.)  Sources advance by 16 rows per tile.
+        const int n_sc = int(P::SC / 16), n_chunks = n_sc + kwh + kwl + vwh + vwl;
+        const unsigned char* cp_ptr[NC];
+        uint32_t cp_step[NC];
+        int ia = int(T0 / n_tiles), iti = int(T0 - int64_t(ia) * n_tiles);    // lane and tile of the next copy
+        {
+            const int64_t row = int64_t(ia / p.HG) * p.c_ls + int64_t(iti) * TILE;
+#pragma unroll
+            for (int j = 0; j < NC; ++j) {
+                int c = lane + 32 * j;
+                const unsigned char* base = p.k_hi;
+                int rb = kwh;
+                if (c < n_sc) {
+                    const int arr = c >> 2;
+                    base = reinterpret_cast<const unsigned char*>(arr == 0 ? static_cast<const void*>(p.k_norms) : arr == 1 ? static_cast<const void*>(p.v_norms)
+                                                                  : arr == 2 ? static_cast<const void*>(p.k_qbits) : arr == 3 ? static_cast<const void*>(p.k_qgamma)
+                                                                  : arr == 4 ? static_cast<const void*>(p.v_qbits) : static_cast<const void*>(p.v_qgamma));
+                    rb = 4; c &= 3;
+                } else {
+                    c -= n_sc;
+                    if (c >= kwh) { c -= kwh; base = p.k_lo; rb = kwl;
+                        if (c >= kwl) { c -= kwl; base = p.v_hi; rb = vwh;
+                            if (c >= vwh) { c -= vwh; base = p.v_lo; rb = vwl; } } }
+                }
+                cp_ptr[j] = base + row * rb + 16 * c;
+                cp_step[j] = lane + 32 * j < n_chunks ? uint32_t(TILE * rb) : 0u;
+            }
+        }
+        auto issue = [&](int stage) {
+            const uint32_t bar = bar0 + 8u * stage, dst = my_area + uint32_t(stage) * P::STAGE + 16u * lane;
+#pragma unroll
+            for (int j = 0; j < NC; ++j) {
+                if (cp_step[j]) cp_async16(dst + 512u * j, cp_ptr[j], 16);
+                cp_ptr[j] += cp_step[j];
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+            if (++iti == n_tiles) {          // the next copy starts the next lane: same rows again (next head group) or the next lane's storage
+                const int64_t jump = ((ia + 1) / p.HG != ia / p.HG ? p.c_ls : 0) - int64_t(n_tiles) * TILE;
+#pragma unroll
+                for (int j = 0; j < NC; ++j) cp_ptr[j] += jump * int64_t(cp_step[j] / TILE);
+                iti = 0; ++ia;
+            }
+        };
+        __syncwarp();
+#pragma unroll 1
+        for (int n = 0; n < min(n_my, NS); ++n) issue(n);
+
+        const Copies cpy{uint32_t(lane * 4), uint32_t((lane & 15) * 8)};
+        const int tokA = tok_of_slot(g);                            // tokens of MMA rows g and g + 8: tokA, tokA + 8
+        const uint32_t a_off = 4u * tokA;
+        const uint32_t p_off = 4u * t;                              // tokens t, t + 4, t + 8, t + 12: k slots 2t, 2t + 1, 2t + 8, 2t + 9
+        // where this lane's bits start: key rows tokA of the first / second part (its share: a quarter of the coordinates), value rows
+        // t (its share: an eighth); byte offset of the word and the bit shift inside it
+        auto word_at = [](uint32_t bit, uint32_t base, uint32_t& sh) -> uint32_t { sh = bit & 31u; return base + (bit >> 5) * 4u; };
+        uint32_t ksh0, ksh1, vsh0, vsh1;
+        const uint32_t o_k = P::SC, o_kl = o_k + 16u * kwh, o_v = o_kl + 16u * kwl, o_vl = o_v + 16u * vwh;
+        const uint32_t k_off0 = word_at(8u * (tokA * kwh) + 2u * kwh * t, o_k, ksh0);
+        const uint32_t k_off1 = word_at(8u * (tokA * kwl) + 2u * kwl * t, o_kl, ksh1);
+        const uint32_t v_off0 = word_at(8u * (t * vwh) + uint32_t(vwh * g), o_v, vsh0);
+        const uint32_t v_off1 = word_at(8u * (t * vwl) + uint32_t(vwl * g), o_vl, vsh1);
+
+        const int tail_ti = (c_len & (TILE - 1)) ? n_tiles - 1 : -1;          // the tile that reaches past the end of the cache
+        int a = int(T0 / n_tiles), ti = int(T0 - int64_t(a) * n_tiles);       // lane and tile being computed
+        int slot = int(T0 / unit) - int((int64_t(a) * n_tiles) / unit);       // partial slot = rank of this warp (CTA) among the lane's
+        int heads_here = 0;
+        uint32_t bq[D / 16][2];
+        uint32_t bu[QM / 16][2];
+        auto load_query = [&]() {
+            heads_here = heads_of(a);
+            const __half* qh = p.st_q16 + (qhead_of(a) + g) * QS;
+            // this lane's coordinates of k-step ks: four in a row
+            const bool split = p.kb_lo != 0;
+#pragma unroll
+            for (int ks = 0; ks < D / 16; ++ks) {
+                const int c = split ? (ks < D / 32 ? t * (D / 8) + 4 * ks : D / 2 + t * (D / 8) + 4 * (ks - D / 32)) : t * (D / 4) + 4 * ks;
+                // (written by the launch before this one while this grid may already have been resident: read at L2, never through a non-coherent path)
+                uint2 x = make_uint2(0u, 0u);
+                if (g < heads_here) x = __ldcg(reinterpret_cast<const uint2*>(qh + c));
+                bq[ks][0] = x.x; bq[ks][1] = x.y;
+            }
+            if (QJL) {
+                // k slot (ks, register hh, half e) of lane t stands for sketch row 4t + 2ks + hh + 16e: the halves of an
+                // operand register are then bits 16 apart in a token's sign word
+#pragma unroll
+                for (int ks = 0; ks < QM / 16; ++ks)
+#pragma unroll
+                    for (int hh = 0; hh < 2; ++hh) {
+                        const int pi = 4 * t + 2 * ks + hh;
+                        bu[ks][hh] = 0u;
+                        if (g < heads_here) {
+                            const unsigned short lo16 = __ldcg(reinterpret_cast<const unsigned short*>(qh + 3 * D + pi));
+                            const unsigned short hi16 = __ldcg(reinterpret_cast<const unsigned short*>(qh + 3 * D + pi + 16));
+                            bu[ks][hh] = uint32_t(lo16) | (uint32_t(hi16) << 16);
+                        }
+                    }
+            }
+        };
+        WarpAcc<D, NZ> st;
+        st.init();
+        load_query();
+        // one partial (up to eight heads of PS floats) to dst: values, sketch rows, maximum, sum
+        auto write_partial = [&](float* dst) {
+            st.finish();
+#pragma unroll
+            for (int off = 4; off < 32; off <<= 1) {
+                st.l[0] += __shfl_xor_sync(0xffffffffu, st.l[0], off);
+                st.l[1] += __shfl_xor_sync(0xffffffffu, st.l[1], off);
+            }
+            if (2 * t < heads_here) {
+                const bool two = 2 * t + 1 < heads_here, split = p.vb_lo != 0;
+                float* h0 = dst + (2 * t) * PS;
+                float* h1 = h0 + PS;
+#pragma unroll
+                for (int mt = 0; mt < D / 16; ++mt) {              // rows g, g + 8 of m-tile mt: two coordinates in a row of this lane's share
+                    const int c = split ? (mt < D / 32 ? g * (D / 16) + 2 * mt : D / 2 + g * (D / 16) + 2 * (mt - D / 32)) : g * (D / 8) + 2 * mt;
+                    *reinterpret_cast<float2*>(h0 + c) = make_float2(st.o[mt][0], st.o[mt][2]);
+                    if (two) *reinterpret_cast<float2*>(h1 + c) = make_float2(st.o[mt][1], st.o[mt][3]);
+                }
+#pragma unroll
+                for (int mz = 0; mz < NZ; ++mz) {
+                    h0[D + 16 * mz + g] = st.z[mz][0]; h0[D + 16 * mz + g + 8] = st.z[mz][2];
+                    if (two) { h1[D + 16 * mz + g] = st.z[mz][1]; h1[D + 16 * mz + g + 8] = st.z[mz][3]; }
+                }
+                if (g == 0) {
+                    h0[D + QM] = st.m[0]; h0[D + QM + 1] = st.l[0];
+                    if (two) { h1[D + QM] = st.m[1]; h1[D + QM + 1] = st.l[1]; }
+                }
+            }
+        };
+        auto slot_ptr = [&]() -> float* { return p.st_part + (int64_t(a) * n_slots + slot) * p.slots * PS; };
+
+#pragma unroll 1
+        for (int n = 0, stage = 0, phase = 0; n < n_my; ++n) {
+            const uint32_t sa = my_area + uint32_t(stage) * P::STAGE;
+            if (!__all_sync(0xffffffffu, mbar_wait(bar0 + 8u * stage, uint32_t(phase)))) {
+                // the copies never landed: record it, drain what is still in flight (bounded), stop - nothing may land in
+                // this CTA's memory after it has gone
+                atomicCAS(p.status, 0, ERR_RING);
+                failed = true;
+                for (int m = n + 1; m < min(n_my, n + NS); ++m) mbar_wait(bar0 + 8u * (m % NS), uint32_t(m / NS) & 1u);
+                break;
+            }
+            const bool partial = ti == tail_ti;
+
+            // ---- scores: S[token][head] = K . q^T ----
+            float s[4] = {0.f, 0.f, 0.f, 0.f};
+            if (kf == F4) key_part<4, D / 16>(s, sa + k_off0, 8u * kwh, ksh0, bq, cpy);
+            else if (kf == F3) key_part<3, D / 16>(s, sa + k_off0, 8u * kwh, ksh0, bq, cpy);
+            else if (kf == F2) key_part<2, D / 16>(s, sa + k_off0, 8u * kwh, ksh0, bq, cpy);
+            else {
+                if (kf == F43) key_part<4, D / 32>(s, sa + k_off0, 8u * kwh, ksh0, bq, cpy);
+                else key_part<2, D / 32>(s, sa + k_off1, 8u * kwl, ksh1, bq + D / 32, cpy);
+                if (kf == F43) key_part<3, D / 32>(s, sa + k_off1, 8u * kwl, ksh1, bq + D / 32, cpy);
+                else key_part<3, D / 32>(s, sa + k_off0, 8u * kwh, ksh0, bq, cpy);
+            }
+            const uint32_t aa = sa + a_off;
+            const float kn0 = ring_f32o<P::O_KN>(aa), kn1 = ring_f32o<P::O_KN + 32>(aa);
+            float vn0 = ring_f32o<P::O_VN>(aa), vn1 = ring_f32o<P::O_VN + 32>(aa);
+            float gv0 = 0.f, gv1 = 0.f;
+            if (QJL) {
+                // sketch term: (c/d) gamma_k * sum_p sign_p (S q)[p]; signs of rows 4t + q (+ 16) sit at bits 12 + q, 28 + q after one shift
+                const uint32_t zs0 = ring32o<P::O_KB>(aa) << (12 - 4 * t), zs1 = ring32o<P::O_KB + 32>(aa) << (12 - 4 * t);
+                float sq[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int ks = 0; ks < QM / 16; ++ks)
+                    mma16816(sq, sign_pair16(zs0 << (3 - 2 * ks)), sign_pair16(zs1 << (3 - 2 * ks)), sign_pair16(zs0 << (2 - 2 * ks)),
+                             sign_pair16(zs1 << (2 - 2 * ks)), bu[ks][0], bu[ks][1]);
+                const float gk0 = ring_f32o<P::O_KG>(aa) * (QJL_C / D), gk1 = ring_f32o<P::O_KG + 32>(aa) * (QJL_C / D);
+                s[0] = fmaf(s[0], kn0, sq[0] * gk0); s[1] = fmaf(s[1], kn0, sq[1] * gk0);
+                s[2] = fmaf(s[2], kn1, sq[2] * gk1); s[3] = fmaf(s[3], kn1, sq[3] * gk1);
+                gv0 = ring_f32o<P::O_VG>(aa); gv1 = ring_f32o<P::O_VG + 32>(aa);
+            } else {
+                s[0] *= kn0; s[1] *= kn0; s[2] *= kn1; s[3] *= kn1;
+            }
+            if (partial) {
+                // the last tile of a lane reaches past the end of the cache: its missing tokens (arbitrary bytes) get no weight
+                __syncwarp();
+                const bool ok0 = ti * TILE + tokA < c_len, ok1 = ti * TILE + tokA + 8 < c_len;
+                vn0 = ok0 ? vn0 : 0.f; vn1 = ok1 ? vn1 : 0.f; gv0 = ok0 ? gv0 : 0.f; gv1 = ok1 ? gv1 : 0.f;
+                s[0] = ok0 ? s[0] : -INFINITY; s[1] = ok0 ? s[1] : -INFINITY;
+                s[2] = ok1 ? s[2] : -INFINITY; s[3] = ok1 ? s[3] : -INFINITY;
+            }
+            float pr[4];
+            softmax_scores<D, NZ>(s, vn0, vn1, fmaxf(gv0, gv1), st, pr);
+            uint32_t bp[2];
+            bp[0] = movm_t(pack_h2(pr[0] * vn0, pr[1] * vn0));
+            bp[1] = movm_t(pack_h2(pr[2] * vn1, pr[3] * vn1));
+
+            // ---- values: O^T[coordinate][head] += V^T . P^T ----
+            if (vf == F4) value_part<4, D / 16>(st.o, sa + v_off0, 4u * vwh, vsh0, bp, cpy);
+            else if (vf == F3) value_part<3, D / 16>(st.o, sa + v_off0, 4u * vwh, vsh0, bp, cpy);
+            else if (vf == F2) value_part<2, D / 16>(st.o, sa + v_off0, 4u * vwh, vsh0, bp, cpy);
+            else if (vf == F43) {
+                value_part<4, D / 32>(st.o, sa + v_off0, 4u * vwh, vsh0, bp, cpy);
+                value_part<3, D / 32>(st.o + D / 32, sa + v_off1, 4u * vwl, vsh1, bp, cpy);
+            } else {
+                value_part<3, D / 32>(st.o, sa + v_off0, 4u * vwh, vsh0, bp, cpy);
+                value_part<2, D / 32>(st.o + D / 32, sa + v_off1, 4u * vwl, vsh1, bp, cpy);
+            }
+            if (QJL) {
+                // sketch rows of the output: z[row][head] += sum_t sign_row(t) * (p_t * gamma_v[t])
+                const uint32_t bz0 = movm_t(pack_h2(pr[0] * gv0, pr[1] * gv0));
+                const uint32_t bz1 = movm_t(pack_h2(pr[2] * gv1, pr[3] * gv1));
+                const uint32_t zv0 = ring32o<P::O_VB>(sa + p_off), zv1 = ring32o<P::O_VB + 16>(sa + p_off);
+                const uint32_t zv2 = ring32o<P::O_VB + 32>(sa + p_off), zv3 = ring32o<P::O_VB + 48>(sa + p_off);
+                // put the two tokens' half-words side by side (row r of the first at bit r, of the second at bit r + 16)
+                const uint32_t x01 = __byte_perm(zv0, zv1, 0x5410) << (7 - g), y01 = __byte_perm(zv0, zv1, 0x7632) << (7 - g);
+                const uint32_t x23 = __byte_perm(zv2, zv3, 0x5410) << (7 - g), y23 = __byte_perm(zv2, zv3, 0x7632) << (7 - g);
+                mma16816(st.z[0], sign_pair16(x01 << 8), sign_pair16(x01), sign_pair16(x23 << 8), sign_pair16(x23), bz0, bz1);
+                mma16816(st.z[NZ ? 1 : 0], sign_pair16(y01 << 8), sign_pair16(y01), sign_pair16(y23 << 8), sign_pair16(y23), bz0, bz1);
+            }
+
+            // ---- the stage is free: ask for the tile NS further on ----
+            if (n + NS < n_my) {
+                __syncwarp();
+                issue(stage);
+            }
+            if (++stage == NS) { stage = 0; phase ^= 1; }
+            if (++ti == n_tiles) {       // the next tile belongs to the next lane
+                if (!fold) {
+                    write_partial(slot_ptr());
+                    ti = 0; ++a; slot = 0;
+                    if (n + 1 < n_my) { st.init(); load_query(); }
+                } else if (n + 1 < n_my) {               // this warp is the CTA's one that crosses into the next lane
+                    write_partial(reinterpret_cast<float*>(gp(P::SPILL)));
+                    if (lane == 0) owner[NW] = a;
+                    ti = 0; ++a;
+                    st.init();
+                    load_query();
+                }
+            }
+        }
+        if (!failed) {
+            if (fold) {
+                __syncwarp();
+                write_partial(reinterpret_cast<float*>(gp(my_area)));        // (the ring is drained: every copy was waited for)
+                if (lane == 0) owner[warp] = a;
+            } else if (ti != 0) write_partial(slot_ptr());
+        }
+    }
+    if (!fold) return;
+
+    // ---------------- fold: one partial per (CTA, lane), from the warps' partials in shared memory ----------------
+    __syncthreads();
+    const int64_t C0 = min(int64_t(blockIdx.x) * unit, total), C1 = min(C0 + unit, total);
+    if (C0 >= C1) return;
+    const int a_first = int(C0 / n_tiles), a_last = int((C1 - 1) / n_tiles);
+    for (int a = a_first; a <= a_last; ++a) {
+        const int heads_here = heads_of(a);
+        const int slot = int(blockIdx.x) - int((int64_t(a) * n_tiles) / unit);
+        float* dst = p.st_part + (int64_t(a) * n_slots + slot) * p.slots * PS;
+        constexpr int NE = D + (QJL ? QM : 0);
+        for (int e = tid; e < heads_here * NE; e += NT) {
+            const int h = e / NE, c = e - h * NE;
+            float m[NW + 1], M = -INFINITY;
+#pragma unroll
+            for (int w = 0; w <= NW; ++w) {
+                const float* src = reinterpret_cast<const float*>(gp(w < NW ? AREA0 + uint32_t(w) * P::AREA : P::SPILL)) + h * PS;
+                m[w] = owner[w] == a ? src[D + QM] : -INFINITY;
+                M = fmaxf(M, m[w]);
+            }
+            float acc = 0.f, sum = 0.f;
+#pragma unroll
+            for (int w = 0; w <= NW; ++w) {
+                if (m[w] == -INFINITY) continue;
+                const float* src = reinterpret_cast<const float*>(gp(w < NW ? AREA0 + uint32_t(w) * P::AREA : P::SPILL)) + h * PS;
+                const float x = ex2(m[w] - M);
+                acc = fmaf(x, src[c], acc);
+                if (c == 0) sum = fmaf(x, src[D + QM + 1], sum);
+            }
+            dst[h * PS + c] = acc;
+            if (c == 0) { dst[h * PS + D + QM] = M; dst[h * PS + D + QM + 1] = sum; }
+        }
+    }
+}
+
+// ---- launch 3: merge --------------------------------------------------------------------------------------
+// A thread per (lane, query head, coordinate), some 512 threads to a block.  At d <= 128, R and S are staged in shared
+// memory before the wait, so the rotation back costs shared-memory reads; at d = 256 (R alone is 256 KB) it reads them
+// at L1 / L2.
+constexpr int sets_per_block(int d) { return 512 / d; }
+template <int D> __host__ __device__ constexpr bool stages_r() { return D <= 128; }
+template <int D> __host__ __device__ constexpr size_t merge_smem() {
+    return (size_t(stages_r<D>() ? (D + QM) * D : 0) + size_t(512 / D) * (2 * MAX_PARTS + D + QM)) * sizeof(float);
+}
+template <int D, bool QJL>
+__global__ void __launch_bounds__(512) lut_merge_kernel(DecodeParams p, int nw) {
+    extern __shared__ __align__(16) unsigned char smem_m[];
+    constexpr int PS = part_stride(D), SPB = 512 / D, NTH = SPB * D;
+    float* rs = reinterpret_cast<float*>(smem_m);                 // [D][D] R, then [32][D] S
+    const int tid = threadIdx.x, set = tid / D, c = tid - set * D;
+    float* s_m = rs + (stages_r<D>() ? (D + QM) * D : 0) + set * (2 * MAX_PARTS + D + QM);
+    float* s_l = s_m + MAX_PARTS;
+    float* s_rot = s_l + MAX_PARTS;
+    float* s_z = s_rot + D;
+    pdl_trigger();
+    if (stages_r<D>()) {
+        const int rows = D + (QJL ? QM : 0);
+        for (int i = tid; i < rows * (D / 4); i += NTH) {      // constants: before the wait
+            const int r = i / (D / 4), k4 = i - r * (D / 4);
+            *reinterpret_cast<float4*>(rs + r * D + 4 * k4) = __ldg(reinterpret_cast<const float4*>(r < D ? p.rot + int64_t(r) * D : p.qjl_proj + int64_t(r - D) * D) + k4);
+        }
+    }
+    pdl_wait();
+    const int L = p.B * p.Hkv * p.HG;
+    const int64_t idx = int64_t(blockIdx.x) * SPB + set;
+    const int a = int(min(idx / p.slots, int64_t(L - 1))), h = int(idx % p.slots);
+    const int kvl = a / p.HG, hg = a - kvl * p.HG, b = kvl / p.Hkv, hkv = kvl - b * p.Hkv;
+    const int heads_here = min(HPG, p.G - hg * HPG);
+    const bool live = idx < int64_t(L) * p.slots && h < heads_here;
+    const int64_t qhead = int64_t(b) * p.Hq + int64_t(hkv) * p.G + hg * HPG + h;
+    const int n_tiles = int((p.c_len + TILE - 1) / TILE);
+    const int n_slots = p.st_npp + p.st_nd;
+    const int64_t unit = p.st_fold ? p.st_range * nw : p.st_range;
+    // the warps (CTAs) whose runs touch this lane's tiles [a * n_tiles, (a + 1) * n_tiles)
+    const int n_pp = n_tiles > 0 ? int((int64_t(a + 1) * n_tiles - 1) / unit) - int((int64_t(a) * n_tiles) / unit) + 1 : 0;
+    const float inv_vs = 1.f / (c < D / 2 || p.vb_lo == 0 ? p.v_scale_hi : p.v_scale_lo);
+    const float* ph = p.st_part + (int64_t(a) * n_slots * p.slots + h) * PS;
+    const int64_t sstride = int64_t(p.slots) * PS;
+    for (int i = c; i < n_slots; i += D) {
+        const bool valid = live && (i < n_pp || i >= p.st_npp);
+        s_m[i] = valid ? __ldcg(ph + i * sstride + D + QM) : -INFINITY;
+        s_l[i] = valid ? __ldcg(ph + i * sstride + D + QM + 1) : 0.f;
+    }
+    __syncthreads();
+    float M = -INFINITY;
+    for (int i = 0; i < n_slots; ++i) M = fmaxf(M, s_m[i]);
+    float Lsum = 0.f, ar = 0.f, ad = 0.f, az = 0.f;
+#pragma unroll 8
+    for (int i = 0; i < n_slots; ++i) {
+        const float mi = s_m[i];
+        const float w = mi == -INFINITY ? 0.f : ex2(mi - M);
+        const float v = mi == -INFINITY ? 0.f : __ldcg(ph + i * sstride + c);
+        Lsum = fmaf(w, s_l[i], Lsum);
+        if (i < p.st_npp) {
+            ar = fmaf(w, v, ar);
+            if (QJL && c < QM && mi != -INFINITY) az = fmaf(w, __ldcg(ph + i * sstride + D + c), az);
+        } else {
+            ad = fmaf(w, v, ad);
+        }
+    }
+    s_rot[c] = ar * inv_vs;
+    if (QJL && c < QM) s_z[c] = az * (QJL_C / D);
+    __syncthreads();
+    // undo the rotation of the packed part (y @ R, rotation.py:68-78) and add (c/d) z @ S (qjl.py:89-92)
+    float v = ad;
+#pragma unroll 8
+    for (int j = 0; j < D; ++j) v = fmaf(s_rot[j], stages_r<D>() ? rs[j * D + c] : __ldg(p.rot + j * D + c), v);
+    if (QJL) {
+#pragma unroll 8
+        for (int i = 0; i < QM; ++i) v = fmaf(s_z[i], stages_r<D>() ? rs[(D + i) * D + c] : __ldg(p.qjl_proj + i * D + c), v);
+    }
+    if (p.n_peers == 0) {
+        if (live) store_from_f32(p.out, p.out_dtype, qhead * D + c, v / Lsum);
+        return;
+    }
+    // fused gather: the head in the result's element type, sent as {payload, epoch} words (the query launch counted the call)
+    __syncthreads();
+    store_from_f32(s_rot, p.out_dtype, c, v / Lsum);
+    __syncthreads();
+    const int es = out_elem_bytes(p.out_dtype), n_words = D * es / 4;
+    if (!live) return;
+    const unsigned long long epoch = static_cast<unsigned long long>(p.epochs[a]) << 32;
+    const int64_t w0 = (int64_t(b) * p.heads_total + p.head_offset + int64_t(hkv) * p.G + hg * HPG + h) * n_words;
+    for (int i = c; i < n_words * p.n_peers; i += D) {
+        const int r = i / n_words, w = i - r * n_words;
+        const unsigned long long x = reinterpret_cast<const uint32_t*>(s_rot)[w] | epoch;
+        asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(p.peer_ll[r] + w0 + w), "l"(x) : "memory");
+    }
+}
+
+// ---- host side ------------------------------------------------------------------------------------------------
+template <int D, bool QJL> static bool fits() {
+    const unsigned sb = dd::probe_smem_base();
+    if (sb == ~0u || sb > LO_BASE || (sb & 15u)) return false;
+    int dev = 0, max_optin = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return false;
+    return size_t(Plan<D, QJL>::SMEM_END - sb) <= size_t(max_optin);
+}
+
+template <int D, bool QJL> static int launch(const DecodeParams& p, cudaStream_t s) {
+    using P = Plan<D, QJL>;
+    const size_t smem = P::SMEM_END - dd::probe_smem_base();
+    static std::atomic<bool> set[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && !set[dev].load(std::memory_order_acquire)) {
+        cudaError_t e = cudaFuncSetAttribute(decode_lut_kernel<D, QJL>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(lut_merge_kernel<D, QJL>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(merge_smem<D>()));
+        if (e != cudaSuccess) return fail(TQ_ERR_LAUNCH, "tq_decode_attn: shared memory %zu B: %s", smem, cudaGetErrorString(e));
+        set[dev].store(true, std::memory_order_release);
+    }
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = p.pdl ? 1 : 0;
+    cudaLaunchConfig_t cfg{};
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const int64_t n_q = int64_t(p.B) * p.Hq;
+    cfg.gridDim = dim3(unsigned((n_q + 7) / 8), unsigned((D / 16 + (QJL ? 2 : 0) + 3) / 4));
+    cfg.blockDim = dim3(128);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, lut_query_kernel<D>, p);
+    if (e == cudaSuccess) {
+        cfg.gridDim = dim3(unsigned(p.st_grid));
+        cfg.blockDim = dim3(P::NT);
+        cfg.dynamicSmemBytes = smem;
+        e = cudaLaunchKernelEx(&cfg, decode_lut_kernel<D, QJL>, p);
+    }
+    if (e == cudaSuccess) {
+        constexpr int SPB = 512 / D;
+        cfg.gridDim = dim3(unsigned((int64_t(p.B) * p.Hkv * p.HG * p.slots + SPB - 1) / SPB));
+        cfg.blockDim = dim3(unsigned(SPB * D));
+        cfg.dynamicSmemBytes = merge_smem<D>();
+        e = cudaLaunchKernelEx(&cfg, lut_merge_kernel<D, QJL>, p, P::NW);
+    }
+    if (e != cudaSuccess) return fail(TQ_ERR_LAUNCH, "tq_decode_attn: %s", cudaGetErrorString(e));
+    return TQ_OK;
+}
+
+}  // namespace lut
+
+static bool lut_width(int hi, int lo) { return lo ? (hi == 4 && lo == 3) || (hi == 3 && lo == 2) : hi >= 2 && hi <= 4; }
+
+bool lut_supported(int d, bool qjl, int kb_hi, int kb_lo, int vb_hi, int vb_lo) {
+    if (!lut_width(kb_hi, kb_lo) || !lut_width(vb_hi, vb_lo)) return false;
+    if (d == 64) return qjl ? lut::fits<64, true>() : lut::fits<64, false>();
+    if (d == 96) return qjl ? lut::fits<96, true>() : lut::fits<96, false>();
+    if (d == 128) return qjl ? lut::fits<128, true>() : lut::fits<128, false>();
+    if (d == 256) return qjl ? lut::fits<256, true>() : lut::fits<256, false>();
+    return false;
+}
+
+StreamPlan lut_plan(int batch, int n_q_heads, int n_kv_heads, int d, int64_t c_len, int64_t dense_len, int sms) {
+    StreamPlan s{};
+    const int nw = d == 256 ? 8 : 16;
+    const int G = n_q_heads / n_kv_heads, hg = (G + HPG - 1) / HPG;
+    const int64_t L = int64_t(batch) * n_kv_heads * hg;
+    const int64_t p_tiles = (c_len + TILE - 1) / TILE, d_tiles = (dense_len + TILE - 1) / TILE;
+    s.grid = sms;
+    const int64_t n_warps = int64_t(s.grid) * nw;
+    s.range = std::max<int64_t>((L * p_tiles + n_warps - 1) / n_warps, 1);
+    // a CTA's run of tiles no longer than a lane: it touches two lanes at most and folds its warps' partials
+    s.fold = p_tiles >= s.range * nw ? 1 : 0;
+    const int64_t unit = s.fold ? s.range * nw : s.range;
+    s.npp = p_tiles > 0 ? int((p_tiles + unit - 1) / unit) + 1 : 0;
+    if (d_tiles > 0) {
+        int64_t nd = std::min<int64_t>(d_tiles, std::max<int64_t>(n_warps / L, 1));
+        s.dt = int((d_tiles + nd - 1) / nd);
+        s.nd = int((d_tiles + s.dt - 1) / s.dt);
+    }
+    s.q16_bytes = (size_t(batch) * n_q_heads * lut::q_stride(d) * sizeof(__half) + 255) / 256 * 256;
+    s.part_bytes = size_t(L) * size_t(s.npp + s.nd) * size_t(std::min(G, HPG)) * lut::part_stride(d) * sizeof(float);
+    s.ok = s.npp + s.nd <= lut::MAX_PARTS && L * p_tiles < (int64_t(1) << 31);
+    return s;
+}
+
+int launch_decode_lut(const DecodeParams& p, cudaStream_t s) {
+    const bool qjl = p.qjl_proj != nullptr;
+    if (p.D == 64) return qjl ? lut::launch<64, true>(p, s) : lut::launch<64, false>(p, s);
+    if (p.D == 96) return qjl ? lut::launch<96, true>(p, s) : lut::launch<96, false>(p, s);
+    if (p.D == 128) return qjl ? lut::launch<128, true>(p, s) : lut::launch<128, false>(p, s);
+    return qjl ? lut::launch<256, true>(p, s) : lut::launch<256, false>(p, s);
+}
+
+}  // namespace tq
