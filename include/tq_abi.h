@@ -256,11 +256,15 @@ int tq_decode_step(const tq_decode_args* a, const void* k_new, const void* v_new
 
 /* Causal attention for t_q query tokens per sequence - the LAST t_q tokens of the cache, appended by the caller
  * beforehand: query i sits at position c_len + sink_len + res_len - t_q + i and sees every cached token up to and
- * including itself.  a->q and a->out are (batch, n_q_heads, t_q, d); workspace, tables and gather are not used.  Caches
+ * including itself.  a->q and a->out are (batch, n_q_heads, t_q, d); tables and gather are not used.  With a workspace of
+ * tq_prefill_workspace_bytes(...) bytes (256-byte aligned, contents irrelevant; more cache lanes than it holds are done
+ * in rounds, one lane at a time at least) the cache's tokens are expanded there once and attended to on the tensor cores;
+ * without one the kernels that unpack as they go run.  Caches
  * with a QJL sketch are refused with TQ_ERR_UNSUPPORTED (their callers take the dense route).  Replaces dense
  * reassembly (cache.py:674-706) + the consumer's masked attention for prefill chunks and multi-token steps; the
  * reference only sketched it for packed keys (kernels.py:558-590, docs/FUSED_ATTENTION_DESIGN.md:281-283). */
 int tq_prefill_attn(const tq_decode_args* a, int t_q, void* stream);
+size_t tq_prefill_workspace_bytes(int batch, int n_q_heads, int n_kv_heads, int d, int64_t total_len, int t_q);
 
 /* Same computation as tq_decode_attn for callers that can neither lend a workspace nor allocate one at call
  * time (a process that gave the whole device to its own memory pool at start-up; a step loop that cannot afford

@@ -550,6 +550,10 @@ class TurboQuantKVCache:
         a = self._fill_decode_args(b, hq, q.dtype, out.dtype, scale)
         a.q, a.out = q.data_ptr(), out.data_ptr()
         a.c_len, a.sink_len, a.res_len = self._compressed_len, self._sink_len, self._fp16_len
+        # scratch for the expanded rows (at most 512 MB): the allocator reuses it in stream order after this call
+        need = _lib.lib().tq_prefill_workspace_bytes(b, hq, a.n_kv_heads, d, self._sink_len + self._compressed_len + self._fp16_len, tq)
+        ws = torch.empty(need, dtype=torch.uint8, device=dev)
+        a.workspace, a.workspace_bytes = ws.data_ptr(), need
         _lib.check(_lib.launch(dev, "tq_prefill_attn", C.byref(a), tq, _lib.stream_ptr(dev)))
         return out
 

@@ -594,7 +594,7 @@ static int g_tune_splits = 0;          // > 0: fixed number of packed splits
 extern int g_tune_dequantize_tc;       // rowops.cu: 0 = dequantize always on the CUDA-core row kernel
 extern int g_tune_prefill_tc;          // prefill.cu: 0 = several-query-token attention always on the mma.sync kernel
 static int g_tune_pdl = 1;             // programmatic dependent launch between consecutive calls
-static int g_tune_lut = 1;             // 0: never take the lookup kernel for the other widths
+static int g_tune_lut = 1;             // 0: never take the lookup kernel of decode_lut.cu; 2: whenever it can (testing)
 static int g_tune_stream = 1;          // 0: never take the streaming kernel
 static int g_tune_stream_min_run = 24; // fewest packed tiles per warp for which the streaming kernel is chosen over the table-lookup kernel (a third of it over the general kernel)
 static int g_tune_stream_max_parts = 40;  // most partials per lane with which it is chosen over the table-lookup kernel (64 over the general kernel)
@@ -765,7 +765,7 @@ int decode_prepare(const tq_decode_args* a, void* workspace, size_t workspace_by
     // everything else the lookup kernel's tables cover (two to four bits, their fractional splits).  The general kernel is one launch instead of three: with whole-byte tables
     // (4-bit keys, 2-bit values) it is the faster one for few tiles (head_dim 64, 16 lanes x 218 tiles: 17 against 29 us;
     // head_dim 128 with sketches, 72 lanes x 230 tiles: 63 against 35 us)
-    bool lut = !direct && !stream && g_tune_lut && !g_tune_force_general && a->c_lane_stride % 16 == 0 &&
+    bool lut = ((!direct && !stream && g_tune_lut) || g_tune_lut == 2) && !g_tune_force_general && a->c_lane_stride % 16 == 0 &&
                aligned(a->k_hi, 16) && aligned(a->v_hi, 16) && aligned(a->k_norms, 16) && aligned(a->v_norms, 16) &&
                (!a->k_bits_lo || aligned(a->k_lo, 16)) && (!a->v_bits_lo || aligned(a->v_lo, 16)) &&
                (!qjl || (aligned(a->k_qjl_bits, 16) && aligned(a->v_qjl_bits, 16) && aligned(a->k_qjl_gamma, 16) && aligned(a->v_qjl_gamma, 16) && aligned(a->qjl_proj, 16))) &&
@@ -774,8 +774,9 @@ int decode_prepare(const tq_decode_args* a, void* workspace, size_t workspace_by
         stp = lut_plan(a->batch, a->n_q_heads, a->n_kv_heads, d, a->c_len, dense_len, sm_count());
         const int64_t tiles = int64_t(a->batch) * a->n_kv_heads * ((a->c_len + TILE - 1) / TILE);
         const bool bytes = a->k_bits_hi == 4 && !a->k_bits_lo && a->v_bits_hi == 2 && !a->v_bits_lo;
-        lut = stp.ok && !(a->c_len > 0 && bytes && tiles < 8000) && lut_supported(d, qjl, a->c_len > 0 ? a->k_bits_hi : 4, a->c_len > 0 ? a->k_bits_lo : 0, a->c_len > 0 ? a->v_bits_hi : 4, a->c_len > 0 ? a->v_bits_lo : 0);
+        lut = stp.ok && !(a->c_len > 0 && bytes && tiles < 8000 && g_tune_lut == 1) && lut_supported(d, qjl, a->c_len > 0 ? a->k_bits_hi : 4, a->c_len > 0 ? a->k_bits_lo : 0, a->c_len > 0 ? a->v_bits_hi : 4, a->c_len > 0 ? a->v_bits_lo : 0);
     }
+    if (lut) stream = false;
     const SplitPlan sp = plan_splits(a->batch, a->n_q_heads, a->n_kv_heads, a->c_len, dense_len, sm_count(), direct);
     const WsLayout wl = ws_layout(a->batch, a->n_q_heads, a->n_kv_heads, d, sp);
     const size_t st_base = align_up(std::max(size_t(a->batch) * a->n_kv_heads * sp.hg * sizeof(int), COUNTER_AREA), 256);
@@ -827,7 +828,7 @@ int decode_prepare(const tq_decode_args* a, void* workspace, size_t workspace_by
     }
     p.pdl = g_tune_pdl;
     p.words_ok = (a->c_len > 0 && aligned(a->k_hi, 4) && aligned(a->v_hi, 4)) ? 1 : 0;   // packed rows readable as 32-bit words
-    p.tables = (direct || stream) ? a->tables : nullptr;
+    p.tables = ((direct || stream) && !lut) ? a->tables : nullptr;
     if (stream || lut) {
         p.st_lut = lut ? 1 : 0; p.st_fold = stp.fold;
         p.st_grid = stp.grid; p.st_npp = stp.npp; p.st_nd = stp.nd; p.st_dt = stp.dt; p.st_range = stp.range;
@@ -836,7 +837,7 @@ int decode_prepare(const tq_decode_args* a, void* workspace, size_t workspace_by
         if (!(p.status = decode_status_ptr())) return fail(TQ_ERR_LAUNCH, "tq_decode_attn: cannot locate the status word");
     }
     *out = p;
-    *direct_out = direct && !stream;
+    *direct_out = direct && !stream && !lut;
     return TQ_OK;
 }
 
@@ -865,7 +866,7 @@ extern "C" int tq_set_tuning(const char* key, int value) {
     if (k == "decode_ctas_per_sm" && value >= 1 && value <= 8) g_tune_ctas_per_sm = value;
     else if (k == "decode_force_general" && (value == 0 || value == 1)) g_tune_force_general = value;
     else if (k == "decode_pdl" && (value == 0 || value == 1)) g_tune_pdl = value;
-    else if (k == "decode_lut" && (value == 0 || value == 1)) g_tune_lut = value;
+    else if (k == "decode_lut" && value >= 0 && value <= 2) g_tune_lut = value;
     else if (k == "decode_stream" && (value == 0 || value == 1)) g_tune_stream = value;
     else if (k == "decode_stream_min_run" && value >= 1 && value <= (1 << 20)) g_tune_stream_min_run = value;
     else if (k == "decode_stream_max_parts" && value >= 1 && value <= 64) g_tune_stream_max_parts = value;

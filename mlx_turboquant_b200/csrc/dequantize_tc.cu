@@ -57,6 +57,7 @@ struct Params {
     void* out; int out_dtype; int64_t out_lane_stride, out_row_stride;
     int n_tiles;
     int* status;
+    float* scales; int64_t scale_lane_stride;       // not null: rows leave without their norms, which are copied here (lane, row)
 };
 
 // ---- PTX wrappers -----------------------------------------------------------------------------------------
@@ -247,6 +248,7 @@ __global__ void __launch_bounds__(NT, 1) dequantize_tc_kernel(Params p) {
                 in_row = ln * p.in_lane_stride + rw;
                 off_next = ln * p.out_lane_stride + rw * p.out_row_stride;
                 nrm_next = __ldg(p.norms + in_row);
+                if (p.scales) { p.scales[ln * p.scale_lane_stride + rw] = nrm_next; nrm_next = 1.f; }
             }
             {   // the same row of the tile PF_AHEAD tiles further on: asked for in L2 now (a packed row is at most 64 bytes, so
                 // every 128-byte line of the tile holds the start of some row)
@@ -411,7 +413,7 @@ __global__ void __launch_bounds__(NT, 1) dequantize_tc_kernel(Params p) {
 }  // namespace dqtc
 
 // Dequantize on the tensor cores when the shape allows; *handled = false leaves the call to the row kernel.
-int tq_dequantize_tc(const tq_dequantize_args* q, cudaStream_t s, bool* handled) {
+int tq_dequantize_tc(const tq_dequantize_args* q, cudaStream_t s, bool* handled, float* scales, int64_t scale_lane_stride) {
     *handled = false;
     const int d = q->d;
     if (d != 64 && d != 96 && d != 128) return TQ_OK;
@@ -441,6 +443,7 @@ int tq_dequantize_tc(const tq_dequantize_args* q, cudaStream_t s, bool* handled)
     p.cent_hi = q->cent_hi; p.cent_lo = q->cent_lo; p.rot = q->rot;
     p.out = q->out; p.out_dtype = q->out_dtype; p.out_lane_stride = q->out_lane_stride; p.out_row_stride = q->out_row_stride;
     p.n_tiles = int(tiles);
+    p.scales = scales; p.scale_lane_stride = scale_lane_stride;
     if (!(p.status = decode_status_ptr())) return fail(TQ_ERR_LAUNCH, "tq_dequantize: cannot locate the status word");
     static bool set[16] = {false};
     static int sms[16] = {0};

@@ -29,6 +29,7 @@ struct RowArgs {
     const float* cent_hi; const float* cent_lo;
     const float* qjl_proj; const uint32_t* qjl_bits_in; const float* qjl_gamma_in;
     void* out; int out_dtype; int64_t out_lane_stride, out_row_stride;
+    float* scales; int64_t scale_lane_stride;      // dequantize: rows leave without their norms, which are copied here (or null)
 };
 
 __global__ void __launch_bounds__(NT) rowops_kernel(RowArgs a) {
@@ -84,6 +85,7 @@ __global__ void __launch_bounds__(NT) rowops_kernel(RowArgs a) {
             if (row < total_rows) {
                 const int64_t o = row / a.n_rows, r = row - o * a.n_rows;
                 nv = a.norms_in[o * a.in_lane_stride + r];
+                if (a.scales) { a.scales[o * a.scale_lane_stride + r] = nv; nv = 1.f; }
             }
             rown[tid] = nv;
         }
@@ -338,8 +340,25 @@ extern "C" int tq_quantize_pack(const tq_quantize_args* q, void* stream) {
 }
 
 namespace tq {
-int tq_dequantize_tc(const tq_dequantize_args* q, cudaStream_t s, bool* handled);      // dequantize_tc.cu
+int tq_dequantize_tc(const tq_dequantize_args* q, cudaStream_t s, bool* handled, float* scales, int64_t scale_lane_stride);      // dequantize_tc.cu
 int g_tune_dequantize_tc = 1;      // 0: always the row kernel (testing)
+
+static int dequantize_rows(const tq_dequantize_args* q, float* scales, int64_t scale_lane_stride, cudaStream_t s) {
+    if (g_tune_dequantize_tc) {
+        bool handled = false;
+        const int rc = tq_dequantize_tc(q, s, &handled, scales, scale_lane_stride);
+        if (handled) return rc;
+    }
+    RowArgs a{};
+    a.mode = MODE_DEQUANT; a.d = q->d; a.inverse = 1; a.n_lanes = q->n_lanes; a.n_rows = q->n_rows;
+    a.rot = q->rot; a.in_hi = q->packed_hi; a.in_lo = q->packed_lo; a.norms_in = q->norms; a.in_lane_stride = q->in_lane_stride;
+    a.bits_hi = q->bits_hi; a.bits_lo = q->bits_lo; a.cent_hi = q->cent_hi; a.cent_lo = q->cent_lo;
+    a.qjl_proj = q->qjl_proj; a.qjl_bits_in = q->qjl_bits; a.qjl_gamma_in = q->qjl_gamma;
+    a.out = q->out; a.out_dtype = q->out_dtype; a.out_lane_stride = q->out_lane_stride; a.out_row_stride = q->out_row_stride;
+    a.scales = scales; a.scale_lane_stride = scale_lane_stride;
+    return launch_rowops(a, s, "tq_dequantize");
+}
+int dequantize_unit(const tq_dequantize_args* q, float* scales, int64_t scale_lane_stride, cudaStream_t s) { return dequantize_rows(q, scales, scale_lane_stride, s); }
 }  // namespace tq
 
 extern "C" int tq_dequantize(const tq_dequantize_args* q, void* stream) {
@@ -351,16 +370,5 @@ extern "C" int tq_dequantize(const tq_dequantize_args* q, void* stream) {
     if (!q->packed_hi || !q->norms || !q->cent_hi || !q->rot || !q->out) return fail(TQ_ERR_INVALID, "tq_dequantize: null pointer");
     if (q->bits_lo && (!q->packed_lo || !q->cent_lo)) return fail(TQ_ERR_INVALID, "tq_dequantize: fractional mode needs packed_lo and cent_lo");
     if (q->qjl_bits && (!q->qjl_proj || !q->qjl_gamma)) return fail(TQ_ERR_INVALID, "tq_dequantize: QJL needs proj and gamma");
-    if (g_tune_dequantize_tc) {
-        bool handled = false;
-        const int rc = tq_dequantize_tc(q, static_cast<cudaStream_t>(stream), &handled);
-        if (handled) return rc;
-    }
-    RowArgs a{};
-    a.mode = MODE_DEQUANT; a.d = q->d; a.inverse = 1; a.n_lanes = q->n_lanes; a.n_rows = q->n_rows;
-    a.rot = q->rot; a.in_hi = q->packed_hi; a.in_lo = q->packed_lo; a.norms_in = q->norms; a.in_lane_stride = q->in_lane_stride;
-    a.bits_hi = q->bits_hi; a.bits_lo = q->bits_lo; a.cent_hi = q->cent_hi; a.cent_lo = q->cent_lo;
-    a.qjl_proj = q->qjl_proj; a.qjl_bits_in = q->qjl_bits; a.qjl_gamma_in = q->qjl_gamma;
-    a.out = q->out; a.out_dtype = q->out_dtype; a.out_lane_stride = q->out_lane_stride; a.out_row_stride = q->out_row_stride;
-    return launch_rowops(a, static_cast<cudaStream_t>(stream), "tq_dequantize");
+    return tq::dequantize_rows(q, nullptr, 0, static_cast<cudaStream_t>(stream));
 }
