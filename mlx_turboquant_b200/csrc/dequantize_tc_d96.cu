@@ -1,0 +1,4 @@
+// The tensor-core dequantize kernels of head_dim 96.
+#include "dequantize_tc.cuh"
+
+TQ_DEQUANTIZE_KERNELS(96)

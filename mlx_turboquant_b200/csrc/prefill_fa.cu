@@ -556,8 +556,8 @@ __global__ void __launch_bounds__(256) fa_dense_rows_kernel(DecodeParams c, int 
 
 }  // namespace fa
 
-// rowops.cu: rows c @ R without their norms (fp16), the norms copied to `scales`
-int dequantize_unit(const tq_dequantize_args* q, float* scales, int64_t scale_lane_stride, cudaStream_t s);
+// rowops.cu: with scales, rows c @ R leave without their norms, which are copied there
+int dequantize_jobs(const tq_dequantize_args* q, int n, float* const* scales, int64_t scale_lane_stride, const int* parts, const float* tab_scale, cudaStream_t s);
 
 namespace fa {
 
@@ -651,20 +651,27 @@ template <int D> static int run(const DecodeParams& c, const void* q, int q_dtyp
             if (int rc = check_launch("tq_prefill_attn")) return rc;
         }
         if (c.c_len > 0) {
+            tq_dequantize_args d[2] = {};
+            float* scales[2] = {kn + c.sink_len, vn + c.sink_len};
+            int parts[2];
+            float tab[2];
             for (int side = 0; side < 2; ++side) {
-                tq_dequantize_args d{};
+                tq_dequantize_args& a = d[side];
                 const int hi = side ? c.vb_hi : c.kb_hi, lo = side ? c.vb_lo : c.kb_lo;
                 const int w_hi = packed_bytes(lo ? D / 2 : D, hi), w_lo = lo ? packed_bytes(D / 2, lo) : 0;
-                d.packed_hi = (side ? c.v_hi : c.k_hi) + int64_t(lane0) * c.c_ls * w_hi;
-                d.packed_lo = lo ? (side ? c.v_lo : c.k_lo) + int64_t(lane0) * c.c_ls * w_lo : nullptr;
-                d.norms = (side ? c.v_norms : c.k_norms) + int64_t(lane0) * c.c_ls;
-                d.n_lanes = n; d.n_rows = c.c_len; d.in_lane_stride = c.c_ls;
-                d.d = D; d.bits_hi = hi; d.bits_lo = lo;
-                d.cent_hi = side ? c.vc_hi : c.kc_hi; d.cent_lo = side ? c.vc_lo : c.kc_lo; d.rot = c.rot;
-                d.out = (side ? v : k) + c.sink_len * D; d.out_dtype = TQ_F16;
-                d.out_lane_stride = int64_t(l.ts) * D; d.out_row_stride = D;
-                if (int rc = dequantize_unit(&d, (side ? vn : kn) + c.sink_len, l.ts, s)) return rc;
+                a.packed_hi = (side ? c.v_hi : c.k_hi) + int64_t(lane0) * c.c_ls * w_hi;
+                a.packed_lo = lo ? (side ? c.v_lo : c.k_lo) + int64_t(lane0) * c.c_ls * w_lo : nullptr;
+                a.norms = (side ? c.v_norms : c.k_norms) + int64_t(lane0) * c.c_ls;
+                a.n_lanes = n; a.n_rows = c.c_len; a.in_lane_stride = c.c_ls;
+                a.d = D; a.bits_hi = hi; a.bits_lo = lo;
+                a.cent_hi = side ? c.vc_hi : c.kc_hi; a.cent_lo = side ? c.vc_lo : c.kc_lo; a.rot = c.rot;
+                a.out = (side ? v : k) + c.sink_len * D; a.out_dtype = TQ_F16;
+                a.out_lane_stride = int64_t(l.ts) * D; a.out_row_stride = D;
+                // fp16 centroids as they are for keys, under their best scale for values (one scale cannot serve two tables: both parts)
+                parts[side] = side && lo ? 2 : 1;
+                tab[side] = side && !lo ? c.v_scale_hi : 1.f;
             }
+            if (int rc = dequantize_jobs(d, 2, scales, l.ts, parts, tab, s)) return rc;
         }
         CUtensorMap maps[2];
         for (int side = 0; side < 2; ++side) {

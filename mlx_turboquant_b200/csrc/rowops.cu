@@ -340,15 +340,22 @@ extern "C" int tq_quantize_pack(const tq_quantize_args* q, void* stream) {
 }
 
 namespace tq {
-int tq_dequantize_tc(const tq_dequantize_args* q, cudaStream_t s, bool* handled, float* scales, int64_t scale_lane_stride);      // dequantize_tc.cu
+int tq_dequantize_tc(const tq_dequantize_args* q, int n_jobs, cudaStream_t s, bool* handled, float* const* scales, int64_t scale_lane_stride,
+                     const int* parts, const float* tab_scale);      // dequantize_tc.cu
 int g_tune_dequantize_tc = 1;      // 0: always the row kernel (testing)
 
-static int dequantize_rows(const tq_dequantize_args* q, float* scales, int64_t scale_lane_stride, cudaStream_t s) {
-    if (g_tune_dequantize_tc) {
-        bool handled = false;
-        const int rc = tq_dequantize_tc(q, s, &handled, scales, scale_lane_stride);
-        if (handled) return rc;
-    }
+static int check_dequantize(const tq_dequantize_args* q) {
+    if (!d_ok(q->d)) return fail(TQ_ERR_UNSUPPORTED, "tq_dequantize: d=%d (need a multiple of 16 in 16..256)", q->d);
+    if (!bits_ok(q->bits_hi) || (q->bits_lo && !bits_ok(q->bits_lo))) return fail(TQ_ERR_INVALID, "Unsupported bit-width: %d/%d. Use 1, 2, 3, or 4.", q->bits_hi, q->bits_lo);
+    if (!dtype_ok(q->out_dtype) || q->n_lanes < 0 || q->n_rows < 0) return fail(TQ_ERR_INVALID, "tq_dequantize: bad dtype or sizes");
+    if (q->n_lanes == 0 || q->n_rows == 0) return TQ_OK;
+    if (!q->packed_hi || !q->norms || !q->cent_hi || !q->rot || !q->out) return fail(TQ_ERR_INVALID, "tq_dequantize: null pointer");
+    if (q->bits_lo && (!q->packed_lo || !q->cent_lo)) return fail(TQ_ERR_INVALID, "tq_dequantize: fractional mode needs packed_lo and cent_lo");
+    if (q->qjl_bits && (!q->qjl_proj || !q->qjl_gamma)) return fail(TQ_ERR_INVALID, "tq_dequantize: QJL needs proj and gamma");
+    return TQ_OK;
+}
+
+static int dequantize_row_kernel(const tq_dequantize_args* q, float* scales, int64_t scale_lane_stride, cudaStream_t s) {
     RowArgs a{};
     a.mode = MODE_DEQUANT; a.d = q->d; a.inverse = 1; a.n_lanes = q->n_lanes; a.n_rows = q->n_rows;
     a.rot = q->rot; a.in_hi = q->packed_hi; a.in_lo = q->packed_lo; a.norms_in = q->norms; a.in_lane_stride = q->in_lane_stride;
@@ -358,17 +365,23 @@ static int dequantize_rows(const tq_dequantize_args* q, float* scales, int64_t s
     a.scales = scales; a.scale_lane_stride = scale_lane_stride;
     return launch_rowops(a, s, "tq_dequantize");
 }
-int dequantize_unit(const tq_dequantize_args* q, float* scales, int64_t scale_lane_stride, cudaStream_t s) { return dequantize_rows(q, scales, scale_lane_stride, s); }
+
+// One or two jobs (the caller has validated them); scales, parts, tab_scale as in tq_dequantize_tc, all null for plain rows.
+int dequantize_jobs(const tq_dequantize_args* q, int n, float* const* scales, int64_t scale_lane_stride, const int* parts, const float* tab_scale, cudaStream_t s) {
+    if (g_tune_dequantize_tc) {
+        bool handled = false;
+        const int rc = tq_dequantize_tc(q, n, s, &handled, scales, scale_lane_stride, parts, tab_scale);
+        if (handled) return rc;
+    }
+    for (int i = 0; i < n; ++i)
+        if (int rc = dequantize_row_kernel(q + i, scales ? scales[i] : nullptr, scale_lane_stride, s)) return rc;
+    return TQ_OK;
+}
 }  // namespace tq
 
 extern "C" int tq_dequantize(const tq_dequantize_args* q, void* stream) {
     if (!q) return fail(TQ_ERR_INVALID, "tq_dequantize: null args");
-    if (!d_ok(q->d)) return fail(TQ_ERR_UNSUPPORTED, "tq_dequantize: d=%d (need a multiple of 16 in 16..256)", q->d);
-    if (!bits_ok(q->bits_hi) || (q->bits_lo && !bits_ok(q->bits_lo))) return fail(TQ_ERR_INVALID, "Unsupported bit-width: %d/%d. Use 1, 2, 3, or 4.", q->bits_hi, q->bits_lo);
-    if (!dtype_ok(q->out_dtype) || q->n_lanes < 0 || q->n_rows < 0) return fail(TQ_ERR_INVALID, "tq_dequantize: bad dtype or sizes");
+    if (int rc = check_dequantize(q)) return rc;
     if (q->n_lanes == 0 || q->n_rows == 0) return TQ_OK;
-    if (!q->packed_hi || !q->norms || !q->cent_hi || !q->rot || !q->out) return fail(TQ_ERR_INVALID, "tq_dequantize: null pointer");
-    if (q->bits_lo && (!q->packed_lo || !q->cent_lo)) return fail(TQ_ERR_INVALID, "tq_dequantize: fractional mode needs packed_lo and cent_lo");
-    if (q->qjl_bits && (!q->qjl_proj || !q->qjl_gamma)) return fail(TQ_ERR_INVALID, "tq_dequantize: QJL needs proj and gamma");
-    return tq::dequantize_rows(q, nullptr, 0, static_cast<cudaStream_t>(stream));
+    return dequantize_jobs(q, 1, nullptr, 0, nullptr, nullptr, static_cast<cudaStream_t>(stream));
 }
