@@ -765,7 +765,7 @@ int decode_prepare(const tq_decode_args* a, void* workspace, size_t workspace_by
     // everything else the lookup kernel's tables cover (two to four bits, their fractional splits).  The general kernel is one launch instead of three: with whole-byte tables
     // (4-bit keys, 2-bit values) it is the faster one for few tiles (head_dim 64, 16 lanes x 218 tiles: 17 against 29 us;
     // head_dim 128 with sketches, 72 lanes x 230 tiles: 63 against 35 us)
-    bool lut = ((!direct && !stream && g_tune_lut) || g_tune_lut == 2) && !g_tune_force_general && a->c_lane_stride % 16 == 0 &&
+    bool lut = ((!direct && !stream && g_tune_lut) || g_tune_lut == 2) && !g_tune_force_general && a->c_lane_stride % 16 == 0 && aligned(a->q, 8) &&
                aligned(a->k_hi, 16) && aligned(a->v_hi, 16) && aligned(a->k_norms, 16) && aligned(a->v_norms, 16) &&
                (!a->k_bits_lo || aligned(a->k_lo, 16)) && (!a->v_bits_lo || aligned(a->v_lo, 16)) &&
                (!qjl || (aligned(a->k_qjl_bits, 16) && aligned(a->v_qjl_bits, 16) && aligned(a->k_qjl_gamma, 16) && aligned(a->v_qjl_gamma, 16) && aligned(a->qjl_proj, 16))) &&

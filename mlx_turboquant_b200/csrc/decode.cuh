@@ -56,7 +56,7 @@ struct DecodeParams {
     int st_lut, st_fold;               // decode_lut.cu runs (decode_stream.cu otherwise); its CTAs fold their warps' partials
     int st_npp, st_nd, st_dt;          // packed-partial slots per lane; dense items per lane and tiles per dense item
     int64_t st_range;                  // packed tiles per warp
-    __half* st_q16;                    // workspace: per query head [rotated | raw | sketch] scaled fp16 query
+    __half* st_q16;                    // workspace: per query head the rotated (stream: | raw) (| sketch) scaled fp16 query
     float* st_part;                    // workspace: partials (lane, slot, head, D + 36)
 };
 

@@ -63,13 +63,18 @@ template <int D, bool QJL> struct Plan {
     static constexpr uint32_t SPILL = AREA0 + NW * AREA;                             // partial of the lane a warp leaves (one warp per CTA can)
     static constexpr uint32_t BARS = SPILL + (PART + 127u) / 128u * 128u;
     static constexpr uint32_t OWNER = BARS + 8u * NW * NS;                           // lane of each warp's partial, then of the spilled one
-    static constexpr uint32_t SMEM_END = OWNER + 4u * (NW + 1) + 60u;
+    static constexpr uint32_t META = (OWNER + 4u * (NW + 1) + 15u) / 16u * 16u;      // per lane of a folding CTA: its heads, first query head, partial slot
+    static constexpr uint32_t QROT = META + 32u;                                     // rotated queries (and sketches) of the CTA's two lanes
+    static constexpr int QR = D + (QJL ? QM : 0);                                    // halves per head there
+    static constexpr uint32_t QLANE = HPG * QR * 2u;                                 // bytes per lane, eight heads
+    static constexpr uint32_t QCAP = 227u * 1024u - QROT < 2u * QLANE ? 227u * 1024u - QROT : 2u * QLANE;
+    static constexpr uint32_t SMEM_END = QROT + QCAP;
     static_assert(SMEM_END <= 227u * 1024u, "shared-memory plan");
     static_assert(STAGE % 16 == 0 && AREA % 128 == 0, "copies need 16-byte alignment");
 };
 
-// Query heads in the workspace, halves: rotated (fp16) | raw, fp16 or the bf16 high part | bf16 low part | sketch
-__host__ __device__ constexpr int q_stride(int d) { return 3 * d + QM; }
+// Query heads in the workspace, halves: rotated | sketch (launches whose CTAs do not rotate their own)
+__host__ __device__ constexpr int q_stride(int d) { return d + QM; }
 __host__ __device__ constexpr int part_stride(int d) { return d + QM + 4; }    // floats per head of a partial: values | sketch rows | max, sum, pad
 
 // ---- PTX wrappers ---------------------------------------------------------------------------------------
@@ -277,6 +282,20 @@ __device__ __forceinline__ void value_part(float (*o)[4], uint32_t addr, uint32_
     }
 }
 
+// Query elements c, c + 1 of a head times scale * log2(e)
+__device__ __forceinline__ float2 q_pair(const DecodeParams& p, int64_t head, int c) {
+    const int64_t e = head * p.D + c;
+    const float f = p.scale * LOG2E;
+    float2 x;
+    if (p.q_dtype == TQ_F32) x = *reinterpret_cast<const float2*>(static_cast<const float*>(p.q) + e);
+    else {
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(static_cast<const uint16_t*>(p.q) + e);
+        if (p.q_dtype == TQ_F16) x = __half22float2(*reinterpret_cast<const __half2*>(&w));
+        else x = make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+    }
+    return make_float2(x.x * f, x.y * f);
+}
+
 // Softmax step on scores that already carry the key norms (and the sketch term); tokens past the end come in with score
 // -inf and norm 0.  pr: the four weights times the value scale.
 template <int D, int NZ>
@@ -298,47 +317,53 @@ __device__ __forceinline__ uint32_t pack_bf2(float lo, float hi) {
 // caches: a tile's rows come in with asynchronous copies and feed the MMAs in their own type.  bf16 rows take the
 // query and the weights as high + low bf16 parts (16 bits between them), so nothing is converted and any magnitude works.
 template <int D, bool BF16>
-__device__ __forceinline__ void dense_run(const DecodeParams& p, int64_t kvl, int tile_lo, int tile_hi, uint32_t stage, const __half* qraw, bool live_q,
+__device__ __forceinline__ void dense_run(const DecodeParams& p, int64_t kvl, int tile_lo, int tile_hi, uint32_t stage, int64_t qhead, bool live_q,
                                           WarpAcc<D, 0>& st, int lane) {
     constexpr int LD = stage_ld<D>(), CPR = D / 8;                       // halves per staged row, 16-byte chunks per row
     const int g = lane >> 2, t = lane & 3;
-    const int64_t n_tok = p.sink_len + p.res_len + (p.k_new ? 1 : 0);
+    const int n_tok = int(p.sink_len + p.res_len) + (p.k_new ? 1 : 0);
     uint32_t bh[D / 16][2], bl[BF16 ? D / 16 : 1][2];
 #pragma unroll
     for (int ks = 0; ks < D / 16; ++ks)
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             const int c = ks * 16 + 2 * t + 8 * u;
-            bh[ks][u] = live_q ? __ldcg(reinterpret_cast<const uint32_t*>(qraw + c)) : 0u;
-            if (BF16) bl[ks][u] = live_q ? __ldcg(reinterpret_cast<const uint32_t*>(qraw + D + c)) : 0u;
+            const float2 x = live_q ? q_pair(p, qhead, c) : make_float2(0.f, 0.f);
+            if (BF16) {
+                bh[ks][u] = pack_bf2(x.x, x.y);
+                bl[ks][u] = pack_bf2(x.x - __uint_as_float(bh[ks][u] << 16), x.y - __uint_as_float(bh[ks][u] & 0xffff0000u));
+            } else {
+                bh[ks][u] = pack_h2(x.x, x.y);
+            }
         }
     const uint32_t vstage = stage + TILE * LD * 2;
-    for (int tile = tile_lo; tile < tile_hi; ++tile) {
-        const int64_t tok0 = int64_t(tile) * TILE;
-        if (int64_t(tile) * TILE >= n_tok) break;
+    // rows of one side of a tile; the warp that owns the new token's tile also stores the row at the end of the recent-token
+    // buffer (the caller's slice assignment, cache.py:632-672); head groups write the same bytes
+    auto load = [&](int tile, uint32_t dst, const void* sink, const void* res, const void* neu, void* res_w) {
+        const int tok0 = tile * TILE, s_len = int(p.sink_len), r_len = int(p.res_len);
+        if (tile < tile_hi && tok0 < n_tok) {
 #pragma unroll 4
-        for (int i = lane; i < TILE * CPR; i += 32) {
-            const int r = i / CPR, c = i - r * CPR;
-            const int64_t tok = tok0 + r, rr = tok - p.sink_len;
-            const bool in_sink = tok < p.sink_len, fresh = rr >= p.res_len;
-            const int64_t e = in_sink ? (kvl * p.sink_ls + tok) * D : fresh ? kvl * D : (kvl * p.res_ls + rr) * D;
-            const uint16_t* kb = static_cast<const uint16_t*>(in_sink ? p.sink_k : fresh ? p.k_new : p.res_k);
-            const uint16_t* vb = static_cast<const uint16_t*>(in_sink ? p.sink_v : fresh ? p.v_new : p.res_v);
-            const int n = tok < n_tok ? 16 : 0;                          // rows past the end are zero-filled
-            const uint16_t* ks = n ? kb + e + c * 8 : reinterpret_cast<const uint16_t*>(p.rot);
-            const uint16_t* vs = n ? vb + e + c * 8 : reinterpret_cast<const uint16_t*>(p.rot);
-            cp_async16(stage + (r * LD + c * 8) * 2, ks, n);
-            cp_async16(vstage + (r * LD + c * 8) * 2, vs, n);
-            // the warp that owns the new token's tile also stores the row at the end of the recent-token buffer (the caller's
-            // slice assignment, cache.py:632-672); head groups write the same bytes
-            if (n && fresh && !in_sink) {
-                const int64_t dst = (kvl * p.res_ls + p.res_len) * D + c * 8;
-                *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.res_k_w) + dst) = __ldg(reinterpret_cast<const uint4*>(ks));
-                *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.res_v_w) + dst) = __ldg(reinterpret_cast<const uint4*>(vs));
+            for (int i = lane; i < TILE * CPR; i += 32) {
+                const int r = i / CPR, c = i - r * CPR, tok = tok0 + r, rr = tok - s_len;
+                const bool in_sink = tok < s_len, fresh = rr >= r_len;
+                const int64_t e = in_sink ? (kvl * p.sink_ls + tok) * D : fresh ? kvl * D : (kvl * p.res_ls + rr) * D;
+                const uint16_t* base = static_cast<const uint16_t*>(in_sink ? sink : fresh ? neu : res);
+                const int n = tok < n_tok ? 16 : 0;                          // rows past the end are zero-filled
+                const uint16_t* src = n ? base + e + c * 8 : reinterpret_cast<const uint16_t*>(p.rot);
+                cp_async16(dst + (r * LD + c * 8) * 2, src, n);
+                if (n && fresh && !in_sink)
+                    *reinterpret_cast<uint4*>(static_cast<uint16_t*>(res_w) + (kvl * p.res_ls + r_len) * D + c * 8) = __ldg(reinterpret_cast<const uint4*>(src));
             }
         }
         cp_async_commit();
-        cp_async_wait<0>();
+    };
+    // the next tile's keys are on their way from when this one's have been used, its values likewise
+    load(tile_lo, stage, p.sink_k, p.res_k, p.k_new, p.res_k_w);
+    load(tile_lo, vstage, p.sink_v, p.res_v, p.v_new, p.res_v_w);
+    for (int tile = tile_lo; tile < tile_hi; ++tile) {
+        const int tok0 = tile * TILE;
+        if (tok0 >= n_tok) break;
+        cp_async_wait<1>();
         __syncwarp();
         float s[4] = {0.f, 0.f, 0.f, 0.f};
         const uint32_t ka = stage + ((lane & 15) * LD + (lane >> 4) * 8) * 2;
@@ -358,6 +383,8 @@ __device__ __forceinline__ void dense_run(const DecodeParams& p, int64_t kvl, in
         const bool ok0 = tok0 + g < n_tok, ok1 = tok0 + g + 8 < n_tok;
         s[0] = ok0 ? s[0] : -INFINITY; s[1] = ok0 ? s[1] : -INFINITY;
         s[2] = ok1 ? s[2] : -INFINITY; s[3] = ok1 ? s[3] : -INFINITY;
+        __syncwarp();
+        load(tile + 1, stage, p.sink_k, p.res_k, p.k_new, p.res_k_w);
         float pr[4];
         softmax_scores<D, 0>(s, 1.f, 1.f, 0.f, st, pr);                 // (value norms are 1)
         uint32_t bp[2], bpl[2] = {0u, 0u};
@@ -369,6 +396,8 @@ __device__ __forceinline__ void dense_run(const DecodeParams& p, int64_t kvl, in
         } else {
             bp[0] = movm_t(pack_h2(pr[0], pr[1])); bp[1] = movm_t(pack_h2(pr[2], pr[3]));
         }
+        cp_async_wait<1>();
+        __syncwarp();
         const uint32_t vaddr = vstage + (((lane & 7) + ((lane >> 4) & 1) * 8) * LD + ((lane >> 3) & 1) * 8) * 2;
 #pragma unroll
         for (int mt = 0; mt < D / 16; ++mt) {
@@ -378,14 +407,53 @@ __device__ __forceinline__ void dense_run(const DecodeParams& p, int64_t kvl, in
             else mma16816(st.o[mt], a[0], a[1], a[2], a[3], bp[0], bp[1]);
         }
         __syncwarp();
+        load(tile + 1, vstage, p.sink_v, p.res_v, p.v_new, p.res_v_w);
     }
+    cp_async_wait<0>();
 }
 
-// ---- launch 1: the queries ------------------------------------------------------------------------------
+// ---- the queries ----------------------------------------------------------------------------------------
 // q_rot[h][j] = sum_k q[h][k] R[j][k] (rotation.py:81-110), u[h][p] = sum_k q[h][k] S[p][k] (qjl.py:70-94), both times
-// scale * log2(e), fp16; the raw query likewise (bf16 caches: high and low bf16 parts).  A warp owns 16 rows of R (or S) as
-// the A operand and eight query heads as the B operand; both are split into fp16 high and 2^-11 low parts (the product of
-// the low parts is below float32 resolution).  Grid (eight heads, groups of four warps' rows).
+// scale * log2(e), fp16.  A warp owns a slab of 16 rows of R (or S) as the A operand and eight query heads as the B operand; both
+// are split into fp16 high and 2^-11 low parts (the product of the low parts is below float32 resolution).
+__device__ __forceinline__ void split_h2(float2 x, uint32_t& h, uint32_t& l) {
+    const __half2 a = __floats2half2_rn(x.x, x.y);
+    const float2 af = __half22float2(a);
+    h = *reinterpret_cast<const uint32_t*>(&a);
+    l = pack_h2((x.x - af.x) * 2048.f, (x.y - af.y) * 2048.f);
+}
+template <int D> __device__ __forceinline__ void load_rows(const DecodeParams& p, int slab, int g, int t, float2 (&rr)[D / 16][4]) {
+    const float* row = slab >= D / 16 ? p.qjl_proj + int64_t(slab - D / 16) * 16 * D : p.rot + int64_t(slab) * 16 * D;
+#pragma unroll
+    for (int ks = 0; ks < D / 16; ++ks)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) rr[ks][r] = __ldg(reinterpret_cast<const float2*>(row + (g + (r & 1) * 8) * D + ks * 16 + 2 * t + (r >> 1) * 8));
+}
+// y: rows g, g + 8 of the slab x heads q0 + 2t, + 1
+template <int D>
+__device__ __forceinline__ void rotate_rows(const DecodeParams& p, int64_t q0, int64_t heads, int g, int t, const float2 (&rr)[D / 16][4], float (&y)[4]) {
+    float2 x[D / 16][2];                                  // head q0 + g: coordinates 16 ks + 2 t, + 1 and the same + 8
+#pragma unroll
+    for (int ks = 0; ks < D / 16; ++ks)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) x[ks][u] = g < heads ? q_pair(p, q0 + g, ks * 16 + 2 * t + 8 * u) : make_float2(0.f, 0.f);
+    float ym[4] = {0.f, 0.f, 0.f, 0.f}, ya[4] = {0.f, 0.f, 0.f, 0.f}, yb[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int ks = 0; ks < D / 16; ++ks) {
+        uint32_t bh[2], bl[2], ah[4], al[4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) split_h2(x[ks][u], bh[u], bl[u]);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) split_h2(rr[ks][r], ah[r], al[r]);
+        mma16816(ym, ah[0], ah[1], ah[2], ah[3], bh[0], bh[1]);
+        mma16816(ya, al[0], al[1], al[2], al[3], bh[0], bh[1]);
+        mma16816(yb, ah[0], ah[1], ah[2], ah[3], bl[0], bl[1]);
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) y[r] = ym[r] + (ya[r] + yb[r]) * (1.f / 2048.f);
+}
+// The launch before the persistent grid when its CTAs do not rotate their own queries: many short lanes, or a fused gather.
+// Grid (eight heads, groups of four warps' slabs).
 template <int D>
 __global__ void __launch_bounds__(128) lut_query_kernel(DecodeParams p) {
     constexpr int QS = q_stride(D), KS = D / 16;
@@ -393,74 +461,29 @@ __global__ void __launch_bounds__(128) lut_query_kernel(DecodeParams p) {
     const int slab = blockIdx.y * 4 + (threadIdx.x >> 5), n_slabs = KS + (p.qjl_proj ? 2 : 0);
     const int64_t n_q = int64_t(p.B) * p.Hq, q0 = int64_t(blockIdx.x) * 8;
     pdl_trigger();
-    auto split = [](float2 x, uint32_t& h, uint32_t& l) {
-        const __half2 a = __floats2half2_rn(x.x, x.y);
-        const float2 af = __half22float2(a);
-        h = *reinterpret_cast<const uint32_t*>(&a);
-        l = pack_h2((x.x - af.x) * 2048.f, (x.y - af.y) * 2048.f);
-    };
-    // this warp's rows of R (or S) as operand fragments: constants, so they are in registers before the wait
-    const bool sk = slab >= KS, live = slab < n_slabs;
-    const float* row = sk && live ? p.qjl_proj + int64_t(slab - KS) * 16 * D : p.rot + int64_t(min(slab, KS - 1)) * 16 * D;
-    uint32_t ah[KS][4], al[KS][4];
-#pragma unroll
-    for (int ks = 0; ks < KS; ++ks)
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-            split(__ldg(reinterpret_cast<const float2*>(row + (g + (r & 1) * 8) * D + ks * 16 + 2 * t + (r >> 1) * 8)), ah[ks][r], al[ks][r]);
+    float2 rr[KS][4];
+    load_rows<D>(p, min(slab, n_slabs - 1), g, t, rr);       // constants, so they are in registers before the wait
     pdl_wait();
     await_gather(p);   // (head-sharded decoding) the peers' heads of an earlier call have arrived
     if (p.n_peers > 0 && blockIdx.y == 0) {           // this call's epoch of every group, for the merge launch
         const int n_groups = p.B * p.Hkv * p.HG;
         for (int i = blockIdx.x * 128 + threadIdx.x; i < n_groups; i += gridDim.x * 128) ++p.epochs[i];
     }
-    const float f = p.scale * LOG2E;
-    float2 x[KS][2];                                  // head q0 + g: coordinates 16 ks + 2 t, + 1 and the same + 8
-#pragma unroll
-    for (int ks = 0; ks < KS; ++ks)
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            x[ks][u] = make_float2(0.f, 0.f);
-            if (q0 + g < n_q) {
-                const int64_t e = (q0 + g) * D + ks * 16 + 2 * t + 8 * u;
-                x[ks][u] = make_float2(load_as_f32(p.q, p.q_dtype, e) * f, load_as_f32(p.q, p.q_dtype, e + 1) * f);
-            }
-        }
-    float ym[4] = {0.f, 0.f, 0.f, 0.f}, yc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int ks = 0; ks < KS; ++ks) {
-        uint32_t bh[2], bl[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            split(x[ks][u], bh[u], bl[u]);
-            if (slab == 0 && q0 + g < n_q) {          // the raw query
-                const int64_t o = (q0 + g) * QS + D + ks * 16 + 2 * t + 8 * u;
-                if (p.dense_dtype == TQ_BF16) {
-                    const uint32_t h = pack_bf2(x[ks][u].x, x[ks][u].y);
-                    *reinterpret_cast<uint32_t*>(p.st_q16 + o) = h;
-                    *reinterpret_cast<uint32_t*>(p.st_q16 + o + D) = pack_bf2(x[ks][u].x - __uint_as_float(h << 16), x[ks][u].y - __uint_as_float(h & 0xffff0000u));
-                } else {
-                    *reinterpret_cast<uint32_t*>(p.st_q16 + o) = bh[u];
-                }
-            }
-        }
-        mma16816(ym, ah[ks][0], ah[ks][1], ah[ks][2], ah[ks][3], bh[0], bh[1]);
-        mma16816(yc, al[ks][0], al[ks][1], al[ks][2], al[ks][3], bh[0], bh[1]);
-        mma16816(yc, ah[ks][0], ah[ks][1], ah[ks][2], ah[ks][3], bl[0], bl[1]);
-    }
-    if (!live) return;
-    const int dst = sk ? 3 * D + (slab - KS) * 16 : slab * 16;
+    float y[4];
+    rotate_rows<D>(p, q0, n_q - q0, g, t, rr, y);
+    if (slab >= n_slabs) return;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {              // rows g, g + 8 of the slab x heads 2t, 2t + 1
         const int64_t h = q0 + 2 * t + (r & 1);
-        if (h < n_q) p.st_q16[h * QS + dst + g + (r >> 1) * 8] = __float2half_rn(ym[r] + yc[r] * (1.f / 2048.f));
+        if (h < n_q) p.st_q16[h * QS + slab * 16 + g + (r >> 1) * 8] = __float2half_rn(y[r]);
     }
 }
 
 // ---- launch 2: the persistent grid ----------------------------------------------------------------------
 __device__ __forceinline__ int fmt_of(int hi, int lo) { return lo ? hi * 10 + lo : hi; }
 
-template <int D, bool QJL>
+// INQ: the CTA rotates the queries of its lanes itself.
+template <int D, bool QJL, bool INQ>
 __global__ void __launch_bounds__(Plan<D, QJL>::NT, 1) decode_lut_kernel(DecodeParams p) {
     using P = Plan<D, QJL>;
     constexpr int NZ = QJL ? QM / 16 : 0, NS = P::NS, NW = P::NW, NT = P::NT, NC = P::NC;
@@ -521,44 +544,78 @@ __global__ void __launch_bounds__(Plan<D, QJL>::NT, 1) decode_lut_kernel(DecodeP
             }
         }
     }
+    const int L = p.B * p.Hkv * p.HG;                          // cache lanes x head groups
+    const int n_tiles = int((p.c_len + TILE - 1) / TILE);      // packed tiles per lane
+    const bool fold = p.st_fold != 0;                          // the warps of the CTA fold their partials of a lane into one
+    const uint32_t total = uint32_t(L) * n_tiles, range = uint32_t(p.st_range), unit = fold ? range * NW : range;       // (below 2^31) unit: tiles behind one partial slot
+    const int n_slots = p.st_npp + p.st_nd;                    // partial slots per lane
+    const int wg = blockIdx.x * NW + warp, n_warps = gridDim.x * NW;
+    const int c_len = int(p.c_len);
+    auto heads_of = [&](int a) { return min(HPG, p.G - (a % p.HG) * HPG); };
+    auto qhead_of = [&](int a) -> int {                        // first query head of lane a
+        const int kvl = a / p.HG, hg = a - kvl * p.HG, b = kvl / p.Hkv, hkv = kvl - b * p.Hkv;
+        return b * p.Hq + hkv * p.G + hg * HPG;
+    };
+    // Everything that follows from the parameters alone is worked out before the wait: integer divisions in code that is cold
+    // in the instruction cache cost 5 us of a small call after it.
+    int a_first = 0, n_la = 0;                                 // (if it folds) the lanes of the CTA's tiles: two at most
+    int4* meta = reinterpret_cast<int4*>(gp(P::META));
+    if (fold) {
+        const uint32_t c0 = min(blockIdx.x * unit, total), c1 = min(c0 + unit, total);
+        a_first = c0 < c1 ? int(c0 / uint32_t(n_tiles)) : 0;
+        n_la = c0 < c1 ? int((c1 - 1) / uint32_t(n_tiles)) - a_first + 1 : 0;
+        if (tid < n_la) meta[tid] = make_int4(heads_of(a_first + tid), qhead_of(a_first + tid), int(blockIdx.x) - int(uint32_t(a_first + tid) * n_tiles / unit), 0);
+    }
+    // uncompressed tokens: items i in [i0, i1) of the L * nd (lane, run of dt tiles) pairs, dealt from the far end: with few
+    // items the warps that have none are the ones whose packed runs are full
+    const uint32_t n_items = uint32_t(L) * p.st_nd, wr = uint32_t(n_warps - 1 - wg);
+    const uint32_t i0 = (wr * n_items + n_warps - 1) / n_warps, i1 = ((wr + 1) * n_items + n_warps - 1) / n_warps;
+    int da = p.st_nd > 0 ? int(i0 / uint32_t(p.st_nd)) : 0, dpart = int(i0) - da * p.st_nd, dheads = heads_of(da), dq = qhead_of(da);
+    // ---------------- queries of the CTA's lanes, by units: sixteen rows of R (or S) x the heads of a lane ----------------
+    constexpr int SLABS = D / 16 + (QJL ? QM / 16 : 0);
+    const int n_units = INQ ? n_la * SLABS : 0;
+    float2 rr[D / 16][4];
+    if (INQ && warp < n_units) load_rows<D>(p, warp % SLABS, g, t, rr);           // constants as well
     __syncthreads();
     pdl_wait();        // the prepared queries, the cache and the workspace are settled from here on
     bool failed = false;
 
-    const int L = p.B * p.Hkv * p.HG;                          // cache lanes x head groups
-    const int n_tiles = int((p.c_len + TILE - 1) / TILE);      // packed tiles per lane
-    const int n_slots = p.st_npp + p.st_nd;                    // partial slots per lane
-    const int wg = blockIdx.x * NW + warp, n_warps = gridDim.x * NW;
-    const int c_len = int(p.c_len);
-    const bool fold = p.st_fold != 0;                          // the warps of the CTA fold their partials of a lane into one
-    const int64_t unit = fold ? p.st_range * NW : p.st_range;  // tiles behind one partial slot
-    auto heads_of = [&](int a) { return min(HPG, p.G - (a % p.HG) * HPG); };
-    auto qhead_of = [&](int a) -> int64_t {                    // first query head of lane a
-        const int kvl = a / p.HG, hg = a - kvl * p.HG, b = kvl / p.Hkv, hkv = kvl - b * p.Hkv;
-        return int64_t(b) * p.Hq + int64_t(hkv) * p.G + hg * HPG;
-    };
+    __half* qrot = reinterpret_cast<__half*>(gp(P::QROT));
+    for (int un = warp; un < n_units; un += NW) {
+        const int la = un / SLABS, slab = un - la * SLABS;
+        const int4 lm = meta[la];
+        if (un != warp) load_rows<D>(p, slab, g, t, rr);
+        float y[4];
+        rotate_rows<D>(p, lm.y, lm.x, g, t, rr, y);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {              // rows g, g + 8 of the slab x heads 2t, 2t + 1
+            const int h = 2 * t + (r & 1);
+            if (h < p.slots) qrot[(la * p.slots + h) * P::QR + slab * 16 + g + (r >> 1) * 8] = __float2half_rn(y[r]);
+        }
+    }
+    if (INQ) __syncthreads();
 
-    // ---------------- uncompressed tokens: items i in [i0, i1) of the L * nd (lane, run of dt tiles) pairs ----------------
-    if (p.st_nd > 0) {
-        const int64_t n_items = int64_t(L) * p.st_nd;
-        // dealt from the far end: with few items the warps that have none are the ones whose packed runs are full
-        const int wr = n_warps - 1 - wg;
-        const int i0 = int((int64_t(wr) * n_items + n_warps - 1) / n_warps), i1 = int((int64_t(wr + 1) * n_items + n_warps - 1) / n_warps);
-        for (int i = i0; i < i1; ++i) {
-            const int a = i / p.st_nd, part = i - a * p.st_nd, heads_here = heads_of(a);
-            const __half* qraw = p.st_q16 + (qhead_of(a) + min(g, heads_here - 1)) * QS + D;
+    // ---------------- uncompressed tokens ----------------
+    {
+        for (uint32_t i = i0; i < i1; ++i) {
+            const int a = da, part = dpart, heads_here = dheads;
+            const int64_t qhead = dq + min(g, heads_here - 1);
+            if (++dpart == p.st_nd) { dpart = 0; ++da; dheads = heads_of(da); dq = qhead_of(da); }
             WarpAcc<D, 0> sd;
             sd.init();
             if (p.dense_dtype == TQ_F16) {
-                dense_run<D, false>(p, a / p.HG, part * p.st_dt, (part + 1) * p.st_dt, my_area, qraw, g < heads_here, sd, lane);
+                dense_run<D, false>(p, a / p.HG, part * p.st_dt, (part + 1) * p.st_dt, my_area, qhead, g < heads_here, sd, lane);
             } else if (p.dense_dtype == TQ_BF16) {
-                dense_run<D, true>(p, a / p.HG, part * p.st_dt, (part + 1) * p.st_dt, my_area, qraw, g < heads_here, sd, lane);
+                dense_run<D, true>(p, a / p.HG, part * p.st_dt, (part + 1) * p.st_dt, my_area, qhead, g < heads_here, sd, lane);
             } else {
                 uint32_t bq[D / 16][2];
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks) {
-                    bq[ks][0] = g < heads_here ? __ldcg(reinterpret_cast<const uint32_t*>(qraw + ks * 16 + 2 * t)) : 0u;
-                    bq[ks][1] = g < heads_here ? __ldcg(reinterpret_cast<const uint32_t*>(qraw + ks * 16 + 2 * t + 8)) : 0u;
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const float2 x = q_pair(p, qhead, ks * 16 + 2 * t + 8 * u);
+                        bq[ks][u] = g < heads_here ? pack_h2(x.x, x.y) : 0u;
+                    }
                 }
                 __half* Ks = reinterpret_cast<__half*>(gp(my_area));
                 dense_tiles<D, 1, 0>(p, a / p.HG, int64_t(part) * p.st_dt, int64_t(part + 1) * p.st_dt, Ks, Ks + TILE * stage_ld<D>(), bq, sd, 0, lane);
@@ -590,8 +647,7 @@ __global__ void __launch_bounds__(Plan<D, QJL>::NT, 1) decode_lut_kernel(DecodeP
     }
 
     // ---------------- packed tokens: flat tiles [T0, T1) of the L * n_tiles ----------------------------------
-    const int64_t total = int64_t(L) * n_tiles;
-    const int64_t T0 = min(int64_t(wg) * p.st_range, total), T1 = min(T0 + p.st_range, total);
+    const uint32_t T0 = min(uint32_t(wg) * range, total), T1 = min(T0 + range, total);
     const int n_my = int(T1 - T0);
     if (n_my > 0) {
         const int kwh = packed_bytes(p.kb_lo ? D / 2 : D, p.kb_hi), kwl = p.kb_lo ? packed_bytes(D / 2, p.kb_lo) : 0;
@@ -601,7 +657,7 @@ __global__ void __launch_bounds__(Plan<D, QJL>::NT, 1) decode_lut_kernel(DecodeP
         const int n_sc = int(P::SC / 16), n_chunks = n_sc + kwh + kwl + vwh + vwl;
         const unsigned char* cp_ptr[NC];
         uint32_t cp_step[NC];
-        int ia = int(T0 / n_tiles), iti = int(T0 - int64_t(ia) * n_tiles);    // lane and tile of the next copy
+        int ia = int(T0 / uint32_t(n_tiles)), iti = int(T0) - ia * n_tiles;    // lane and tile of the next copy
         {
             const int64_t row = int64_t(ia / p.HG) * p.c_ls + int64_t(iti) * TILE;
 #pragma unroll
@@ -659,14 +715,14 @@ __global__ void __launch_bounds__(Plan<D, QJL>::NT, 1) decode_lut_kernel(DecodeP
         const uint32_t v_off1 = word_at(8u * (t * vwl) + uint32_t(vwl * g), o_vl, vsh1);
 
         const int tail_ti = (c_len & (TILE - 1)) ? n_tiles - 1 : -1;          // the tile that reaches past the end of the cache
-        int a = int(T0 / n_tiles), ti = int(T0 - int64_t(a) * n_tiles);       // lane and tile being computed
-        int slot = int(T0 / unit) - int((int64_t(a) * n_tiles) / unit);       // partial slot = rank of this warp (CTA) among the lane's
+        int a = int(T0 / uint32_t(n_tiles)), ti = int(T0) - a * n_tiles;       // lane and tile being computed
+        int slot = int(T0 / unit) - int(uint32_t(a) * n_tiles / unit);       // partial slot = rank of this warp (CTA) among the lane's
         int heads_here = 0;
         uint32_t bq[D / 16][2];
         uint32_t bu[QM / 16][2];
         auto load_query = [&]() {
-            heads_here = heads_of(a);
-            const __half* qh = p.st_q16 + (qhead_of(a) + g) * QS;
+            heads_here = fold ? meta[a - a_first].x : heads_of(a);
+            const __half* qh = INQ ? qrot + ((a - a_first) * p.slots + g) * P::QR : p.st_q16 + (qhead_of(a) + g) * QS;
             // this lane's coordinates of k-step ks: four in a row
             const bool split = p.kb_lo != 0;
 #pragma unroll
@@ -674,7 +730,7 @@ __global__ void __launch_bounds__(Plan<D, QJL>::NT, 1) decode_lut_kernel(DecodeP
                 const int c = split ? (ks < D / 32 ? t * (D / 8) + 4 * ks : D / 2 + t * (D / 8) + 4 * (ks - D / 32)) : t * (D / 4) + 4 * ks;
                 // (written by the launch before this one while this grid may already have been resident: read at L2, never through a non-coherent path)
                 uint2 x = make_uint2(0u, 0u);
-                if (g < heads_here) x = __ldcg(reinterpret_cast<const uint2*>(qh + c));
+                if (g < heads_here) x = INQ ? *reinterpret_cast<const uint2*>(qh + c) : __ldcg(reinterpret_cast<const uint2*>(qh + c));
                 bq[ks][0] = x.x; bq[ks][1] = x.y;
             }
             if (QJL) {
@@ -687,8 +743,8 @@ __global__ void __launch_bounds__(Plan<D, QJL>::NT, 1) decode_lut_kernel(DecodeP
                         const int pi = 4 * t + 2 * ks + hh;
                         bu[ks][hh] = 0u;
                         if (g < heads_here) {
-                            const unsigned short lo16 = __ldcg(reinterpret_cast<const unsigned short*>(qh + 3 * D + pi));
-                            const unsigned short hi16 = __ldcg(reinterpret_cast<const unsigned short*>(qh + 3 * D + pi + 16));
+                            const unsigned short* z = reinterpret_cast<const unsigned short*>(qh + D + pi);
+                            const unsigned short lo16 = INQ ? z[0] : __ldcg(z), hi16 = INQ ? z[16] : __ldcg(z + 16);
                             bu[ks][hh] = uint32_t(lo16) | (uint32_t(hi16) << 16);
                         }
                     }
@@ -841,130 +897,207 @@ __global__ void __launch_bounds__(Plan<D, QJL>::NT, 1) decode_lut_kernel(DecodeP
 
     // ---------------- fold: one partial per (CTA, lane), from the warps' partials in shared memory ----------------
     __syncthreads();
-    const int64_t C0 = min(int64_t(blockIdx.x) * unit, total), C1 = min(C0 + unit, total);
-    if (C0 >= C1) return;
-    const int a_first = int(C0 / n_tiles), a_last = int((C1 - 1) / n_tiles);
-    for (int a = a_first; a <= a_last; ++a) {
-        const int heads_here = heads_of(a);
-        const int slot = int(blockIdx.x) - int((int64_t(a) * n_tiles) / unit);
-        float* dst = p.st_part + (int64_t(a) * n_slots + slot) * p.slots * PS;
-        constexpr int NE = D + (QJL ? QM : 0);
-        for (int e = tid; e < heads_here * NE; e += NT) {
-            const int h = e / NE, c = e - h * NE;
-            float m[NW + 1], M = -INFINITY;
+    // (the tables are free: every warp has left its loop)  Weights: a warp per (lane, head), lane w of it = partial w.
+    constexpr int NE = D + (QJL ? QM : 0), FW = 20;
+    float* fw = reinterpret_cast<float*>(gp(TAB_B));
+    auto partial_of = [&](int w, int h) -> const float* {
+        return reinterpret_cast<const float*>(gp(w < NW ? AREA0 + uint32_t(w) * P::AREA : P::SPILL)) + h * PS;
+    };
+    auto dst_of = [&](int la) -> float* {
+        return p.st_part + (int64_t(a_first + la) * n_slots + meta[la].z) * p.slots * PS;
+    };
+    for (int i = warp; i < n_la * p.slots; i += NW) {
+        const int la = i >= p.slots ? 1 : 0, h = i - la * p.slots;
+        const bool mine = lane <= NW && owner[lane <= NW ? lane : 0] == a_first + la && h < meta[la].x;
+        const float* src = partial_of(lane <= NW ? lane : 0, h);
+        const float m = mine ? src[D + QM] : -INFINITY, l = mine ? src[D + QM + 1] : 0.f;
+        float M = m;
 #pragma unroll
-            for (int w = 0; w <= NW; ++w) {
-                const float* src = reinterpret_cast<const float*>(gp(w < NW ? AREA0 + uint32_t(w) * P::AREA : P::SPILL)) + h * PS;
-                m[w] = owner[w] == a ? src[D + QM] : -INFINITY;
-                M = fmaxf(M, m[w]);
-            }
-            float acc = 0.f, sum = 0.f;
+        for (int off = 16; off; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
+        const float w = m == -INFINITY ? 0.f : ex2(m - M);
+        float sum = w * l;
 #pragma unroll
-            for (int w = 0; w <= NW; ++w) {
-                if (m[w] == -INFINITY) continue;
-                const float* src = reinterpret_cast<const float*>(gp(w < NW ? AREA0 + uint32_t(w) * P::AREA : P::SPILL)) + h * PS;
-                const float x = ex2(m[w] - M);
-                acc = fmaf(x, src[c], acc);
-                if (c == 0) sum = fmaf(x, src[D + QM + 1], sum);
-            }
-            dst[h * PS + c] = acc;
-            if (c == 0) { dst[h * PS + D + QM] = M; dst[h * PS + D + QM + 1] = sum; }
+        for (int off = 16; off; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+        if (lane <= NW) fw[i * FW + lane] = w;
+        if (lane == 0 && h < meta[la].x) *reinterpret_cast<float2*>(dst_of(la) + h * PS + D + QM) = make_float2(M, sum);
+    }
+    __syncthreads();
+    for (int e = tid; e < n_la * p.slots * (NE / 4); e += NT) {
+        const int i = e / (NE / 4), c = 4 * (e - i * (NE / 4)), la = i >= p.slots ? 1 : 0, h = i - la * p.slots;
+        if (h >= meta[la].x) continue;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w <= NW; ++w) {
+            const float x = fw[i * FW + w];
+            // (a partial of another lane has weight 0 and may hold anything: skipped, not multiplied)
+            const float4 v = x != 0.f ? *reinterpret_cast<const float4*>(partial_of(w, h) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            acc.x = fmaf(x, v.x, acc.x); acc.y = fmaf(x, v.y, acc.y); acc.z = fmaf(x, v.z, acc.z); acc.w = fmaf(x, v.w, acc.w);
         }
+        *reinterpret_cast<float4*>(dst_of(la) + h * PS + c) = acc;
     }
 }
 
 // ---- launch 3: merge --------------------------------------------------------------------------------------
-// A thread per (lane, query head, coordinate), some 512 threads to a block.  At d <= 128, R and S are staged in shared
-// memory before the wait, so the rotation back costs shared-memory reads; at d = 256 (R alone is 256 KB) it reads them
-// at L1 / L2.
-constexpr int sets_per_block(int d) { return 512 / d; }
-template <int D> __host__ __device__ constexpr bool stages_r() { return D <= 128; }
-template <int D> __host__ __device__ constexpr size_t merge_smem() {
-    return (size_t(stages_r<D>() ? (D + QM) * D : 0) + size_t(512 / D) * (2 * MAX_PARTS + D + QM)) * sizeof(float);
-}
+// Latency is all there is to it: one round trip for the partials' maxima and sums together with the first sixteen partials
+// of every thread, one step of weights, one of sums, one of rotation.  A block takes `rp` (lane, query head) rows at a time
+// (1, 2 or 4): its NG groups of D threads share a row's slots NG / rp ways.  The rotation back (y @ R, rotation.py:68-78; plus
+// (c/d) z @ S for the sketches, qjl.py:89-92) is float32: thread (k group, column) holds its quarter of the column of R in
+// registers from before the wait.  (R staged in shared memory by every block, a thread per coordinate over all slots: 12 to
+// 20 us per launch whatever the size; now 5 to 7.)  d = 256: two blocks share a row's columns.
+template <int D> __host__ __device__ constexpr int merge_cols() { return D > 128 ? 128 : D; }
+template <int D> __host__ __device__ constexpr int merge_threads() { return 4 * merge_cols<D>(); }
 template <int D, bool QJL>
-__global__ void __launch_bounds__(512) lut_merge_kernel(DecodeParams p, int nw) {
-    extern __shared__ __align__(16) unsigned char smem_m[];
-    constexpr int PS = part_stride(D), SPB = 512 / D, NTH = SPB * D;
-    float* rs = reinterpret_cast<float*>(smem_m);                 // [D][D] R, then [32][D] S
-    const int tid = threadIdx.x, set = tid / D, c = tid - set * D;
-    float* s_m = rs + (stages_r<D>() ? (D + QM) * D : 0) + set * (2 * MAX_PARTS + D + QM);
-    float* s_l = s_m + MAX_PARTS;
-    float* s_rot = s_l + MAX_PARTS;
-    float* s_z = s_rot + D;
+__global__ void __launch_bounds__(merge_threads<D>(), 1) lut_merge_kernel(DecodeParams p, int nw, int rp) {
+    constexpr int PS = part_stride(D), NT = merge_threads<D>(), NCOL = merge_cols<D>(), NG = NT / D, KR = D / 4, SR = QJL ? QM / 4 : 0, U = 16;
+    __shared__ float s_w[4][MAX_PARTS], s_il[4];
+    __shared__ __align__(16) float s_a[4][D + QM], s_p[2][NG][D], s_o[4][4][NCOL];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     pdl_trigger();
-    if (stages_r<D>()) {
-        const int rows = D + (QJL ? QM : 0);
-        for (int i = tid; i < rows * (D / 4); i += NTH) {      // constants: before the wait
-            const int r = i / (D / 4), k4 = i - r * (D / 4);
-            *reinterpret_cast<float4*>(rs + r * D + 4 * k4) = __ldg(reinterpret_cast<const float4*>(r < D ? p.rot + int64_t(r) * D : p.qjl_proj + int64_t(r - D) * D) + k4);
-        }
-    }
-    pdl_wait();
-    const int L = p.B * p.Hkv * p.HG;
-    const int64_t idx = int64_t(blockIdx.x) * SPB + set;
-    const int a = int(min(idx / p.slots, int64_t(L - 1))), h = int(idx % p.slots);
-    const int kvl = a / p.HG, hg = a - kvl * p.HG, b = kvl / p.Hkv, hkv = kvl - b * p.Hkv;
-    const int heads_here = min(HPG, p.G - hg * HPG);
-    const bool live = idx < int64_t(L) * p.slots && h < heads_here;
-    const int64_t qhead = int64_t(b) * p.Hq + int64_t(hkv) * p.G + hg * HPG + h;
+    const int n0 = blockIdx.y * NCOL, kg = tid / NCOL, oc = tid - kg * NCOL;       // rotation: k group, output column
+    float rr[KR], sr[SR ? SR : 1];
+#pragma unroll
+    for (int j = 0; j < KR; ++j) rr[j] = __ldg(p.rot + (kg * KR + j) * D + n0 + oc);
+#pragma unroll
+    for (int j = 0; j < SR; ++j) sr[j] = __ldg(p.qjl_proj + (kg * SR + j) * D + n0 + oc);
     const int n_tiles = int((p.c_len + TILE - 1) / TILE);
     const int n_slots = p.st_npp + p.st_nd;
-    const int64_t unit = p.st_fold ? p.st_range * nw : p.st_range;
-    // the warps (CTAs) whose runs touch this lane's tiles [a * n_tiles, (a + 1) * n_tiles)
-    const int n_pp = n_tiles > 0 ? int((int64_t(a + 1) * n_tiles - 1) / unit) - int((int64_t(a) * n_tiles) / unit) + 1 : 0;
-    const float inv_vs = 1.f / (c < D / 2 || p.vb_lo == 0 ? p.v_scale_hi : p.v_scale_lo);
-    const float* ph = p.st_part + (int64_t(a) * n_slots * p.slots + h) * PS;
-    const int64_t sstride = int64_t(p.slots) * PS;
-    for (int i = c; i < n_slots; i += D) {
-        const bool valid = live && (i < n_pp || i >= p.st_npp);
-        s_m[i] = valid ? __ldcg(ph + i * sstride + D + QM) : -INFINITY;
-        s_l[i] = valid ? __ldcg(ph + i * sstride + D + QM + 1) : 0.f;
-    }
-    __syncthreads();
-    float M = -INFINITY;
-    for (int i = 0; i < n_slots; ++i) M = fmaxf(M, s_m[i]);
-    float Lsum = 0.f, ar = 0.f, ad = 0.f, az = 0.f;
-#pragma unroll 8
-    for (int i = 0; i < n_slots; ++i) {
-        const float mi = s_m[i];
-        const float w = mi == -INFINITY ? 0.f : ex2(mi - M);
-        const float v = mi == -INFINITY ? 0.f : __ldcg(ph + i * sstride + c);
-        Lsum = fmaf(w, s_l[i], Lsum);
-        if (i < p.st_npp) {
-            ar = fmaf(w, v, ar);
-            if (QJL && c < QM && mi != -INFINITY) az = fmaf(w, __ldcg(ph + i * sstride + D + c), az);
-        } else {
-            ad = fmaf(w, v, ad);
+    const uint32_t unit = uint32_t(p.st_fold ? p.st_range * nw : p.st_range);       // (fewer than 2^31 tiles in all)
+    const uint32_t n_rows = uint32_t(p.B * p.Hkv * p.HG * p.slots), slots = uint32_t(p.slots);
+    const int sstride = p.slots * PS;
+    const int sg = tid / D, c = tid - sg * D, ns = NG / rp, r_of = sg / ns, part = sg - r_of * ns;      // sums: row of the pass, share of its slots
+    for (uint32_t row0 = blockIdx.x * uint32_t(rp); row0 < n_rows; row0 += gridDim.x * uint32_t(rp)) {
+        auto row_ptr = [&](int r) -> const float* {                   // the row's first partial
+            const uint32_t i = min(row0 + r, n_rows - 1), a = i / slots;
+            return p.st_part + (int64_t(a) * n_slots * p.slots + (i - a * slots)) * PS;
+        };
+        auto row_live = [&](int r) -> bool {
+            const uint32_t i = row0 + r, a = i / slots;
+            return i < n_rows && int(i - a * slots) < min(HPG, p.G - int(a % uint32_t(p.HG)) * HPG);
+        };
+        const float* src = row_ptr(r_of) + c;
+        const uint32_t wa = min(row0 + min(warp, rp - 1), n_rows - 1) / slots;
+        // the warps (CTAs) whose runs touch this lane's tiles [wa * n_tiles, (wa + 1) * n_tiles)
+        const int n_pp = n_tiles > 0 ? int(((wa + 1) * uint32_t(n_tiles) - 1) / unit) - int((wa * uint32_t(n_tiles)) / unit) + 1 : 0;
+        const bool live = row_live(min(warp, rp - 1));
+        const float* ml_src = row_ptr(min(warp, rp - 1)) + D + QM;
+        if (row0 == blockIdx.x * uint32_t(rp)) pdl_wait();            // (everything above only needs the parameters)
+        float v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = part + ns * u < n_slots ? __ldcg(src + (part + ns * u) * sstride) : 0.f;
+        if (warp < rp) {
+            constexpr int NI = (MAX_PARTS + 31) / 32;
+            float2 ml[NI];
+            float M = -INFINITY, sum = 0.f;
+#pragma unroll
+            for (int k = 0; k < NI; ++k) {
+                ml[k] = make_float2(-INFINITY, 0.f);
+                if (32 * k >= n_slots) continue;
+                const int j = lane + 32 * k;
+                const bool valid = live && j < n_slots && (j < n_pp || j >= p.st_npp);
+                ml[k] = valid ? __ldcg(reinterpret_cast<const float2*>(ml_src + j * sstride)) : make_float2(-INFINITY, 0.f);
+            }
+#pragma unroll
+            for (int k = 0; k < NI; ++k) M = fmaxf(M, ml[k].x);
+#pragma unroll
+            for (int off = 16; off; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
+#pragma unroll
+            for (int k = 0; k < NI; ++k) {
+                if (32 * k >= n_slots) continue;
+                const int j = lane + 32 * k;
+                const float w = ml[k].x == -INFINITY ? 0.f : ex2(ml[k].x - M);
+                sum = fmaf(w, ml[k].y, sum);
+                if (j < n_slots) s_w[warp][j] = w;
+            }
+#pragma unroll
+            for (int off = 16; off; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+            if (lane == 0) s_il[warp] = 1.f / sum;
         }
-    }
-    s_rot[c] = ar * inv_vs;
-    if (QJL && c < QM) s_z[c] = az * (QJL_C / D);
-    __syncthreads();
-    // undo the rotation of the packed part (y @ R, rotation.py:68-78) and add (c/d) z @ S (qjl.py:89-92)
-    float v = ad;
+        __syncthreads();
+        // weighted sums: the packed part in rotated space, the uncompressed part.  A slot without a partial has weight 0 and
+        // whatever bytes the workspace holds: it is skipped, not multiplied.
+        float ar = 0.f, ad = 0.f;
+        auto add = [&](int i, float x) {
+            const float w = i < n_slots ? s_w[r_of][i] : 0.f;
+            const float y = w != 0.f ? w * x : 0.f;
+            if (i < p.st_npp) ar += y; else ad += y;
+        };
+#pragma unroll
+        for (int u = 0; u < U; ++u) add(part + ns * u, v[u]);
+#pragma unroll 1
+        for (int i0 = part + ns * U; i0 < n_slots; i0 += ns * U) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = i0 + ns * u < n_slots ? __ldcg(src + (i0 + ns * u) * sstride) : 0.f;
+#pragma unroll
+            for (int u = 0; u < U; ++u) add(i0 + ns * u, v[u]);
+        }
+        s_p[0][sg][c] = ar;
+        s_p[1][sg][c] = ad;
+        if (QJL) {
+            for (int e = tid; e < rp * QM; e += NT) {
+                const int r = e / QM, z = e - r * QM;
+                const float* zs = row_ptr(r) + D + z;
+                float az = 0.f;
 #pragma unroll 8
-    for (int j = 0; j < D; ++j) v = fmaf(s_rot[j], stages_r<D>() ? rs[j * D + c] : __ldg(p.rot + j * D + c), v);
-    if (QJL) {
-#pragma unroll 8
-        for (int i = 0; i < QM; ++i) v = fmaf(s_z[i], stages_r<D>() ? rs[(D + i) * D + c] : __ldg(p.qjl_proj + i * D + c), v);
-    }
-    if (p.n_peers == 0) {
-        if (live) store_from_f32(p.out, p.out_dtype, qhead * D + c, v / Lsum);
-        return;
-    }
-    // fused gather: the head in the result's element type, sent as {payload, epoch} words (the query launch counted the call)
-    __syncthreads();
-    store_from_f32(s_rot, p.out_dtype, c, v / Lsum);
-    __syncthreads();
-    const int es = out_elem_bytes(p.out_dtype), n_words = D * es / 4;
-    if (!live) return;
-    const unsigned long long epoch = static_cast<unsigned long long>(p.epochs[a]) << 32;
-    const int64_t w0 = (int64_t(b) * p.heads_total + p.head_offset + int64_t(hkv) * p.G + hg * HPG + h) * n_words;
-    for (int i = c; i < n_words * p.n_peers; i += D) {
-        const int r = i / n_words, w = i - r * n_words;
-        const unsigned long long x = reinterpret_cast<const uint32_t*>(s_rot)[w] | epoch;
-        asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(p.peer_ll[r] + w0 + w), "l"(x) : "memory");
+                for (int i = 0; i < p.st_npp; ++i) {
+                    const float w = s_w[r][i];
+                    const float x = __ldcg(zs + i * sstride);
+                    az += w != 0.f ? w * x : 0.f;
+                }
+                s_a[r][D + z] = az * (QJL_C / D);
+            }
+        }
+        __syncthreads();
+        for (int e = tid; e < rp * D; e += NT) {
+            const int r = e / D, k = e - r * D;
+            float x = 0.f;
+            for (int q = 0; q < ns; ++q) x += s_p[0][r * ns + q][k];
+            s_a[r][k] = x * (1.f / (p.vb_lo != 0 && k >= D / 2 ? p.v_scale_lo : p.v_scale_hi));
+        }
+        __syncthreads();
+        for (int r = 0; r < rp; ++r) {
+            float x = 0.f, y = 0.f;
+#pragma unroll
+            for (int j = 0; j < KR; j += 4) {
+                const float4 q = *reinterpret_cast<const float4*>(&s_a[r][kg * KR + j]);
+                x = fmaf(q.x, rr[j], x); y = fmaf(q.y, rr[j + 1], y); x = fmaf(q.z, rr[j + 2], x); y = fmaf(q.w, rr[j + 3], y);
+            }
+#pragma unroll
+            for (int j = 0; j < SR; ++j) x = fmaf(s_a[r][D + kg * SR + j], sr[j], x);
+            s_o[kg][r][oc] = x + y;
+        }
+        __syncthreads();
+        for (int e = tid; e < rp * (NCOL / 2); e += NT) {              // two columns each
+            const int r = e / (NCOL / 2), o0 = 2 * (e - r * (NCOL / 2)), col = n0 + o0;
+            if (!row_live(r)) continue;
+            float o[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                float x = (s_o[0][r][o0 + u] + s_o[1][r][o0 + u]) + (s_o[2][r][o0 + u] + s_o[3][r][o0 + u]);
+                for (int q = 0; q < ns; ++q) x += s_p[1][r * ns + q][col + u];
+                o[u] = x * s_il[r];
+            }
+            const int ir = int(row0) + r;
+            const int a = ir / p.slots, h = ir - a * p.slots, kvl = a / p.HG, hg = a - kvl * p.HG, b = kvl / p.Hkv, hkv = kvl - b * p.Hkv;
+            const int head = hkv * p.G + hg * HPG + h;
+            if (p.n_peers == 0) {
+                const int64_t at = (int64_t(b) * p.Hq + head) * D + col;
+                store_from_f32(p.out, p.out_dtype, at, o[0]);
+                store_from_f32(p.out, p.out_dtype, at + 1, o[1]);
+                continue;
+            }
+            // fused gather: the two elements in the result's type, sent to every peer as {payload, epoch} words (the query launch
+            // counted the call)
+            const unsigned long long epoch = static_cast<unsigned long long>(p.epochs[a]) << 32;
+            const int64_t at = (int64_t(b) * p.heads_total + p.head_offset + head) * D + col;
+            const bool f32 = p.out_dtype == TQ_F32;
+            const uint32_t w0 = f32 ? __float_as_uint(o[0]) : p.out_dtype == TQ_F16 ? pack_h2(o[0], o[1]) : pack_bf2(o[0], o[1]), w1 = __float_as_uint(o[1]);
+            for (int q = 0; q < p.n_peers; ++q) {
+                unsigned long long* dst = p.peer_ll[q] + (f32 ? at : at / 2);
+                asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(dst), "l"(w0 | epoch) : "memory");
+                if (f32) asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(dst + 1), "l"(w1 | epoch) : "memory");
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -985,8 +1118,8 @@ template <int D, bool QJL> static int launch(const DecodeParams& p, cudaStream_t
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !set[dev].load(std::memory_order_acquire)) {
-        cudaError_t e = cudaFuncSetAttribute(decode_lut_kernel<D, QJL>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(lut_merge_kernel<D, QJL>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(merge_smem<D>()));
+        cudaError_t e = cudaFuncSetAttribute(decode_lut_kernel<D, QJL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_lut_kernel<D, QJL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return fail(TQ_ERR_LAUNCH, "tq_decode_attn: shared memory %zu B: %s", smem, cudaGetErrorString(e));
         set[dev].store(true, std::memory_order_release);
     }
@@ -998,21 +1131,31 @@ template <int D, bool QJL> static int launch(const DecodeParams& p, cudaStream_t
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const int64_t n_q = int64_t(p.B) * p.Hq;
-    cfg.gridDim = dim3(unsigned((n_q + 7) / 8), unsigned((D / 16 + (QJL ? 2 : 0) + 3) / 4));
-    cfg.blockDim = dim3(128);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, lut_query_kernel<D>, p);
+    cudaError_t e = cudaSuccess;
+    // CTAs that touch two lanes at most rotate those lanes' queries themselves: it takes them 2 us, a launch 5 (with four
+    // lanes: 8)
+    const bool inq = p.n_peers == 0 && !p.await_ll && (p.c_len == 0 || (p.st_fold && 2u * uint32_t(p.slots) * P::QR * 2u <= P::QCAP));
+    if (!inq) {
+        cfg.gridDim = dim3(unsigned((n_q + 7) / 8), unsigned((D / 16 + (QJL ? 2 : 0) + 3) / 4));
+        cfg.blockDim = dim3(128);
+        e = cudaLaunchKernelEx(&cfg, lut_query_kernel<D>, p);
+    }
     if (e == cudaSuccess) {
         cfg.gridDim = dim3(unsigned(p.st_grid));
         cfg.blockDim = dim3(P::NT);
         cfg.dynamicSmemBytes = smem;
-        e = cudaLaunchKernelEx(&cfg, decode_lut_kernel<D, QJL>, p);
+        e = inq ? cudaLaunchKernelEx(&cfg, decode_lut_kernel<D, QJL, true>, p) : cudaLaunchKernelEx(&cfg, decode_lut_kernel<D, QJL, false>, p);
     }
     if (e == cudaSuccess) {
-        constexpr int SPB = 512 / D;
-        cfg.gridDim = dim3(unsigned((int64_t(p.B) * p.Hkv * p.HG * p.slots + SPB - 1) / SPB));
-        cfg.blockDim = dim3(unsigned(SPB * D));
-        cfg.dynamicSmemBytes = merge_smem<D>();
-        e = cudaLaunchKernelEx(&cfg, lut_merge_kernel<D, QJL>, p, P::NW);
+        // one row at a time spreads few rows over the SMs and many slots over a block; else as many as the groups share evenly
+        const int64_t rows = int64_t(p.B) * p.Hkv * p.HG * p.slots;
+        constexpr int NG = merge_threads<D>() / D;
+        const int n_slots = p.st_npp + p.st_nd;
+        const int rp = rows <= p.st_grid || n_slots > 32 ? 1 : std::min(NG, n_slots > 16 ? 2 : 4);
+        cfg.gridDim = dim3(unsigned(std::min<int64_t>((rows + rp - 1) / rp, 4 * int64_t(p.st_grid))), D / merge_cols<D>());
+        cfg.blockDim = dim3(merge_threads<D>());
+        cfg.dynamicSmemBytes = 0;
+        e = cudaLaunchKernelEx(&cfg, lut_merge_kernel<D, QJL>, p, P::NW, rp);
     }
     if (e != cudaSuccess) return fail(TQ_ERR_LAUNCH, "tq_decode_attn: %s", cudaGetErrorString(e));
     return TQ_OK;
@@ -1051,7 +1194,7 @@ StreamPlan lut_plan(int batch, int n_q_heads, int n_kv_heads, int d, int64_t c_l
     }
     s.q16_bytes = (size_t(batch) * n_q_heads * lut::q_stride(d) * sizeof(__half) + 255) / 256 * 256;
     s.part_bytes = size_t(L) * size_t(s.npp + s.nd) * size_t(std::min(G, HPG)) * lut::part_stride(d) * sizeof(float);
-    s.ok = s.npp + s.nd <= lut::MAX_PARTS && L * p_tiles < (int64_t(1) << 31);
+    s.ok = s.npp + s.nd <= lut::MAX_PARTS && (L + 1) * (p_tiles + 1) < (int64_t(1) << 31) && L < (int64_t(1) << 20) && dense_len < (int64_t(1) << 30);
     return s;
 }
 
