@@ -762,19 +762,27 @@ int decode_prepare(const tq_decode_args* a, void* workspace, size_t workspace_by
         const int max_parts = direct ? std::min(g_tune_stream_max_parts, 64) : 64;
         stream = stp.range >= min_run && stp.npp + stp.nd <= max_parts && stream_supported(d, qjl);
     }
-    // everything else the lookup kernel's tables cover (two to four bits, their fractional splits).  The general kernel is one launch instead of three: with whole-byte tables
-    // (4-bit keys, 2-bit values) it is the faster one for few tiles (head_dim 64, 16 lanes x 218 tiles: 17 against 29 us;
-    // head_dim 128 with sketches, 72 lanes x 230 tiles: 63 against 35 us)
-    bool lut = ((!direct && !stream && g_tune_lut) || g_tune_lut == 2) && !g_tune_force_general && a->c_lane_stride % 16 == 0 && aligned(a->q, 8) &&
+    // The lookup kernel: everything else its tables cover (two to four bits, their fractional splits), and of the 4-bit-key /
+    // 2-bit-value calls those that are not its rivals' best.  Per call:
+    //   * table-lookup (direct) kernel: many lanes - 256 x 31 tiles 54.7 against 44.1 us, 384 x 62 72.7 / 42.7, 128 x 375 56.9 / 50.5;
+    //     few or short ones stay (16 x 1000 22.7 / 33.2, 64 x 94 21.9 / 25.9)
+    //   * streaming kernel: until its runs are long enough to pay for two partials per warp - 128 x 512 68.0 / 63.9, with sketches
+    //     64 x 500 72.8 / 51.5, 128 x 512 at d = 96 72 / 63; beyond it stays (128 x 1024 95.1 / 97.9)
+    //   * general kernel: d = 64 without sketches and few tiles, where it is one launch of little code (48 x 63 12.0 / 15.6,
+    //     64 x 188 21.5 / 18.9); d = 96, d = 256 and sketches are faster here at any size (8 x 125 16.3 / 15.3, 36.8 / 31.6, 32.6 / 22.8)
+    const int64_t kv_lanes = int64_t(a->batch) * a->n_kv_heads, tiles = kv_lanes * ((a->c_len + TILE - 1) / TILE);
+    const bool bytes = a->c_len > 0 && a->k_bits_hi == 4 && !a->k_bits_lo && a->v_bits_hi == 2 && !a->v_bits_lo;
+    const bool lut_best = !bytes ? true : stream ? stp.range < g_tune_stream_min_run * 3 / 2 && kv_lanes <= 148 : direct ? kv_lanes >= 256 || (kv_lanes >= 64 && tiles >= 16000)
+                                                                                 : d != 64 || qjl || tiles >= 10000;
+    bool lut = ((lut_best && g_tune_lut) || g_tune_lut == 2) && !g_tune_force_general && a->c_lane_stride % 16 == 0 && aligned(a->q, 8) &&
                aligned(a->k_hi, 16) && aligned(a->v_hi, 16) && aligned(a->k_norms, 16) && aligned(a->v_norms, 16) &&
                (!a->k_bits_lo || aligned(a->k_lo, 16)) && (!a->v_bits_lo || aligned(a->v_lo, 16)) &&
                (!qjl || (aligned(a->k_qjl_bits, 16) && aligned(a->v_qjl_bits, 16) && aligned(a->k_qjl_gamma, 16) && aligned(a->v_qjl_gamma, 16) && aligned(a->qjl_proj, 16))) &&
                (a->sink_len == 0 || (aligned(a->sink_k, 16) && aligned(a->sink_v, 16))) && (!a->res_k || (aligned(a->res_k, 16) && aligned(a->res_v, 16)));
     if (lut) {
-        stp = lut_plan(a->batch, a->n_q_heads, a->n_kv_heads, d, a->c_len, dense_len, sm_count());
-        const int64_t tiles = int64_t(a->batch) * a->n_kv_heads * ((a->c_len + TILE - 1) / TILE);
-        const bool bytes = a->k_bits_hi == 4 && !a->k_bits_lo && a->v_bits_hi == 2 && !a->v_bits_lo;
-        lut = stp.ok && !(a->c_len > 0 && bytes && tiles < 8000 && g_tune_lut == 1) && lut_supported(d, qjl, a->c_len > 0 ? a->k_bits_hi : 4, a->c_len > 0 ? a->k_bits_lo : 0, a->c_len > 0 ? a->v_bits_hi : 4, a->c_len > 0 ? a->v_bits_lo : 0);
+        const StreamPlan lp = lut_plan(a->batch, a->n_q_heads, a->n_kv_heads, d, a->c_len, dense_len, sm_count());
+        lut = lp.ok && lut_supported(d, qjl, a->c_len > 0 ? a->k_bits_hi : 4, a->c_len > 0 ? a->k_bits_lo : 0, a->c_len > 0 ? a->v_bits_hi : 4, a->c_len > 0 ? a->v_bits_lo : 0);
+        if (lut) stp = lp;
     }
     if (lut) stream = false;
     const SplitPlan sp = plan_splits(a->batch, a->n_q_heads, a->n_kv_heads, a->c_len, dense_len, sm_count(), direct);

@@ -714,6 +714,9 @@ size_t prefill_fa_workspace(int batch, int n_q_heads, int n_kv_heads, int d, int
 // Whether the two-step kernel takes the call with this workspace; the caller has validated the arguments.
 bool prefill_fa_applicable(const tq_decode_args* a, int t_q) {
     const int64_t total = a->c_len + a->sink_len + a->res_len;
+    // (a float32 query would be rounded to fp16 beside the rounding of the expanded rows; 16-bit queries are exact: float32 callers
+    // stay with the kernels that multiply the rotated query with the centroids, one rounding fewer)
+    if (a->q_dtype == TQ_F32) return false;
     if (!a->workspace || !aligned(a->workspace, 256) || total >= (int64_t(1) << 30) || !fa::encoder()) return false;
     if (a->c_len > 0 && ((a->k_bits_lo && a->k_bits_lo != a->k_bits_hi - 1) || (a->v_bits_lo && a->v_bits_lo != a->v_bits_hi - 1))) return false;
     if (!aligned(a->out, 16) || !aligned(a->rot, 16)) return false;
