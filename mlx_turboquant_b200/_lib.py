@@ -193,6 +193,23 @@ except AttributeError:                                    # pragma: no cover - o
     _raw_stream = None
 
 
+_cuda_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)      # (initialised: some tensor is on the GPU already)
+
+
+def here(*tensors: torch.Tensor) -> int | None:
+    """The current stream's handle when every tensor is on the current CUDA device, else None: the cheap check of the calls
+    that a decode loop makes thousands of times (a few hundred nanoseconds); ``require_cuda`` and ``launch`` do the rest."""
+    idx = _cuda_device()
+    for t in tensors:
+        if t.get_device() != idx:
+            return None
+    return stream_ptr_of(idx)
+
+
+def stream_ptr_of(idx: int) -> int:
+    return _raw_stream(idx) if _raw_stream is not None else torch.cuda.current_stream(idx).cuda_stream
+
+
 def stream_ptr(device: torch.device) -> int:
     if _raw_stream is not None:
         return _raw_stream(device.index if device.index is not None else torch.cuda.current_device())

@@ -146,6 +146,8 @@ class TurboQuantKVCache:
         self._dense_len = 0
         self._dargs = self._dargs_key = self._ws_key = None     # decode argument block kept between attend() calls
         self._ws_need = 0
+        self._last_ws = None        # workspace the argument block points to
+        self._step = None           # what the last fused decode step was checked against (see decode_step)
         self._tables = None         # prebuilt constants of the decode kernel (shared between caches of the same shape)
         self.offset = 0
 
@@ -213,7 +215,7 @@ class TurboQuantKVCache:
         if dev is not None and self._device is not None and dev != self._device:
             raise RuntimeError(f"state tensors are on {dev}, this cache is bound to {self._device}")
         v = tuple(v) + (None,) * (14 - n)
-        self._dargs = self._dargs_key = self._ws_key = None     # the cached decode arguments pointed into the old arrays
+        self._dargs = self._dargs_key = self._ws_key = self._step = None     # the cached decode arguments pointed into the old arrays
         self.keys, self.values = v[0], v[1]
         def own(t):
             """Adopt a packed array as storage: contiguous, token capacity padded to a multiple of 16."""
@@ -518,6 +520,8 @@ class TurboQuantKVCache:
             self._ws_key = ws_key
         ws = kernels.decode_workspace(dev, self._ws_need)
         a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+        self._last_ws = ws
+        self._step = None                            # (a gather or a wait may be set now)
         if _new is None:
             _lib.check(_lib.launch(dev, "tq_decode_attn", C.byref(a), _lib.stream_ptr(dev)))
         else:      # append the token's rows and attend over them in the same launch
@@ -562,6 +566,38 @@ class TurboQuantKVCache:
         """One decode step: ``update(keys, values)`` followed by ``attend(queries)``, as ONE kernel launch when the new token
         simply joins the recent-token buffer (no growth, no compression due, not a sink token, same dtype as the buffer):
         the kernel stores the token's rows itself and attends over them.  Any other step takes the two calls."""
+        # A loop's next step differs from the last fused one by three addresses and the lengths: everything that was checked
+        # and filled in then is recognised by shapes, types and the identity of the buffers (3 us of host work instead of 12).
+        p = self._step
+        if p is not None and out is None:
+            q_shape, kv_shape, q_dt, kv_dt, sc, k_buf, v_buf, k_hi, v_hi, k_q, sink, a, ref = p
+            n = self._fp16_len + 1
+            if (queries.shape == q_shape and keys.shape == kv_shape and values.shape == kv_shape and queries.dtype is q_dt and keys.dtype is kv_dt
+                    and values.dtype is kv_dt and scale == sc and self.keys is k_buf and self.values is v_buf and self._k.hi is k_hi
+                    and self._v.hi is v_hi and self._k.qbits is k_q and self.sink_keys is sink and self._dargs is a and n <= self._fp16_capacity
+                    and self.offset >= self.fp16_sink_size
+                    and (n <= self.residual_window * 2 if self.chunk_size <= 0 else n < self.residual_window + self.chunk_size)
+                    and queries.is_contiguous() and keys.is_contiguous() and values.is_contiguous()):
+                stream = _lib.here(queries, keys, values, k_buf)
+                ws = None if stream is None else kernels.workspace_of(self._device.index, stream)
+                if ws is not None:
+                    c_len, s_len = self._compressed_len, self._sink_len
+                    ws_key = (c_len, (s_len + n + 15) >> 4)
+                    if ws_key != self._ws_key:
+                        self._ws_need = _lib.lib().tq_decode_workspace_bytes(q_shape[0], q_shape[1], a.n_kv_heads, self.head_dim, c_len, ws_key[1] << 4)
+                        self._ws_key = ws_key
+                    if ws.numel() >= self._ws_need:
+                        if ws is not self._last_ws:
+                            a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+                            self._last_ws = ws
+                        res = torch.empty_like(queries)
+                        a.q, a.out, a.c_len, a.sink_len, a.res_len = queries.data_ptr(), res.data_ptr(), c_len, s_len, n - 1
+                        rc = _lib.lib().tq_decode_step(ref, keys.data_ptr(), values.data_ptr(), stream)
+                        if rc != 0:
+                            _lib.check(rc)
+                        self._fp16_len = n
+                        self.offset += 1
+                        return res
         t_new = keys.shape[2] if keys.dim() == 4 else 0
         fast = (t_new == 1 and self.keys is not None and self.offset >= self.fp16_sink_size
                 and self._fp16_len + 1 <= self._fp16_capacity and keys.dtype == self.keys.dtype and values.dtype == self.values.dtype
@@ -578,6 +614,9 @@ class TurboQuantKVCache:
         if keys.device != self._device or values.device != self._device:
             raise RuntimeError(f"this cache lives on {self._device}; got tensors on {keys.device}")
         res = self.attend(queries, scale=scale, out=out, _new=(keys, values))
+        if out is None and res.dtype == queries.dtype:
+            self._step = (queries.shape, keys.shape, queries.dtype, keys.dtype, scale, self.keys, self.values, self._k.hi, self._v.hi,
+                          self._k.qbits, self.sink_keys, self._dargs, C.byref(self._dargs))
         self._fp16_len += 1
         self.offset += 1
         return res

@@ -30,15 +30,29 @@ class TurboQuantMSE:
         self.d, self.bits, self.seed = d, bits, seed
         self.rotation = get_rotation_matrix(d, seed, device)
         self.centroids, self.boundaries = get_codebook(d, bits, device)
+        self._rows = None
+
+    def _codec(self) -> kernels.RowCodec:
+        c = self._rows
+        if c is None or c.of[0] is not self.rotation or c.of[1] is not self.centroids or c.of[2] is not self.boundaries:
+            c = self._rows = kernels.RowCodec(self.d, self.bits, self.rotation, self.centroids, self.boundaries)
+        return c
 
     def quantize(self, x: torch.Tensor) -> QuantizedTensor:
         """(..., d) -> packed (..., d*bits/8) uint8 + norms (...) float32; a bare (d,) vector works too."""
+        res = self._codec().quantize(x)
+        if res is not None:
+            return QuantizedTensor(res[0], res[1], self.bits, self.d)
         lead = x.shape[:-1]
         flat = x.reshape(-1, self.d)
         packed, _, norms = kernels.quantize_pack(flat, self.rotation, self.boundaries, self.bits)
         return QuantizedTensor(packed.reshape(*lead, -1), norms.reshape(lead), self.bits, self.d)
 
     def dequantize(self, qt: QuantizedTensor) -> torch.Tensor:
+        if qt.bits == self.bits and qt.d == self.d:
+            out = self._codec().dequantize(qt.packed_indices, qt.norms)
+            if out is not None:
+                return out
         lead = qt.norms.shape
         n = qt.norms.numel()
         out = kernels.dequantize(qt.packed_indices.reshape(n, -1), qt.norms.reshape(n), self.centroids,
