@@ -96,6 +96,8 @@ typedef struct {
 /* TurboQuantMSE.quantize / cache._quantize_kv(_fractional) (quantizer.py:54-85, cache.py:232-274);
  * metal_quantize_4bit (kernels.py:363-409). */
 int tq_quantize_pack(const tq_quantize_args* a, void* stream);
+/* n independent calls of the above, one after the other on the stream. */
+int tq_quantize_pack_many(const tq_quantize_args* a, int n, void* stream);
 
 /* The tensor-core quantize kernel (fp16 rows, d = 128) and the 4-bit-key / 2-bit-value decode kernel wait on
  * mbarriers with an iteration limit; if a wait ever runs out the kernel drains and finishes, and this returns the
@@ -120,6 +122,24 @@ typedef struct {
 /* TurboQuantMSE.dequantize / cache._dequantize_kv(_fractional) / metal_dequantize
  * (quantizer.py:87-109, cache.py:276-343, kernels.py:313-360). */
 int tq_dequantize(const tq_dequantize_args* a, void* stream);
+/* Keys and values of a cache in one call: the two share d, rot and out_dtype. */
+int tq_dequantize_pair(const tq_dequantize_args* k, const tq_dequantize_args* v, void* stream);
+
+/* Dense keys and values [sink | middle | recent] (update_and_fetch, cache.py:620-706) into k_out / v_out, (lanes, out_rows, d)
+ * of out_dtype: up to three parts of rows are copied (and widened to float32) in one launch - part i to rows
+ * [dst_row, dst_row + rows) of every lane, its own lanes lane_stride rows apart - and, if k and v are given, packed rows are
+ * dequantized by tq_dequantize_pair.  All pointers 16-byte aligned, d a multiple of 8. */
+typedef struct {
+    const void* k; const void* v; int dtype;
+    int64_t rows, lane_stride, dst_row;
+} tq_fetch_part;
+typedef struct {
+    tq_fetch_part part[3];
+    int64_t lanes, out_rows;
+    int d, out_dtype;
+    void* k_out; void* v_out;
+} tq_fetch_args;
+int tq_fetch_dense(const tq_fetch_args* a, const tq_dequantize_args* k, const tq_dequantize_args* v, void* stream);
 
 /* ---- QJL sketch ---------------------------------------------------------------------------- */
 

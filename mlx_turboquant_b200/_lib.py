@@ -43,6 +43,14 @@ class DequantizeArgs(C.Structure):
     ]
 
 
+class FetchPart(C.Structure):
+    _fields_ = [("k", _vp), ("v", _vp), ("dtype", _i), ("rows", _i64), ("lane_stride", _i64), ("dst_row", _i64)]
+
+
+class FetchArgs(C.Structure):
+    _fields_ = [("part", FetchPart * 3), ("lanes", _i64), ("out_rows", _i64), ("d", _i), ("out_dtype", _i), ("k_out", _vp), ("v_out", _vp)]
+
+
 TQ_MAX_PEERS = 8
 
 
@@ -87,7 +95,10 @@ PROTOTYPES = {
     "tq_quantize_from_rotated": (_i, [_vp, _i64, _i, _vp, _i, _vp, _i, _vp, _vp, _vp]),
     "tq_rotate": (_i, [_vp, _i, _vp, _vp, _i64, _i, _i, _vp]),
     "tq_quantize_pack": (_i, [C.POINTER(QuantizeArgs), _vp]),
+    "tq_quantize_pack_many": (_i, [C.POINTER(QuantizeArgs), _i, _vp]),
     "tq_dequantize": (_i, [C.POINTER(DequantizeArgs), _vp]),
+    "tq_dequantize_pair": (_i, [C.POINTER(DequantizeArgs), C.POINTER(DequantizeArgs), _vp]),
+    "tq_fetch_dense": (_i, [C.POINTER(FetchArgs), C.POINTER(DequantizeArgs), C.POINTER(DequantizeArgs), _vp]),
     "tq_qjl_quantize": (_i, [_vp, _vp, _vp, _vp, _i64, _i, _i, _vp]),
     "tq_qjl_dequantize": (_i, [_vp, _vp, _vp, _vp, _i64, _i, _i, _vp]),
     "tq_qk_scores": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i64, _i64, _vp, _vp]),
@@ -175,9 +186,9 @@ def launch(dev: torch.device, name: str, *args) -> int:
     shared-memory plan, static scratch) are keyed on it; tensors on ``cuda:1`` handed over while ``cuda:0`` is current
     would be dereferenced on the wrong GPU.  ``stream`` arguments must already belong to ``dev`` (``stream_ptr(dev)``).
     """
-    fn = getattr(lib(), name)
+    fn = getattr(_lib or lib(), name)
     idx = dev.index if dev.index is not None else torch.cuda.current_device()
-    if idx == torch.cuda.current_device():
+    if idx == _cuda_device():
         return fn(*args)
     with torch.cuda.device(idx):
         return fn(*args)

@@ -10,8 +10,8 @@ written against the reference keeps working.  What differs is where the work hap
   preallocated packed storage that grows geometrically - no per-drain concatenation;
 * ``update`` + ``attend`` compute a decode step directly on the packed storage (the path the
   reference only prototyped); ``update_and_fetch`` still returns the dense
-  ``[sink | dequantized middle | recent]`` tensors for callers that run their own attention,
-  building the dense middle lazily and incrementally;
+  ``[sink | dequantized middle | recent]`` tensors for callers that run their own attention, the
+  middle dequantized straight into the result;
 * the QJL sketch (sign bits + residual norm per token) is kept, so the correction survives a
   state reload instead of being baked into a transient dense tensor.
 """
@@ -62,6 +62,9 @@ def _rotated_projection(d: int, m: int, rotation_seed: int, device) -> torch.Ten
     return _proj_rot_cache[key]
 
 
+_bound: dict[tuple, tuple] = {}     # (device, settings) -> constants of a cache (see TurboQuantKVCache._bind)
+
+
 class _Side:
     """Packed storage of one side (keys or values): codes, norms and the optional QJL sketch."""
 
@@ -72,6 +75,56 @@ class _Side:
         self.hi = self.lo = self.norms = self.qbits = self.qgamma = None
         self.cent_hi = self.cent_lo = self.bnd_hi = self.bnd_lo = None
         self.fp16_scale_hi = self.fp16_scale_lo = 0.0
+        self.q_block = self.r_block = b""              # argument blocks of quantize / dequantize with the constants filled in
+
+    def constants(self) -> tuple:
+        return (self.cent_hi, self.bnd_hi, self.fp16_scale_hi, self.cent_lo, self.bnd_lo, self.fp16_scale_lo, self.q_block, self.r_block)
+
+    def adopt(self, c: tuple) -> None:
+        self.cent_hi, self.bnd_hi, self.fp16_scale_hi, self.cent_lo, self.bnd_lo, self.fp16_scale_lo, self.q_block, self.r_block = c
+
+    def fill_blocks(self, d: int, rotation, proj, proj_rot) -> None:
+        q, r = _lib.QuantizeArgs(), _lib.DequantizeArgs()
+        for a in (q, r):
+            a.d, a.rot, a.bits_hi, a.bits_lo = d, rotation.data_ptr(), self.bits_hi, self.bits_lo
+            a.cent_hi, a.cent_lo = self.cent_hi.data_ptr(), _lib.ptr(self.cent_lo)
+        q.bnd_hi, q.bnd_lo = self.bnd_hi.data_ptr(), _lib.ptr(self.bnd_lo)
+        q.qjl_proj_rot, r.qjl_proj = _lib.ptr(proj_rot), _lib.ptr(proj)
+        r.out_row_stride = d
+        self.q_block, self.r_block = bytes(q), bytes(r)
+
+    def quantize_job(self, a, x: torch.Tensor, at: int) -> torch.Tensor:
+        """Fills ``a``: rows x (B, H, T, D) to tokens [at, at + T) of the packed storage; returns what must stay alive until
+        the launch."""
+        b, h, t, d = x.shape
+        if x.dtype not in _lib._DTYPES:
+            x = x.to(torch.float32)
+        st = x.stride()
+        if st[3] != 1 or (b > 1 and h > 1 and st[0] != h * st[1]):
+            x = x.contiguous()
+            st = x.stride()
+        C.memmove(C.addressof(a), self.q_block, len(self.q_block))
+        cap = self.hi.shape[2]
+        a.x, a.x_dtype, a.n_lanes, a.n_rows = x.data_ptr(), _lib.dtype_code(x.dtype), b * h, t
+        a.x_lane_stride, a.x_row_stride = (st[1] if h > 1 else st[0] if b > 1 else 0), (st[2] if t > 1 else d)
+        a.packed_hi, a.norms, a.out_lane_stride = self.hi.data_ptr() + at * self.hi.shape[3], self.norms.data_ptr() + 4 * at, cap
+        if self.lo is not None:
+            a.packed_lo = self.lo.data_ptr() + at * self.lo.shape[3]
+        if a.qjl_proj_rot and self.qbits is not None:
+            a.qjl_bits, a.qjl_gamma = self.qbits.data_ptr() + 4 * at, self.qgamma.data_ptr() + 4 * at
+        return x
+
+    def dequantize_job(self, n: int, at: int, out_ptr: int, out_rows: int, d: int, with_qjl: bool) -> "_lib.DequantizeArgs":
+        """Argument block: tokens [at, at + n) as float32 rows, every lane's ``out_rows`` rows from the last one's."""
+        a = _lib.DequantizeArgs.from_buffer_copy(self.r_block)
+        a.packed_hi, a.norms = self.hi.data_ptr() + at * self.hi.shape[3], self.norms.data_ptr() + 4 * at
+        if self.lo is not None:
+            a.packed_lo = self.lo.data_ptr() + at * self.lo.shape[3]
+        if with_qjl:
+            a.qjl_bits, a.qjl_gamma = self.qbits.data_ptr() + 4 * at, self.qgamma.data_ptr() + 4 * at
+        a.n_lanes, a.n_rows, a.in_lane_stride = self.hi.shape[0] * self.hi.shape[1], n, self.hi.shape[2]
+        a.out, a.out_dtype, a.out_lane_stride = out_ptr, _lib.TQ_F32, out_rows * d
+        return a
 
     def load_tables(self, d: int, device) -> None:
         self.cent_hi, self.bnd_hi = get_codebook(d, self.bits_hi, device)
@@ -147,6 +200,7 @@ class TurboQuantKVCache:
         self._dargs = self._dargs_key = self._ws_key = None     # decode argument block kept between attend() calls
         self._ws_need = 0
         self._last_ws = None        # workspace the argument block points to
+        self._many = None           # likewise for several query tokens: what the block was filled for, the block
         self._step = None           # what the last fused decode step was checked against (see decode_step)
         self._tables = None         # prebuilt constants of the decode kernel (shared between caches of the same shape)
         self.offset = 0
@@ -159,6 +213,14 @@ class TurboQuantKVCache:
             return
         self._device = device
         d = self.head_dim
+        # constants shared by every cache of these settings on the device (a fresh cache per prompt pays a lookup, not 25 us)
+        key = (device, d, self.rotation_seed, self.key_bits, self.value_bits, self.qjl_correction, self.qjl_n_proj)
+        known = _bound.get(key)
+        if known is not None:
+            self._rotation, self._tables, self._qjl_proj, self._qjl_proj_rot, k, v = known
+            self._k.adopt(k)
+            self._v.adopt(v)
+            return
         self._rotation = get_rotation_matrix(d, self.rotation_seed, device)
         self._k.load_tables(d, device)
         self._v.load_tables(d, device)
@@ -168,6 +230,9 @@ class TurboQuantKVCache:
         if self.qjl_correction:
             self._qjl_proj = get_projection_matrix(d, self.qjl_n_proj, device=device)
             self._qjl_proj_rot = _rotated_projection(d, self.qjl_n_proj, self.rotation_seed, device)
+        for side in (self._k, self._v):
+            side.fill_blocks(d, self._rotation, self._qjl_proj, self._qjl_proj_rot)
+        _bound[key] = (self._rotation, self._tables, self._qjl_proj, self._qjl_proj_rot, self._k.constants(), self._v.constants())
 
     @property
     def rotation(self):
@@ -215,7 +280,7 @@ class TurboQuantKVCache:
         if dev is not None and self._device is not None and dev != self._device:
             raise RuntimeError(f"state tensors are on {dev}, this cache is bound to {self._device}")
         v = tuple(v) + (None,) * (14 - n)
-        self._dargs = self._dargs_key = self._ws_key = self._step = None     # the cached decode arguments pointed into the old arrays
+        self._dargs = self._dargs_key = self._ws_key = self._step = self._many = None     # the cached decode arguments pointed into the old arrays
         self.keys, self.values = v[0], v[1]
         def own(t):
             """Adopt a packed array as storage: contiguous, token capacity padded to a multiple of 16."""
@@ -291,12 +356,6 @@ class TurboQuantKVCache:
         return total
 
     # ---- compression ------------------------------------------------------------------------------
-    def _qjl_args(self, side: _Side):
-        if not self.qjl_correction:
-            return None
-        return dict(proj_rot=self._qjl_proj_rot, cent_hi=side.cent_hi, cent_lo=side.cent_lo,
-                    bits=side.qbits, gamma=side.qgamma)
-
     def _due(self, length: int) -> int:
         """How many of ``length`` recent tokens the schedule compresses now (cache.py:497-533).  The reference drains one chunk
         per loop iteration while the buffer holds ``residual_window + chunk_size``; tokens are quantized independently, so
@@ -328,13 +387,14 @@ class TurboQuantKVCache:
         old = min(n, have)                     # of the n, those that sit in the buffer
         if n > 0:
             at = self._compressed_len
+            jobs, alive = (_lib.QuantizeArgs * 4)(), []
             for side, buf, new in ((self._k, self.keys, k_new), (self._v, self.values, v_new)):
                 side.reserve(b, h, d, at + n, at, dev, self.qjl_correction)
-                for rows, where in ((buf[:, :, :old] if old else None, at), (new[:, :, :n - old] if n > old else None, at + old)):
-                    if rows is not None:
-                        kernels.quantize_pack(rows, self._rotation, side.bnd_hi, side.bits_hi, side.bnd_lo, side.bits_lo,
-                                              out_hi=side.hi, out_lo=side.lo, out_norms=side.norms, out_offset=where,
-                                              qjl=self._qjl_args(side))
+                if old:
+                    alive.append(side.quantize_job(jobs[len(alive)], buf[:, :, :old], at))
+                if n > old:
+                    alive.append(side.quantize_job(jobs[len(alive)], new[:, :, :n - old] if n - old < t_new else new, at + old))
+            _lib.check(_lib.launch(dev, "tq_quantize_pack_many", jobs, len(alive), _lib.stream_ptr(dev)))
             # A long prefill would leave buffers sized for the whole prompt; they get the size a fresh cache would get for what
             # remains instead (batch 64 x 32K tokens: 17 GB per layer otherwise).
             small = max(length - n, self.residual_window * 2) + 256
@@ -352,10 +412,17 @@ class TurboQuantKVCache:
                 tail = buf[:, :, old:have]
                 buf[:, :, :kept] = tail.clone() if old < kept else tail
         if n - old < t_new:
-            self._append(self.keys, self.values, k_new[:, :, n - old:], v_new[:, :, n - old:], kept)
+            if n > old:
+                k_new, v_new = k_new[:, :, n - old:], v_new[:, :, n - old:]
+            self._append(self.keys, self.values, k_new, v_new, kept)
         self._fp16_capacity = cap
         self._fp16_len = length - n
         self._compressed_len += n
+        # blocks that were filled for buffers since replaced must not keep those alive
+        if self._step is not None and (self._step[5] is not self.keys or self._step[7] is not self._k.hi):
+            self._step = None
+        if self._many is not None and (self._many[0][8] is not self.keys or self._many[0][5] is not self._k.hi):
+            self._many = None
 
     def _route_sink(self, keys, values):
         """Peel the tokens that belong to the permanent sink off the head of the batch (cache.py:577-618)."""
@@ -367,8 +434,9 @@ class TurboQuantKVCache:
             return keys, values
         if self.sink_keys is None:
             b, h, _, d = keys.shape
-            self.sink_keys = torch.zeros((b, h, self.fp16_sink_size, d), dtype=keys.dtype, device=keys.device)
-            self.sink_values = torch.zeros((b, h, self.fp16_sink_size, d), dtype=values.dtype, device=values.device)
+            new = torch.empty if n_sink == self.fp16_sink_size else torch.zeros        # (rows without a token yet read as zeros)
+            self.sink_keys = new((b, h, self.fp16_sink_size, d), dtype=keys.dtype, device=keys.device)
+            self.sink_values = new((b, h, self.fp16_sink_size, d), dtype=values.dtype, device=values.device)
         self._append(self.sink_keys, self.sink_values, keys[:, :, :n_sink], values[:, :, :n_sink], self.offset)
         self._sink_len = self.offset + n_sink
         return keys[:, :, n_sink:], values[:, :, n_sink:]
@@ -377,13 +445,14 @@ class TurboQuantKVCache:
     def _append(k_buf, v_buf, k_new, v_new, row0: int) -> None:
         """k_buf[:, :, row0:row0+T] = k_new (same for values): one library launch when the layout allows it."""
         b, h, t_new, d = k_new.shape
-        _lib.require_cuda(k_buf, v_buf, k_new, v_new)
-        lane = k_new.stride(1)
-        if (k_new.dtype == k_buf.dtype == v_new.dtype == v_buf.dtype and k_new.stride() == v_new.stride()
-                and k_new.stride(3) == 1 and k_new.stride(2) == d and (b == 1 or k_new.stride(0) == h * lane) and lane % d == 0
-                and (d * k_buf.element_size()) % 16 == 0 and (lane >= t_new * d or h == 1)):
-            rc = _lib.launch(k_buf.device, "tq_append_tokens", k_new.data_ptr(), v_new.data_ptr(), k_buf.data_ptr(), v_buf.data_ptr(),
-                             b * h, t_new, d * k_buf.element_size(), max(lane // d, t_new), k_buf.shape[2], row0, _lib.stream_ptr(k_buf.device))
+        dev = _lib.require_cuda(k_buf, v_buf, k_new, v_new)
+        st, size = k_new.stride(), k_buf.element_size()
+        lane = st[1]
+        if (k_new.dtype == k_buf.dtype == v_new.dtype == v_buf.dtype and st == v_new.stride()
+                and st[3] == 1 and st[2] == d and (b == 1 or st[0] == h * lane) and lane % d == 0
+                and (d * size) % 16 == 0 and (lane >= t_new * d or h == 1)):
+            rc = _lib.launch(dev, "tq_append_tokens", k_new.data_ptr(), v_new.data_ptr(), k_buf.data_ptr(), v_buf.data_ptr(),
+                             b * h, t_new, d * size, max(lane // d, t_new), k_buf.shape[2], row0, _lib.stream_ptr(dev))
             if rc == 0:
                 return
             if rc != -2:                      # anything but "layout not supported" is an error
@@ -397,6 +466,8 @@ class TurboQuantKVCache:
         The state-changing half of ``update_and_fetch`` (cache.py:632-672) without building any dense
         output; pair it with :meth:`attend`.
         """
+        if self._append_step(keys, values):
+            return
         dev = _lib.require_cuda(keys, values)
         self._bind(dev)
         t_total = keys.shape[2]
@@ -404,6 +475,28 @@ class TurboQuantKVCache:
         if keys_rest.shape[2] > 0 or (self.keys is not None and self._due(self._fp16_len) > 0):
             self._take(keys_rest, values_rest)
         self.offset += t_total
+
+    def _append_step(self, keys: torch.Tensor, values: torch.Tensor) -> bool:
+        """The everyday step: tokens that simply join the recent-token buffer (no sink, no growth, nothing due)."""
+        buf = self.keys
+        if (buf is None or self.offset < self.fp16_sink_size or keys.dim() != 4 or keys.shape != values.shape or keys.dtype is not buf.dtype
+                or values.dtype is not buf.dtype or self.values.dtype is not buf.dtype or not keys.is_contiguous() or not values.is_contiguous()):
+            return False
+        b, h, t, d = keys.shape
+        have, cap = self._fp16_len, self._fp16_capacity
+        if have + t > cap or cap != buf.shape[2] or t == 0 or self._due(have + t) > 0 or buf.shape[0] != b or buf.shape[1] != h or buf.shape[3] != d:
+            return False
+        stream = _lib.here(keys, values, buf)
+        if stream is None or not buf.is_contiguous() or not self.values.is_contiguous():
+            return False
+        rc = _lib.lib().tq_append_tokens(keys.data_ptr(), values.data_ptr(), buf.data_ptr(), self.values.data_ptr(), b * h, t,
+                                         d * buf.element_size(), t, cap, have, stream)
+        if rc == -2:                          # (layout not supported)
+            return False
+        _lib.check(rc)
+        self._fp16_len = have + t
+        self.offset += t
+        return True
 
     # ---- dense output ------------------------------------------------------------------------------
     def _ensure_dense(self) -> None:
@@ -424,13 +517,9 @@ class TurboQuantKVCache:
                 if old is not None and self._dense_len > 0:
                     new[:, :, :self._dense_len] = old[:, :, :self._dense_len]
                 setattr(self, name, new)
-        for side, out in ((k, self._dense_k), (v, self._dense_v)):
-            qjl = None
-            if self.qjl_correction and side.qbits is not None:
-                qjl = dict(proj=self._qjl_proj, bits=side.qbits, gamma=side.qgamma)
-            kernels.dequantize_rows(side.hi, side.lo, side.norms, self._rotation, side.cent_hi, side.bits_hi,
-                                    side.cent_lo, side.bits_lo, d, n_rows=n, in_offset=self._dense_len,
-                                    out=out, out_offset=self._dense_len, qjl=qjl)
+        jobs = [side.dequantize_job(n, self._dense_len, out.data_ptr() + 4 * d * self._dense_len, out.shape[2], d, self.qjl_correction and side.qbits is not None)
+                for side, out in ((k, self._dense_k), (v, self._dense_v))]
+        _lib.check(_lib.launch(dev, "tq_dequantize_pair", C.byref(jobs[0]), C.byref(jobs[1]), _lib.stream_ptr(dev)))
         self._dense_len = self._compressed_len
 
     def update_and_fetch(self, keys: torch.Tensor, values: torch.Tensor):
@@ -440,6 +529,9 @@ class TurboQuantKVCache:
         the input dtype until a compressed part exists and float32 afterwards.
         """
         self.update(keys, values)
+        out = self._fetch()
+        if out is not None:
+            return out
         self._ensure_dense()
         pk, pv = [], []
         if self._sink_len > 0:
@@ -456,6 +548,44 @@ class TurboQuantKVCache:
         if len(pk) == 1:
             return pk[0], pv[0]
         return torch.cat(pk, dim=2), torch.cat(pv, dim=2)
+
+    def _fetch(self):
+        """The dense result in one library call: the packed middle is dequantized straight to its place in the result, the
+        uncompressed regions are copied around it.  None: a single region (returned as the view it is) or layouts the copy
+        kernel does not take.  With sketches and at head_dim 256, where dequantizing costs more than copying (16.8 million
+        values: 41 to 65 us against 20), the middle is kept expanded and only the newly compressed tokens are dequantized."""
+        s_len, c_len, r_len = self._sink_len, self._compressed_len, self._fp16_len
+        if (s_len > 0) + (c_len > 0) + (r_len > 0) < 2:
+            return None
+        ref = self.keys if r_len > 0 else self.sink_keys
+        b, h, _, d = ref.shape
+        dt = torch.float32 if c_len > 0 else ref.dtype
+        if dt not in _lib._DTYPES or d % 8:
+            return None
+        a = _lib.FetchArgs()
+        rows = s_len + c_len + r_len
+        for i, (n, k, v, at) in enumerate(((s_len, self.sink_keys, self.sink_values, 0), (r_len, self.keys, self.values, s_len + c_len))):
+            if n > 0:
+                if k.dtype != v.dtype or k.dtype not in _lib._DTYPES or (dt != torch.float32 and k.dtype != dt) or not k.is_contiguous() or not v.is_contiguous():
+                    return None
+                p = a.part[i]
+                p.k, p.v, p.dtype, p.rows, p.lane_stride, p.dst_row = k.data_ptr(), v.data_ptr(), _lib.dtype_code(k.dtype), n, k.shape[2], at
+        dev = self._device
+        out_k, out_v = torch.empty((b, h, rows, d), dtype=dt, device=dev), torch.empty((b, h, rows, d), dtype=dt, device=dev)
+        a.lanes, a.out_rows, a.d, a.out_dtype, a.k_out, a.v_out = b * h, rows, d, _lib.dtype_code(dt), out_k.data_ptr(), out_v.data_ptr()
+        jk = jv = None
+        if c_len > 0:
+            if self.qjl_correction or d == 256:
+                self._ensure_dense()
+                p = a.part[2]
+                p.k, p.v, p.dtype, p.rows, p.lane_stride, p.dst_row = self._dense_k.data_ptr(), self._dense_v.data_ptr(), _lib.TQ_F32, c_len, self._dense_k.shape[2], s_len
+            else:
+                jk, jv = (C.byref(side.dequantize_job(c_len, 0, o.data_ptr() + 4 * d * s_len, rows, d, False)) for side, o in ((self._k, out_k), (self._v, out_v)))
+        rc = _lib.launch(dev, "tq_fetch_dense", C.byref(a), jk, jv, _lib.stream_ptr(dev))
+        if rc == -2:
+            return None
+        _lib.check(rc)
+        return out_k, out_v
 
     # ---- attention on the packed cache -----------------------------------------------------------
     def attend(self, queries: torch.Tensor, scale: float | None = None, out_dtype=None, gather=None,
@@ -551,7 +681,15 @@ class TurboQuantKVCache:
             out = torch.empty((b, hq, tq, d), dtype=out_dtype or q.dtype, device=dev)
         elif out.device != dev or tuple(out.shape) != (b, hq, tq, d) or not out.is_contiguous() or out.dtype not in _lib._DTYPES:
             raise ValueError("out must be a contiguous float16 / bfloat16 / float32 tensor of the queries' shape on their device")
-        a = self._fill_decode_args(b, hq, q.dtype, out.dtype, scale)
+        # (kept between calls like a decode step's; the buffers it holds keep their addresses from being handed out again)
+        k, v = self._k, self._v
+        key = (b, hq, q.dtype, out.dtype, scale, k.hi, v.hi, k.qbits, self.keys, self.values, self.sink_keys, self._fp16_capacity)
+        kept = self._many
+        if kept is not None and all(x is y for x, y in zip(kept[0][5:11], key[5:11])) and kept[0][:5] == key[:5] and kept[0][11] == key[11]:
+            a = kept[1]
+        else:
+            a = self._fill_decode_args(b, hq, q.dtype, out.dtype, scale)
+            self._many = (key, a)
         a.q, a.out = q.data_ptr(), out.data_ptr()
         a.c_len, a.sink_len, a.res_len = self._compressed_len, self._sink_len, self._fp16_len
         # scratch for the expanded rows (at most 512 MB): the allocator reuses it in stream order after this call

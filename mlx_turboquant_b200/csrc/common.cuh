@@ -19,6 +19,7 @@ int fail(int code, const char* fmt, ...);
 int check_launch(const char* what);
 
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0; }
+inline bool dtype_ok(int t) { return t == TQ_F16 || t == TQ_BF16 || t == TQ_F32; }
 inline bool bits_ok(int b) { return b >= 1 && b <= 4; }
 // bytes per packed row of n codes
 __host__ __device__ inline int packed_bytes(int n_codes, int bits) { return n_codes * bits / 8; }

@@ -89,6 +89,9 @@ int tq_dequantize_tc(const tq_dequantize_args* q, int n_jobs, cudaStream_t s, bo
             return TQ_OK;
     }
     *handled = true;
+    // Two jobs of few tiles run side by side on half the SMs each: a CTA's set-up (R as operand tiles, 8 us) is then paid once
+    // (65,536 rows a side at d = 128: 39 us one after the other, 27 side by side); long ones balance better one after the other.
+    const bool share = n_jobs == 2 && std::max(p[0].n_tiles, p[1].n_tiles) <= 16 * n_sms;
     for (int i = 0; i < n_jobs; ++i) {
         std::atomic<uint64_t>& bits = set[dev][d == 64 ? 0 : d == 96 ? 1 : d == 128 ? 2 : 3];
         const uint64_t bit = uint64_t(1) << (p[i].bits_hi * 8 + p[i].bits_lo - 8 + (p[i].qjl_bits ? 32 : 0));
@@ -98,7 +101,8 @@ int tq_dequantize_tc(const tq_dequantize_args* q, int n_jobs, cudaStream_t s, bo
             bits.fetch_or(bit, std::memory_order_release);
         }
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(unsigned(d == 256 ? 2 * std::min(p[i].n_tiles, n_sms / 2) : std::min(p[i].n_tiles, n_sms)));
+        const int ctas = share ? n_sms / 2 : n_sms;
+        cfg.gridDim = dim3(unsigned(d == 256 ? 2 * std::min(p[i].n_tiles, ctas / 2) : std::min(p[i].n_tiles, ctas)));
         cfg.blockDim = dim3(dqtc::NT);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = s;
@@ -106,7 +110,7 @@ int tq_dequantize_tc(const tq_dequantize_args* q, int n_jobs, cudaStream_t s, bo
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = i > 0 ? 1 : 0;
+        cfg.numAttrs = 1;
         const cudaError_t e = cudaLaunchKernelEx(&cfg, k[i], p[i], maps[i]);
         if (e != cudaSuccess) return fail(TQ_ERR_LAUNCH, "tq_dequantize: %s", cudaGetErrorString(e));
     }

@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(NT, 1) dequantize_tc_kernel(const __grid_const
     // d = 256: CTAs with an even number own output columns 0 .. 127, the others 128 .. 255 of the same tiles
     constexpr int SPLIT = D == 256 ? 2 : 1;
     const int first = blockIdx.x / SPLIT, stride = gridDim.x / SPLIT, col_base = (blockIdx.x % SPLIT) * NC;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (p.follows) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     // ---------------- set-up: barriers, tensor memory, centroid tables, R as two fp16 B tiles, S ------------------------
     if (tid == 0) {
@@ -505,6 +505,10 @@ __global__ void __launch_bounds__(NT, 1) dequantize_tc_kernel(const __grid_const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (!p.follows) {          // the set-up read constants only; the second job may start once everything before this one has ended
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
     const uint32_t tmem_base = slot[0];
 
     const Waiter wait_bar{sbase + P::OFF_BAR, slot, p.status};

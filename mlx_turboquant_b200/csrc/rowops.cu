@@ -293,7 +293,6 @@ static int launch_rowops(const RowArgs& a, cudaStream_t s, const char* what) {
 }
 
 static bool d_ok(int d) { return d >= 16 && d <= 256 && d % 16 == 0; }
-static bool dtype_ok(int t) { return t == TQ_F16 || t == TQ_BF16 || t == TQ_F32; }
 
 }  // namespace tq
 
@@ -337,6 +336,13 @@ extern "C" int tq_quantize_pack(const tq_quantize_args* q, void* stream) {
     a.y_out = q->y_out; a.qjl_proj_rot = q->qjl_proj_rot; a.qjl_bits_out = q->qjl_bits; a.qjl_gamma_out = q->qjl_gamma;
     a.cent_hi = q->cent_hi; a.cent_lo = q->cent_lo;
     return launch_rowops(a, s, "tq_quantize_pack");
+}
+
+extern "C" int tq_quantize_pack_many(const tq_quantize_args* q, int n, void* stream) {
+    if (n < 0 || (n > 0 && !q)) return fail(TQ_ERR_INVALID, "tq_quantize_pack_many: null args");
+    for (int i = 0; i < n; ++i)
+        if (int rc = tq_quantize_pack(q + i, stream)) return rc;
+    return TQ_OK;
 }
 
 namespace tq {
@@ -384,4 +390,17 @@ extern "C" int tq_dequantize(const tq_dequantize_args* q, void* stream) {
     if (int rc = check_dequantize(q)) return rc;
     if (q->n_lanes == 0 || q->n_rows == 0) return TQ_OK;
     return dequantize_jobs(q, 1, nullptr, 0, nullptr, nullptr, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int tq_dequantize_pair(const tq_dequantize_args* k, const tq_dequantize_args* v, void* stream) {
+    if (!k || !v) return fail(TQ_ERR_INVALID, "tq_dequantize_pair: null args");
+    tq_dequantize_args q[2];
+    int n = 0;
+    for (const tq_dequantize_args* a : {k, v}) {
+        if (int rc = check_dequantize(a)) return rc;
+        if (a->n_lanes > 0 && a->n_rows > 0) q[n++] = *a;
+    }
+    if (n == 0) return TQ_OK;
+    if (n == 2 && (q[0].d != q[1].d || q[0].rot != q[1].rot || q[0].out_dtype != q[1].out_dtype)) return fail(TQ_ERR_INVALID, "tq_dequantize_pair: the two must share d, rot and out_dtype");
+    return dequantize_jobs(q, n, nullptr, 0, nullptr, nullptr, static_cast<cudaStream_t>(stream));
 }
