@@ -30,6 +30,12 @@
 //   last warp    one thread keeps the operand stages full with tiled TMA copies (cp.async.bulk.tensor, 3-D tensor map
 //                (column, row, lane), 128-byte swizzle as the MMA descriptors expect; rows past a lane's end and
 //                columns past d read as zeros)
+// head_dim 256 (DC = 256, no sketch): R does not fit beside the rows, so four CTAs share a 128-row tile, 64 output columns
+// each (a fractional width's halves are two such slices, so every slice has one width).  The contraction runs over 256
+// columns in two halves of one operand stage each; all terms of R sit side by side in ONE operand (fp16: [R_hi | R_lo],
+// bf16: [R_1 | R_2 | R_3], N = 128 / 192), because sixteen dependent MMAs take the same time at any width, and the epilogue
+// adds the accumulators.  The rows' norms have slots of their own, so that stages are free as soon as the MMAs have read
+// them.  A tile is fetched from memory once and three times from L2.  (524,288 rows at 4 bits: 4602 us in the CUDA-core row kernel before, 230 here; 3.5 bits 4576 / 255, bf16 4595 / 256.)
 // Every mbarrier wait is bounded: on a timeout the kernel raises a status word, drains and frees its TMEM.
 #include <algorithm>
 #include <cstdlib>
@@ -78,6 +84,10 @@ constexpr int SK_LD = 32;                                  // QJL: bytes per sta
 constexpr int OFF_SKETCH = (OFF_MISC + 64 + 127) / 128 * 128;   // QJL: one 32-row staging buffer per epilogue warp
 constexpr int SMEM_BYTES = OFF_SKETCH + TQ_QJL_EPI_WARPS * 32 * SK_LD;
 static_assert(SMEM_BYTES <= 227 * 1024, "shared-memory plan");
+
+constexpr int SLICE = 64, NSQ_SLOTS = 8;                   // head_dim 256: output columns of a CTA, norm slots
+constexpr int OFF_NSQ256 = OFF_PT, OFF_NRMBAR256 = OFF_NSQ256 + NSQ_SLOTS * TM * 4;     // (there is no sketch)
+static_assert(NSQ_SLOTS * TM * 4 + NSQ_SLOTS * 8 <= DMAX * QM * 4, "head_dim 256: norm slots");
 
 struct Params {
     int d, bf16, a_stages;
@@ -311,6 +321,7 @@ __device__ __forceinline__ void store_words(uint8_t* dst, const uint32_t (&words
 struct EpiCtx {
     const Params& p; unsigned char* smem; uint32_t tmem_base, bar_accfull, bar_accfree, bar_afree, bar_nrm;
     volatile int* abort_flag; int warp, lane;
+    uint8_t* dst; int nb; bool write_norms;        // head_dim 256: the slice's first byte, bytes of a packed row, this slice writes the norms
 };
 
 // QJL: the residual of sixteen coordinates (normalised rotated value minus its centroid) enters the 32 projections and
@@ -414,7 +425,7 @@ __device__ __forceinline__ uint32_t sketch_bits(const Sketch& sk) {
 // instruction cache.  SPLITACC: the high and low products sit in two accumulators lo_off columns apart and are combined
 // here (y = hi + 2^-11 lo), sixteen coordinates per pair of loads; otherwise one 32-column load per step.
 // NCH: the number of chunks when it is known at compile time (1 or 2: a single step whose shape folds), 0 = nch_rt.
-template <int BITS, bool QJL, bool SPLITACC, int NCH>
+template <int BITS, bool QJL, bool SPLITACC, int NCH, int TERMS = 2>
 __device__ __forceinline__ void quantize_part(uint32_t t_row, int col0, int nch_rt, int lo_off, const RowCtx& rc, const float (&sb)[7], const float* raw,
                                               const float* cent, uint8_t* dst, bool live, Sketch& sk, float& ee) {
     constexpr int NW = 2 * 16 * BITS / 32;                                          // words of a step: BITS
@@ -443,9 +454,17 @@ __device__ __forceinline__ void quantize_part(uint32_t t_row, int col0, int nch_
                     uint32_t (&lo)[16] = *reinterpret_cast<uint32_t (*)[16]>(v + 16);
                     tmem_ld16(t_row + col0 + (c0 + c) * 16, hi);
                     tmem_ld16(t_row + lo_off + col0 + (c0 + c) * 16, lo);
-                    tmem_ld_wait();
+                    if constexpr (TERMS == 3) {                                     // three bf16 terms of equal weight, smallest first
+                        uint32_t t3[16];
+                        tmem_ld16(t_row + 2 * lo_off + col0 + (c0 + c) * 16, t3);
+                        tmem_ld_wait();
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(fmaf(__uint_as_float(v[16 + i]), 1.f / 2048.f, __uint_as_float(v[i])));
+                        for (int i = 0; i < 16; ++i) v[i] = __float_as_uint((__uint_as_float(t3[i]) + __uint_as_float(v[16 + i])) + __uint_as_float(v[i]));
+                    } else {
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(fmaf(__uint_as_float(v[16 + i]), 1.f / 2048.f, __uint_as_float(v[i])));
+                    }
                 }
                 quantize16<BITS>(vc, rc, sb, raw, g0, g1);
                 put_group<BITS, NW>(w, 2 * c, g0);
@@ -456,6 +475,8 @@ __device__ __forceinline__ void quantize_part(uint32_t t_row, int col0, int nch_
         if (live) store_words<NW>(dst + c0 * 2 * BITS, w, nc * 2 * BITS);
     }
 }
+
+__device__ __forceinline__ uint32_t sbase_of(const EpiCtx& e) { return static_cast<uint32_t>(__cvta_generic_to_shared(e.smem)); }
 
 // BH bits for coordinates [0, half), BL for [half, d) (BL == 0: BH for all of them, half = d).  Three shapes:
 //   fp16 rows (SPLITACC): two accumulators per tile (high and low products: two independent chains of MMAs instead of
@@ -475,12 +496,12 @@ template <bool QJL, bool SPLITACC> struct EpiShape {
 };
 // DC: head_dim when it is known at compile time (the chunk shares, row widths and store shapes then fold), 0 = read it
 // from the parameters.
-template <int BH, int BL, bool QJL, bool SPLITACC, int DC>
+template <int BH, int BL, bool QJL, bool SPLITACC, int DC, int TERMS = 2>
 __device__ __forceinline__ void epilogue_loop(const EpiCtx& e) {
     using Sh = EpiShape<QJL, SPLITACC>;
     const Params& p = e.p;
     const int group = e.warp / Sh::WPG, quad = e.warp & 3, part = (e.warp % Sh::WPG) >> 2, row_in_tile = quad * 32 + e.lane;
-    const int d = DC ? DC : p.d, half = BL ? d / 2 : d;
+    const int d = DC == 256 ? SLICE : DC ? DC : p.d, half = BL ? d / 2 : d;
     const int nch_h = half / 16, nch_l = BL ? (d - half) / 16 : 0;                   // chunks of sixteen coordinates per bit width
     // this thread's chunks: [h0, h1) of the first width, [l0, l1) of the second
     // (share q of n chunks: [ceil(q n / SPLIT), ceil((q + 1) n / SPLIT)); the second width is dealt from the other end so
@@ -505,18 +526,28 @@ __device__ __forceinline__ void epilogue_loop(const EpiCtx& e) {
     const int nb_h = half * BH / 8, nb_l = BL ? (d - half) * BL / 8 : 0;            // bytes of a packed row (per width)
     int s = group % a_stages;                                                       // operand stage of iteration `it`
     // (cache lane, tile inside the lane) of the group's current tile, advanced by the group's tile stride: one division here
-    const uint32_t first_tile = blockIdx.x + uint32_t(group) * gridDim.x, stride_tiles = uint32_t(Sh::GROUPS) * gridDim.x;
+    constexpr uint32_t CPT = DC == 256 ? 4 : 1;                                     // CTAs per tile
+    const uint32_t first_tile = (blockIdx.x + uint32_t(group) * gridDim.x) / CPT, stride_tiles = uint32_t(Sh::GROUPS) * gridDim.x / CPT;
     uint32_t lane_o = first_tile / tpl, tl = first_tile - lane_o * tpl;
     const uint32_t step_o = stride_tiles / tpl, step_t = stride_tiles - step_o * tpl;
     for (int64_t tile = first_tile, it = group; tile < p.n_tiles; tile += stride_tiles, it += Sh::GROUPS) {
         const int a = int(it % Sh::STAGES);
         if (!mbar_wait(e.bar_accfull + 8 * a, uint32_t(it / Sh::STAGES) & 1u, e.abort_flag, 3)) break;
-        if (!mbar_wait(e.bar_nrm + 8 * s, uint32_t(it / a_stages) & 1u, e.abort_flag, 5)) break;     // sums of squares written
-        tc_fence_after();
-        const float* nsq = reinterpret_cast<const float*>(e.smem + OFF_NSQ) + s * 2 * TM;
-        const float nrm = sqrtf(nsq[row_in_tile] + nsq[TM + row_in_tile]);
-        mbar_arrive(e.bar_afree + 8 * s);                       // norm slots of this stage are free again
-        s = (s + Sh::GROUPS) % a_stages;
+        float nrm;
+        if constexpr (DC == 256) {
+            const int q = int(it % NSQ_SLOTS);
+            if (!mbar_wait(sbase_of(e) + OFF_NRMBAR256 + 8 * q, uint32_t(it / NSQ_SLOTS) & 1u, e.abort_flag, 5)) break;
+            tc_fence_after();
+            // (the slot is written again eight tiles on, by which time this tile's accumulator has been freed and used again)
+            nrm = sqrtf(reinterpret_cast<const float*>(e.smem + OFF_NSQ256)[q * TM + row_in_tile]);
+        } else {
+            if (!mbar_wait(e.bar_nrm + 8 * s, uint32_t(it / a_stages) & 1u, e.abort_flag, 5)) break;     // sums of squares written
+            tc_fence_after();
+            const float* nsq = reinterpret_cast<const float*>(e.smem + OFF_NSQ) + s * 2 * TM;
+            nrm = sqrtf(nsq[row_in_tile] + nsq[TM + row_in_tile]);
+            mbar_arrive(e.bar_afree + 8 * s);                       // norm slots of this stage are free again
+            s = (s + Sh::GROUPS) % a_stages;
+        }
         const float nden = fmaxf(nrm, 1e-10f);                  // cache.py:237-238 guards the zero vector the same way
         rc.rinv = 1.f / nden;
         rc.rbin = rc.rinv * 256.f;
@@ -537,13 +568,16 @@ __device__ __forceinline__ void epilogue_loop(const EpiCtx& e) {
         }
         // with head_dim 128 and quarter shares every thread has two chunks of an integer width, or one of each fractional width
         constexpr int NCH_H = (DC == 128 && Sh::SPLIT == 4) ? (BL ? 1 : 2) : 0, NCH_L = (DC == 128 && Sh::SPLIT == 4) ? 1 : 0;
+        if constexpr (DC == 256)
+            quantize_part<BH, QJL, SPLITACC, 1, TERMS>(t_row, h0 * 16, 1, SLICE, rc, sb_h, raw_h, cent_h, e.dst + orow * e.nb + h0 * 2 * BH, live, sk, ee);
+        else
         quantize_part<BH, QJL, SPLITACC, NCH_H>(t_row, h0 * 16, h1 - h0, d, rc, sb_h, raw_h, cent_h, p.p_hi + orow * nb_h + h0 * 2 * BH, live, sk, ee);
         if (BL) quantize_part<(BL ? BL : 1), QJL, SPLITACC, NCH_L>(t_row, half + l0 * 16, l1 - l0, d, rc, sb_l, raw_l, cent_l, p.p_lo + orow * nb_l + l0 * 2 * BL, live, sk, ee);
         tc_fence_before();
         mbar_arrive(e.bar_accfree + 8 * a);                     // the accumulator may be overwritten
         uint32_t zb = 0;
         if (QJL) zb = sketch_bits(sk);                          // (every lane of the warp takes part)
-        if (live && part == 0) {
+        if (live && part == 0 && (DC != 256 || e.write_norms)) {
             p.norms[orow] = nrm;
             if (QJL) {
                 if (nrm == 0.f) zb = 0xffffffffu;               // zero row: the reference's residual is exactly 0, and 0 >= 0
@@ -582,12 +616,47 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
             // one arrival (the issuing thread, with the byte count) fills a stage; it is free again once the MMAs have
             // committed, the norm warps have read the rows and the tile's epilogue group has read the norms
             mbar_init(bar_full + 8 * s, 1);
-            mbar_init(bar_afree + 8 * s, 1 + N_NORM + N_EPI / Sh::GROUPS);
+            mbar_init(bar_afree + 8 * s, 1 + N_NORM + (DC == 256 ? 0 : N_EPI / Sh::GROUPS));
             mbar_init(bar_nrm + 8 * s, N_NORM);
         }
+        if (DC == 256)
+            for (int q = 0; q < NSQ_SLOTS; ++q) mbar_init(sbase + OFF_NRMBAR256 + 8 * q, N_NORM);
         for (int a = 0; a < ACC_STAGES; ++a) { mbar_init(bar_accfull + 8 * a, 1); mbar_init(bar_accfree + 8 * a, N_EPI / Sh::GROUPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    // head_dim 256: this CTA's slice of the columns, its width and its bytes of a packed row
+    const int slice = DC == 256 ? int(blockIdx.x & 3u) : 0;
+    const bool in_lo = DC == 256 && p.bits_lo != 0 && slice >= 2;
+    const int slice_bits = in_lo ? p.bits_lo : p.bits_hi;
+    const uint32_t tile0 = DC == 256 ? blockIdx.x >> 2 : blockIdx.x, tile_step = DC == 256 ? gridDim.x >> 2 : gridDim.x;
+    if constexpr (DC == 256) {
+        // operand rows: term t of slice row j at row 64 t + j, K-blocks of (64 TERMS) rows x 128 bytes
+        const int terms = bf16 ? 3 : 2, kb_bytes = terms * SLICE * 128;
+        unsigned char* rbase = smem + (bf16 ? OFF_R3 : OFF_R1);
+        for (int idx = tid; idx < SLICE * 32; idx += NT) {
+            const int j = idx >> 5, c = idx & 31, kblk = c >> 3, cc = c & 7;
+            const float* src = p.rot + (slice * SLICE + j) * 256 + c * 8;
+            const float4 f0 = __ldg(reinterpret_cast<const float4*>(src)), f1 = __ldg(reinterpret_cast<const float4*>(src + 4));
+            float v[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+            for (int t = 0; t < terms; ++t) {
+                __align__(16) uint16_t w[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if (bf16) {
+                        const __nv_bfloat16 h = __float2bfloat16_rn(v[i]);
+                        w[i] = __bfloat16_as_ushort(h);
+                        v[i] -= __bfloat162float(h);                          // exact
+                    } else {
+                        const __half h = __float2half_rn(v[i]);
+                        w[i] = __half_as_ushort(h);
+                        v[i] = (v[i] - __half2float(h)) * 2048.f;
+                    }
+                }
+                const int r = t * SLICE + j;
+                *reinterpret_cast<uint4*>(rbase + kblk * kb_bytes + r * 128 + ((cc ^ (r & 7)) << 4)) = *reinterpret_cast<const uint4*>(w);
+            }
+        }
+    } else
     // R -> operand tiles (swizzled K-major): B[n = j][k] = R[j][k], rows j < d, 16-byte chunks c < d / 8
     for (int idx = tid; idx < d * (d / 8); idx += NT) {
         const int j = idx / (d / 8), c = idx - j * (d / 8);      // row j, chunk c (8 elements) of the row
@@ -634,10 +703,10 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
         float* raw = reinterpret_cast<float*>(smem + OFF_BND);
         if (tid < 64) {
             const int which = tid >> 4, i = tid & 15;                    // 0 / 1: boundaries hi / lo, 2 / 3: centroids hi / lo
-            const int bits = (which & 1) ? p.bits_lo : p.bits_hi;
+            const int bits = DC == 256 ? slice_bits : (which & 1) ? p.bits_lo : p.bits_hi;
             float val = which < 2 ? INFINITY : 0.f;
             if (which < 2) {
-                const float* src = which ? p.bnd_lo : p.bnd_hi;
+                const float* src = (DC == 256 ? in_lo : which != 0) ? p.bnd_lo : p.bnd_hi;
                 if (src != nullptr && bits > 0 && i < (1 << bits) - 1) val = src[i];
             } else if (QJL) {
                 const float* src = (which & 1) ? p.cent_lo : p.cent_hi;
@@ -667,7 +736,7 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
             }
         }
         __syncthreads();
-        if (p.bits_hi == 4) build_bins(reinterpret_cast<float2*>(smem + OFF_BINS), raw, 15, tid, NT);
+        if ((DC == 256 ? slice_bits : p.bits_hi) == 4) build_bins(reinterpret_cast<float2*>(smem + OFF_BINS), raw, 15, tid, NT);
     }
     if (warp == EPI_WARPS) {              // one warp owns the TMEM allocation: 4 stages x 128 columns
         tmem_alloc(sbase + OFF_MISC, 512);
@@ -682,9 +751,29 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
 
     if (warp < EPI_WARPS) {
         // ======================= epilogue: row = 32 * (warp % 4) + lane; groups and column halves as in EpiShape =======================
-        EpiCtx e{p, smem, tmem_base, bar_accfull, bar_accfree, bar_afree, bar_nrm, abort_flag, warp, lane};
-        const int key = p.bits_hi * 8 + p.bits_lo;
-        switch (key) {
+        EpiCtx e{p, smem, tmem_base, bar_accfull, bar_accfree, bar_afree, bar_nrm, abort_flag, warp, lane, nullptr, 0, true};
+        if constexpr (DC == 256) {
+            const int coords = p.bits_lo ? 128 : 256;                      // of a packed row of this slice's width
+            e.nb = coords * slice_bits / 8;
+            e.dst = (in_lo ? p.p_lo : p.p_hi) + (slice * SLICE - (in_lo ? 128 : 0)) * slice_bits / 8;
+            e.write_norms = slice == 0;
+            if (bf16) {
+                switch (slice_bits) {
+                    case 4: epilogue_loop<4, 0, false, true, 256, 3>(e); break;
+                    case 3: epilogue_loop<3, 0, false, true, 256, 3>(e); break;
+                    case 2: epilogue_loop<2, 0, false, true, 256, 3>(e); break;
+                    default: epilogue_loop<1, 0, false, true, 256, 3>(e); break;
+                }
+            } else {
+                switch (slice_bits) {
+                    case 4: epilogue_loop<4, 0, false, true, 256, 2>(e); break;
+                    case 3: epilogue_loop<3, 0, false, true, 256, 2>(e); break;
+                    case 2: epilogue_loop<2, 0, false, true, 256, 2>(e); break;
+                    default: epilogue_loop<1, 0, false, true, 256, 2>(e); break;
+                }
+            }
+        } else
+        switch (p.bits_hi * 8 + p.bits_lo) {
             case 4 * 8 + 0: epilogue_loop<4, 0, QJL, SPLITACC, DC>(e); break;
             case 3 * 8 + 0: epilogue_loop<3, 0, QJL, SPLITACC, DC>(e); break;
             case 2 * 8 + 0: epilogue_loop<2, 0, QJL, SPLITACC, DC>(e); break;
@@ -696,6 +785,31 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
         }
     } else if (warp == EPI_WARPS) {
         // ======================= MMA issue: one elected thread =======================
+        if (DC == 256) {
+            if (lane == 0) {
+                const int terms = bf16 ? 3 : 2, kb_bytes = terms * SLICE * 128;
+                const uint32_t idesc = make_idesc(terms * SLICE, bf16), rb = sbase + (bf16 ? OFF_R3 : OFF_R1);
+                int it = 0, hit = 0;
+                bool ok = true;
+                for (int64_t tile = tile0; ok && tile < p.n_tiles; tile += tile_step, ++it) {
+                    const int a = it % ACCS;
+                    if (it >= ACCS && !mbar_wait(bar_accfree + 8 * a, uint32_t((it / ACCS) - 1) & 1u, abort_flag, 2)) break;
+                    for (int kh = 0; kh < 2; ++kh, ++hit) {
+                        const int s = hit % a_stages;
+                        ok = mbar_wait(bar_full + 8 * s, uint32_t(hit / a_stages) & 1u, abort_flag, 1);
+                        if (!ok) break;
+                        tc_fence_after();
+                        for (int ks = 0; ks < 8; ++ks) {
+                            const int kblk = kh * 2 + (ks >> 2);
+                            umma_f16(tmem_base + a * Sh::STAGE_COLS, smem_desc(sbase + OFF_A + s * OPER_BYTES, ks >> 2, ks & 3), smem_desc(rb + kblk * kb_bytes, 0, ks & 3), idesc,
+                                     (kh | ks) ? 1u : 0u);
+                        }
+                        umma_commit(bar_afree + 8 * s);
+                    }
+                    if (ok) umma_commit(bar_accfull + 8 * a);
+                }
+            }
+        } else
         if (lane == 0) {
             const uint32_t idesc = make_idesc(SPLITACC ? 2 * d : d, bf16);
             const int ksteps = d / 16;
@@ -740,6 +854,25 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
         __syncwarp();
     } else if (warp == EPI_WARPS + 1 + N_NORM / 32) {
         // ======================= TMA issue: one thread keeps the operand stages full =======================
+        if (DC == 256) {
+            if (lane == 0) {
+                const uint32_t tpl = uint32_t(p.tiles_per_lane);
+                int hit = 0;
+                bool ok = true;
+                for (int64_t tile = tile0; ok && tile < p.n_tiles; tile += tile_step) {
+                    const uint32_t t32 = uint32_t(tile), o = t32 / tpl, tl = t32 - o * tpl;
+                    for (int kh = 0; kh < 2 && ok; ++kh, ++hit) {
+                        const int s = hit % a_stages;
+                        if (hit >= a_stages) ok = mbar_wait(bar_afree + 8 * s, uint32_t((hit / a_stages) - 1) & 1u, abort_flag, 6);
+                        if (!ok) break;
+                        const uint32_t a_tile = sbase + OFF_A + s * OPER_BYTES;
+                        mbar_expect_tx(bar_full + 8 * s, OPER_BYTES);
+                        tma_load_3d(a_tile, &tmap, kh * 128, int(tl * TM), int(o), bar_full + 8 * s);
+                        tma_load_3d(a_tile + KBLK_BYTES, &tmap, kh * 128 + 64, int(tl * TM), int(o), bar_full + 8 * s);
+                    }
+                }
+            }
+        } else
         if (lane == 0) {
             const uint32_t tpl = uint32_t(p.tiles_per_lane);
             int it = 0;
@@ -759,12 +892,14 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
         // thread -> row 32 nw + lane, both 64-column blocks: eight consecutive rows hit eight different 16-byte columns
         // of the swizzled tile, so the 128-bit reads are free of bank conflicts
         const int nw = warp - (EPI_WARPS + 1), r = nw * 32 + lane;
-        int it = 0;
-        for (int64_t tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x, ++it) {
+        constexpr int KH = DC == 256 ? 2 : 1;
+        int it = 0;                                                        // operand stages so far: KH per tile
+        float a = 0.f, b = 0.f;
+        for (int64_t tile = tile0; tile < p.n_tiles; tile += (KH == 1 || (it & 1)) ? tile_step : 0, ++it) {
             const int s = it % a_stages;
             if (!mbar_wait(bar_full + 8 * s, uint32_t(it / a_stages) & 1u, abort_flag, 7)) break;
             const unsigned char* rowp = smem + OFF_A + s * OPER_BYTES + r * 128;
-            float a = 0.f, b = 0.f;
+            if (KH == 1 || !(it & 1)) a = b = 0.f;
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
                 const uint4 v = *reinterpret_cast<const uint4*>(rowp + ((c ^ (r & 7)) << 4));
@@ -790,9 +925,17 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
                     }
                 }
             }
+            if constexpr (DC == 256) {
+                if (it & 1) {
+                    const int q = (it >> 1) % NSQ_SLOTS;
+                    reinterpret_cast<float*>(smem + OFF_NSQ256)[q * TM + r] = a + b;
+                    mbar_arrive(sbase + OFF_NRMBAR256 + 8 * q);
+                }
+            } else {
             float* nsq = reinterpret_cast<float*>(smem + OFF_NSQ) + s * 2 * TM;
             nsq[r] = a; nsq[TM + r] = b;
             mbar_arrive(bar_nrm + 8 * s);        // release: the epilogue reads the sums after waiting on this barrier
+            }
             mbar_arrive(bar_afree + 8 * s);      // this thread is done reading the stage
         }
     }
@@ -811,13 +954,13 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
 
 using namespace tq;
 
-// Takes the call when it fits the tensor-core kernel: fp16 / bf16 rows, d in {64, 96, 128}, 16-byte aligned rows, no
+// Takes the call when it fits the tensor-core kernel: fp16 / bf16 rows, d in {64, 96, 128} or 256 without a sketch, 16-byte aligned rows, no
 // rotated-row output, a bit-width pair the epilogue is compiled for.  Otherwise reports "not handled" and the caller uses
 // the general CUDA-core kernel.
 int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled) {
     *handled = false;
     const int d = q->d;
-    if ((d != 64 && d != 96 && d != 128) || (q->x_dtype != TQ_F16 && q->x_dtype != TQ_BF16) || q->y_out) return TQ_OK;
+    if ((d != 64 && d != 96 && d != 128 && (d != 256 || q->qjl_bits)) || (q->x_dtype != TQ_F16 && q->x_dtype != TQ_BF16) || q->y_out) return TQ_OK;
     const bool frac = q->bits_lo != 0;
     if (frac && (q->bits_hi != q->bits_lo + 1)) return TQ_OK;                  // the reference's fractional widths only
     if (!aligned(q->x, 16) || q->x_row_stride % 8 || q->x_lane_stride % 8 || !aligned(q->rot, 16)) return TQ_OK;
@@ -838,6 +981,7 @@ int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled
     if (dev < 0 || dev >= 16) return TQ_OK;
     if (!attr_set[dev]) {
         cudaError_t e = cudaFuncSetAttribute(tc::quantize_tc_kernel<false, true, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(tc::quantize_tc_kernel<false, true, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(tc::quantize_tc_kernel<false, true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(tc::quantize_tc_kernel<false, false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(tc::quantize_tc_kernel<true, false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
@@ -876,8 +1020,9 @@ int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled
     p.rot = q->rot; p.bnd_hi = q->bnd_hi; p.bnd_lo = q->bnd_lo; p.bits_hi = q->bits_hi; p.bits_lo = q->bits_lo;
     p.p_hi = q->packed_hi; p.p_lo = q->packed_lo; p.norms = q->norms; p.out_lane_stride = q->out_lane_stride;
     p.qjl_proj_rot = q->qjl_proj_rot; p.cent_hi = q->cent_hi; p.cent_lo = q->cent_lo; p.qjl_bits = q->qjl_bits; p.qjl_gamma = q->qjl_gamma;
-    const unsigned grid = unsigned(std::min<int64_t>(p.n_tiles, sms[dev]));
-    if (qjl) tc::quantize_tc_kernel<true, false, 0><<<grid, tc::n_threads(true), tc::SMEM_BYTES, s>>>(p, tmap);
+    const unsigned grid = d == 256 ? 4 * unsigned(std::min<int64_t>(p.n_tiles, sms[dev] / 4)) : unsigned(std::min<int64_t>(p.n_tiles, sms[dev]));
+    if (d == 256) tc::quantize_tc_kernel<false, true, 256><<<grid, tc::n_threads(false), tc::SMEM_BYTES, s>>>(p, tmap);
+    else if (qjl) tc::quantize_tc_kernel<true, false, 0><<<grid, tc::n_threads(true), tc::SMEM_BYTES, s>>>(p, tmap);
     else if (p.bf16) tc::quantize_tc_kernel<false, false, 0><<<grid, tc::n_threads(false), tc::SMEM_BYTES, s>>>(p, tmap);
     else if (d == 128) tc::quantize_tc_kernel<false, true, 128><<<grid, tc::n_threads(false), tc::SMEM_BYTES, s>>>(p, tmap);
     else tc::quantize_tc_kernel<false, true, 0><<<grid, tc::n_threads(false), tc::SMEM_BYTES, s>>>(p, tmap);
