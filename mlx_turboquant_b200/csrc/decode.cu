@@ -765,15 +765,22 @@ int decode_prepare(const tq_decode_args* a, void* workspace, size_t workspace_by
     // The lookup kernel: everything else its tables cover (two to four bits, their fractional splits), and of the 4-bit-key /
     // 2-bit-value calls those that are not its rivals' best.  Per call:
     //   * table-lookup (direct) kernel: many lanes - 256 x 31 tiles 54.7 against 44.1 us, 384 x 62 72.7 / 42.7, 128 x 375 56.9 / 50.5;
-    //     few or short ones stay (16 x 1000 22.7 / 33.2, 64 x 94 21.9 / 25.9)
+    //     few or short ones stay (16 x 1000 22.7 / 33.2, 64 x 94 21.9 / 25.9).  Its uncompressed tokens cost more when they are
+    //     not fp16 (here bfloat16 rows feed the MMAs as they are): then from 64 lanes (128 x 109 50.8 / 37.5, 64 x 28 25.1 / 22.7)
     //   * streaming kernel: until its runs are long enough to pay for two partials per warp - 128 x 512 68.0 / 63.9, with sketches
-    //     64 x 500 72.8 / 51.5, 128 x 512 at d = 96 72 / 63; beyond it stays (128 x 1024 95.1 / 97.9)
+    //     64 x 500 72.8 / 51.5, 128 x 512 at d = 96 72 / 63; beyond it stays (128 x 1024 95.1 / 97.9) -
+    //     and while the uncompressed tokens are a large share, larger still when they are not fp16 (1632 x 56 131 / 121, bfloat16
+    //     247 / 128, 1024 x 234 222 / 182; 256 x 1000 161 / 179)
     //   * general kernel: d = 64 without sketches and few tiles, where it is one launch of little code (48 x 63 12.0 / 15.6,
     //     64 x 188 21.5 / 18.9); d = 96, d = 256 and sketches are faster here at any size (8 x 125 16.3 / 15.3, 36.8 / 31.6, 32.6 / 22.8)
     const int64_t kv_lanes = int64_t(a->batch) * a->n_kv_heads, tiles = kv_lanes * ((a->c_len + TILE - 1) / TILE);
     const bool bytes = a->c_len > 0 && a->k_bits_hi == 4 && !a->k_bits_lo && a->v_bits_hi == 2 && !a->v_bits_lo;
-    const bool lut_best = !bytes ? true : stream ? stp.range < g_tune_stream_min_run * 3 / 2 && kv_lanes <= 148 : direct ? kv_lanes >= 256 || (kv_lanes >= 64 && tiles >= 16000)
-                                                                                 : d != 64 || qjl || tiles >= 10000;
+    const bool fp16 = a->dense_dtype == TQ_F16;
+    const int64_t p_tiles = (a->c_len + TILE - 1) / TILE, d_tiles = (dense_len + TILE - 1) / TILE;
+    const bool lut_best = !bytes ? true
+        : stream ? (stp.range < g_tune_stream_min_run * 3 / 2 && kv_lanes <= 148) || p_tiles * 24 < (fp16 ? 6 : 37) * d_tiles * g_tune_stream_min_run
+        : direct ? kv_lanes >= (fp16 ? 256 : 64) || (kv_lanes >= 64 && tiles >= 16000)
+        : d != 64 || qjl || !fp16 || tiles >= 10000;
     bool lut = ((lut_best && g_tune_lut) || g_tune_lut == 2) && !g_tune_force_general && a->c_lane_stride % 16 == 0 && aligned(a->q, 8) &&
                aligned(a->k_hi, 16) && aligned(a->v_hi, 16) && aligned(a->k_norms, 16) && aligned(a->v_norms, 16) &&
                (!a->k_bits_lo || aligned(a->k_lo, 16)) && (!a->v_bits_lo || aligned(a->v_lo, 16)) &&
