@@ -41,27 +41,28 @@ namespace fa {
 
 constexpr uint32_t WAIT_LIMIT = 4u << 20;
 constexpr int ERR_WAIT = 111;
-constexpr int TM = 128, NSC = 4;                       // rows per query tile, tiles' norms in flight
+constexpr int TM = 128, NSC = 8;                       // rows per query tile, tiles' norms in flight
 
 template <int D> struct Plan {
     static constexpr int NQ = D == 256 ? 1 : 2;        // query tiles per CTA
-    static constexpr int TN = D == 256 ? 64 : 128;     // tokens per key tile
-    static constexpr int SB = NQ == 1 ? 2 : 1;         // score buffers per query tile
+    static constexpr int TN = 64;                      // tokens per key tile
+    static constexpr int SB = 2;                       // score buffers per query tile
+    static constexpr int ST = D == 256 ? 2 : 4;        // key tiles (and value tiles) in flight
     static constexpr int NBLK = (D + 63) / 64;         // 64-column blocks of a row
     static constexpr int DP = NBLK * 64;               // columns of O (d = 96: the last 32 are zeros)
-    static constexpr int NT = NQ * 128 + 64;           // softmax warps, MMA warp, TMA warp
+    static constexpr int NT = NQ * 128 + 96;           // softmax warps, MMA warp, a TMA warp for keys and norms, one for values
     static constexpr uint32_t QBLK = TM * 128u, KBLK = TN * 128u;            // bytes of a 64-column block
     static constexpr uint32_t Q_TILE = NBLK * QBLK, K_TILE = NBLK * KBLK;
-    static constexpr uint32_t OFF_Q = 0, OFF_K = NQ * Q_TILE, OFF_V = OFF_K + 2 * K_TILE;
-    static constexpr uint32_t OFF_SC = OFF_V + 2 * K_TILE;                   // float [NSC][2][TN]: key norms, value norms
+    static constexpr uint32_t OFF_Q = 0, OFF_K = NQ * Q_TILE, OFF_V = OFF_K + ST * K_TILE;
+    static constexpr uint32_t OFF_SC = OFF_V + ST * K_TILE;                  // float [NSC][2][TN]: key norms, value norms
     static constexpr uint32_t OFF_BAR = OFF_SC + NSC * 2 * TN * 4;
-    static constexpr uint32_t OFF_SLOT = OFF_BAR + 256;                      // [0] tensor-memory base, [1] abort
+    static constexpr uint32_t OFF_SLOT = OFF_BAR + 336;                      // [0] tensor-memory base, [1] abort
     static constexpr size_t NEED = OFF_SLOT + 16 + 1024, SMEM = NEED > 116 * 1024 ? NEED : 116 * 1024;      // one CTA per SM: it takes all of the tensor memory
     static constexpr uint32_t COL_O = NQ * SB * TN;                          // scores first, then the accumulators
     static_assert(COL_O + NQ * DP <= 512, "tensor memory");
     static_assert(SMEM <= 227 * 1024, "shared memory");
 };
-enum Bars { K_FULL = 0, K_FREE = 2, V_FULL = 4, V_FREE = 6, SC_FULL = 8, SC_FREE = 12, S_FULL = 16, P_FULL = 18, O_DONE = 20 };
+enum Bars { K_FULL = 0, K_FREE = 4, V_FULL = 8, V_FREE = 12, SC_FULL = 16, SC_FREE = 24, S_FULL = 32, P_FULL = 36, O_DONE = 40 };       // (42 of 8 bytes)
 
 struct Params {
     const void* q; int q_dtype; float f;               // scale * log2(e)
@@ -102,22 +103,24 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
+// The tensor core's instructions take their operands from uniform registers.  A whole warp in uniform control flow computes
+// them there and one elected lane issues; with a single thread in a divergent branch every operand is moved over one by one
+// (70 cycles per instruction: the issuing thread, not the products, was what the softmax warps waited for).
 // D = A.B (+ D when accumulate != 0), both operands through shared-memory descriptors
 __device__ __forceinline__ void umma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    const uint32_t zero = 0;
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(zero), "r"(zero), "r"(zero), "r"(zero) : "memory");
+    asm volatile("{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
 }
 // the same with A in tensor memory (two fp16 per 32-bit column)
 __device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    const uint32_t zero = 0;
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-                 ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(zero), "r"(zero), "r"(zero), "r"(zero) : "memory");
+    asm volatile("{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -187,7 +190,7 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(Params p, const __gr
     unsigned char* smem = smem_raw + (sbase - raw_addr);
     volatile uint32_t* slot = reinterpret_cast<volatile uint32_t*>(smem + P::OFF_SLOT);
     auto bar = [&](int which) -> uint32_t { return sbase + P::OFF_BAR + 8u * uint32_t(which); };
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);      // (uniform)
 
     // blockIdx.x = row block x split, the latest query rows (the longest runs of tiles) first
     const int n_blocks = gridDim.x / p.n_splits, split = blockIdx.x % p.n_splits, blk = n_blocks - 1 - int(blockIdx.x) / p.n_splits;
@@ -207,10 +210,11 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(Params p, const __gr
     const int t_lo = split * per, n = max(0, min(t_lo + per, n_all) - t_lo);
 
     if (tid == 0) {
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < 4; ++i) {
             mbar_init(bar(K_FULL + i), 1); mbar_init(bar(K_FREE + i), 1); mbar_init(bar(V_FULL + i), 1); mbar_init(bar(V_FREE + i), 1);
-            mbar_init(bar(S_FULL + i), 1); mbar_init(bar(P_FULL + i), 128); mbar_init(bar(O_DONE + i), 1);
+            mbar_init(bar(S_FULL + i), 1); mbar_init(bar(P_FULL + i), 128);
         }
+        for (int i = 0; i < 2; ++i) mbar_init(bar(O_DONE + i), 1);
         for (int i = 0; i < NSC; ++i) { mbar_init(bar(SC_FULL + i), 1); mbar_init(bar(SC_FREE + i), NQ * 128); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         slot[1] = 0u;
@@ -235,7 +239,7 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(Params p, const __gr
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = slot[0];
+    const uint32_t tmem = __shfl_sync(0xffffffffu, slot[0], 0);
 
     auto wait_bar = [&](int which, int phase) -> bool {
         const uint32_t addr = bar(which);
@@ -248,38 +252,48 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(Params p, const __gr
         return false;
     };
     // score buffer of (query tile q, key tile j) and the phase of its barriers
-    auto sbuf = [](int q, int j) { return NQ == 2 ? q : (j & 1); };
-    auto sph = [](int j) { return NQ == 2 ? j : (j >> 1); };
+    constexpr int SB = P::SB, ST = P::ST;
+    auto sbuf = [](int q, int j) { return q * SB + j % SB; };
+    auto sph = [](int j) { return j / SB; };
 
     if (warp == NQ * 4 + 1) {
-        // ======================= loads: one thread =======================
+        // ======================= keys and norms: one thread (a key tile is free as soon as its scores are computed, long before =====
+        // ======================= the value tile: each of the two rings is kept full by a thread of its own) =======================
         if (lane == 0) {
             const float* kn = p.kn + int64_t(lane_c) * p.ts;
             const float* vn = p.vn + int64_t(lane_c) * p.ts;
             for (int j = 0; j < n; ++j) {
-                const int row = (t_lo + j) * TN, s = j % NSC, st = j & 1;
+                const int row = (t_lo + j) * TN, s = j % NSC, st = j % ST;
+                if (j >= ST && !wait_bar(K_FREE + st, j / ST - 1)) break;
+                mbar_expect_tx(bar(K_FULL + st), P::K_TILE);
+                for (int x = 0; x < P::NBLK; ++x) tma_load_3d(sbase + P::OFF_K + st * P::K_TILE + x * P::KBLK, &kmap, x * 64, row, lane_c, bar(K_FULL + st));
                 if (j >= NSC && !wait_bar(SC_FREE + s, j / NSC - 1)) break;
                 const uint32_t sc = sbase + P::OFF_SC + s * 2 * TN * 4;
                 mbar_expect_tx(bar(SC_FULL + s), 2 * TN * 4);
                 bulk_g2s(sc, kn + row, TN * 4, bar(SC_FULL + s));
                 bulk_g2s(sc + TN * 4, vn + row, TN * 4, bar(SC_FULL + s));
-                if (j >= 2 && !wait_bar(K_FREE + st, (j >> 1) - 1)) break;
-                mbar_expect_tx(bar(K_FULL + st), P::K_TILE);
-                for (int x = 0; x < P::NBLK; ++x) tma_load_3d(sbase + P::OFF_K + st * P::K_TILE + x * P::KBLK, &kmap, x * 64, row, lane_c, bar(K_FULL + st));
-                if (j >= 2 && !wait_bar(V_FREE + st, (j >> 1) - 1)) break;
+            }
+        }
+        __syncwarp();
+    } else if (warp == NQ * 4 + 2) {
+        // ======================= values: one thread =======================
+        if (lane == 0) {
+            for (int j = 0; j < n; ++j) {
+                const int row = (t_lo + j) * TN, st = j % ST;
+                if (j >= ST && !wait_bar(V_FREE + st, j / ST - 1)) break;
                 mbar_expect_tx(bar(V_FULL + st), P::K_TILE);
                 for (int x = 0; x < P::NBLK; ++x) tma_load_3d(sbase + P::OFF_V + st * P::K_TILE + x * P::KBLK, &vmap, x * 64, row, lane_c, bar(V_FULL + st));
             }
         }
         __syncwarp();
     } else if (warp == NQ * 4) {
-        // ======================= MMA issue: one thread =======================
-        if (lane == 0 && n > 0) {
+        // ======================= MMA issue: one warp, uniform =======================
+        if (n > 0) {
             auto issue_qk = [&](int q, int j) {                    // S = Q K^T of key tile j
                 const uint32_t s = tmem + sbuf(q, j) * TN;
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks)
-                    umma_ss(s, desc_k(sbase + P::OFF_Q + q * P::Q_TILE, P::QBLK, ks), desc_k(sbase + P::OFF_K + (j & 1) * P::K_TILE, P::KBLK, ks),
+                    umma_ss(s, desc_k(sbase + P::OFF_Q + q * P::Q_TILE, P::QBLK, ks), desc_k(sbase + P::OFF_K + (j % ST) * P::K_TILE, P::KBLK, ks),
                             idesc_of(TN, false), ks > 0 ? 1u : 0u);
                 umma_commit(bar(S_FULL + sbuf(q, j)));
             };
@@ -287,32 +301,33 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(Params p, const __gr
                 const uint32_t a = tmem + sbuf(q, j) * TN;
 #pragma unroll
                 for (int ks = 0; ks < TN / 16; ++ks)
-                    umma_ts(tmem + P::COL_O + q * DP, a + ks * 8, desc_mn(sbase + P::OFF_V + (j & 1) * P::K_TILE, P::KBLK, ks), idesc_of(DP, true),
+                    umma_ts(tmem + P::COL_O + q * DP, a + ks * 8, desc_mn(sbase + P::OFF_V + (j % ST) * P::K_TILE, P::KBLK, ks), idesc_of(DP, true),
                             (j > 0 || ks > 0) ? 1u : 0u);
                 umma_commit(bar(O_DONE + q));
             };
+            auto wait_all = [&](int which, int phase) -> bool { return __all_sync(0xffffffffu, wait_bar(which, phase)); };
             bool ok = true;
-            for (int j = 0; j < min(n, P::SB) && ok; ++j) {
-                ok = wait_bar(K_FULL + (j & 1), 0);
+            for (int j = 0; j < min(n, SB) && ok; ++j) {
+                ok = wait_all(K_FULL + j % ST, 0);
                 if (!ok) break;
                 tc_fence_after();
                 for (int q = 0; q < NQ; ++q) issue_qk(q, j);
-                umma_commit(bar(K_FREE + (j & 1)));
+                umma_commit(bar(K_FREE + j % ST));
             }
             for (int j = 0; j < n && ok; ++j) {
-                ok = wait_bar(V_FULL + (j & 1), j >> 1);
-                const int jn = j + P::SB;                          // the key tile whose scores go where P of tile j sits now
+                ok = wait_all(V_FULL + j % ST, j / ST);
+                const int jn = j + SB;                             // the key tile whose scores go where P of tile j sits now
                 for (int q = 0; q < NQ && ok; ++q) {
-                    ok = wait_bar(P_FULL + sbuf(q, j), sph(j));
+                    ok = wait_all(P_FULL + sbuf(q, j), sph(j));
                     if (!ok) break;
                     tc_fence_after();
                     issue_pv(q, j);
-                    if (q == NQ - 1) umma_commit(bar(V_FREE + (j & 1)));
+                    if (q == NQ - 1) umma_commit(bar(V_FREE + j % ST));
                     if (jn < n) {                                  // (the tensor core takes one thread's products in order)
-                        if (q == 0) ok = wait_bar(K_FULL + (jn & 1), jn >> 1);
+                        if (q == 0) ok = wait_all(K_FULL + jn % ST, jn / ST);
                         if (!ok) break;
                         issue_qk(q, jn);
-                        if (q == NQ - 1) umma_commit(bar(K_FREE + (jn & 1)));
+                        if (q == NQ - 1) umma_commit(bar(K_FREE + jn % ST));
                     }
                 }
             }
@@ -428,6 +443,8 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(Params p, const __gr
         float l0, l1, l_sum;
         upk(add2(l2a, l2b), l0, l1);
         l_sum = l0 + l1;
+        // (the last scores only say that the products of tile n - 3 are done, and a parity wait may not run two phases ahead)
+        if (ok && n > 1) ok = wait_bar(O_DONE + q, n - 2);
         if (ok && n > 0) ok = wait_bar(O_DONE + q, n - 1);
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
