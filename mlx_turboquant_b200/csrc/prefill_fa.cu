@@ -56,13 +56,13 @@ template <int D> struct Plan {
     static constexpr uint32_t OFF_Q = 0, OFF_K = NQ * Q_TILE, OFF_V = OFF_K + ST * K_TILE;
     static constexpr uint32_t OFF_SC = OFF_V + ST * K_TILE;                  // float [NSC][2][TN]: key norms, value norms
     static constexpr uint32_t OFF_BAR = OFF_SC + NSC * 2 * TN * 4;
-    static constexpr uint32_t OFF_SLOT = OFF_BAR + 336;                      // [0] tensor-memory base, [1] abort
+    static constexpr uint32_t OFF_SLOT = OFF_BAR + 352;                      // [0] tensor-memory base, [1] abort
     static constexpr size_t NEED = OFF_SLOT + 16 + 1024, SMEM = NEED > 116 * 1024 ? NEED : 116 * 1024;      // one CTA per SM: it takes all of the tensor memory
     static constexpr uint32_t COL_O = NQ * SB * TN;                          // scores first, then the accumulators
     static_assert(COL_O + NQ * DP <= 512, "tensor memory");
     static_assert(SMEM <= 227 * 1024, "shared memory");
 };
-enum Bars { K_FULL = 0, K_FREE = 4, V_FULL = 8, V_FREE = 12, SC_FULL = 16, SC_FREE = 24, S_FULL = 32, P_FULL = 36, O_DONE = 40 };       // (42 of 8 bytes)
+enum Bars { K_FULL = 0, K_FREE = 4, V_FULL = 8, V_FREE = 12, SC_FULL = 16, SC_FREE = 24, S_FULL = 32, P_FULL = 36, O_DONE = 40, ALL_DONE = 42 };       // (44 of 8 bytes)
 
 struct Params {
     const void* q; int q_dtype; float f;               // scale * log2(e)
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(Params p, const __gr
             mbar_init(bar(K_FULL + i), 1); mbar_init(bar(K_FREE + i), 1); mbar_init(bar(V_FULL + i), 1); mbar_init(bar(V_FREE + i), 1);
             mbar_init(bar(S_FULL + i), 1); mbar_init(bar(P_FULL + i), 128);
         }
-        for (int i = 0; i < 2; ++i) mbar_init(bar(O_DONE + i), 1);
+        for (int i = 0; i < 2; ++i) { mbar_init(bar(O_DONE + i), 1); mbar_init(bar(ALL_DONE + i), 1); }
         for (int i = 0; i < NSC; ++i) { mbar_init(bar(SC_FULL + i), 1); mbar_init(bar(SC_FREE + i), NQ * 128); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         slot[1] = 0u;
@@ -304,6 +304,7 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(Params p, const __gr
                     umma_ts(tmem + P::COL_O + q * DP, a + ks * 8, desc_mn(sbase + P::OFF_V + (j % ST) * P::K_TILE, P::KBLK, ks), idesc_of(DP, true),
                             (j > 0 || ks > 0) ? 1u : 0u);
                 umma_commit(bar(O_DONE + q));
+                if (j == n - 1) umma_commit(bar(ALL_DONE + q));    // (a barrier of its own: a parity wait on O_DONE could be two phases early or one late)
             };
             auto wait_all = [&](int which, int phase) -> bool { return __all_sync(0xffffffffu, wait_bar(which, phase)); };
             bool ok = true;
@@ -443,9 +444,7 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(Params p, const __gr
         float l0, l1, l_sum;
         upk(add2(l2a, l2b), l0, l1);
         l_sum = l0 + l1;
-        // (the last scores only say that the products of tile n - 3 are done, and a parity wait may not run two phases ahead)
-        if (ok && n > 1) ok = wait_bar(O_DONE + q, n - 2);
-        if (ok && n > 0) ok = wait_bar(O_DONE + q, n - 1);
+        if (ok && n > 0) ok = wait_bar(ALL_DONE + q, 0);
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
         float* part = nullptr;
