@@ -111,15 +111,17 @@ __device__ __forceinline__ void tmem_relinquish() { asm volatile("tcgen05.relinq
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
+// (issued by one elected lane of a warp in uniform control flow: the operands then come straight from uniform registers, where a
+// single thread in a divergent branch moves each of them over, 70 cycles per instruction)
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    const uint32_t zero = 0;
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(zero), "r"(zero), "r"(zero), "r"(zero) : "memory");
+        "{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
@@ -434,7 +436,7 @@ __global__ void __launch_bounds__(NT, 1) dequantize_tc_kernel(const __grid_const
     unsigned char* smem = smem_raw + (sbase - raw_addr);
     volatile uint32_t* slot = reinterpret_cast<volatile uint32_t*>(smem + P::OFF_SLOT);
     auto bar = [&](int which) -> uint32_t { return sbase + P::OFF_BAR + 8u * uint32_t(which); };
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);      // (warp: uniform)
     // d = 256: CTAs with an even number own output columns 0 .. 127, the others 128 .. 255 of the same tiles
     constexpr int SPLIT = D == 256 ? 2 : 1;
     const int first = blockIdx.x / SPLIT, stride = gridDim.x / SPLIT, col_base = (blockIdx.x % SPLIT) * NC;
@@ -509,22 +511,23 @@ __global__ void __launch_bounds__(NT, 1) dequantize_tc_kernel(const __grid_const
         asm volatile("griddepcontrol.wait;" ::: "memory");
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
-    const uint32_t tmem_base = slot[0];
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, slot[0], 0);
 
     const Waiter wait_bar{sbase + P::OFF_BAR, slot, p.status};
     const int n_mine = p.n_tiles > first ? (p.n_tiles - first + stride - 1) / stride : 0;
 
     if (warp == MMA_W) {
-        // ======================= MMA issue: one thread =======================
-        if (lane == 0) {
+        // ======================= MMA issue: one warp, uniform =======================
+        {
+            auto wait_all = [&](int which, int phase) { return bool(__all_sync(0xffffffffu, wait_bar(which, phase))); };
             bool ok = true;
             for (int it = 0; it < n_mine && ok; ++it) {
                 const int st = it & 1;
                 const uint32_t acc = tmem_base + uint32_t(st) * 256u;
-                if (it >= 2) ok = wait_bar(ACC_FREE + st, (it >> 1) - 1);
+                if (it >= 2) ok = wait_all(ACC_FREE + st, (it >> 1) - 1);
                 for (int part = 0; part < p.parts && ok; ++part) {
                     const int s = it * p.parts + part, bf = s % P::NB;
-                    ok = wait_bar(A_FULL + bf, s / P::NB);
+                    ok = wait_all(A_FULL + bf, s / P::NB);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t a = sbase + P::OFF_A + bf * P::A_TILE;

@@ -142,23 +142,25 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
 // D = A.B (+ D when accumulate != 0)
+// (issued by one elected lane of a warp in uniform control flow: the operands then come straight from uniform registers, where a
+// single thread in a divergent branch moves each of them over, 70 cycles per instruction)
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    const uint32_t zero = 0;
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(zero), "r"(zero), "r"(zero), "r"(zero) : "memory");
+        "{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
 // D = A.B + 2^-11 D
 __device__ __forceinline__ void umma_f16_scaled11(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
-    const uint32_t zero = 0, one = 1;
+    const uint32_t one = 1;
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p, 11;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(one), "r"(zero), "r"(zero), "r"(zero), "r"(zero) : "memory");
+        "{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, 11;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(one) : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -596,7 +598,7 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
     constexpr int ACCS = Sh::STAGES, NT = Sh::NT, EPI_WARPS = Sh::EW, N_EPI = Sh::N_EPI;
     extern __shared__ __align__(1024) unsigned char smem[];
     const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // (warp: uniform)
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + OFF_MISC + 4);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_MISC);
     const int d = DC ? DC : p.d, a_stages = p.a_stages;
@@ -746,7 +748,7 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const uint32_t oper_bytes = d > 64 ? OPER_BYTES : KBLK_BYTES;        // bytes one tile's copies deliver
 
     if (warp < EPI_WARPS) {
@@ -785,18 +787,19 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
         }
     } else if (warp == EPI_WARPS) {
         // ======================= MMA issue: one elected thread =======================
+        auto wait_all = [&](uint32_t bar, uint32_t parity, volatile int* flag, int code) { return bool(__all_sync(0xffffffffu, mbar_wait(bar, parity, flag, code))); };
         if (DC == 256) {
-            if (lane == 0) {
+            {
                 const int terms = bf16 ? 3 : 2, kb_bytes = terms * SLICE * 128;
                 const uint32_t idesc = make_idesc(terms * SLICE, bf16), rb = sbase + (bf16 ? OFF_R3 : OFF_R1);
                 int it = 0, hit = 0;
                 bool ok = true;
                 for (int64_t tile = tile0; ok && tile < p.n_tiles; tile += tile_step, ++it) {
                     const int a = it % ACCS;
-                    if (it >= ACCS && !mbar_wait(bar_accfree + 8 * a, uint32_t((it / ACCS) - 1) & 1u, abort_flag, 2)) break;
+                    if (it >= ACCS && !wait_all(bar_accfree + 8 * a, uint32_t((it / ACCS) - 1) & 1u, abort_flag, 2)) break;
                     for (int kh = 0; kh < 2; ++kh, ++hit) {
                         const int s = hit % a_stages;
-                        ok = mbar_wait(bar_full + 8 * s, uint32_t(hit / a_stages) & 1u, abort_flag, 1);
+                        ok = wait_all(bar_full + 8 * s, uint32_t(hit / a_stages) & 1u, abort_flag, 1);
                         if (!ok) break;
                         tc_fence_after();
                         for (int ks = 0; ks < 8; ++ks) {
@@ -810,31 +813,21 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
                 }
             }
         } else
-        if (lane == 0) {
+        {
             const uint32_t idesc = make_idesc(SPLITACC ? 2 * d : d, bf16);
             const int ksteps = d / 16;
             int it = 0;
             for (int64_t tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x, ++it) {
                 const int a = it % ACCS, s = it % a_stages;
-                if (it >= ACCS && !mbar_wait(bar_accfree + 8 * a, uint32_t((it / ACCS) - 1) & 1u, abort_flag, 2)) break;
-                if (!mbar_wait(bar_full + 8 * s, uint32_t(it / a_stages) & 1u, abort_flag, 1)) break;
+                if (it >= ACCS && !wait_all(bar_accfree + 8 * a, uint32_t((it / ACCS) - 1) & 1u, abort_flag, 2)) break;
+                if (!wait_all(bar_full + 8 * s, uint32_t(it / a_stages) & 1u, abort_flag, 1)) break;
                 tc_fence_after();
                 const uint32_t a_tile = sbase + OFF_A + s * OPER_BYTES;
                 const uint32_t d_acc = tmem_base + a * Sh::STAGE_COLS;
                 if (SPLITACC) {
                     // columns [0, d): x.R_hi, columns [d, 2 d): 2^11 x.R_lo; the operand's K-blocks are 32 KB apart
-#ifdef EXP_TWO_MMA
-                    const uint32_t idesc1 = make_idesc(d, bf16);
-                    for (int ks = 0; ks < ksteps; ++ks) {
-                        const uint64_t da = smem_desc(a_tile, ks >> 2, ks & 3);
-                        const uint32_t rb = sbase + OFF_R1 + (ks >> 2) * KBLK_BYTES;
-                        umma_f16(d_acc, da, smem_desc(rb, ks >> 2, ks & 3), idesc1, ks ? 1u : 0u);
-                        umma_f16(d_acc + d, da, smem_desc(rb + d * 128, ks >> 2, ks & 3), idesc1, ks ? 1u : 0u);
-                    }
-#else
                     for (int ks = 0; ks < ksteps; ++ks)
                         umma_f16(d_acc, smem_desc(a_tile, ks >> 2, ks & 3), smem_desc(sbase + OFF_R1 + (ks >> 2) * KBLK_BYTES, ks >> 2, ks & 3), idesc, ks ? 1u : 0u);
-#endif
                 } else if (!bf16) {
                     for (int ks = 0; ks < ksteps; ++ks)            // 2^11-scaled low products first
                         umma_f16(d_acc, smem_desc(a_tile, ks >> 2, ks & 3), smem_desc(sbase + OFF_R2, ks >> 2, ks & 3), idesc, ks ? 1u : 0u);
