@@ -96,7 +96,7 @@ typedef struct {
 /* TurboQuantMSE.quantize / cache._quantize_kv(_fractional) (quantizer.py:54-85, cache.py:232-274);
  * metal_quantize_4bit (kernels.py:363-409). */
 int tq_quantize_pack(const tq_quantize_args* a, void* stream);
-/* n independent calls of the above, one after the other on the stream. */
+/* n independent calls of the above (their rows and results do not overlap): the launches may run side by side. */
 int tq_quantize_pack_many(const tq_quantize_args* a, int n, void* stream);
 
 /* The tensor-core quantize kernel (fp16 rows, d = 128) and the 4-bit-key / 2-bit-value decode kernel wait on

@@ -91,6 +91,7 @@ static_assert(NSQ_SLOTS * TM * 4 + NSQ_SLOTS * 8 <= DMAX * QM * 4, "head_dim 256
 
 struct Params {
     int d, bf16, a_stages;
+    int follows;                                 // runs beside the launch before it and ends after it
     int64_t n_rows, n_tiles, tiles_per_lane;     // tiles never cross cache lanes; tile = lane * tiles_per_lane + tile in lane
     const float* rot;
     const float* bnd_hi; const float* bnd_lo; int bits_hi, bits_lo;
@@ -603,6 +604,7 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_MISC);
     const int d = DC ? DC : p.d, a_stages = p.a_stages;
     const bool bf16 = p.bf16 != 0;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");        // (an independent job of the same call takes the SMs this one leaves idle)
     // barriers: full[3] (TMA -> MMA, norms), a_free[3] (MMA commit + norm warps + the epilogue's norm read -> TMA),
     //           nrm[3] (norm warps -> epilogue), acc_full[4] (MMA commit -> epilogue group), acc_free[4] (epilogue group -> MMA)
     const uint32_t bar_full = sbase + OFF_BAR, bar_afree = bar_full + 8 * A_STAGES_MAX, bar_nrm = bar_afree + 8 * A_STAGES_MAX;
@@ -610,6 +612,7 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
 
     if (sbase & 1023u) {                  // the swizzled operand tiles need 1024-byte alignment (uniform across the CTA)
         if (tid == 0) atomicCAS(&g_status, 0, 9);
+        if (p.follows) asm volatile("griddepcontrol.wait;" ::: "memory");
         return;
     }
     if (tid == 0) {
@@ -939,6 +942,7 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
         tc_fence_after();
         tmem_dealloc(tmem_base, 512);
     }
+    if (p.follows) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 }  // namespace tc
@@ -950,7 +954,7 @@ using namespace tq;
 // Takes the call when it fits the tensor-core kernel: fp16 / bf16 rows, d in {64, 96, 128} or 256 without a sketch, 16-byte aligned rows, no
 // rotated-row output, a bit-width pair the epilogue is compiled for.  Otherwise reports "not handled" and the caller uses
 // the general CUDA-core kernel.
-int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled) {
+int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled, bool follows) {
     *handled = false;
     const int d = q->d;
     if ((d != 64 && d != 96 && d != 128 && (d != 256 || q->qjl_bits)) || (q->x_dtype != TQ_F16 && q->x_dtype != TQ_BF16) || q->y_out) return TQ_OK;
@@ -1004,6 +1008,7 @@ int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled
     if (r != CUDA_SUCCESS) return TQ_OK;
 
     tc::Params p{};
+    p.follows = follows ? 1 : 0;
     p.d = d; p.bf16 = q->x_dtype == TQ_BF16 ? 1 : 0; p.a_stages = p.bf16 ? 2 : 3;
     p.n_rows = q->n_rows;
     p.tiles_per_lane = (q->n_rows + tc::TM - 1) / tc::TM;
@@ -1013,11 +1018,21 @@ int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled
     p.p_hi = q->packed_hi; p.p_lo = q->packed_lo; p.norms = q->norms; p.out_lane_stride = q->out_lane_stride;
     p.qjl_proj_rot = q->qjl_proj_rot; p.cent_hi = q->cent_hi; p.cent_lo = q->cent_lo; p.qjl_bits = q->qjl_bits; p.qjl_gamma = q->qjl_gamma;
     const unsigned grid = d == 256 ? 4 * unsigned(std::min<int64_t>(p.n_tiles, sms[dev] / 4)) : unsigned(std::min<int64_t>(p.n_tiles, sms[dev]));
-    if (d == 256) tc::quantize_tc_kernel<false, true, 256><<<grid, tc::n_threads(false), tc::SMEM_BYTES, s>>>(p, tmap);
-    else if (qjl) tc::quantize_tc_kernel<true, false, 0><<<grid, tc::n_threads(true), tc::SMEM_BYTES, s>>>(p, tmap);
-    else if (p.bf16) tc::quantize_tc_kernel<false, false, 0><<<grid, tc::n_threads(false), tc::SMEM_BYTES, s>>>(p, tmap);
-    else if (d == 128) tc::quantize_tc_kernel<false, true, 128><<<grid, tc::n_threads(false), tc::SMEM_BYTES, s>>>(p, tmap);
-    else tc::quantize_tc_kernel<false, true, 0><<<grid, tc::n_threads(false), tc::SMEM_BYTES, s>>>(p, tmap);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(unsigned(tc::n_threads(qjl)));
+    cfg.dynamicSmemBytes = tc::SMEM_BYTES;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = follows ? 1 : 0;
+    if (d == 256) cudaLaunchKernelEx(&cfg, tc::quantize_tc_kernel<false, true, 256>, p, tmap);
+    else if (qjl) cudaLaunchKernelEx(&cfg, tc::quantize_tc_kernel<true, false, 0>, p, tmap);
+    else if (p.bf16) cudaLaunchKernelEx(&cfg, tc::quantize_tc_kernel<false, false, 0>, p, tmap);
+    else if (d == 128) cudaLaunchKernelEx(&cfg, tc::quantize_tc_kernel<false, true, 128>, p, tmap);
+    else cudaLaunchKernelEx(&cfg, tc::quantize_tc_kernel<false, true, 0>, p, tmap);
     *handled = true;
     return check_launch("tq_quantize_pack (tensor core)");
 }

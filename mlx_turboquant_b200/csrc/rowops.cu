@@ -310,9 +310,13 @@ extern "C" int tq_rotate(const void* x, int x_dtype, const float* rot, float* ou
     return launch_rowops(a, static_cast<cudaStream_t>(stream), "tq_rotate");
 }
 
-int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled);
+int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled, bool follows);
 
-extern "C" int tq_quantize_pack(const tq_quantize_args* q, void* stream) {
+// follows: the launch before this one is a quantize of the same call on the tensor cores, and this one does not depend on it;
+// on return whether the next one may follow in turn.
+static int quantize_pack(const tq_quantize_args* q, void* stream, bool& follows) {
+    const bool after = follows;
+    follows = false;
     if (!q) return fail(TQ_ERR_INVALID, "tq_quantize_pack: null args");
     if (!d_ok(q->d)) return fail(TQ_ERR_UNSUPPORTED, "tq_quantize_pack: d=%d (need a multiple of 16 in 16..256)", q->d);
     if (!bits_ok(q->bits_hi) || (q->bits_lo && !bits_ok(q->bits_lo))) return fail(TQ_ERR_INVALID, "Unsupported bit-width: %d/%d. Use 1, 2, 3, or 4.", q->bits_hi, q->bits_lo);
@@ -326,7 +330,8 @@ extern "C" int tq_quantize_pack(const tq_quantize_args* q, void* stream) {
     if (q->qjl_bits && (!q->qjl_proj_rot || !q->qjl_gamma || !q->cent_hi || (q->bits_lo && !q->cent_lo))) return fail(TQ_ERR_INVALID, "tq_quantize_pack: QJL needs proj, gamma and centroids");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     bool handled = false;
-    int rc = tq_quantize_pack_tc(q, s, &handled);
+    int rc = tq_quantize_pack_tc(q, s, &handled, after);
+    follows = handled;
     if (handled) return rc;
     RowArgs a{};
     a.mode = MODE_QUANT; a.d = q->d; a.n_lanes = q->n_lanes; a.n_rows = q->n_rows;
@@ -338,10 +343,18 @@ extern "C" int tq_quantize_pack(const tq_quantize_args* q, void* stream) {
     return launch_rowops(a, s, "tq_quantize_pack");
 }
 
+extern "C" int tq_quantize_pack(const tq_quantize_args* q, void* stream) {
+    bool follows = false;
+    return quantize_pack(q, stream, follows);
+}
+
 extern "C" int tq_quantize_pack_many(const tq_quantize_args* q, int n, void* stream) {
     if (n < 0 || (n > 0 && !q)) return fail(TQ_ERR_INVALID, "tq_quantize_pack_many: null args");
+    // keys and values, buffered and new rows: each is a launch of few tiles in a decode loop or a prefill piece; every one but the
+    // first may start while the one before it still runs
+    bool follows = false;
     for (int i = 0; i < n; ++i)
-        if (int rc = tq_quantize_pack(q + i, stream)) return rc;
+        if (int rc = quantize_pack(q + i, stream, follows)) return rc;
     return TQ_OK;
 }
 
