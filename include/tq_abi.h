@@ -99,9 +99,9 @@ int tq_quantize_pack(const tq_quantize_args* a, void* stream);
 /* n independent calls of the above (their rows and results do not overlap): the launches may run side by side. */
 int tq_quantize_pack_many(const tq_quantize_args* a, int n, void* stream);
 
-/* The tensor-core quantize kernel (fp16 rows, d = 128) and the 4-bit-key / 2-bit-value decode kernel wait on
+/* The tensor-core kernels (quantize, dequantize, several-query attention) and the decode kernels wait on
  * mbarriers with an iteration limit; if a wait ever runs out the kernel drains and finishes, and this returns the
- * code of the first such wait on the current device (quantize 1-9, decode 101-103 and 106-108, several-query-token attention 104, dequantize 105, gather wait 201; 0 = none).  Synchronises the
+ * code of the first such wait on the current device (quantize 1-9, decode 101-103 and 106-110, several-query-token attention 104 and 111, dequantize 105, gather wait 201; 0 = none).  Synchronises the
  * device; no reference counterpart. */
 int tq_device_status(void);
 /* Back to 0 (after the caller has dealt with a reported time-out). */
@@ -338,6 +338,7 @@ float tq_fp16_table_scale(const float* centroids_host, int n);
  *   "decode_stream" 0/1 (the persistent streaming kernel for 4-bit keys / 2-bit values at d = 96 / 128 may be chosen, default, or never),
  *   "decode_stream_min_run" 1.. (fewest packed 16-token tiles per warp of the persistent grid for which it is chosen over the
  *   table-lookup kernel, default 24; over the general kernel a third of that),
+ *   "decode_lut" 0/1/2 (the lookup kernel is never chosen, where it is the faster one, default, or whenever it can run),
  *   "decode_stream_max_parts" 1..64 (most partial results per lane with which it is chosen over the table-lookup kernel; default 40).
  * Changing them changes tq_decode_workspace_bytes for the same sizes. */
 int tq_set_tuning(const char* key, int value);
@@ -345,7 +346,8 @@ int tq_set_tuning(const char* key, int value);
 /* Which kernel tq_decode_attn would run for these arguments under the current tuning (no launch; no reference counterpart):
  * 0 = general kernel (any width, d = 64 / 96 / 128 / 256), 1 = table-lookup kernel (4-bit keys / 2-bit values, d = 128: one CTA
  * per (sequence, KV head, split)), 2 = streaming kernel (the same widths at d = 96 / 128, sign sketches allowed: persistent
- * grid, chosen when the packed tokens of all lanes give every warp a long run).  Negative: the arguments are invalid
+ * grid, chosen when the packed tokens of all lanes give every warp a long run), 3 = lookup kernel (2 to 4 bits and the splits
+ * 4 | 3 and 3 | 2, d = 64 / 96 / 128 / 256, sign sketches allowed).  Negative: the arguments are invalid
  * (tq_last_error has the text). */
 int tq_decode_kernel_choice(const tq_decode_args* a);
 

@@ -14,7 +14,7 @@
 // Persistent CTAs (one per SM) walk the 128-row tiles, 17 warps:
 //   * warps 8-15 turn a tile's codes into fp16 A tiles (high parts, then low parts;
 //     K-major, 128-byte swizzle) in a ring of buffers and stage the rows' norms, offsets, sign words;
-//   * one thread of warp 16 issues the tcgen05.mma: c_hi [R_hi | R_lo] as one product per K step, then c_lo R_hi, into
+//   * warp 16 (in uniform control flow, one elected lane) issues the tcgen05.mma: c_hi [R_hi | R_lo] as one product per K step, then c_lo R_hi, into
 //     accumulator pair t & 1 - R sits in shared memory as MN-major B tiles built once per CTA (d = 256: a CTA owns 128 of
 //     the output columns);
 //   * warps 0-7 (two groups of four, alternating tiles) read both accumulators, a row per thread, combine, scale and stage
@@ -26,8 +26,8 @@
 // products (0.4 us of a tile's 2.6 at d = 128) nor by memory (1.7 us).  Eight producer warps: with four, one per scheduler,
 // the chains of a chunk do not overlap (166 us).  Measured at 134 million coordinates, float32 / fp16 results, against the
 // four-warp table-lookup kernel before (d = 256 and sketches: the row kernel):
-//   d = 128: 4 bits 146 / 133 us (163 / 150), 3.5 bits 146 / 134 (326 / 314), 3 bits 152 / 150 (165 / 156), 2 bits 137 / 122 (162 / 140)
-//   d = 64: 4 bits 171 / 165 (228 / 215), 3.5 bits 182 / 176 (524 / 523);  d = 256: 4 bits 349 / 346 (3804 / 3793)
+//   d = 128: 4 bits 132 / 118 us (163 / 150), 3.5 bits 138 / 122 (326 / 314), 3 bits 145 / 136 (165 / 156), 2 bits 128 / 108 (162 / 140)
+//   d = 64: 4 bits 177 / 173 (228 / 215), 3.5 bits 185 / 178 (524 / 523);  d = 256: 4 bits 300 / 289 (3804 / 3793)
 #pragma once
 
 #include <cuda.h>

@@ -1,4 +1,4 @@
-// Fused quantize kernel on the 5th-generation tensor cores (tcgen05 + TMEM) for fp16 / bf16 rows with d in {64, 96, 128}:
+// Fused quantize kernel on the 5th-generation tensor cores (tcgen05 + TMEM) for fp16 / bf16 rows with d in {64, 96, 128, 256}:
 //   norm -> rotation (128 rows x d x d contraction per tile) -> Lloyd-Max boundary search -> bit-pack (+ QJL sketch).
 //
 // The rotation has to be float32-accurate (a code flips whenever a rotated value crosses a boundary), so the rows are
@@ -25,7 +25,7 @@
 //                outcome bits straight into the packed word; at 4 bits one lookup in a 513-bin table (bin -> nearest
 //                boundary + count below; see build_bins).  Fractional widths: the threads of a row take chunks of
 //                either width, so they finish together.
-//   warp  E      allocates TMEM, issues the MMAs (one elected thread) and commits them to mbarriers
+//   warp  E      allocates TMEM, issues the MMAs (in uniform control flow, one elected lane) and commits them to mbarriers
 //   next four    norms: read each tile back from shared memory for the rows' sums of squares
 //   last warp    one thread keeps the operand stages full with tiled TMA copies (cp.async.bulk.tensor, 3-D tensor map
 //                (column, row, lane), 128-byte swizzle as the MMA descriptors expect; rows past a lane's end and
@@ -35,7 +35,7 @@
 // columns in two halves of one operand stage each; all terms of R sit side by side in ONE operand (fp16: [R_hi | R_lo],
 // bf16: [R_1 | R_2 | R_3], N = 128 / 192), because sixteen dependent MMAs take the same time at any width, and the epilogue
 // adds the accumulators.  The rows' norms have slots of their own, so that stages are free as soon as the MMAs have read
-// them.  A tile is fetched from memory once and three times from L2.  (524,288 rows at 4 bits: 4602 us in the CUDA-core row kernel before, 230 here; 3.5 bits 4576 / 255, bf16 4595 / 256.)
+// them.  A tile is fetched from memory once and three times from L2.  (524,288 rows at 4 bits: 4602 us in the CUDA-core row kernel before, 244 here; 3.5 bits 4576 / 254, bf16 4595 / 252.)
 // Every mbarrier wait is bounded: on a timeout the kernel raises a status word, drains and frees its TMEM.
 #include <algorithm>
 #include <cstdlib>
