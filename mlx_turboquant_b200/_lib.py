@@ -186,9 +186,10 @@ def launch(dev: torch.device, name: str, *args) -> int:
     shared-memory plan, static scratch) are keyed on it; tensors on ``cuda:1`` handed over while ``cuda:0`` is current
     would be dereferenced on the wrong GPU.  ``stream`` arguments must already belong to ``dev`` (``stream_ptr(dev)``).
     """
-    fn = getattr(_lib or lib(), name)
-    idx = dev.index if dev.index is not None else torch.cuda.current_device()
-    if idx == _cuda_device():
+    fn = getattr(lib(), name)
+    current = torch.cuda.current_device()
+    idx = dev.index if dev.index is not None else current
+    if idx == current:
         return fn(*args)
     with torch.cuda.device(idx):
         return fn(*args)
