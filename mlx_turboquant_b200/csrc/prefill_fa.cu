@@ -617,12 +617,12 @@ template <int D> static Layout layout(int n_lanes, int G, int64_t total, int t_q
     l.QT = TM / l.GP;
     l.n_blocks = (t_q + P::NQ * l.QT - 1) / (P::NQ * l.QT);
     l.ts = int((total + 127) / 128 * 128);
-    // key ranges per row block: as many as shorten the whole launch, a CTA costing its tiles and some four more for set-up,
-    // first scores and the partials
+    // key ranges per row block: as many as shorten the whole launch, a CTA costing its tiles and some twelve more for set-up,
+    // first scores and the partials (with four, 512 queries x 32 lanes over 16,384 tokens were split for a merge of 34 us and no gain)
     const int64_t tiles = (total + P::TN - 1) / P::TN, ctas = int64_t(l.n_blocks) * n_lanes * hg, sms = sm_count();
     double best = 0.0;
     for (int s = 1; s <= 16 && (s == 1 || tiles >= 2 * s); ++s) {
-        const double t = double((ctas * s + sms - 1) / sms) * (double((tiles + s - 1) / s) + 4.0) + (s > 1 ? 3.0 : 0.0);
+        const double t = double((ctas * s + sms - 1) / sms) * (double((tiles + s - 1) / s) + 12.0) + (s > 1 ? 8.0 : 0.0);
         if (s == 1 || t < best) { best = t; l.n_splits = s; }
     }
     const size_t rows = size_t(n_lanes) * l.ts;
