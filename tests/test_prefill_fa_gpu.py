@@ -1,0 +1,55 @@
+"""The two-step attention for several query tokens where its tiles can go wrong: key counts around multiples of 64 and 128, query
+counts around a block's rows, key ranges split over CTAs, every head_dim, lanes done in rounds for want of workspace.  Reference:
+float32 attention over the cache's dense rows."""
+
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(d, b, hq, hkv, t, tq, dtype, kb=3.5, vb=4):
+    from mlx_turboquant_b200 import TurboQuantKVCache
+    g = torch.Generator(device="cuda").manual_seed(d + t + tq)
+    c = TurboQuantKVCache(head_dim=d, num_kv_heads=hkv, key_bits=kb, value_bits=vb, residual_window=16, fp16_sink_size=5)
+    k, v = (torch.randn(b, hkv, t, d, device="cuda", generator=g) for _ in range(2))
+    k, v = k.to(dtype), (v * torch.exp(torch.randn(b, hkv, t, 1, device="cuda", generator=g))).to(dtype)
+    q = (torch.randn(b, hq, tq, d, device="cuda", generator=g) / d ** 0.5).to(dtype)
+    dk, dv = (x.float().repeat_interleave(hq // hkv, 1) for x in c.update_and_fetch(k, v))
+    s = (q.float() @ dk.transpose(-1, -2)) * d ** -0.5
+    pos = torch.arange(t, device="cuda")
+    s = s.masked_fill(pos[None, :] > (t - tq + torch.arange(tq, device="cuda"))[:, None], float("-inf"))
+    return c, q, torch.softmax(s, -1) @ dv
+
+
+def _check(out, ref):
+    from mlx_turboquant_b200 import _lib
+    err = float((out.float() - ref).abs().max() / ref.abs().max())
+    assert err < 1e-3, err
+    assert _lib.lib().tq_device_status() == 0
+
+
+@pytest.mark.parametrize("d", (64, 96, 128, 256))
+@pytest.mark.parametrize("dtype", (torch.float16, torch.bfloat16))
+@pytest.mark.parametrize("b,hq,hkv,t,tq", ((1, 4, 4, 64, 2), (2, 4, 2, 65, 65), (1, 8, 1, 127, 33), (1, 8, 2, 129, 64), (2, 16, 1, 1500, 3), (1, 4, 4, 3001, 257),
+                                            (3, 12, 4, 640, 129)))
+def test_tile_and_block_edges(d, dtype, b, hq, hkv, t, tq):
+    c, q, ref = _case(d, b, hq, hkv, t, tq, dtype)
+    _check(c.attend(q, out_dtype=torch.float32), ref)
+
+
+@pytest.mark.parametrize("d", (64, 128, 256))
+def test_lanes_in_rounds(d):
+    from mlx_turboquant_b200 import _lib
+    c, q, ref = _case(d, 3, 8, 4, 700, 40, torch.float16, 4, 2)
+    out = torch.empty(3, 8, 40, d, device="cuda")
+    a = c._fill_decode_args(3, 8, q.dtype, out.dtype, None)
+    a.q, a.out, a.c_len, a.sink_len, a.res_len = q.data_ptr(), out.data_ptr(), c._compressed_len, c._sink_len, c._fp16_len
+    need = _lib.lib().tq_prefill_workspace_bytes(1, 2, 1, d, 700, 40)        # one lane's
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+    a.workspace, a.workspace_bytes = ws.data_ptr(), need
+    _lib.check(_lib.lib().tq_prefill_attn(C.byref(a), 40, torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    _check(out, ref)
