@@ -75,3 +75,11 @@ def test_decode_steps_append_and_attend(dtype):
         assert torch.equal(o1, c2.attend(q))
     assert torch.equal(c1.keys[:, :, :c1._fp16_len], c2.keys[:, :, :c2._fp16_len])
     assert np.isfinite(host(o1.float())).all()
+
+
+@pytest.mark.parametrize("d,b,hq,hkv,t,qjl,bf16", ((128, 64, 8, 4, 90, False, False), (128, 16, 8, 4, 120, False, True), (96, 2, 8, 4, 300, False, False),
+                                                   (256, 1, 8, 2, 300, False, False), (128, 2, 8, 4, 250, True, False), (64, 2, 4, 2, 200, False, True)))
+def test_four_and_two_bits_where_this_kernel_is_the_faster_one(oracle, d, b, hq, hkv, t, qjl, bf16):
+    rs = np.random.RandomState(d + b)
+    c, q, ref = _case(oracle, rs, b, hq, hkv, t, d, 4, 2, 32, 8, qjl=qjl, bf16=bf16)
+    _run(c, q, ref)
