@@ -609,7 +609,9 @@ struct Layout {
     int GP, QT, n_blocks, n_splits, ts;
     size_t k, v, kn, vn, part, bytes;
 };
-template <int D> static Layout layout(int n_lanes, int G, int64_t total, int t_q) {
+// n_splits 0: chosen here, for a call (or its first round); a later round of fewer lanes keeps the first one's: left to itself it may
+// choose more ranges, whose partials can outweigh the rows it saves (13 sequences of 120,026 tokens at d = 128: 711 MB of 537).
+template <int D> static Layout layout(int n_lanes, int G, int64_t total, int t_q, int n_splits = 0) {
     using P = Plan<D>;
     Layout l{};
     const int g = std::min(G, HPG), hg = (G + HPG - 1) / HPG;
@@ -621,7 +623,8 @@ template <int D> static Layout layout(int n_lanes, int G, int64_t total, int t_q
     // first scores and the partials (with four, 512 queries x 32 lanes over 16,384 tokens were split for a merge of 34 us and no gain)
     const int64_t tiles = (total + P::TN - 1) / P::TN, ctas = int64_t(l.n_blocks) * n_lanes * hg, sms = sm_count();
     double best = 0.0;
-    for (int s = 1; s <= 16 && (s == 1 || tiles >= 2 * s); ++s) {
+    l.n_splits = n_splits;
+    for (int s = 1; n_splits == 0 && s <= 16 && (s == 1 || tiles >= 2 * s); ++s) {
         const double t = double((ctas * s + sms - 1) / sms) * (double((tiles + s - 1) / s) + 12.0) + (s > 1 ? 8.0 : 0.0);
         if (s == 1 || t < best) { best = t; l.n_splits = s; }
     }
@@ -642,13 +645,29 @@ template <int D> static size_t workspace(int lanes, int G, int64_t total, int t_
     return std::max(std::min(all, WS_CAP), one);
 }
 
+// The rounds of a call with ws_bytes of workspace: cache lanes of a round (the last one may have fewer) and key ranges of all of them.
+template <int D> static int first_round(int lanes, int G, int64_t total, int t_q, size_t ws_bytes, int& n_splits) {
+    int chunk = lanes;
+    while (chunk > 1 && layout<D>(chunk, G, total, t_q).bytes > ws_bytes) chunk = (chunk + 1) / 2;
+    n_splits = layout<D>(chunk, G, total, t_q).n_splits;
+    return chunk;
+}
+
+template <int D> static size_t most_used(int lanes, int G, int64_t total, int t_q, size_t ws_bytes) {
+    int n_splits;
+    const int chunk = first_round<D>(lanes, G, total, t_q, ws_bytes, n_splits);
+    size_t most = 0;
+    for (int lane0 = 0; lane0 < lanes; lane0 += chunk) most = std::max(most, layout<D>(std::min(chunk, lanes - lane0), G, total, t_q, n_splits).bytes);
+    return most;
+}
+
 template <int D> static int run(const DecodeParams& c, const void* q, int q_dtype, void* out, int out_dtype, int t_q, int64_t q_pos0, unsigned char* ws,
                                 size_t ws_bytes, cudaStream_t s) {
     using P = Plan<D>;
     const int64_t total = c.sink_len + c.c_len + c.res_len;
     const int lanes = c.B * c.Hkv;
-    int chunk = lanes;
-    while (chunk > 1 && layout<D>(chunk, c.G, total, t_q).bytes > ws_bytes) chunk = (chunk + 1) / 2;
+    int n_splits;
+    const int chunk = first_round<D>(lanes, c.G, total, t_q, ws_bytes, n_splits);
     static std::atomic<bool> set[64];
     int dev = 0;
     cudaGetDevice(&dev);
@@ -659,7 +678,8 @@ template <int D> static int run(const DecodeParams& c, const void* q, int q_dtyp
     }
     for (int lane0 = 0; lane0 < lanes; lane0 += chunk) {
         const int n = std::min(chunk, lanes - lane0);
-        const Layout l = layout<D>(n, c.G, total, t_q);
+        const Layout l = layout<D>(n, c.G, total, t_q, n_splits);
+        if (l.bytes > ws_bytes) return fail(TQ_ERR_INVALID, "tq_prefill_attn: workspace %zu B < %zu B", ws_bytes, l.bytes);
         __half* k = reinterpret_cast<__half*>(ws + l.k);
         __half* v = reinterpret_cast<__half*>(ws + l.v);
         float* kn = reinterpret_cast<float*>(ws + l.kn);
@@ -755,4 +775,15 @@ int launch_prefill_fa(const DecodeParams& c, const void* q, int q_dtype, void* o
 
 extern "C" size_t tq_prefill_workspace_bytes(int batch, int n_q_heads, int n_kv_heads, int d, int64_t total_len, int t_q) {
     return tq::prefill_fa_workspace(batch, n_q_heads, n_kv_heads, d, total_len, t_q);
+}
+
+extern "C" size_t tq_prefill_workspace_used(int batch, int n_q_heads, int n_kv_heads, int d, int64_t total_len, int t_q, size_t workspace_bytes) {
+    using namespace tq;
+    if (prefill_fa_workspace(batch, n_q_heads, n_kv_heads, d, total_len, t_q) == 0 ||
+        workspace_bytes < prefill_fa_workspace(1, n_q_heads / n_kv_heads, 1, d, total_len, t_q)) return 0;
+    const int lanes = batch * n_kv_heads, g = n_q_heads / n_kv_heads;
+    if (d == 64) return fa::most_used<64>(lanes, g, total_len, t_q, workspace_bytes);
+    if (d == 96) return fa::most_used<96>(lanes, g, total_len, t_q, workspace_bytes);
+    if (d == 128) return fa::most_used<128>(lanes, g, total_len, t_q, workspace_bytes);
+    return fa::most_used<256>(lanes, g, total_len, t_q, workspace_bytes);
 }

@@ -41,13 +41,15 @@ def test_tile_and_block_edges(d, dtype, b, hq, hkv, t, tq):
 
 
 @pytest.mark.parametrize("d", (64, 128, 256))
-def test_lanes_in_rounds(d):
+@pytest.mark.parametrize("b,hkv,lent", ((3, 4, 1), (5, 2, 3)))              # one lane at a time; three at a time, the last round has one
+def test_lanes_in_rounds(d, b, hkv, lent):
     from mlx_turboquant_b200 import _lib
-    c, q, ref = _case(d, 3, 8, 4, 700, 40, torch.float16, 4, 2)
-    out = torch.empty(3, 8, 40, d, device="cuda")
-    a = c._fill_decode_args(3, 8, q.dtype, out.dtype, None)
+    c, q, ref = _case(d, b, 2 * hkv, hkv, 700, 40, torch.float16, 4, 2)
+    out = torch.empty(b, 2 * hkv, 40, d, device="cuda")
+    a = c._fill_decode_args(b, 2 * hkv, q.dtype, out.dtype, None)
     a.q, a.out, a.c_len, a.sink_len, a.res_len = q.data_ptr(), out.data_ptr(), c._compressed_len, c._sink_len, c._fp16_len
-    need = _lib.lib().tq_prefill_workspace_bytes(1, 2, 1, d, 700, 40)        # one lane's
+    need = _lib.lib().tq_prefill_workspace_bytes(lent, 2, 1, d, 700, 40)
+    assert need < _lib.lib().tq_prefill_workspace_bytes(b, 2 * hkv, hkv, d, 700, 40)
     ws = torch.empty(need, dtype=torch.uint8, device="cuda")
     a.workspace, a.workspace_bytes = ws.data_ptr(), need
     _lib.check(_lib.lib().tq_prefill_attn(C.byref(a), 40, torch.cuda.current_stream().cuda_stream))
