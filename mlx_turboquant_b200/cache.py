@@ -100,7 +100,9 @@ class _Side:
         if x.dtype not in _lib._DTYPES:
             x = x.to(torch.float32)
         st = x.stride()
-        if st[3] != 1 or (b > 1 and h > 1 and st[0] != h * st[1]):
+        # (one stride per lane and per row; an expanded axis, stride 0, is laid out: the tensor-core kernel does not take it)
+        if (st[3] != 1 or (b > 1 and h > 1 and st[0] != h * st[1]) or (h > 1 and st[1] == 0) or (b > 1 and st[0] == 0)
+                or (t > 1 and st[2] == 0)):
             x = x.contiguous()
             st = x.stride()
         C.memmove(C.addressof(a), self.q_block, len(self.q_block))

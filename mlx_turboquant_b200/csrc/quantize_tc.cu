@@ -961,6 +961,7 @@ int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled
     const bool frac = q->bits_lo != 0;
     if (frac && (q->bits_hi != q->bits_lo + 1)) return TQ_OK;                  // the reference's fractional widths only
     if (!aligned(q->x, 16) || q->x_row_stride % 8 || q->x_lane_stride % 8 || !aligned(q->rot, 16)) return TQ_OK;
+    if ((q->n_rows > 1 && q->x_row_stride <= 0) || (q->n_lanes > 1 && q->x_lane_stride <= 0)) return TQ_OK;     // the same rows again and again: no tensor map
     if (q->n_rows >= (int64_t(1) << 31) || q->n_lanes >= (int64_t(1) << 31)) return TQ_OK;
     static int disabled = -1;
     if (disabled < 0) {
@@ -999,7 +1000,9 @@ int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled
     // the 128-byte-swizzled layout the MMA descriptors describe; rows past a lane's end and columns past d read as zeros.
     CUtensorMap tmap{};
     const cuuint64_t dims[3] = {cuuint64_t(d), cuuint64_t(q->n_rows), cuuint64_t(q->n_lanes)};
-    const cuuint64_t strides[2] = {cuuint64_t(q->x_row_stride) * 2, cuuint64_t(q->x_lane_stride ? q->x_lane_stride : q->x_row_stride * q->n_rows) * 2};   // bytes, multiples of 16
+    // bytes, multiples of 16 (a single row or lane: any stride will do)
+    const int64_t row_stride = q->n_rows > 1 ? q->x_row_stride : d, lane_stride = q->n_lanes > 1 ? q->x_lane_stride : row_stride * q->n_rows;
+    const cuuint64_t strides[2] = {cuuint64_t(row_stride) * 2, cuuint64_t(lane_stride) * 2};
     const cuuint32_t box[3] = {64, cuuint32_t(tc::TM), 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = encode(&tmap, q->x_dtype == TQ_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(q->x),

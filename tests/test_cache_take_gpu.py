@@ -53,3 +53,18 @@ def test_newcomers_of_another_dtype_take_the_buffers():
     c.update(x[:, :, :10].half(), x[:, :, :10].half())
     c.update(x[:, :, 10:60], x[:, :, 10:60])
     assert c.keys.dtype == torch.float16 and torch.equal(c.keys[:, :, :c._fp16_len], x[:, :, 44:60].half())
+
+
+@pytest.mark.parametrize("d", (64, 128, 256))
+@pytest.mark.parametrize("axis", (0, 1))
+def test_expanded_newcomers_equal_their_copies(d, axis):
+    from mlx_turboquant_b200 import TurboQuantKVCache, kernels
+    shape, full = ((1, 1, 300, d), (3, 1, 300, d) if axis == 0 else (1, 3, 300, d))
+    k, v = (torch.randn(*shape, device="cuda").half() for _ in range(2))
+    cs = [TurboQuantKVCache(head_dim=d, num_kv_heads=full[1], residual_window=16, fp16_sink_size=4) for _ in range(2)]
+    cs[0].update(k.expand(full), v.expand(full))
+    cs[1].update(k.expand(full).contiguous(), v.expand(full).contiguous())
+    assert all(x is y is None or torch.equal(x, y) for x, y in zip(cs[0].state, cs[1].state))
+    c = cs[1]
+    got, want = (kernels.quantize_pack(x, c._rotation, c._k.bnd_hi, 4) for x in (k.expand(full), k.expand(full).contiguous()))
+    assert (got[0] == want[0]).float().mean() > 0.999 and torch.allclose(got[2], want[2], rtol=1e-5)     # (the row kernel takes the expanded one)
