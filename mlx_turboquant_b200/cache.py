@@ -452,7 +452,7 @@ class TurboQuantKVCache:
         lane = st[1]
         if (k_new.dtype == k_buf.dtype == v_new.dtype == v_buf.dtype and st == v_new.stride()
                 and st[3] == 1 and st[2] == d and (b == 1 or st[0] == h * lane) and lane % d == 0
-                and (d * size) % 16 == 0 and (lane >= t_new * d or h == 1)):
+                and (d * size) % 16 == 0 and (lane >= t_new * d or b * h == 1)):
             rc = _lib.launch(dev, "tq_append_tokens", k_new.data_ptr(), v_new.data_ptr(), k_buf.data_ptr(), v_buf.data_ptr(),
                              b * h, t_new, d * size, max(lane // d, t_new), k_buf.shape[2], row0, _lib.stream_ptr(dev))
             if rc == 0:
