@@ -322,6 +322,7 @@ class TurboQuantKVCache:
     def meta_state(self, v):
         self.offset = int(v["offset"])
         self._compressed_len = int(v["compressed_len"])
+        self._dense_len = min(self._dense_len, self._compressed_len)     # (what is compressed after a rewind is expanded anew)
         if "fp16_sink_size" in v:
             self.fp16_sink_size = int(v["fp16_sink_size"])
         if "sink_len" in v:

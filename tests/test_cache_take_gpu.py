@@ -68,3 +68,18 @@ def test_expanded_newcomers_equal_their_copies(d, axis):
     c = cs[1]
     got, want = (kernels.quantize_pack(x, c._rotation, c._k.bnd_hi, 4) for x in (k.expand(full), k.expand(full).contiguous()))
     assert (got[0] == want[0]).float().mean() > 0.999 and torch.allclose(got[2], want[2], rtol=1e-5)     # (the row kernel takes the expanded one)
+
+
+@pytest.mark.parametrize("d,qjl", ((256, False), (64, True), (64, False)))
+def test_a_second_continuation_does_not_see_the_first_one(d, qjl):
+    from mlx_turboquant_b200 import TurboQuantKVCache
+    x = [torch.randn(1, 2, 40, d, device="cuda").half() for _ in range(3)]
+    make = lambda: TurboQuantKVCache(head_dim=d, num_kv_heads=2, residual_window=0, qjl_correction=qjl)   # noqa: E731
+    c, ref = make(), make()
+    c.update_and_fetch(x[0], x[0])
+    mark = c.meta_state
+    c.update_and_fetch(x[1], x[1])
+    c.meta_state = mark
+    ref.update(x[0], x[0])
+    got, want = c.update_and_fetch(x[2], x[2]), ref.update_and_fetch(x[2], x[2])
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])

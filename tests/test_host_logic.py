@@ -255,3 +255,14 @@ def test_gather_slot_ledger():
         led.use(2)
     with pytest.raises(IndexError):
         led.use(3)
+
+
+def test_rewinding_the_counters_drops_the_expanded_rows_behind_them():
+    from mlx_turboquant_b200 import TurboQuantKVCache
+    c = TurboQuantKVCache(head_dim=256)
+    c._compressed_len = c._dense_len = 100
+    m = c.meta_state
+    c.meta_state = dict(m, compressed_len="40")
+    assert c._dense_len == 40
+    c.meta_state = dict(m, compressed_len="100")          # forward again: rows 40 .. 99 are expanded anew
+    assert c._dense_len == 40
