@@ -695,10 +695,14 @@ class TurboQuantKVCache:
             self._many = (key, a)
         a.q, a.out = q.data_ptr(), out.data_ptr()
         a.c_len, a.sink_len, a.res_len = self._compressed_len, self._sink_len, self._fp16_len
-        # scratch for the expanded rows (at most 512 MB): the allocator reuses it in stream order after this call
-        need = _lib.lib().tq_prefill_workspace_bytes(b, hq, a.n_kv_heads, d, self._sink_len + self._compressed_len + self._fp16_len, tq)
-        ws = torch.empty(need, dtype=torch.uint8, device=dev)
-        a.workspace, a.workspace_bytes = ws.data_ptr(), need
+        # Scratch for the expanded rows; the allocator reuses it in stream order after this call. On a card without room for it the
+        # lanes are done one at a time, or by the kernels that need none; those take float32 queries anyway.
+        ws = None
+        if q.dtype != torch.float32:
+            total = self._sink_len + self._compressed_len + self._fp16_len
+            need = _lib.lib().tq_prefill_workspace_bytes
+            ws = kernels.scratch(dev, lambda: need(b, hq, a.n_kv_heads, d, total, tq), lambda: need(1, hq // a.n_kv_heads, 1, d, total, tq))
+        a.workspace, a.workspace_bytes = (None, 0) if ws is None else (ws.data_ptr(), ws.numel())
         _lib.check(_lib.launch(dev, "tq_prefill_attn", C.byref(a), tq, _lib.stream_ptr(dev)))
         return out
 

@@ -272,6 +272,16 @@ def workspace_of(index: int, stream: int) -> torch.Tensor | None:
     return _workspaces.get((index, stream))
 
 
+def scratch(device: torch.device, *sizes) -> torch.Tensor | None:
+    """A buffer of the first of these sizes (callables) that the device has room for, or None."""
+    for size in sizes:
+        try:
+            return torch.empty(size(), dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:
+            pass
+    return None
+
+
 _decode_tables: dict[tuple, torch.Tensor | None] = {}
 
 

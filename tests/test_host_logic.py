@@ -266,3 +266,18 @@ def test_rewinding_the_counters_drops_the_expanded_rows_behind_them():
     assert c._dense_len == 40
     c.meta_state = dict(m, compressed_len="100")          # forward again: rows 40 .. 99 are expanded anew
     assert c._dense_len == 40
+
+
+def test_scratch_falls_back_to_what_fits(monkeypatch):
+    import torch
+    from mlx_turboquant_b200 import kernels
+    empty, room = torch.empty, [0]
+
+    def limited(n, **kw):
+        if n > room[0]:
+            raise torch.OutOfMemoryError("no room")
+        return empty(n, **kw)
+    monkeypatch.setattr(torch, "empty", limited)
+    for room[0], want in ((100, 100), (99, 10), (9, None)):
+        got = kernels.scratch(torch.device("cpu"), lambda: 100, lambda: 10)
+        assert (None if got is None else got.numel()) == want

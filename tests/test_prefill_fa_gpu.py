@@ -55,3 +55,21 @@ def test_lanes_in_rounds(d, b, hkv, lent):
     _lib.check(_lib.lib().tq_prefill_attn(C.byref(a), 40, torch.cuda.current_stream().cuda_stream))
     torch.cuda.synchronize()
     _check(out, ref)
+
+
+@pytest.mark.parametrize("d,kb,vb", ((128, 4, 2), (128, 3.5, 3.5), (64, 4, 4), (256, 4, 2)))
+@pytest.mark.parametrize("dtype", (torch.float16, torch.bfloat16))
+@pytest.mark.parametrize("room", ("one lane", "none"))
+def test_a_card_without_room_for_the_scratch(monkeypatch, d, kb, vb, dtype, room):
+    from mlx_turboquant_b200 import kernels
+    c, q, ref = _case(d, 2, 8, 2, 900, 80, dtype, kb, vb)
+    full = kernels.scratch
+    monkeypatch.setattr(kernels, "scratch", lambda dev, *sizes: full(dev, sizes[-1]) if room == "one lane" else None)
+    _check(c.attend(q, out_dtype=torch.float32), ref)
+
+
+def test_float32_queries_need_no_scratch(monkeypatch):
+    from mlx_turboquant_b200 import kernels
+    c, q, ref = _case(128, 1, 8, 2, 500, 70, torch.float32, 4, 2)
+    monkeypatch.setattr(kernels, "scratch", lambda *a: pytest.fail("scratch asked for"))
+    _check(c.attend(q), ref)
