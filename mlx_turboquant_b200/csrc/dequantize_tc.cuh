@@ -71,7 +71,7 @@ template <int D> struct Plan {
     static_assert(SMEM <= 227 * 1024 && OFF_S % 1024 == 0 && 2 * (NC / 8) * 2 * 32 * 8 <= 8 * STG, "shared-memory plan");
     static_assert(RBLK % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
 };
-enum Bars { A_FULL = 0, A_FREE = 4, ACC_FULL = 8, ACC_FREE = 10 };
+enum Bars { A_FULL = 0, A_FREE = 4, ACC_FULL = 8, ACC_FREE = 10, DRAIN = 12 };
 
 struct Params {
     const uint8_t* packed_hi; const uint8_t* packed_lo; const float* norms;
@@ -446,6 +446,7 @@ __global__ void __launch_bounds__(NT, 1) dequantize_tc_kernel(const __grid_const
     if (tid == 0) {
         for (int i = 0; i < P::NB; ++i) { mbar_init(bar(A_FULL + i), PROD_T); mbar_init(bar(A_FREE + i), 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(bar(ACC_FULL + i), 1); mbar_init(bar(ACC_FREE + i), EPI_T); }
+        mbar_init(bar(DRAIN), 1);
         fence_barrier_init();
         slot[1] = 0u;
     }
@@ -539,6 +540,10 @@ __global__ void __launch_bounds__(NT, 1) dequantize_tc_kernel(const __grid_const
                     umma_commit(bar(A_FREE + bf));
                 }
                 if (ok) umma_commit(bar(ACC_FULL + st));
+            }
+            if (!ok) {             // a wait ran out: the products in flight end (bounded) before their memory is given up
+                umma_commit(bar(DRAIN));
+                for (uint32_t i = 0; i < WAIT_LIMIT && !mbar_try(bar(DRAIN), 0); ++i) {}
             }
         }
         __syncwarp();

@@ -59,13 +59,13 @@ template <int D> struct Plan {
     static constexpr uint32_t OFF_Q = 0, OFF_K = NQ * Q_TILE, OFF_V = OFF_K + ST * K_TILE;
     static constexpr uint32_t OFF_SC = OFF_V + ST * K_TILE;                  // float [NSC][2][TN]: key norms, value norms
     static constexpr uint32_t OFF_BAR = OFF_SC + NSC * 2 * TN * 4;
-    static constexpr uint32_t OFF_SLOT = OFF_BAR + 352;                      // [0] tensor-memory base, [1] abort
+    static constexpr uint32_t OFF_SLOT = OFF_BAR + 368;                      // [0] tensor-memory base, [1] abort
     static constexpr size_t NEED = OFF_SLOT + 16 + 1024, SMEM = NEED > 116 * 1024 ? NEED : 116 * 1024;      // one CTA per SM: it takes all of the tensor memory
     static constexpr uint32_t COL_O = NQ * SB * TN;                          // scores first, then the accumulators
     static_assert(COL_O + NQ * DP <= 512, "tensor memory");
     static_assert(SMEM <= 227 * 1024, "shared memory");
 };
-enum Bars { K_FULL = 0, K_FREE = 4, V_FULL = 8, V_FREE = 12, SC_FULL = 16, SC_FREE = 24, S_FULL = 32, P_FULL = 36, O_DONE = 40, ALL_DONE = 42 };       // (44 of 8 bytes)
+enum Bars { K_FULL = 0, K_FREE = 4, V_FULL = 8, V_FREE = 12, SC_FULL = 16, SC_FREE = 24, S_FULL = 32, P_FULL = 36, O_DONE = 40, ALL_DONE = 42, DRAIN = 44 };       // (45 of 8 bytes)
 
 struct Params {
     const void* q; int q_dtype; float f;               // scale * log2(e)
@@ -218,6 +218,7 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(Params p, const __gr
             mbar_init(bar(S_FULL + i), 1); mbar_init(bar(P_FULL + i), 128);
         }
         for (int i = 0; i < 2; ++i) { mbar_init(bar(O_DONE + i), 1); mbar_init(bar(ALL_DONE + i), 1); }
+        mbar_init(bar(DRAIN), 1);
         for (int i = 0; i < NSC; ++i) { mbar_init(bar(SC_FULL + i), 1); mbar_init(bar(SC_FREE + i), NQ * 128); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         slot[1] = 0u;
@@ -254,6 +255,10 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(Params p, const __gr
         atomicCAS(p.status, 0, ERR_WAIT);
         return false;
     };
+    // copies and products end (bounded) before their memory is given up, also after a wait that ran out
+    auto drain = [&](int which, int phase) {
+        for (uint32_t i = 0; i < WAIT_LIMIT && !mbar_try(bar(which), uint32_t(phase & 1)); ++i) {}
+    };
     // score buffer of (query tile q, key tile j) and the phase of its barriers
     constexpr int SB = P::SB, ST = P::ST;
     auto sbuf = [](int q, int j) { return q * SB + j % SB; };
@@ -265,28 +270,36 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(Params p, const __gr
         if (lane == 0) {
             const float* kn = p.kn + int64_t(lane_c) * p.ts;
             const float* vn = p.vn + int64_t(lane_c) * p.ts;
+            int nk = 0, nsc = 0;                                   // copies asked for so far
             for (int j = 0; j < n; ++j) {
                 const int row = (t_lo + j) * TN, s = j % NSC, st = j % ST;
                 if (j >= ST && !wait_bar(K_FREE + st, j / ST - 1)) break;
+                nk = j + 1;
                 mbar_expect_tx(bar(K_FULL + st), P::K_TILE);
                 for (int x = 0; x < P::NBLK; ++x) tma_load_3d(sbase + P::OFF_K + st * P::K_TILE + x * P::KBLK, &kmap, x * 64, row, lane_c, bar(K_FULL + st));
                 if (j >= NSC && !wait_bar(SC_FREE + s, j / NSC - 1)) break;
                 const uint32_t sc = sbase + P::OFF_SC + s * 2 * TN * 4;
+                nsc = j + 1;
                 mbar_expect_tx(bar(SC_FULL + s), 2 * TN * 4);
                 bulk_g2s(sc, kn + row, TN * 4, bar(SC_FULL + s));
                 bulk_g2s(sc + TN * 4, vn + row, TN * 4, bar(SC_FULL + s));
             }
+            for (int j = max(0, nk - ST); j < nk; ++j) drain(K_FULL + j % ST, j / ST);
+            for (int j = max(0, nsc - NSC); j < nsc; ++j) drain(SC_FULL + j % NSC, j / NSC);
         }
         __syncwarp();
     } else if (warp == NQ * 4 + 2) {
         // ======================= values: one thread =======================
         if (lane == 0) {
+            int nv = 0;
             for (int j = 0; j < n; ++j) {
                 const int row = (t_lo + j) * TN, st = j % ST;
                 if (j >= ST && !wait_bar(V_FREE + st, j / ST - 1)) break;
+                nv = j + 1;
                 mbar_expect_tx(bar(V_FULL + st), P::K_TILE);
                 for (int x = 0; x < P::NBLK; ++x) tma_load_3d(sbase + P::OFF_V + st * P::K_TILE + x * P::KBLK, &vmap, x * 64, row, lane_c, bar(V_FULL + st));
             }
+            for (int j = max(0, nv - ST); j < nv; ++j) drain(V_FULL + j % ST, j / ST);
         }
         __syncwarp();
     } else if (warp == NQ * 4) {
@@ -335,6 +348,7 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(Params p, const __gr
                     }
                 }
             }
+            if (!ok) { umma_commit(bar(DRAIN)); drain(DRAIN, 0); }
         }
         __syncwarp();
     } else {

@@ -124,6 +124,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     atomicCAS(&g_status, 0, code);
     return false;
 }
+// What this thread's last copies or products were to complete, also after a wait that ran out (bounded, whatever the flag says):
+// nothing may land in shared or tensor memory that the CTA has given up.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
+    for (uint32_t i = 0; i < WAIT_LIMIT && !mbar_try(bar, parity); ++i) {}
+}
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes) : "memory");
@@ -609,6 +614,7 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
     //           nrm[3] (norm warps -> epilogue), acc_full[4] (MMA commit -> epilogue group), acc_free[4] (epilogue group -> MMA)
     const uint32_t bar_full = sbase + OFF_BAR, bar_afree = bar_full + 8 * A_STAGES_MAX, bar_nrm = bar_afree + 8 * A_STAGES_MAX;
     const uint32_t bar_accfull = bar_nrm + 8 * A_STAGES_MAX, bar_accfree = bar_accfull + 8 * ACC_STAGES;      // (ACCS of the 4 slots are used)
+    const uint32_t bar_drain = bar_accfree + 8 * ACC_STAGES;              // products in flight when a wait ran out
 
     if (sbase & 1023u) {                  // the swizzled operand tiles need 1024-byte alignment (uniform across the CTA)
         if (tid == 0) atomicCAS(&g_status, 0, 9);
@@ -626,6 +632,7 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
         }
         if (DC == 256)
             for (int q = 0; q < NSQ_SLOTS; ++q) mbar_init(sbase + OFF_NRMBAR256 + 8 * q, N_NORM);
+        mbar_init(bar_drain, 1);
         for (int a = 0; a < ACC_STAGES; ++a) { mbar_init(bar_accfull + 8 * a, 1); mbar_init(bar_accfree + 8 * a, N_EPI / Sh::GROUPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -789,17 +796,17 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
             default: break;               // the host only launches the combinations above
         }
     } else if (warp == EPI_WARPS) {
-        // ======================= MMA issue: one elected thread =======================
+        // ======================= MMA issue: the whole warp in uniform control flow, one elected lane issues =======================
+        bool ok = true;
         auto wait_all = [&](uint32_t bar, uint32_t parity, volatile int* flag, int code) { return bool(__all_sync(0xffffffffu, mbar_wait(bar, parity, flag, code))); };
         if (DC == 256) {
             {
                 const int terms = bf16 ? 3 : 2, kb_bytes = terms * SLICE * 128;
                 const uint32_t idesc = make_idesc(terms * SLICE, bf16), rb = sbase + (bf16 ? OFF_R3 : OFF_R1);
                 int it = 0, hit = 0;
-                bool ok = true;
                 for (int64_t tile = tile0; ok && tile < p.n_tiles; tile += tile_step, ++it) {
                     const int a = it % ACCS;
-                    if (it >= ACCS && !wait_all(bar_accfree + 8 * a, uint32_t((it / ACCS) - 1) & 1u, abort_flag, 2)) break;
+                    if (it >= ACCS && !(ok = wait_all(bar_accfree + 8 * a, uint32_t((it / ACCS) - 1) & 1u, abort_flag, 2))) break;
                     for (int kh = 0; kh < 2; ++kh, ++hit) {
                         const int s = hit % a_stages;
                         ok = wait_all(bar_full + 8 * s, uint32_t(hit / a_stages) & 1u, abort_flag, 1);
@@ -822,8 +829,8 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
             int it = 0;
             for (int64_t tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x, ++it) {
                 const int a = it % ACCS, s = it % a_stages;
-                if (it >= ACCS && !wait_all(bar_accfree + 8 * a, uint32_t((it / ACCS) - 1) & 1u, abort_flag, 2)) break;
-                if (!wait_all(bar_full + 8 * s, uint32_t(it / a_stages) & 1u, abort_flag, 1)) break;
+                if (it >= ACCS && !(ok = wait_all(bar_accfree + 8 * a, uint32_t((it / ACCS) - 1) & 1u, abort_flag, 2))) break;
+                if (!(ok = wait_all(bar_full + 8 * s, uint32_t(it / a_stages) & 1u, abort_flag, 1))) break;
                 tc_fence_after();
                 const uint32_t a_tile = sbase + OFF_A + s * OPER_BYTES;
                 const uint32_t d_acc = tmem_base + a * Sh::STAGE_COLS;
@@ -847,6 +854,7 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
                 umma_commit(bar_accfull + 8 * a);    // the accumulator is complete: its epilogue group may read it
             }
         }
+        if (!ok) { umma_commit(bar_drain); mbar_drain(bar_drain, 0); }
         __syncwarp();
     } else if (warp == EPI_WARPS + 1 + N_NORM / 32) {
         // ======================= TMA issue: one thread keeps the operand stages full =======================
@@ -867,6 +875,7 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
                         tma_load_3d(a_tile + KBLK_BYTES, &tmap, kh * 128 + 64, int(tl * TM), int(o), bar_full + 8 * s);
                     }
                 }
+                for (int h = hit > a_stages ? hit - a_stages : 0; h < hit; ++h) mbar_drain(bar_full + 8 * (h % a_stages), uint32_t(h / a_stages) & 1u);
             }
         } else
         if (lane == 0) {
@@ -881,6 +890,7 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
                 tma_load_3d(a_tile, &tmap, 0, int(tl * TM), int(o), bar_full + 8 * s);                              // columns 0..63
                 if (d > 64) tma_load_3d(a_tile + KBLK_BYTES, &tmap, 64, int(tl * TM), int(o), bar_full + 8 * s);    // columns 64..127 (zeros past d)
             }
+            for (int i = it > a_stages ? it - a_stages : 0; i < it; ++i) mbar_drain(bar_full + 8 * (i % a_stages), uint32_t(i / a_stages) & 1u);
         }
         __syncwarp();
     } else {
