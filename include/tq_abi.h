@@ -285,9 +285,9 @@ int tq_decode_step(const tq_decode_args* a, const void* k_new, const void* v_new
  * reference only sketched it for packed keys (kernels.py:558-590, docs/FUSED_ATTENTION_DESIGN.md:281-283). */
 int tq_prefill_attn(const tq_decode_args* a, int t_q, void* stream);
 size_t tq_prefill_workspace_bytes(int batch, int n_q_heads, int n_kv_heads, int d, int64_t total_len, int t_q);
-/* The most bytes that any round of such a call uses of a workspace of workspace_bytes (0: too small to be used at all).  Host
+/* The most bytes that any round of such a call (c_len packed, dense_len uncompressed tokens) uses of a workspace of workspace_bytes (0: too small to be used at all).  Host
  * arithmetic, no device needed; at most workspace_bytes. */
-size_t tq_prefill_workspace_used(int batch, int n_q_heads, int n_kv_heads, int d, int64_t total_len, int t_q, size_t workspace_bytes);
+size_t tq_prefill_workspace_used(int batch, int n_q_heads, int n_kv_heads, int d, int64_t c_len, int64_t dense_len, int t_q, size_t workspace_bytes);
 
 /* Same computation as tq_decode_attn for callers that can neither lend a workspace nor allocate one at call
  * time (a process that gave the whole device to its own memory pool at start-up; a step loop that cannot afford

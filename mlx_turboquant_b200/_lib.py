@@ -110,7 +110,7 @@ PROTOTYPES = {
     "tq_decode_step": (_i, [C.POINTER(DecodeArgs), _vp, _vp, _vp]),
     "tq_prefill_attn": (_i, [C.POINTER(DecodeArgs), _i, _vp]),
     "tq_prefill_workspace_bytes": (_sz, [_i, _i, _i, _i, _i64, _i]),
-    "tq_prefill_workspace_used": (_sz, [_i, _i, _i, _i, _i64, _i, _sz]),
+    "tq_prefill_workspace_used": (_sz, [_i, _i, _i, _i, _i64, _i64, _i, _sz]),
     "tq_decode_attn_static": (_i, [C.POINTER(DecodeArgs), _vp]),
     "tq_set_tuning": (_i, [C.c_char_p, _i]),
     "tq_decode_kernel_choice": (_i, [C.POINTER(DecodeArgs)]),

@@ -73,3 +73,27 @@ def test_float32_queries_need_no_scratch(monkeypatch):
     c, q, ref = _case(128, 1, 8, 2, 500, 70, torch.float32, 4, 2)
     monkeypatch.setattr(kernels, "scratch", lambda *a: pytest.fail("scratch asked for"))
     _check(c.attend(q), ref)
+
+
+@pytest.mark.parametrize("d", (64, 96, 128, 256))
+@pytest.mark.parametrize("kb,vb", ((4, 2), (3.5, 3.5), (2, 4)))
+@pytest.mark.parametrize("loud", (1.0, 8.0))
+def test_as_close_to_64_bits_as_the_kernel_that_unpacks_as_it_goes(d, kb, vb, loud):
+    """The same operands rounded to fp16 (rotated queries, centroids, weights) and float32 sums: no further off, up to the scatter of
+    some 10,000 outputs' root mean square."""
+    from mlx_turboquant_b200 import TurboQuantKVCache, kernels
+    g = torch.Generator(device="cuda").manual_seed(7)
+    t, tq, h = 2500, 60, 2
+    c = TurboQuantKVCache(head_dim=d, num_kv_heads=h, key_bits=kb, value_bits=vb, residual_window=64, fp16_sink_size=10)
+    k, v = ((torch.randn(1, h, t, d, device="cuda", generator=g) * torch.exp(0.5 * torch.randn(1, h, t, 1, device="cuda", generator=g))).half() for _ in range(2))
+    q = (torch.randn(1, 4 * h, tq, d, device="cuda", generator=g) * loud / d ** 0.5).half()
+    dk, dv = (x.double().repeat_interleave(4, 1) for x in c.update_and_fetch(k, v))
+    s = (q.double() @ dk.transpose(-1, -2)) * d ** -0.5
+    s = s.masked_fill(torch.arange(t, device="cuda")[None, :] > (t - tq + torch.arange(tq, device="cuda"))[:, None], float("-inf"))
+    ref = torch.softmax(s, -1) @ dv
+    err = []
+    for tc in (1, 0):
+        kernels.set_tuning("prefill_tc", tc)
+        err.append(float((c.attend(q, out_dtype=torch.float32) - ref).norm() / ref.norm()))
+    kernels.set_tuning("prefill_tc", 1)
+    assert err[0] < 1.1 * err[1], err
