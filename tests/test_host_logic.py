@@ -281,3 +281,19 @@ def test_scratch_falls_back_to_what_fits(monkeypatch):
     for room[0], want in ((100, 100), (99, 10), (9, None)):
         got = kernels.scratch(torch.device("cpu"), lambda: 100, lambda: 10)
         assert (None if got is None else got.numel()) == want
+
+
+def test_fp16_value_tables_have_no_mean_error():
+    """A weighted sum of N tokens keeps the mean error of a coordinate and shrinks with sqrt(N) itself: the fp16 copy of a table has to
+    be free of it (1e-6 of a coordinate's deviation is 2e-4 of a sum over 40,000 tokens, what all other roundings are together)."""
+    from math import erf, sqrt
+    from mlx_turboquant_b200.cache import _fp16_scale
+    from mlx_turboquant_b200.codebook import get_codebook_host
+    for d in (64, 96, 128, 256):
+        for bits in (1, 2, 3, 4):
+            c, b = (x.astype(np.float64) * sqrt(d) for x in get_codebook_host(d, bits))
+            p = np.diff([0.0] + [0.5 * (1 + erf(x / sqrt(2))) for x in b] + [1.0])
+            s = np.float32(_fp16_scale(d, bits))
+            err = ((get_codebook_host(d, bits)[0] * s).astype(np.float16).astype(np.float64) / np.float64(s)) * sqrt(d) - c
+            assert abs((p * err).sum()) < 2.5e-7 and sqrt((p * err * err).sum()) < 1.3e-4, (d, bits)
+    assert [_fp16_scale(128, b) for b in (2, 3, 4)] == [1.49676513671875, 1.2477874755859375, 1.447540283203125]      # symmetric tables: as they were
