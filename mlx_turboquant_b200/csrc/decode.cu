@@ -700,6 +700,61 @@ template <int D, bool QJL> static int launch_decode(const DecodeParams& p, cudaS
     return TQ_OK;
 }
 
+// Whether the lookup kernel of decode_lut.cu takes a call that its tables cover.  Times in us, rival / lookup kernel, on caches that do
+// not come from L2; "lanes" are (sequence, KV head) pairs, lanes x packed tiles of 16 tokens where two numbers are given.  Lines between
+// the rivals' waves of CTAs move with the number of SMs.
+struct LutRivals {
+    int64_t c_len, lanes, p_tiles, d_tiles, run;       // run: packed tiles per warp of the streaming kernel
+    int sms, d, G, dense_dtype;
+    bool qjl, direct, stream, bytes;                   // which rival would run; 4-bit keys and 2-bit values
+};
+static bool lut_is_best(const LutRivals& r) {
+    const bool fp16 = r.dense_dtype == TQ_F16, bf16 = r.dense_dtype == TQ_BF16;
+    if (r.c_len == 0) {
+        // Only uncompressed tokens; the rival is the general kernel: one launch, a CTA per lane or a few, so that it wins with few tokens
+        // (d = 128, 20 tokens: 8.3 / 10.0, float32 19.3 / 24.4) and with lanes that just do not fit a wave; here bfloat16 rows feed the
+        // MMAs as they are (200 tokens of 8 lanes: 24.0 / 10.6, fp16 13.1 / 10.3, float32 36 / 25), many lanes of few heads cost
+        // little (2048 lanes of 1 head: 63 / 35, of 8: 100 / 110).
+        const int64_t L = r.lanes, T = r.d_tiles, sms = r.sms;
+        if (r.d == 256) {                              // (eight warps per CTA and 292 floats a partial: 128 lanes of 8 heads 24.6 / 52.7)
+            if (bf16) return 4 * L <= sms || T >= 20 || (T >= 12 && !(r.G > 4 && 2 * L > sms && L <= sms)) || (r.G <= 4 && L > (r.G > 2 ? 2 : 1) * sms);
+            if (fp16) return (16 * L <= sms && (T >= 12 || r.G > 4)) || (r.G > 4 && T >= 12 && 4 * L <= sms) || (r.G == 1 && L > 2 * sms);
+            return (T >= 12 && (4 * L <= sms || (T < 20 && 2 * L <= sms))) || (T <= 4 && r.G <= 2 && L > sms);
+        }
+        if (L <= 4) return true;                       // (a handful of lanes: within 2 us either way, float32 4; 8 heads 17.0 / 13.6)
+        if (bf16) return !(T < (r.d == 64 ? 14 : 12) && L > sms && (r.G > 4 ? L <= 4 * sms : r.d == 64 && r.G > 2 && L <= 2 * sms));
+        if (fp16 && r.G > 4) return 2 * L <= sms || (T >= 20 && L > sms);
+        if (fp16) return (T >= 12 && 8 * L <= 7 * sms) || L > (r.G > 2 ? 4 : 2) * sms || (T >= 20 && L > sms);
+        return (T >= 12 && 10 * L <= 11 * sms) || (T >= 20 && L <= 2 * sms) || (T <= 4 && r.G <= 4 && L > 2 * sms) || (L > 8 * sms && r.G <= 2 && r.d != 96);
+    }
+    if (!r.bytes) return true;                         // (other widths: the general kernel, code by code)
+    const int64_t tiles = r.lanes * r.p_tiles;
+    if (r.stream)
+        // Until its runs are long enough to pay for two partials per warp (128 x 600 at d = 128 1.00 / 0.97, x 1000 1.00 / 1.04; with
+        // sketches 64 x 607 73 / 57; d = 96 128 x 524 62 / 52), float32 only with sketches (64 x 607 87 / 78, without 54 / 65); and while
+        // the uncompressed tokens are a large share, larger still in bfloat16 (1632 x 56 131 / 121, bfloat16 864 x 150 171 / 121,
+        // 368 x 608 169 / 165; float32 242 / 268).
+        return (r.run < g_tune_stream_min_run * 3 / 2 && r.lanes <= r.sms && (fp16 || bf16 || r.qjl)) ||
+               ((fp16 || bf16) && r.p_tiles * 24 < (fp16 ? 6 : 37) * r.d_tiles * g_tune_stream_min_run);
+    if (r.direct)
+        // Its CTAs come two to an SM, at least one per lane and one for the uncompressed tokens: beyond a wave of them it pays to fold.
+        // fp16, 4 heads: 256 x 64 1.00 / 1.13, 320 x 64 1.00 / 0.94, 512 x 64 1.00 / 0.80; 1 head: 192 x 64 1.00 / 0.96, 256 x 64 1.00 / 0.91.
+        // bfloat16: 96 x 64 1.00 / 1.03, 128 x 64 1.00 / 0.86, 320 x 64 1.00 / 0.69; 80 x 5 1.00 / 0.91.  float32 rows are converted through
+        // shared memory here: 72 x 71 30.3 / 50.5, 352 x 122 115 / 118, 256 x 28 89 / 82, 1024 x 28 268 / 220.
+        return fp16 ? r.lanes > (r.G <= 2 ? 3 * r.sms / 2 : 2 * r.sms) : bf16 ? 5 * r.lanes > 4 * r.sms || (5 * r.lanes > 2 * r.sms && r.p_tiles < 16)
+                                                                              : 2 * r.lanes > 3 * r.sms && r.p_tiles < 64;
+    // The general kernel: d = 64, where it is one launch of little code, while the tiles are few (fp16 96 x 50 13.1 / 17.5, 128 x 91
+    // 23.5 / 20.4, 400 x 17 33.7 / 29.9; bfloat16 24 x 53 16.6 / 15.1, 96 x 50 17.1 / 18.6; float32 32 x 67 24.1 / 21.4, 32 x 899 29.1 / 33.0,
+    // 96 x 355 37.9 / 36.5), a single head per lane even with sketches (96 x 50 18.1 / 19.5) or at d = 96 (32 x 20 13.9 / 14.9, 32 x 298
+    // 22.6 / 21.3); everything else is faster here (d = 96, 4 heads 32 x 96 19.9 / 18.9, sketches 37.6 / 21.2).
+    if (r.d == 64 && !r.qjl) {
+        if (fp16) return tiles >= 10000 || r.lanes > 2 * r.sms;
+        if (bf16) return tiles >= 10000 || r.lanes > r.sms || r.lanes < 40;
+        return tiles < 4500 || tiles >= 30000 || r.lanes <= 8 || 2 * r.lanes > 3 * r.sms;
+    }
+    return !(fp16 && r.G == 1 && r.d <= 96 && tiles < (r.qjl ? r.d == 64 ? 5000 : 0 : 7000));
+}
+
 // Validates the arguments, picks the path and the split plan and fills the kernel parameters.
 int decode_prepare(const tq_decode_args* a, void* workspace, size_t workspace_bytes, DecodeParams* out, bool* direct_out,
                    const void* k_new, const void* v_new) {
@@ -764,25 +819,10 @@ int decode_prepare(const tq_decode_args* a, void* workspace, size_t workspace_by
         const int max_parts = direct ? std::min(g_tune_stream_max_parts, 64) : 64;
         stream = stp.range >= min_run && stp.npp + stp.nd <= max_parts && stream_supported(d, qjl);
     }
-    // The lookup kernel: everything else its tables cover (two to four bits, their fractional splits), and of the 4-bit-key /
-    // 2-bit-value calls those that are not its rivals' best.  Per call:
-    //   * table-lookup (direct) kernel: many lanes - 256 x 31 tiles 54.7 against 44.1 us, 384 x 62 72.7 / 42.7, 128 x 375 56.9 / 50.5;
-    //     few or short ones stay (16 x 1000 22.7 / 33.2, 64 x 94 21.9 / 25.9).  Its uncompressed tokens cost more when they are
-    //     not fp16 (here bfloat16 rows feed the MMAs as they are): then from 64 lanes (128 x 109 50.8 / 37.5, 64 x 28 25.1 / 22.7)
-    //   * streaming kernel: until its runs are long enough to pay for two partials per warp - 128 x 512 68.0 / 63.9, with sketches
-    //     64 x 500 72.8 / 51.5, 128 x 512 at d = 96 72 / 63; beyond it stays (128 x 1024 95.1 / 97.9) -
-    //     and while the uncompressed tokens are a large share, larger still when they are not fp16 (1632 x 56 131 / 121, bfloat16
-    //     247 / 128, 1024 x 234 222 / 182; 256 x 1000 161 / 179)
-    //   * general kernel: d = 64 without sketches and few tiles, where it is one launch of little code (48 x 63 12.0 / 15.6,
-    //     64 x 188 21.5 / 18.9); d = 96, d = 256 and sketches are faster here at any size (8 x 125 16.3 / 15.3, 36.8 / 31.6, 32.6 / 22.8)
-    const int64_t kv_lanes = int64_t(a->batch) * a->n_kv_heads, tiles = kv_lanes * ((a->c_len + TILE - 1) / TILE);
-    const bool bytes = a->c_len > 0 && a->k_bits_hi == 4 && !a->k_bits_lo && a->v_bits_hi == 2 && !a->v_bits_lo;
-    const bool fp16 = a->dense_dtype == TQ_F16;
-    const int64_t p_tiles = (a->c_len + TILE - 1) / TILE, d_tiles = (dense_len + TILE - 1) / TILE;
-    const bool lut_best = !bytes ? true
-        : stream ? (stp.range < g_tune_stream_min_run * 3 / 2 && kv_lanes <= 148) || p_tiles * 24 < (fp16 ? 6 : 37) * d_tiles * g_tune_stream_min_run
-        : direct ? kv_lanes >= (fp16 ? 256 : 64) || (kv_lanes >= 64 && tiles >= 16000)
-        : d != 64 || qjl || !fp16 || tiles >= 10000;
+    const LutRivals r{a->c_len, int64_t(a->batch) * a->n_kv_heads, (a->c_len + TILE - 1) / TILE, (dense_len + TILE - 1) / TILE, stp.range,
+                      sm_count(), d, a->n_q_heads / a->n_kv_heads, a->dense_dtype, qjl, direct, stream,
+                      a->k_bits_hi == 4 && !a->k_bits_lo && a->v_bits_hi == 2 && !a->v_bits_lo};
+    const bool lut_best = lut_is_best(r);
     bool lut = ((lut_best && g_tune_lut) || g_tune_lut == 2) && !g_tune_force_general && a->c_lane_stride % 16 == 0 && aligned(a->q, 8) &&
                aligned(a->k_hi, 16) && aligned(a->v_hi, 16) && aligned(a->k_norms, 16) && aligned(a->v_norms, 16) &&
                (!a->k_bits_lo || aligned(a->k_lo, 16)) && (!a->v_bits_lo || aligned(a->v_lo, 16)) &&

@@ -83,3 +83,13 @@ def test_four_and_two_bits_where_this_kernel_is_the_faster_one(oracle, d, b, hq,
     rs = np.random.RandomState(d + b)
     c, q, ref = _case(oracle, rs, b, hq, hkv, t, d, 4, 2, 32, 8, qjl=qjl, bf16=bf16)
     _run(c, q, ref)
+
+
+@pytest.mark.parametrize("d,b,hq,hkv,t,rw,dt,want", ((128, 12, 12, 6, 300, 32, "bf16", 1), (128, 16, 8, 4, 120, 32, "fp32", 1), (128, 32, 16, 8, 60, 16, "fp16", 3),
+                                                     (256, 16, 32, 4, 30, 64, "fp16", 0), (256, 4, 8, 1, 200, 128, "fp16", 3), (64, 6, 8, 4, 20, 64, "fp16", 0),
+                                                     (96, 6, 8, 4, 20, 64, "fp32", 0), (128, 6, 8, 4, 20, 64, "bf16", 3), (64, 4, 8, 8, 200, 32, "fp32", 3)))
+def test_calls_that_other_kernels_do_faster_stay_with_them(oracle, d, b, hq, hkv, t, rw, dt, want):
+    """4-bit keys / 2-bit values, and caches without packed tokens: one launch of little code, or a wave of CTAs, is faster than this kernel's two."""
+    rs = np.random.RandomState(d + b + t)
+    c, q, ref = _case(oracle, rs, b, hq, hkv, t, d, 4, 2, rw, 8, dtype=np.float32 if dt == "fp32" else np.float16, bf16=dt == "bf16")
+    _run(c, q, ref, want)
