@@ -797,16 +797,16 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
         }
     } else if (warp == EPI_WARPS) {
         // ======================= MMA issue: the whole warp in uniform control flow, one elected lane issues =======================
-        bool ok = true;
         auto wait_all = [&](uint32_t bar, uint32_t parity, volatile int* flag, int code) { return bool(__all_sync(0xffffffffu, mbar_wait(bar, parity, flag, code))); };
         if (DC == 256) {
             {
                 const int terms = bf16 ? 3 : 2, kb_bytes = terms * SLICE * 128;
                 const uint32_t idesc = make_idesc(terms * SLICE, bf16), rb = sbase + (bf16 ? OFF_R3 : OFF_R1);
                 int it = 0, hit = 0;
+                bool ok = true;
                 for (int64_t tile = tile0; ok && tile < p.n_tiles; tile += tile_step, ++it) {
                     const int a = it % ACCS;
-                    if (it >= ACCS && !(ok = wait_all(bar_accfree + 8 * a, uint32_t((it / ACCS) - 1) & 1u, abort_flag, 2))) break;
+                    if (it >= ACCS && !wait_all(bar_accfree + 8 * a, uint32_t((it / ACCS) - 1) & 1u, abort_flag, 2)) break;
                     for (int kh = 0; kh < 2; ++kh, ++hit) {
                         const int s = hit % a_stages;
                         ok = wait_all(bar_full + 8 * s, uint32_t(hit / a_stages) & 1u, abort_flag, 1);
@@ -829,8 +829,8 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
             int it = 0;
             for (int64_t tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x, ++it) {
                 const int a = it % ACCS, s = it % a_stages;
-                if (it >= ACCS && !(ok = wait_all(bar_accfree + 8 * a, uint32_t((it / ACCS) - 1) & 1u, abort_flag, 2))) break;
-                if (!(ok = wait_all(bar_full + 8 * s, uint32_t(it / a_stages) & 1u, abort_flag, 1))) break;
+                if (it >= ACCS && !wait_all(bar_accfree + 8 * a, uint32_t((it / ACCS) - 1) & 1u, abort_flag, 2)) break;
+                if (!wait_all(bar_full + 8 * s, uint32_t(it / a_stages) & 1u, abort_flag, 1)) break;
                 tc_fence_after();
                 const uint32_t a_tile = sbase + OFF_A + s * OPER_BYTES;
                 const uint32_t d_acc = tmem_base + a * Sh::STAGE_COLS;
@@ -854,7 +854,7 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
                 umma_commit(bar_accfull + 8 * a);    // the accumulator is complete: its epilogue group may read it
             }
         }
-        if (!ok) { umma_commit(bar_drain); mbar_drain(bar_drain, 0); }
+        if (__any_sync(0xffffffffu, *abort_flag != 0)) { umma_commit(bar_drain); mbar_drain(bar_drain, 0); }
         __syncwarp();
     } else if (warp == EPI_WARPS + 1 + N_NORM / 32) {
         // ======================= TMA issue: one thread keeps the operand stages full =======================
