@@ -129,8 +129,8 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 // The tensor core's instructions take their operands from uniform registers.  A whole warp in uniform control flow computes
-// them there and one elected lane issues; with a single thread in a divergent branch every operand is moved over one by one
-// (70 cycles per instruction: the issuing thread, not the products, was what the softmax warps waited for).
+// them there and one elected lane issues; with a single thread in a divergent branch every operand is moved over one by one (the
+// issuing thread, not the products, was what the softmax warps waited for; quantize of bfloat16 rows went from 154 to 121 us).
 // D = A.B (+ D when accumulate != 0), both operands through shared-memory descriptors
 __device__ __forceinline__ void umma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -1136,6 +1136,19 @@ bool prefill_fa_applicable(const tq_decode_args* a, int t_q) {
     }
     if (!aligned(a->q, 4) || !aligned(a->out, 16) || !aligned(a->rot, 16)) return false;
     return a->workspace_bytes >= prefill_fa_least(a->n_q_heads / a->n_kv_heads, a->d, total, t_q);
+}
+
+// Whether prefill_tc.cu, which unpacks as it goes, is the faster one of two that take the call: with a single block of 128 query rows
+// per lane nothing is unpacked twice there, and the expansion here costs as much as the attention.  Its time goes by waves of CTAs, a
+// lane each, this one's by lanes x tokens; us on 148 SMs, fa / tc, 4-bit keys and 2-bit values at d = 128 (other widths: always fa):
+// 64 lanes x 8192 195 / 292, 112 x 8192 313 / 330, 128 x 8192 387 / 331, 112 x 16384 604 / 521, 128 x 4000 187 / 199, 160 x 8192 499 / 632,
+// 224 x 8192 627 / 640, 256 x 8192 770 / 658.
+bool prefill_tc_faster(const tq_decode_args* a, int t_q) {
+    const int g = a->n_q_heads / a->n_kv_heads, gp = g <= 1 ? 1 : g <= 2 ? 2 : g <= 4 ? 4 : 8;
+    if (a->d != 128 || a->k_bits_hi != 4 || a->k_bits_lo || a->v_bits_hi != 2 || a->v_bits_lo || t_q > fa::TM / gp) return false;
+    const int64_t lanes = int64_t(a->batch) * a->n_kv_heads * fa::groups_of(g), total = a->c_len + a->sink_len + a->res_len, sms = fa::sm_count();
+    const double fa_us = 20.0 + 3.2e-4 * double(lanes) * double(total), tc_us = double((lanes + sms - 1) / sms) * (100.0 + 0.0265 * double(total));
+    return tc_us < fa_us;
 }
 
 int launch_prefill_fa(const DecodeParams& c, const void* q, int q_dtype, void* out, int out_dtype, int t_q, int64_t q_pos0, void* ws, size_t ws_bytes,

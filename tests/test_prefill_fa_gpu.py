@@ -97,3 +97,20 @@ def test_as_close_to_64_bits_as_the_kernel_that_unpacks_as_it_goes(d, kb, vb, lo
         err.append(float((c.attend(q, out_dtype=torch.float32) - ref).norm() / ref.norm()))
     kernels.set_tuning("prefill_tc", 1)
     assert err[0] < 1.1 * err[1], err
+
+
+@pytest.mark.parametrize("b,tq,unpacks", ((16, 16, True), (16, 33, False), (8, 16, False)))
+def test_a_block_of_query_rows_over_many_long_lanes_unpacks_as_it_goes(monkeypatch, b, tq, unpacks):
+    """128 query rows per lane: where waves of one CTA per lane are the faster way, the result is that kernel's, bit for bit (it is what
+    runs without scratch); other calls take the expansion."""
+    from mlx_turboquant_b200 import TurboQuantKVCache, _lib, kernels
+    g = torch.Generator(device="cuda").manual_seed(2)
+    c = TurboQuantKVCache(head_dim=128, num_kv_heads=8, key_bits=4, value_bits=2, fp16_sink_size=128)
+    x = torch.randn(b, 8, 8192, 128, device="cuda", generator=g).half()
+    c.update(x, x)
+    q = torch.randn(b, 32, tq, 128, device="cuda", generator=g).half() / 11
+    got = c.attend(q, out_dtype=torch.float32)
+    monkeypatch.setattr(kernels, "scratch", lambda *a: None)
+    want = c.attend(q, out_dtype=torch.float32)
+    assert torch.equal(got, want) == unpacks and (got - want).abs().max() < 1e-3 * want.abs().max()
+    assert _lib.lib().tq_device_status() == 0
