@@ -13,12 +13,9 @@ template <> Kernel kernel_of<256>(int, int, bool);
 }  // namespace dqtc
 
 // One or two jobs that share head_dim, rotation and result type (keys and values of a cache), on the tensor cores when
-// every job's layout allows; *handled = false leaves the call to the row kernel.  scales (one pointer per job, or null): rows
-// leave without their norms, which go there (lane stride in floats); parts / tab_scale: centroids as fp16 high and low parts
-// (2, the default) or as high parts of tab_scale times them (1).  The second job's launch does not wait for the first: its
+// every job's layout allows; *handled = false leaves the call to the row kernel.  The second job's launch does not wait for the first: its
 // CTAs take the SMs that the first one's last tiles leave idle.
-int tq_dequantize_tc(const tq_dequantize_args* q, int n_jobs, cudaStream_t s, bool* handled, float* const* scales, int64_t scale_lane_stride,
-                     const int* parts, const float* tab_scale) {
+int tq_dequantize_tc(const tq_dequantize_args* q, int n_jobs, cudaStream_t s, bool* handled) {
     *handled = false;
     const int d = q[0].d;
     if ((d != 64 && d != 96 && d != 128 && d != 256) || n_jobs < 1 || n_jobs > 2) return TQ_OK;
@@ -50,8 +47,6 @@ int tq_dequantize_tc(const tq_dequantize_args* q, int n_jobs, cudaStream_t s, bo
         j.cent_hi = a.cent_hi; j.cent_lo = a.cent_lo; j.rot = a.rot;
         j.qjl_proj = a.qjl_proj; j.qjl_bits = a.qjl_bits; j.qjl_gamma = a.qjl_gamma;
         j.out = a.out; j.out_dtype = a.out_dtype; j.out_lane_stride = a.out_lane_stride; j.out_row_stride = a.out_row_stride;
-        j.parts = parts ? parts[i] : 2; j.tab_scale = tab_scale ? tab_scale[i] : 1.f;
-        j.scales = scales ? scales[i] : nullptr; j.scale_lane_stride = scale_lane_stride;
         j.n_tiles = int((total + dqtc::TM - 1) / dqtc::TM);
         j.follows = i; j.status = status;
         k[i] = d == 64 ? dqtc::kernel_of<64>(a.bits_hi, a.bits_lo, a.qjl_bits != nullptr) : d == 96 ? dqtc::kernel_of<96>(a.bits_hi, a.bits_lo, a.qjl_bits != nullptr)

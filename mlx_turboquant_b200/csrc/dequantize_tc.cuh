@@ -8,8 +8,7 @@
 // is a dense 128 x d x d contraction per 128 rows.  To stay float32-faithful on fp16 operands both factors are split,
 // c = c_hi + 2^-11 c_lo and R = R_hi + 2^-11 R_lo, and three products are kept: c_hi R_hi in one accumulator,
 // c_hi R_lo + c_lo R_hi in a second one that the epilogue adds with weight 2^-11 (the fourth product is below float32
-// resolution).  The unit rows of the prefill kernel drop c_lo: its operands were fp16 centroids before, value tables under
-// the scale that makes fp16 hold them best (tq_fp16_table_scale).
+// resolution).
 //
 // Persistent CTAs (one per SM) walk the 128-row tiles, 17 warps:
 //   * warps 8-15 turn a tile's codes into fp16 A tiles (high parts, then low parts;
@@ -22,8 +21,8 @@
 //     the accumulators in the register layout of mma.sync fragments instead, which compute the correction on +-1 operands.
 // Every mbarrier wait is bounded (status 105); tensor memory is freed on every path.
 //
-// Bound by the shared-memory pipe (operand tiles in, results through the staging) and the producers' instructions, not by the
-// products (0.4 us of a tile's 2.6 at d = 128) nor by memory (1.7 us).  Eight producer warps: with four, one per scheduler,
+// No pipe is full: at d = 128 (4 bits, float32 results) memory runs at 68 % of a copy, issue slots are 51 % busy, the tensor pipe
+// 45 %, shared memory 30 %; what is left is the hand-over between the three roles of a tile.  Eight producer warps: with four, one per scheduler,
 // the chains of a chunk do not overlap (166 us).  Measured at 134 million coordinates, float32 / fp16 results, against the
 // four-warp table-lookup kernel before (d = 256 and sketches: the row kernel):
 //   d = 128: 4 bits 132 / 118 us (163 / 150), 3.5 bits 138 / 122 (326 / 314), 3 bits 145 / 136 (165 / 156), 2 bits 128 / 108 (162 / 140)
@@ -80,8 +79,6 @@ struct Params {
     const float* cent_hi; const float* cent_lo; const float* rot;
     const float* qjl_proj; const uint32_t* qjl_bits; const float* qjl_gamma;     // null: no correction
     void* out; int out_dtype; int64_t out_lane_stride, out_row_stride;
-    int parts; float tab_scale;                               // 2: high and low parts of the centroids, 1: high parts of tab_scale times the centroids
-    float* scales; int64_t scale_lane_stride;                 // not null: rows leave without their norms, which are copied here (lane, row)
     int n_tiles;
     int follows;                                              // the second of a pair: it may run beside the first and ends after it
     int* status;
@@ -112,7 +109,7 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
 // (issued by one elected lane of a warp in uniform control flow: the operands then come straight from uniform registers, where a
-// single thread in a divergent branch moves each of them over, 70 cycles per instruction)
+// single thread in a divergent branch moves each of them over one by one)
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -314,14 +311,9 @@ __device__ __forceinline__ void produce(const Params& job, unsigned char* smem, 
             const int64_t ir = int64_t(ln) * job.in_lane_stride + rw;
             in_row = int(ir);
             row.y = uint32_t((int64_t(ln) * job.out_lane_stride + int64_t(rw) * job.out_row_stride) >> 3);
-            float nrm = __ldg(job.norms + ir);
+            row.x = __float_as_uint(__ldg(job.norms + ir));
             if (QJL) { row.z = __ldg(job.qjl_bits + ir); row.w = __float_as_uint(__ldg(job.qjl_gamma + ir) * (QJL_C / D)); }
             else { row.z = ln; row.w = rw; }
-            if (job.scales) {
-                if (D != 256 || (blockIdx.x & 1) == 0) job.scales[int64_t(ln) * job.scale_lane_stride + rw] = nrm;
-                nrm = 1.f / job.tab_scale;
-            }
-            row.x = __float_as_uint(nrm);
         }
         const int r0 = __shfl_sync(0xffffffffu, in_row, 0);
         run = __all_sync(0xffffffffu, (in_row == r0 + lane && r0 >= 0) || lane >= RW);
@@ -367,7 +359,7 @@ __device__ __forceinline__ void produce(const Params& job, unsigned char* smem, 
         if (run && active) each<NK>([&](auto kc) { w[decltype(kc)::v] = load_run(kc); });
     }
     for (int it = 0; it < n_mine; ++it) {
-        const int sub = it * job.parts;
+        const int sub = it * 2;
         const uint4 row_cur = row;
         const int row_in = in_row;
         const bool run_cur = run, more = it + 1 < n_mine;
@@ -378,11 +370,10 @@ __device__ __forceinline__ void produce(const Params& job, unsigned char* smem, 
         if (more && run && active) each<NK>([&](auto kc) { wn[decltype(kc)::v] = load_run(kc); });
         // one pass writes the high and the low parts when the ring has room for both, else a pass each
         constexpr bool ONE_PASS = P::NB > 1;
-        for (int part = 0; part < job.parts; part += ONE_PASS ? 2 : 1) {
+        for (int part = 0; part < 2; part += ONE_PASS ? 2 : 1) {
             const int n0 = sub + part, bf = n0 % P::NB, bf2 = (n0 + 1) % P::NB;
-            const bool both = ONE_PASS && job.parts == 2;
             if (n0 / P::NB > 0) ok = wait_bar(A_FREE + bf, n0 / P::NB - 1);        // the products that read the buffer's previous tile have completed
-            if (ok && both && (n0 + 1) / P::NB > 0) ok = wait_bar(A_FREE + bf2, (n0 + 1) / P::NB - 1);
+            if (ok && ONE_PASS && (n0 + 1) / P::NB > 0) ok = wait_bar(A_FREE + bf2, (n0 + 1) / P::NB - 1);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) return;
             // (the products of tile it - 4 or a later one have completed; they could start only after the rows of tile it - 6 had been
@@ -409,7 +400,7 @@ __device__ __forceinline__ void produce(const Params& job, unsigned char* smem, 
                         const uint4 hi = tab.template lookup<0>(x);
                         if (active) *reinterpret_cast<uint4*>(d) = hi;
                     }
-                    if (ONE_PASS ? both : part == 1) {
+                    if (ONE_PASS || part == 1) {
                         const uint4 lo = tab.template lookup<2>(x);
                         if (active) *reinterpret_cast<uint4*>(ONE_PASS ? d + a2 : d) = lo;
                     }
@@ -419,7 +410,7 @@ __device__ __forceinline__ void produce(const Params& job, unsigned char* smem, 
             });
             fence_proxy_async();
             mbar_arrive(sbase + P::OFF_BAR + 8u * (A_FULL + bf));
-            if (both) mbar_arrive(sbase + P::OFF_BAR + 8u * (A_FULL + bf2));
+            if (ONE_PASS) mbar_arrive(sbase + P::OFF_BAR + 8u * (A_FULL + bf2));
         }
 #pragma unroll
         for (int k = 0; k < NK; ++k) w[k] = wn[k];
@@ -459,7 +450,7 @@ __global__ void __launch_bounds__(NT, 1) dequantize_tc_kernel(const __grid_const
         const float* src = which ? p.cent_lo : p.cent_hi;
         const int bits = which ? p.bits_lo : p.bits_hi;
         float c = 0.f;
-        if (src != nullptr && bits > 0 && k < (1 << bits)) c = src[k] * p.tab_scale;
+        if (src != nullptr && bits > 0 && k < (1 << bits)) c = src[k];
         const __half hi = __float2half_rn(c);
         const __half lo = __float2half_rn((c - __half2float(hi)) * 2048.f);
         reinterpret_cast<uint32_t*>(smem + P::OFF_CTAB)[tid] = uint32_t(__half_as_ushort(hi)) | (uint32_t(__half_as_ushort(lo)) << 16);
@@ -526,8 +517,8 @@ __global__ void __launch_bounds__(NT, 1) dequantize_tc_kernel(const __grid_const
                 const int st = it & 1;
                 const uint32_t acc = tmem_base + uint32_t(st) * 256u;
                 if (it >= 2) ok = wait_all(ACC_FREE + st, (it >> 1) - 1);
-                for (int part = 0; part < p.parts && ok; ++part) {
-                    const int s = it * p.parts + part, bf = s % P::NB;
+                for (int part = 0; part < 2 && ok; ++part) {
+                    const int s = it * 2 + part, bf = s % P::NB;
                     ok = wait_all(A_FULL + bf, s / P::NB);
                     if (!ok) break;
                     tc_fence_after();

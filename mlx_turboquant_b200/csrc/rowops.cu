@@ -29,7 +29,6 @@ struct RowArgs {
     const float* cent_hi; const float* cent_lo;
     const float* qjl_proj; const uint32_t* qjl_bits_in; const float* qjl_gamma_in;
     void* out; int out_dtype; int64_t out_lane_stride, out_row_stride;
-    float* scales; int64_t scale_lane_stride;      // dequantize: rows leave without their norms, which are copied here (or null)
 };
 
 __global__ void __launch_bounds__(NT) rowops_kernel(RowArgs a) {
@@ -85,7 +84,6 @@ __global__ void __launch_bounds__(NT) rowops_kernel(RowArgs a) {
             if (row < total_rows) {
                 const int64_t o = row / a.n_rows, r = row - o * a.n_rows;
                 nv = a.norms_in[o * a.in_lane_stride + r];
-                if (a.scales) { a.scales[o * a.scale_lane_stride + r] = nv; nv = 1.f; }
             }
             rown[tid] = nv;
         }
@@ -359,8 +357,7 @@ extern "C" int tq_quantize_pack_many(const tq_quantize_args* q, int n, void* str
 }
 
 namespace tq {
-int tq_dequantize_tc(const tq_dequantize_args* q, int n_jobs, cudaStream_t s, bool* handled, float* const* scales, int64_t scale_lane_stride,
-                     const int* parts, const float* tab_scale);      // dequantize_tc.cu
+int tq_dequantize_tc(const tq_dequantize_args* q, int n_jobs, cudaStream_t s, bool* handled);      // dequantize_tc.cu
 int g_tune_dequantize_tc = 1;      // 0: always the row kernel (testing)
 
 static int check_dequantize(const tq_dequantize_args* q) {
@@ -374,26 +371,25 @@ static int check_dequantize(const tq_dequantize_args* q) {
     return TQ_OK;
 }
 
-static int dequantize_row_kernel(const tq_dequantize_args* q, float* scales, int64_t scale_lane_stride, cudaStream_t s) {
+static int dequantize_row_kernel(const tq_dequantize_args* q, cudaStream_t s) {
     RowArgs a{};
     a.mode = MODE_DEQUANT; a.d = q->d; a.inverse = 1; a.n_lanes = q->n_lanes; a.n_rows = q->n_rows;
     a.rot = q->rot; a.in_hi = q->packed_hi; a.in_lo = q->packed_lo; a.norms_in = q->norms; a.in_lane_stride = q->in_lane_stride;
     a.bits_hi = q->bits_hi; a.bits_lo = q->bits_lo; a.cent_hi = q->cent_hi; a.cent_lo = q->cent_lo;
     a.qjl_proj = q->qjl_proj; a.qjl_bits_in = q->qjl_bits; a.qjl_gamma_in = q->qjl_gamma;
     a.out = q->out; a.out_dtype = q->out_dtype; a.out_lane_stride = q->out_lane_stride; a.out_row_stride = q->out_row_stride;
-    a.scales = scales; a.scale_lane_stride = scale_lane_stride;
     return launch_rowops(a, s, "tq_dequantize");
 }
 
-// One or two jobs (the caller has validated them); scales, parts, tab_scale as in tq_dequantize_tc, all null for plain rows.
-int dequantize_jobs(const tq_dequantize_args* q, int n, float* const* scales, int64_t scale_lane_stride, const int* parts, const float* tab_scale, cudaStream_t s) {
+// One or two jobs (the caller has validated them).
+static int dequantize_jobs(const tq_dequantize_args* q, int n, cudaStream_t s) {
     if (g_tune_dequantize_tc) {
         bool handled = false;
-        const int rc = tq_dequantize_tc(q, n, s, &handled, scales, scale_lane_stride, parts, tab_scale);
+        const int rc = tq_dequantize_tc(q, n, s, &handled);
         if (handled) return rc;
     }
     for (int i = 0; i < n; ++i)
-        if (int rc = dequantize_row_kernel(q + i, scales ? scales[i] : nullptr, scale_lane_stride, s)) return rc;
+        if (int rc = dequantize_row_kernel(q + i, s)) return rc;
     return TQ_OK;
 }
 }  // namespace tq
@@ -402,7 +398,7 @@ extern "C" int tq_dequantize(const tq_dequantize_args* q, void* stream) {
     if (!q) return fail(TQ_ERR_INVALID, "tq_dequantize: null args");
     if (int rc = check_dequantize(q)) return rc;
     if (q->n_lanes == 0 || q->n_rows == 0) return TQ_OK;
-    return dequantize_jobs(q, 1, nullptr, 0, nullptr, nullptr, static_cast<cudaStream_t>(stream));
+    return dequantize_jobs(q, 1, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int tq_dequantize_pair(const tq_dequantize_args* k, const tq_dequantize_args* v, void* stream) {
@@ -415,5 +411,5 @@ extern "C" int tq_dequantize_pair(const tq_dequantize_args* k, const tq_dequanti
     }
     if (n == 0) return TQ_OK;
     if (n == 2 && (q[0].d != q[1].d || q[0].rot != q[1].rot || q[0].out_dtype != q[1].out_dtype)) return fail(TQ_ERR_INVALID, "tq_dequantize_pair: the two must share d, rot and out_dtype");
-    return dequantize_jobs(q, n, nullptr, 0, nullptr, nullptr, static_cast<cudaStream_t>(stream));
+    return dequantize_jobs(q, n, static_cast<cudaStream_t>(stream));
 }
