@@ -2,9 +2,10 @@
 // fractional split (4 | 3 or 3 | 2 bits), head_dim 64 / 96 / 128 / 256, with or without the QJL sign sketches.
 //
 // One persistent CTA per SM; the packed 16-token tiles of ALL cache lanes (sequence, KV head, head group) are dealt out as
-// one flat sequence, an equal contiguous run per warp (as decode_stream.cu does for 4-bit keys / 2-bit values).  Three
-// launches chained with programmatic dependent launch: lut_query_kernel (rotates the queries once, on mma.sync),
-// decode_lut_kernel, lut_merge_kernel (log-sum-exp merge, rotation back, normalisation).
+// one flat sequence, an equal contiguous run per warp (as decode_stream.cu does for 4-bit keys / 2-bit values).  Two
+// launches chained with programmatic dependent launch: decode_lut_kernel and lut_merge_kernel (log-sum-exp merge, rotation
+// back, normalisation).  A CTA rotates the queries of its lanes itself where it has two lanes at most; many short lanes, and a
+// fused gather, have lut_query_kernel rotate all of them in a launch before (on mma.sync).
 //
 // Operands.  What bounds a decode step at these widths is how packed codes become fp16 operand registers, so no code is
 // ever looked at on its own: one shared-memory lookup turns a PAIR of codes (4 bits: a byte; 3 bits: a six-bit field) or

@@ -149,7 +149,7 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
 }
 // D = A.B (+ D when accumulate != 0)
 // (issued by one elected lane of a warp in uniform control flow: the operands then come straight from uniform registers, where a
-// single thread in a divergent branch moves each of them over, 70 cycles per instruction)
+// single thread in a divergent branch moves each of them over one by one)
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
