@@ -220,7 +220,7 @@ typedef struct {
 /* Ordering on the stream.  tq_decode_attn is launched with programmatic stream serialisation (unless the "decode_pdl"
  * tuning knob is 0): its CTAs may become resident while the preceding kernel on the stream is still finishing.  Before
  * that kernel has completed they read only rot, the centroid tables and `tables` (which the preceding kernel must not
- * write) and ask for lines of the packed arrays in L2 (harmless whoever is writing them); q, the cache contents, the
+ * write) and ask for lines of the cache's arrays in L2 (harmless whoever is writing them); q, the cache contents, the
  * workspace and the output are touched only after the preceding kernel has completed and its writes are visible. */
 
 /* Bytes of the constants buffer for tq_decode_args.tables (host arithmetic); 0 when no kernel uses prebuilt constants
@@ -342,6 +342,7 @@ float tq_fp16_table_scale(const float* centroids_host, int n);
  *   "decode_stream_min_run" 1.. (fewest packed 16-token tiles per warp of the persistent grid for which it is chosen over the
  *   table-lookup kernel, default 24; over the general kernel a third of that),
  *   "decode_lut" 0/1/2 (the lookup kernel is never chosen, where it is the faster one, default, or whenever it can run),
+ *   "decode_lane" 0/1/2 (the one-launch kernel likewise), "decode_lane_ctas" 0 (auto)..16 (its CTAs per cache lane: 1 to 6, 8, 12, 16),
  *   "decode_stream_max_parts" 1..64 (most partial results per lane with which it is chosen over the table-lookup kernel; default 40).
  * Changing them changes tq_decode_workspace_bytes for the same sizes. */
 int tq_set_tuning(const char* key, int value);
@@ -353,6 +354,9 @@ int tq_set_tuning(const char* key, int value);
  * 4 | 3 and 3 | 2, d = 64 / 96 / 128 / 256, sign sketches allowed).  Negative: the arguments are invalid
  * (tq_last_error has the text). */
 int tq_decode_kernel_choice(const tq_decode_args* a);
+/* Whether tq_decode_attn would do the call in one launch, a cluster of CTAs per cache lane merging on chip, in the place of the kernel that
+ * tq_decode_kernel_choice names (which keeps its workspace requirement): the CTAs per lane, or 0.  Negative: the arguments are invalid. */
+int tq_decode_one_launch(const tq_decode_args* a);
 
 #ifdef __cplusplus
 }

@@ -3,8 +3,9 @@
 //
 // This file: the host side (argument checks, split plan, workspace layout, launch) and the GENERAL kernel, which
 // handles every bit width (1-4, fractional splits) and d in {64, 96, 128, 256}.  4-bit keys with 2-bit values at
-// d = 128 take the table-lookup kernel of decode_direct.cu instead, and the same widths at d = 96 / 128 (sign sketches
-// allowed) the persistent streaming kernel of decode_stream.cu once every warp of its grid gets a long run of tiles.
+// d = 128 take the table-lookup kernel of decode_direct.cu instead, the same widths at d = 96 / 128 (sign sketches
+// allowed) the persistent streaming kernel of decode_stream.cu once every warp of its grid gets a long run of tiles, other widths
+// the lookup kernel of decode_lut.cu; small and middling calls of any of them one launch of clusters (decode_lane.cu).
 //
 // decode_attn_kernel, grid (splits, kv_heads * head_groups, batch).  Every CTA
 //   1. rotates the query heads of its GQA group once (q @ R^T, float32), folds scale*log2(e) in and keeps
@@ -597,6 +598,8 @@ extern int g_tune_dequantize_tc;       // rowops.cu: 0 = dequantize always on th
 extern int g_tune_prefill_tc;          // prefill.cu: 0 = several-query-token attention always on the mma.sync kernel
 static int g_tune_pdl = 1;             // programmatic dependent launch between consecutive calls
 static int g_tune_lut = 1;             // 0: never take the lookup kernel of decode_lut.cu; 2: whenever it can (testing)
+static int g_tune_lane = 1;            // 0: never take the one-launch kernel of decode_lane.cu; 2: whenever it can (testing)
+static int g_tune_lane_ctas = 0;       // > 0: its CTAs per lane
 static int g_tune_stream = 1;          // 0: never take the streaming kernel
 static int g_tune_stream_min_run = 24; // fewest packed tiles per warp for which the streaming kernel is chosen over the table-lookup kernel (a third of it over the general kernel)
 static int g_tune_stream_max_parts = 40;  // most partials per lane with which it is chosen over the table-lookup kernel (64 over the general kernel)
@@ -706,7 +709,7 @@ template <int D, bool QJL> static int launch_decode(const DecodeParams& p, cudaS
 struct LutRivals {
     int64_t c_len, lanes, p_tiles, d_tiles, run;       // run: packed tiles per warp of the streaming kernel
     int sms, d, G, dense_dtype;
-    bool qjl, direct, stream, bytes;                   // which rival would run; 4-bit keys and 2-bit values
+    bool qjl, direct, stream, bytes, wide;             // which rival would run; 4-bit keys and 2-bit values; 6.5 bits or more a pair
 };
 static bool lut_is_best(const LutRivals& r) {
     const bool fp16 = r.dense_dtype == TQ_F16, bf16 = r.dense_dtype == TQ_BF16;
@@ -753,6 +756,27 @@ static bool lut_is_best(const LutRivals& r) {
         return tiles < 4500 || tiles >= 30000 || r.lanes <= 8 || 2 * r.lanes > 3 * r.sms;
     }
     return !(fp16 && r.G == 1 && r.d <= 96 && tiles < (r.qjl ? r.d == 64 ? 5000 : 0 : 7000));
+}
+
+// Whether the one-launch kernel of decode_lane.cu takes a call that it can run: its plan's cost against what the other kernel takes, in us
+// (both fitted to 965 measured calls, log errors 0.06 to 0.12; other / one launch).  Lookup kernel: 8 lanes x 48 + 16 tiles at d = 96 16.6 /
+// 8.4, 3 x 369 27.9 / 14.3, 160 x 67 40.3 / 28.4, 32 x 737 38.0 / 32.8, 64 x 1108 59.3 / 58.4, 8 x 1825 at d = 256 55.3 / 77.8, 736 x 102 73.6
+// / 109.  Table-lookup kernel: 8 x 38 tiles 11.9 / 8.4, 8 x 2048 17.0 / 33.8; bfloat16 4 x 113 23.2 / 11.3.  General kernel: 8.7 / 8.5,
+// 16.8 / 12.2, 216 x 49 at d = 64 23.4 / 13.6.  Streaming kernel: while its warps' runs are short (256 x 109 tiles at d = 96 36.2 / 26.2, 248
+// x 218 50.3 / 42.1; 448 x 641 at d = 128 157 / 255).  Of those calls 597 go to one launch, five of them more than 3 % slower.
+static bool lane_is_best(const LutRivals& r, const LanePlan& ln, const StreamPlan* lut, bool stream) {
+    if (!lut && stream && r.run >= 2 * g_tune_stream_min_run) return false;
+    const int heads = std::min(r.G, HPG);
+    const double dd = r.d / 128.0, tiles = double(r.p_tiles + r.d_tiles), lanes = double(r.lanes * ((r.G + HPG - 1) / HPG)), per_sm = lanes * tiles / r.sms;
+    const double bf16 = r.dense_dtype == TQ_BF16, many = r.G > 4, qjl = r.qjl, wide = r.wide;
+    double other;
+    if (lut) other = 5.0 + 14.7 * dd + 3.1 * qjl + many * dd + (lut->fold ? 0.0 : 0.4 + 0.0137 * dd * lanes * heads) + bf16 + (r.d == 256 ? 2.3 : 0.0) +
+                     per_sm * (0.026 + 0.070 * dd + 0.029 * dd * qjl + 0.011 * dd * wide);
+    else if (stream) other = (r.d == 96 ? 24.0 : 43.0) + per_sm * (0.058 + 0.020 * qjl) + 0.004 * lanes * heads;
+    else if (r.direct) other = 9.1 + 0.42 * std::min(r.G, 4) + 6.2 * bf16 + 5.0 * many + 0.095 * per_sm + 11.3 * std::max(0.0, 2.0 * lanes / r.sms - 1.0);
+    else other = 7.9 + (r.d == 96 ? 4.9 : 0.0) + 3.9 * many + 1.8 * bf16 + 0.25 * std::min(r.G, 4) + 0.063 * per_sm + 0.0055 * tiles + 0.026 * lanes +
+                 9.7 * std::max(0.0, lanes / r.sms - 1.0);
+    return ln.cost + 1.2 * many < 0.9 * other;
 }
 
 // Validates the arguments, picks the path and the split plan and fills the kernel parameters.
@@ -821,19 +845,26 @@ int decode_prepare(const tq_decode_args* a, void* workspace, size_t workspace_by
     }
     const LutRivals r{a->c_len, int64_t(a->batch) * a->n_kv_heads, (a->c_len + TILE - 1) / TILE, (dense_len + TILE - 1) / TILE, stp.range,
                       sm_count(), d, a->n_q_heads / a->n_kv_heads, a->dense_dtype, qjl, direct, stream,
-                      a->k_bits_hi == 4 && !a->k_bits_lo && a->v_bits_hi == 2 && !a->v_bits_lo};
+                      a->k_bits_hi == 4 && !a->k_bits_lo && a->v_bits_hi == 2 && !a->v_bits_lo,
+                      a->k_bits_hi + (a->k_bits_lo ? a->k_bits_lo : a->k_bits_hi) + a->v_bits_hi + (a->v_bits_lo ? a->v_bits_lo : a->v_bits_hi) >= 13};
     const bool lut_best = lut_is_best(r);
-    bool lut = ((lut_best && g_tune_lut) || g_tune_lut == 2) && !g_tune_force_general && a->c_lane_stride % 16 == 0 && aligned(a->q, 8) &&
+    const bool tab = !g_tune_force_general && a->c_lane_stride % 16 == 0 && aligned(a->q, 8) &&            // (rows that the lookup kernels' copies take)
                aligned(a->k_hi, 16) && aligned(a->v_hi, 16) && aligned(a->k_norms, 16) && aligned(a->v_norms, 16) &&
                (!a->k_bits_lo || aligned(a->k_lo, 16)) && (!a->v_bits_lo || aligned(a->v_lo, 16)) &&
                (!qjl || (aligned(a->k_qjl_bits, 16) && aligned(a->v_qjl_bits, 16) && aligned(a->k_qjl_gamma, 16) && aligned(a->v_qjl_gamma, 16) && aligned(a->qjl_proj, 16))) &&
                (a->sink_len == 0 || (aligned(a->sink_k, 16) && aligned(a->sink_v, 16))) && (!a->res_k || (aligned(a->res_k, 16) && aligned(a->res_v, 16)));
+    bool lut = ((lut_best && g_tune_lut) || g_tune_lut == 2) && tab;
     if (lut) {
         const StreamPlan lp = lut_plan(a->batch, a->n_q_heads, a->n_kv_heads, d, a->c_len, dense_len, sm_count());
         lut = lp.ok && lut_supported(d, qjl, a->c_len > 0 ? a->k_bits_hi : 4, a->c_len > 0 ? a->k_bits_lo : 0, a->c_len > 0 ? a->v_bits_hi : 4, a->c_len > 0 ? a->v_bits_lo : 0);
         if (lut) stp = lp;
     }
     if (lut) stream = false;
+    LanePlan ln{};
+    if (g_tune_lane && tab && a->c_len > 0 && a->dense_dtype != TQ_F32 && lut_supported(d, qjl, a->k_bits_hi, a->k_bits_lo, a->v_bits_hi, a->v_bits_lo)) {
+        ln = lane_plan(r.lanes * ((r.G + HPG - 1) / HPG), d, qjl, a->k_bits_hi, a->k_bits_lo, a->v_bits_hi, a->v_bits_lo, a->c_len, dense_len, g_tune_lane_ctas);
+        if (g_tune_lane == 1 && !lane_is_best(r, ln, lut ? &stp : nullptr, stream)) ln.c = 0;
+    }
     const SplitPlan sp = plan_splits(a->batch, a->n_q_heads, a->n_kv_heads, a->c_len, dense_len, sm_count(), direct);
     const WsLayout wl = ws_layout(a->batch, a->n_q_heads, a->n_kv_heads, d, sp);
     const size_t st_base = align_up(std::max(size_t(a->batch) * a->n_kv_heads * sp.hg * sizeof(int), COUNTER_AREA), 256);
@@ -893,6 +924,10 @@ int decode_prepare(const tq_decode_args* a, void* workspace, size_t workspace_by
         p.st_part = reinterpret_cast<float*>(ws + st_base + stp.q16_bytes);
         if (!(p.status = decode_status_ptr())) return fail(TQ_ERR_LAUNCH, "tq_decode_attn: cannot locate the status word");
     }
+    if (ln.c > 0) {        // (in the place of the kernel chosen above, whose requirements hold as before)
+        p.ln_c = ln.c; p.ln_per_sm = ln.per_sm; p.ln_pw = ln.pw; p.ln_dw = ln.dw; p.ln_ns = ln.ns;
+        if (!(p.status = decode_status_ptr())) return fail(TQ_ERR_LAUNCH, "tq_decode_attn: cannot locate the status word");
+    }
     *out = p;
     *direct_out = direct && !stream && !lut;
     return TQ_OK;
@@ -904,6 +939,7 @@ int decode_launch(const DecodeParams& p0, bool direct, cudaStream_t s) {
         if (int rc = launch_gather_wait(p.await_ll, p.await_epochs, p.await_words, p.await_out, p.await_polls, s)) return rc;
         p.await_ll = nullptr;
     }
+    if (p.ln_c > 0) return launch_decode_lane(p, s);
     if (p.st_grid > 0) return p.st_lut ? launch_decode_lut(p, s) : launch_decode_stream(p, s);
     if (direct) return launch_decode_direct(p, s);
     const bool qjl = p.qjl_proj != nullptr;
@@ -924,6 +960,8 @@ extern "C" int tq_set_tuning(const char* key, int value) {
     else if (k == "decode_force_general" && (value == 0 || value == 1)) g_tune_force_general = value;
     else if (k == "decode_pdl" && (value == 0 || value == 1)) g_tune_pdl = value;
     else if (k == "decode_lut" && value >= 0 && value <= 2) g_tune_lut = value;
+    else if (k == "decode_lane" && value >= 0 && value <= 2) g_tune_lane = value;
+    else if (k == "decode_lane_ctas" && value >= 0 && value <= 16) g_tune_lane_ctas = value;
     else if (k == "decode_stream" && (value == 0 || value == 1)) g_tune_stream = value;
     else if (k == "decode_stream_min_run" && value >= 1 && value <= (1 << 20)) g_tune_stream_min_run = value;
     else if (k == "decode_stream_max_parts" && value >= 1 && value <= 64) g_tune_stream_max_parts = value;
@@ -940,6 +978,13 @@ extern "C" int tq_decode_kernel_choice(const tq_decode_args* a) {
     bool direct = false;
     if (decode_prepare(a, a ? a->workspace : nullptr, a ? a->workspace_bytes : 0, &p, &direct)) return -1;
     return p.st_grid > 0 ? (p.st_lut ? 3 : 2) : direct ? 1 : 0;
+}
+
+extern "C" int tq_decode_one_launch(const tq_decode_args* a) {
+    DecodeParams p;
+    bool direct = false;
+    if (decode_prepare(a, a ? a->workspace : nullptr, a ? a->workspace_bytes : 0, &p, &direct)) return -1;
+    return p.ln_c > 0 ? p.ln_c : 0;
 }
 
 extern "C" int tq_gather_wait(const unsigned long long* ll, const unsigned* epochs, int64_t n_words, void* out, void* stream) {

@@ -56,6 +56,7 @@ struct DecodeParams {
     int st_lut, st_fold;               // decode_lut.cu runs (decode_stream.cu otherwise); its CTAs fold their warps' partials
     int st_npp, st_nd, st_dt;          // packed-partial slots per lane; dense items per lane and tiles per dense item
     int64_t st_range;                  // packed tiles per warp
+    int ln_c, ln_per_sm, ln_pw, ln_dw, ln_ns;      // decode_lane.cu: CTAs per lane (0: another kernel runs) and SM, a lane's warps with packed / uncompressed tiles, ring stages
     __half* st_q16;                    // workspace: per query head the rotated (stream: | raw) (| sketch) scaled fp16 query
     float* st_part;                    // workspace: partials (lane, slot, head, D + 36)
 };
@@ -103,6 +104,10 @@ int launch_decode_stream(const DecodeParams& p, cudaStream_t s);
 bool lut_supported(int d, bool qjl, int kb_hi, int kb_lo, int vb_hi, int vb_lo);
 StreamPlan lut_plan(int batch, int n_q_heads, int n_kv_heads, int d, int64_t c_len, int64_t dense_len, int sms);
 int launch_decode_lut(const DecodeParams& p, cudaStream_t s);
+// decode_lane.cu: the lookup kernel's operands in one launch, a cluster of CTAs per lane.
+struct LanePlan { int c, per_sm, pw, dw, ns; double cost; };       // (c = 0: it does not take the call)
+LanePlan lane_plan(int64_t lanes, int d, bool qjl, int kb_hi, int kb_lo, int vb_hi, int vb_lo, int64_t c_len, int64_t dense_len, int force_c);
+int launch_decode_lane(const DecodeParams& p, cudaStream_t s);
 int launch_gather_wait(const unsigned long long* ll, const unsigned* epochs, int64_t n_words, void* out, int max_polls, cudaStream_t s);
 int* decode_status_ptr();          // device address of the status word on the current device (null on error)
 int decode_status_host();          // code of the first bounded wait that ran out on this device (0 = none), -1 on error

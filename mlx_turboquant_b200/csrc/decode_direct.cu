@@ -662,9 +662,20 @@ unsigned probe_smem_base() {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return ~0u;
     if (!have[dev].load(std::memory_order_acquire)) {
+        // (on a stream of its own, so that a first call made while another stream is being captured does not end the capture)
         unsigned v = ~0u;
-        smem_base_probe<<<1, 32, 1024>>>();
-        if (cudaGetLastError() != cudaSuccess || cudaMemcpyFromSymbol(&v, g_probe_base, sizeof(v)) != cudaSuccess) return ~0u;
+        cudaStream_t st = nullptr;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return ~0u;
+        bool ok = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess;
+        if (ok) {
+            smem_base_probe<<<1, 32, 1024, st>>>();
+            ok = cudaGetLastError() == cudaSuccess && cudaMemcpyFromSymbolAsync(&v, g_probe_base, sizeof(v), 0, cudaMemcpyDeviceToHost, st) == cudaSuccess;
+            ok = cudaStreamSynchronize(st) == cudaSuccess && ok;
+            cudaStreamDestroy(st);
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (!ok) return ~0u;
         cache[dev].store(v, std::memory_order_relaxed);
         have[dev].store(true, std::memory_order_release);
     }

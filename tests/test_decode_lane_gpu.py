@@ -1,0 +1,139 @@
+"""The one-launch decode kernel (a cluster of CTAs per cache lane) against the oracle: every code format and head_dim, every cluster size,
+tiles that do and do not fill the warps, head groups, regions, appends, and that the rule for it leaves long contexts alone."""
+
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+import test_decode_gpu as general
+import test_decode_lut_gpu as lookup
+from test_decode_gpu import _case, _check
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture()
+def lane():
+    """lane(ctas): the kernel for every call that it can run, with so many CTAs per lane (0: its own choice)."""
+    from mlx_turboquant_b200.kernels import set_tuning
+
+    def force(ctas):
+        set_tuning("decode_lane", 2)
+        set_tuning("decode_lane_ctas", ctas)
+    yield force
+    set_tuning("decode_lane", 1)
+    set_tuning("decode_lane_ctas", 0)
+
+
+def _run(c, q, ref, ctas=0):
+    from mlx_turboquant_b200 import _lib
+    out = c.attend(q, out_dtype=torch.float32)
+    got = _lib.lib().tq_decode_one_launch(C.byref(c._dargs))
+    assert got == ctas if ctas else got > 0
+    _check(out, ref)
+    assert _lib.lib().tq_device_status() == 0
+
+
+@pytest.mark.parametrize("d", (64, 96, 128, 256))
+@pytest.mark.parametrize("kb,vb", ((4, 2), (4, 4), (3, 2), (2, 3), (3.5, 2.5), (2.5, 3.5), (2, 2)))
+@pytest.mark.parametrize("qjl", (False, True))
+def test_every_format(oracle, lane, d, kb, vb, qjl):
+    rs = np.random.RandomState(d + int(10 * kb + vb))
+    c, q, ref = _case(oracle, rs, 2, 8, 4, 333, d, kb, vb, 32, 8, qjl=qjl, bf16=qjl)
+    lane(0)
+    _run(c, q, ref)
+
+
+@pytest.mark.parametrize("d", (64, 96, 128, 256))
+@pytest.mark.parametrize("ctas", (1, 2, 3, 4, 5, 6, 8, 12, 16))
+def test_every_cluster_size(oracle, lane, d, ctas):
+    """More warps than tiles, and a few tiles per warp; d / ctas columns per CTA with remainders."""
+    rs = np.random.RandomState(d + ctas)
+    lane(ctas)
+    for t in (100, 900):
+        c, q, ref = _case(oracle, rs, 1, 12, 2, t, d, 3, 4, 16, 4, bf16=ctas % 2 == 0, qjl=d != 128)
+        _run(c, q, ref, ctas)
+
+
+@pytest.mark.parametrize("b,hq,hkv,t,rw,sink", ((1, 8, 8, 49, 16, 4), (3, 48, 3, 700, 16, 4), (70, 16, 16, 90, 16, 4), (1, 4, 1, 33, 0, 0), (2, 8, 2, 400, 0, 8),
+                                                  (2, 8, 2, 400, 150, 0), (1, 8, 1, 1000, 128, 128)))
+@pytest.mark.parametrize("bf16", (False, True))
+def test_heads_lanes_and_regions(oracle, lane, b, hq, hkv, t, rw, sink, bf16):
+    rs = np.random.RandomState(b + t)
+    c, q, ref = _case(oracle, rs, b, hq, hkv, t, 128, 4, 2, rw, sink, bf16=bf16)
+    lane(0)
+    _run(c, q, ref)
+
+
+@pytest.mark.parametrize("v_scale", (1e5, 1e-6))
+def test_value_norms_far_outside_the_fp16_range(oracle, lane, v_scale):
+    rs = np.random.RandomState(13)
+    c, q, ref = _case(oracle, rs, 2, 8, 8, 600, 128, 3, 3, 32, 16, dtype=np.float32, v_scale=v_scale, bf16=True, qjl=True)
+    lane(3)
+    _run(c, q, ref, 3)
+
+
+def test_steps_append(lane):
+    """The appended token counts, and its rows are in the buffer: steps equal update followed by attend; across a drain too."""
+    from mlx_turboquant_b200 import TurboQuantKVCache
+    g = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda n, h=4: torch.randn(2, h, n, 96, device="cuda", generator=g).bfloat16()  # noqa: E731
+    cs = [TurboQuantKVCache(head_dim=96, num_kv_heads=4, key_bits=3.5, value_bits=3, residual_window=32, fp16_sink_size=16) for _ in range(2)]
+    k, v = r(300), r(300)
+    for c in cs:
+        c.update(k, v)
+    lane(4)
+    for _ in range(40):
+        kn, vn, q = r(1), r(1), r(1, 16) / 96 ** 0.5
+        o = cs[0].decode_step(q, kn, vn)
+        cs[1].update(kn, vn)
+        assert torch.equal(o, cs[1].attend(q))
+    n = cs[0]._fp16_len
+    assert n == cs[1]._fp16_len and torch.equal(cs[0].keys[:, :, :n], cs[1].keys[:, :, :n]) and torch.equal(cs[0].values[:, :, :n], cs[1].values[:, :, :n])
+
+
+def test_what_it_leaves_to_the_others(oracle, lane):
+    """float32 rows, caches without packed tokens and, by its rule, long contexts of many lanes."""
+    from mlx_turboquant_b200 import _lib
+    from mlx_turboquant_b200.kernels import set_tuning
+    lane(0)
+    takes = lambda c: _lib.lib().tq_decode_one_launch(C.byref(c._dargs))  # noqa: E731
+    for t, dtype in ((300, np.float32), (20, np.float16)):
+        c, q, ref = _case(oracle, np.random.RandomState(t), 2, 8, 2, t, 128, 4, 2, 32, 8, dtype=dtype)
+        _check(c.attend(q, out_dtype=torch.float32), ref)
+        assert takes(c) == 0
+    set_tuning("decode_lane", 1)
+    from mlx_turboquant_b200 import TurboQuantKVCache
+    for b, t, want in ((8, 16384, False), (1, 600, True)):
+        c = TurboQuantKVCache(head_dim=128, num_kv_heads=8, key_bits=4, value_bits=2, residual_window=128, fp16_sink_size=128)
+        x = torch.randn(b, 8, t, 128, device="cuda").half()
+        c.update(x, x)
+        c.attend(torch.zeros(b, 32, 1, 128, device="cuda").half())
+        assert (takes(c) > 0) == want
+
+
+@pytest.fixture()
+def off():
+    from mlx_turboquant_b200.kernels import set_tuning
+    set_tuning("decode_lane", 0)
+    yield
+    set_tuning("decode_lane", 1)
+
+
+@pytest.mark.parametrize("d", (64, 96, 128, 256))
+@pytest.mark.parametrize("kb,vb", ((4, 4), (3, 2), (2, 3), (3.5, 2.5), (2.5, 3.5), (2, 2)))
+@pytest.mark.parametrize("qjl", (False, True))
+def test_the_lookup_kernel_where_this_one_would_take_the_call(oracle, off, d, kb, vb, qjl):
+    lookup.test_every_format(oracle, d, kb, vb, qjl)
+
+
+@pytest.mark.parametrize("b,hq,hkv,t", ((1, 8, 1, 2500), (3, 48, 3, 700), (70, 16, 16, 90), (2, 12, 4, 130)))
+def test_lookup_kernel_lanes_and_folds(oracle, off, b, hq, hkv, t):
+    lookup.test_lanes_runs_and_folds(oracle, b, hq, hkv, t, True)
+
+
+@pytest.mark.parametrize("t", (129, 300, 2500))
+def test_the_table_lookup_kernel(oracle, off, t):
+    general.test_k4v2_direct_path_lengths(oracle, t)
