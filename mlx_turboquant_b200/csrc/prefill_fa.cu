@@ -26,15 +26,15 @@
 //
 // fa_kernel: a CTA owns NQ (2; 1 at d = 256) tiles of 128 rows = 128 / GP query tokens x the GP query heads of a GQA group, and a
 // range of key tiles (TN tokens each), packed tokens first:
-//   * 4 NQ softmax warps, a row per thread: tcgen05.ld of the row's TN scores into registers, one multiply-add each
-//     (packed in pairs), maximum, ex2, P (fp16) back into tensor memory over the scores it came from;
+//   * 8 NQ softmax warps, two rows' shares per thread: tcgen05.ld of the scores as mma.sync fragments, one multiply-add each (packed in
+//     pairs), ex2, P (fp16) back into tensor memory over the scores it came from; a row's reference maximum is looked at through its sum;
 //   * one warp issues S = Q K^T (both operands in shared memory) and O += P V (P from tensor memory), the tiles of the two
 //     query blocks alternating so that one block's softmax runs under the other's products;
 //   * one thread each keeps four key tiles (and eight tiles' norms) and four value tiles in flight (tiled TMA, bulk copies); scores
 //     are two key tiles ahead of the softmax;
 //   * between the two regions the softmax warps leave O as high and low fp16 parts where the scores were, the MMA warp multiplies
 //     them with R's parts in place (three products, the small ones first) and the raw queries replace the rotated ones.
-//   512 queries x 32 lanes over 16,384 tokens at d = 128: 700 us = 775 TFLOP/s (350 with the unpacking inside the kernel).
+//   512 queries x 32 lanes over 16,384 tokens at d = 128: 610 us = 880 TFLOP/s (350 with the unpacking inside the kernel).
 //
 // Every mbarrier wait is bounded; a wait that runs out leaves status 111 (tq_device_status) and raises a flag that ends
 // every other wait; copies and products in flight are waited for (bounded), tensor memory is freed on every path.
@@ -65,7 +65,7 @@ template <int D> struct Plan {
     static constexpr int ST = D == 256 ? 2 : 4;        // key tiles (and value tiles) in flight
     static constexpr int NBLK = (D + 63) / 64;         // 64-column blocks of a row
     static constexpr int DP = NBLK * 64;               // columns of O (d = 96: the last 32 are zeros)
-    static constexpr int NT = NQ * 128 + 96;           // softmax warps, MMA warp, a TMA warp for keys and norms, one for values
+    static constexpr int SW = NQ * 8, NT = SW * 32 + 96;      // softmax warps; MMA warp, a TMA warp for keys and norms, one for values
     static constexpr uint32_t QBLK = TM * 128u, KBLK = TN * 128u;            // bytes of a 64-column block
     static constexpr uint32_t Q_TILE = NBLK * QBLK, K_TILE = NBLK * KBLK;
     static constexpr uint32_t OFF_Q = 0, OFF_K = NQ * Q_TILE, OFF_V = OFF_K + ST * K_TILE;
@@ -73,7 +73,8 @@ template <int D> struct Plan {
     static constexpr uint32_t OFF_R = D == 64 ? OFF_SC + NSC * 2 * TN * 4 : OFF_K;      // R (see below): through the key ring where it has no room of its own
     static constexpr uint32_t OFF_BAR = OFF_SC + NSC * 2 * TN * 4 + (D == 64 ? 2 * 64 * 128 : 0);
     static constexpr uint32_t OFF_SLOT = OFF_BAR + 464;                      // [0] tensor-memory base, [1] abort
-    static constexpr size_t NEED = OFF_SLOT + 16 + 1024, SMEM = NEED > 116 * 1024 ? NEED : 116 * 1024;      // one CTA per SM: it takes all of the tensor memory
+    static constexpr uint32_t OFF_ROW = OFF_SLOT + 16;                       // float2 [NQ * 128]: sum and maximum of a row
+    static constexpr size_t NEED = OFF_ROW + NQ * TM * 8 + 1024, SMEM = NEED > 116 * 1024 ? NEED : 116 * 1024;      // one CTA per SM: it takes all of the tensor memory
     static constexpr uint32_t COL_O = NQ * SB * TN;                          // scores first, then the accumulators
     // rotation of the packed tokens' sums: they sit in tensor memory as A operands (high parts and low parts, two per column) where
     // scores were (d = 256: the low parts behind the accumulator), R as RC columns at a time, high, then low parts, passes taking turns
@@ -173,6 +174,42 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
                    "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
                  : "memory");
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+                 : "memory");
+}
+// Sixteen rows as mma.sync accumulator fragments: of eight columns, lane 4 g + t holds columns 2 t, + 1 of row g (r[0], r[1]) and of row g + 8
+// (r[2], r[3]).  64 columns; 32 of them; and, stored, 64 fp16 values: columns 2 t, + 1 of each row packed into r[0], r[1].
+__device__ __forceinline__ void tmem_ld_frag64(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                 : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_st_frag32(uint32_t taddr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st_half64(uint32_t taddr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+                 : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // two float32 at once
@@ -257,19 +294,19 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(const __grid_constan
     if (tid == 0) {
         for (int i = 0; i < 4; ++i) {
             mbar_init(bar(K_FULL + i), 1); mbar_init(bar(K_FREE + i), 1); mbar_init(bar(V_FULL + i), 1); mbar_init(bar(V_FREE + i), 1);
-            mbar_init(bar(S_FULL + i), 1); mbar_init(bar(P_FULL + i), 128);
+            mbar_init(bar(S_FULL + i), 1); mbar_init(bar(P_FULL + i), 256);
         }
         for (int i = 0; i < 2; ++i) { mbar_init(bar(O_DONE + i), 1); mbar_init(bar(ALL_DONE + i), 1); }
         mbar_init(bar(DRAIN), 1);
         for (int i = 0; i < 2; ++i) {
-            mbar_init(bar(ROT_IN + i), 1); mbar_init(bar(ROT_A + i), 128); mbar_init(bar(ROT_OUT + i), 1); mbar_init(bar(Q_FULL + i), 1);
+            mbar_init(bar(ROT_IN + i), 1); mbar_init(bar(ROT_A + i), 256); mbar_init(bar(ROT_OUT + i), 1); mbar_init(bar(Q_FULL + i), 1);
             mbar_init(bar(R_FULL + i), 1); mbar_init(bar(R_DONE + i), 1);
         }
-        for (int i = 0; i < NSC; ++i) { mbar_init(bar(SC_FULL + i), 1); mbar_init(bar(SC_FREE + i), NQ * 128); }
+        for (int i = 0; i < NSC; ++i) { mbar_init(bar(SC_FULL + i), 1); mbar_init(bar(SC_FREE + i), NQ * 256); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         slot[1] = 0u;
     }
-    if (warp == NQ * 4) {
+    if (warp == P::SW) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + P::OFF_SLOT), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -298,7 +335,7 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(const __grid_constan
     auto sbuf = [](int q, int j) { return q * SB + j % SB; };
     auto sph = [](int j) { return j / SB; };
 
-    if (warp == NQ * 4 + 1) {
+    if (warp == P::SW + 1) {
         // ======================= keys and norms: one thread (a key tile is free as soon as its scores are computed, long before =====
         // ======================= the value tile: each of the two rings is kept full by a thread of its own) =======================
         if (lane == 0) {
@@ -354,7 +391,7 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(const __grid_constan
             for (int j = max(0, nsc - NSC); j < nsc; ++j) drain(SC_FULL + j % NSC, j / NSC);
         }
         __syncwarp();
-    } else if (warp == NQ * 4 + 2) {
+    } else if (warp == P::SW + 2) {
         // ======================= values: one thread =======================
         if (lane == 0) {
             int nv = 0, nr = 0;
@@ -382,7 +419,7 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(const __grid_constan
             for (int j = max(0, nv - ST); j < nv; ++j) drain(V_FULL + j % ST, j / ST);
         }
         __syncwarp();
-    } else if (warp == NQ * 4) {
+    } else if (warp == P::SW) {
         // ======================= MMA issue: one warp, uniform =======================
         if (n > 0) {
             auto issue_qk = [&](int q, int j) {                    // S = Q K^T of key tile j
@@ -460,17 +497,28 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(const __grid_constan
         }
         __syncwarp();
     } else {
-        // ======================= softmax: a row per thread =======================
-        const int q = warp >> 2, m = tid;                          // (rows of query tile q: threads 128 q ... )
-        const uint32_t t_row = tmem + (uint32_t((warp & 3) * 32) << 16);
+        // ======================= softmax: two rows per thread, sixteen columns of each =======================
+        // Scores are read as mma.sync fragments: lane 4 g + t of a warp holds columns 8 r + 2 t, + 1 of rows g and g + 8 of its sixteen, so that it
+        // needs the norms of 16 tokens a side, not of all 64.  Two warps share the 32 lanes of a quarter of tensor memory: four per scheduler
+        // hide one another's latencies.  (A row per thread in half as many warps read every norm in every thread: 760 shared-memory wavefronts
+        // per key tile beside 1035 of operands and 256 of copies; with those the shared-memory pipe was 90 % busy: 667 -> 610 us for 512 queries x 32
+        // lanes over 16,384 tokens at d = 128, of 1280 cycles of products per key tile and 1700 in all.  Scores of two key tiles in one product of
+        // 128 columns, 1024 cycles, take a query tile's two score buffers at once: 660 us.)
+        const int q = warp >> 3, hh = (warp >> 2) & 1, g = lane >> 2, t2 = 2 * (lane & 3);       // query tile; half of the 32 lanes
+        const uint32_t t_row = tmem + (uint32_t((warp & 3) * 32) << 16), t_frag = t_row + (uint32_t(16 * hh) << 16);
+        const int m = q * TM + (warp & 3) * 32 + lane, mf = q * TM + (warp & 3) * 32 + 16 * hh + g;       // this thread's row where a thread has one; first of its two
         const bool valid = row_valid(m);
-        const int pos = p.q_pos0 + row_token(m), pos0 = p.q_pos0 + tq0 + q * p.QT;
-        int last = valid ? limit_p(pos) : -1;                      // the last token of the region (packed tokens first) that this row sees
+        const int pos0 = p.q_pos0 + tq0 + q * p.QT;
+        auto sync_q = [&]() { asm volatile("barrier.sync %0, 256;" ::"r"(1 + q) : "memory"); };       // the warps of the query tile
+        int last[2];                                               // the last token of the region (packed tokens first) that each row sees
+#pragma unroll
+        for (int k = 0; k < 2; ++k) last[k] = row_valid(mf + 8 * k) ? limit_p(p.q_pos0 + row_token(mf + 8 * k)) : -1;
         int full_upto = limit_p(pos0);                             // tokens every row of the query tile sees
-        // A row that has seen no token yet keeps m_ref = -1e30 with a bias of lvsc and asks for a reference at its first one (t_thr).
-        float m_ref = -1e30f, vsc = 1.f, vthr = 0.f;               // (vthr 0: the first tile with a non-zero value norm picks the scale)
-        float lvsc = 0.f, bias = 0.f, t_thr = -INFINITY;           // log2(vsc); lvsc - m_ref (0 before the first tile); MAX_SLACK + lvsc
-        u64 l2a = pk(0.f, 0.f), l2b = l2a;
+        // A row that has seen no token yet keeps m_ref = -1e30, has lvsc for a bias and asks for a reference at its first one.
+        float vsc = 1.f, vthr = 0.f, lvsc = 0.f;                   // (vthr 0: the first tile with a non-zero value norm picks the scale); log2(vsc)
+        float m_ref[2] = {-1e30f, -1e30f};
+        u64 l2[2] = {pk(0.f, 0.f), pk(0.f, 0.f)};                  // this thread's share of the rows' sums
+        auto bias_of = [&](int k) { return m_ref[k] > -1e30f ? lvsc - m_ref[k] : lvsc; };
         bool ok = true;
         for (int j = 0; j <= n; ++j) {
             if (j == n_p) {
@@ -492,18 +540,17 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(const __grid_constan
                     }
                     const float sc = stage_scale(__float_as_uint(mx));
 #pragma unroll 1
-                    for (int c0 = 0; c0 < DP; c0 += 64) {
-                        uint32_t o[64], hi[32], lo[32];
+                    for (int c0 = 32 * hh; c0 < DP; c0 += 64) {
+                        uint32_t o[32], hi[16], lo[16];
                         tmem_ld32(o_row + c0, o);
-                        tmem_ld32(o_row + c0 + 32, o + 32);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int i = 0; i < 64; i += 2) {
+                        for (int i = 0; i < 32; i += 2) {
                             const float u = sc * (c0 + i < D / 2 ? p.v_inv_hi : p.v_inv_lo);
                             split2(__uint_as_float(o[i]) * u, __uint_as_float(o[i + 1]) * u, hi[i / 2], lo[i / 2]);
                         }
-                        tmem_st32(a_row + c0 / 2, hi);
-                        tmem_st32(a_row + P::COL_LO + c0 / 2, lo);
+                        tmem_st16(a_row + c0 / 2, hi);
+                        tmem_st16(a_row + P::COL_LO + c0 / 2, lo);
                     }
                     tmem_st_wait();
                     tc_fence_before();
@@ -513,7 +560,7 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(const __grid_constan
                     tc_fence_after();
                     const float is = 1.f / sc;
 #pragma unroll 1
-                    for (int c0 = 0; c0 < DP; c0 += 32) {
+                    for (int c0 = 32 * hh; c0 < DP; c0 += 64) {
                         uint32_t o[32];
                         tmem_ld32(o_row + c0, o);
                         tmem_ld_wait();
@@ -522,8 +569,12 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(const __grid_constan
                         tmem_st32(o_row + c0, o);
                     }
                     tmem_st_wait();
+                    tc_fence_before();
+                    sync_q();                                      // (the other warp of these lanes has done the other columns)
+                    tc_fence_after();
                 }
-                last = valid ? limit_d(pos) : -1;
+#pragma unroll
+                for (int k = 0; k < 2; ++k) last[k] = row_valid(mf + 8 * k) ? limit_d(p.q_pos0 + row_token(mf + 8 * k)) : -1;
                 full_upto = limit_d(pos0);
             }
             if (j == n) break;
@@ -531,115 +582,154 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(const __grid_constan
             ok = wait_bar(SC_FULL + s, j / NSC) && wait_bar(S_FULL + sbuf(q, j), sph(j));
             if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
             tc_fence_after();
-            const float* kn = reinterpret_cast<const float*>(smem + P::OFF_SC) + s * 2 * TN;
+            const float* kn = reinterpret_cast<const float*>(smem + P::OFF_SC) + s * 2 * TN + t2;
             const float* vn = kn + TN;
-            const uint32_t s_col = t_row + sbuf(q, j) * TN;
-            uint32_t v[TN];
+            const uint32_t s_col = t_frag + sbuf(q, j) * TN;
+            constexpr int NR = TN / 8;
+            uint32_t v[4 * NR];                                    // of eight columns: two of row g, two of row g + 8
+            tmem_ld_frag64(s_col, v);
+            u64 nv[NR];
 #pragma unroll
-            for (int i = 0; i < TN / 32; ++i) tmem_ld32(s_col + 32 * i, v + 32 * i);
-            float vmax = 0.f;
-#pragma unroll
-            for (int i = 0; i < TN / 32; ++i) vmax = fmaxf(vmax, vn[lane + 32 * i]);
-#pragma unroll
-            for (int off = 16; off; off >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, off));
+            for (int r = 0; r < NR; ++r) nv[r] = *reinterpret_cast<const u64*>(kn + 8 * r);
             tmem_ld_wait();
             // t = score * key norm - reference + log2(value scale)
-            const u64 bias2 = pk(bias, bias);
-            float mx = -INFINITY;
 #pragma unroll
-            for (int i = 0; i < TN; i += 4) {
-                const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(kn + i);
-                const u64 a = fma2(pk(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), k4.x, bias2);
-                const u64 c = fma2(pk(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])), k4.y, bias2);
-                float x0, x1, x2, x3;
-                upk(a, x0, x1); upk(c, x2, x3);
-                v[i] = __float_as_uint(x0); v[i + 1] = __float_as_uint(x1); v[i + 2] = __float_as_uint(x2); v[i + 3] = __float_as_uint(x3);
+            for (int k = 0; k < 2; ++k) {
+                uint32_t* x = v + 2 * k;
+                const float bias = bias_of(k);
+                const u64 b2 = pk(bias, bias);
+#pragma unroll
+                for (int r = 0; r < NR; ++r) {
+                    float x0, x1;
+                    upk(fma2(pk(__uint_as_float(x[4 * r]), __uint_as_float(x[4 * r + 1])), nv[r], b2), x0, x1);
+                    x[4 * r] = __float_as_uint(x0); x[4 * r + 1] = __float_as_uint(x1);
+                }
             }
             if (base + TN > full_upto + 1) {                       // some token of the tile is hidden from some row, or past the end
-                const int lim = last - base;
 #pragma unroll
-                for (int i = 0; i < TN; ++i) v[i] = i <= lim ? v[i] : 0xff800000u;
+                for (int k = 0; k < 2; ++k) {
+                    uint32_t* x = v + 2 * k;
+                    const int lim = last[k] - base - t2;
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) { x[4 * r] = 8 * r <= lim ? x[4 * r] : 0xff800000u; x[4 * r + 1] = 8 * r + 1 <= lim ? x[4 * r + 1] : 0xff800000u; }
+                }
             }
+            // Weights, their sums, P = weight * value norm (both carry the value scale) as fp16.  A row needs another reference when a weight
+            // exceeds 2^MAX_SLACK, which its sum then does too: the sums are looked at behind the exponentials and no maximum is taken in the
+            // common case.  The lanes share the check of the tile's norms, eight tokens' pairs each.
+            const float2 v2 = *reinterpret_cast<const float2*>(vn + 8 * g);
+            float vmax = fmaxf(v2.x, v2.y);
 #pragma unroll
-            for (int i = 0; i < TN; i += 2) mx = fmaxf(fmaxf(mx, __uint_as_float(v[i])), __uint_as_float(v[i + 1]));
-            // Reference maximum / value scale: refreshed for the whole warp when any row needs it (rare after the first tile):
-            // the row's sums and its O in tensor memory are rescaled.
-            if (__any_sync(0xffffffffu, mx > t_thr || vmax > vthr)) {
-                const float mn = fmaxf(fmaxf(m_ref, mx - bias), -1e30f);
-                float a = ex2(m_ref - mn);
-                m_ref = mn;
+            for (int r = 0; r < NR; ++r) nv[r] = *reinterpret_cast<const u64*>(vn + 8 * r);
+            uint32_t w[2 * NR];
+            u64 ls[2];
+#pragma unroll 1
+            for (int pass = 0;; ++pass) {
+                ls[0] = ls[1] = pk(0.f, 0.f);
+#pragma unroll
+                for (int r = 0; r < NR; ++r)
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const u64 x = pk(ex2(__uint_as_float(v[4 * r + 2 * k])), ex2(__uint_as_float(v[4 * r + 2 * k + 1])));
+                        ls[k] = add2(ls[k], x);
+                        float x0, x1;
+                        upk(mul2(x, nv[r]), x0, x1);
+                        w[2 * r + k] = pack_h2(x0, x1);
+                    }
+                bool again = vmax > vthr;
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    float x0, x1;
+                    upk(ls[k], x0, x1);
+                    again = again || x0 + x1 > (m_ref[k] > -1e30f ? float(1 << int(MAX_SLACK)) * vsc : last[k] >= base ? -1.f : INFINITY);      // (a row's first token: always)
+                }
+                if (pass > 0 || !__any_sync(0xffffffffu, again)) break;
+                // Reference maximum / value scale: refreshed for the whole warp when any row needs it (rare after the first tile):
+                // the rows' sums and their O in tensor memory are rescaled.
+                float a[2], bias[2] = {bias_of(0), bias_of(1)}, mx[2] = {-INFINITY, -INFINITY}, ratio = 1.f;
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) mx[k] = fmaxf(fmaxf(mx[k], __uint_as_float(v[4 * r + 2 * k])), __uint_as_float(v[4 * r + 2 * k + 1]));
+#pragma unroll
+                    for (int off = 1; off < 4; off <<= 1) mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], off));
+                }
+#pragma unroll
+                for (int off = 16; off; off >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, off));
                 if (vmax > vthr) {
                     int eb = (__float_as_int(vmax) >> 23) & 0xff;
                     eb = min(max(eb, 16), 240);
                     const float nsc = __int_as_float((261 - eb) << 23);    // the largest value norm lands in [128, 256)
-                    a *= nsc / vsc;
+                    ratio = nsc / vsc;
                     vsc = nsc;
                     vthr = VSC_CAP / nsc;
                     lvsc = float(134 - eb);
                 }
-                const bool seen = m_ref > -1e30f;
-                const float nb = seen ? lvsc - m_ref : lvsc, delta = nb - bias;
-                bias = nb;
-                t_thr = seen ? MAX_SLACK + lvsc : -INFINITY;
-                const u64 a2 = pk(a, a);
-                l2a = mul2(l2a, a2); l2b = mul2(l2b, a2);
 #pragma unroll
-                for (int i = 0; i < TN; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) + delta);
+                for (int k = 0; k < 2; ++k) {
+                    const float mn = fmaxf(fmaxf(m_ref[k], mx[k] - bias[k]), -1e30f);
+                    a[k] = ex2(m_ref[k] - mn) * ratio;
+                    m_ref[k] = mn;
+                    const float delta = bias_of(k) - bias[k];
+                    l2[k] = mul2(l2[k], pk(a[k], a[k]));
+                    uint32_t* x = v + 2 * k;
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) {
+                        x[4 * r] = __float_as_uint(__uint_as_float(x[4 * r]) + delta);
+                        x[4 * r + 1] = __float_as_uint(__uint_as_float(x[4 * r + 1]) + delta);
+                    }
+                }
                 if (j > 0) {
                     ok = wait_bar(O_DONE + q, j - 1);
                     if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
                     tc_fence_after();
 #pragma unroll 1
                     for (int c0 = 0; c0 < DP; c0 += 32) {
-                        uint32_t o[32];
-                        tmem_ld32(t_row + P::COL_O + q * DP + c0, o);
+                        uint32_t o[16];
+                        tmem_ld_frag32(t_frag + P::COL_O + q * DP + c0, o);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * a);
-                        tmem_st32(t_row + P::COL_O + q * DP + c0, o);
+                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * a[(i >> 1) & 1]);
+                        tmem_st_frag32(t_frag + P::COL_O + q * DP + c0, o);
                     }
                     tmem_st_wait();
                 }
             }
-            // weights, their sum, P = weight * value norm (both carry the value scale) as fp16 over the scores
-#pragma unroll
-            for (int h = 0; h < TN / 64; ++h) {
-                uint32_t w[32];
-#pragma unroll
-                for (int i = 0; i < 64; i += 4) {
-                    const int e = 64 * h + i;
-                    const ulonglong2 n4 = *reinterpret_cast<const ulonglong2*>(vn + e);
-                    const u64 x = pk(ex2(__uint_as_float(v[e])), ex2(__uint_as_float(v[e + 1]))), y = pk(ex2(__uint_as_float(v[e + 2])), ex2(__uint_as_float(v[e + 3])));
-                    l2a = add2(l2a, x); l2b = add2(l2b, y);
-                    float x0, x1, y0, y1;
-                    upk(mul2(x, n4.x), x0, x1); upk(mul2(y, n4.y), y0, y1);
-                    w[i / 2] = pack_h2(x0, x1); w[i / 2 + 1] = pack_h2(y0, y1);
-                }
-                tmem_st32(s_col + 32 * h, w);
-            }
+            if (!ok) break;
+            l2[0] = add2(l2[0], ls[0]);
+            l2[1] = add2(l2[1], ls[1]);
+            tmem_st_half64(s_col, w);
             tmem_st_wait();
             tc_fence_before();
             mbar_arrive(bar(P_FULL + sbuf(q, j)));
             mbar_arrive(bar(SC_FREE + s));
         }
-        // ---- the row's result ----
-        float l0, l1, l_sum;
-        upk(add2(l2a, l2b), l0, l1);
-        l_sum = l0 + l1;
+        // ---- the rows' results: a row per thread from here on, each warp every other 32 columns ----
+        float2* const s_row = reinterpret_cast<float2*>(smem + P::OFF_ROW);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            float l0, l1;
+            upk(l2[k], l0, l1);
+            l0 += l1;
+#pragma unroll
+            for (int off = 1; off < 4; off <<= 1) l0 += __shfl_xor_sync(0xffffffffu, l0, off);
+            if ((lane & 3) == 0) s_row[mf + 8 * k] = make_float2(l0, m_ref[k]);
+        }
+        sync_q();
+        const float l_sum = s_row[m].x, m_row = s_row[m].y;
         if (ok && n > n_p) ok = wait_bar(ALL_DONE + q, 0);
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
         float* part = nullptr;
         if (p.n_splits > 1) {
             part = p.part + (((int64_t(y) * p.n_blk + blk) * p.n_splits + split) * (NQ * TM) + m) * (D + 4);
-            part[D] = n > 0 && ok ? m_ref - lvsc : -INFINITY;
-            part[D + 1] = n > 0 && ok ? l_sum : 0.f;
+            if (hh == 0) *reinterpret_cast<float2*>(part + D) = n > 0 && ok ? make_float2(m_row - lvsc, l_sum) : make_float2(-INFINITY, 0.f);
         }
         if (n > 0 && ok) {
             const float il = 1.f / l_sum;
             const int64_t o0 = valid ? row_q_index(m) : 0;
 #pragma unroll 1
-            for (int c0 = 0; c0 < D; c0 += 32) {
+            for (int c0 = 32 * hh; c0 < D; c0 += 64) {
                 uint32_t o[32];
                 tmem_ld32(t_row + P::COL_O + q * DP + c0, o);
                 tmem_ld_wait();
@@ -675,7 +765,7 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(const __grid_constan
     // ---------------- teardown: every loop above is bounded, so every thread gets here ----------------
     tc_fence_before();
     __syncthreads();
-    if (warp == NQ * 4) {
+    if (warp == P::SW) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     }
