@@ -165,6 +165,11 @@ int tq_qk_scores(const float* q_rot, const uint8_t* packed, const float* norms, 
  * (cache.py:632-672, 577-618). */
 int tq_append_tokens(const void* k_new, const void* v_new, void* k_buf, void* v_buf, int64_t lanes, int64_t t_new,
                      int64_t row_bytes, int64_t src_lane_stride, int64_t dst_lane_stride, int64_t dst_row0, void* stream);
+/* A whole buffer in one launch: of every lane's `capacity` rows the first `kept` come from an older buffer (k_old / v_old: its first row to
+ * keep, lanes old_lane_stride rows apart), the next t_new from the caller's rows, and the rest become zeros.  The new buffer must not
+ * overlap its sources; otherwise as above. */
+int tq_fill_tokens(const void* k_old, const void* v_old, int64_t kept, int64_t old_lane_stride, const void* k_new, const void* v_new, int64_t t_new,
+                   int64_t src_lane_stride, void* k_buf, void* v_buf, int64_t lanes, int64_t row_bytes, int64_t capacity, void* stream);
 
 /* ---- decode attention over [fp16 sink | packed middle | fp16 residual] ------------------- */
 

@@ -103,6 +103,7 @@ PROTOTYPES = {
     "tq_qjl_dequantize": (_i, [_vp, _vp, _vp, _vp, _i64, _i, _i, _vp]),
     "tq_qk_scores": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i64, _i64, _vp, _vp]),
     "tq_append_tokens": (_i, [_vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i64, _vp]),
+    "tq_fill_tokens": (_i, [_vp, _vp, _i64, _i64, _vp, _vp, _i64, _i64, _vp, _vp, _i64, _i64, _i64, _vp]),
     "tq_decode_workspace_bytes": (_sz, [_i, _i, _i, _i, _i64, _i64]),
     "tq_decode_tables_bytes": (_sz, [_i, _i, _i]),
     "tq_decode_tables_build": (_i, [_i, _vp, _vp, _i, _vp, _i, _f, _vp, _sz, _vp]),
@@ -143,6 +144,24 @@ def lib():
             fn.restype, fn.argtypes = res, args
         _lib = handle
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host path (csrc/host.cpp): checks, allocations and launches of the calls that are mostly host work.  Its functions return
+    None for anything but the plain case (the callers in this package then take their own path) and a negative status as it is."""
+    global _host
+    if _host is None:
+        lib()                                             # (the module is linked against the library)
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise RuntimeError(f"the native host module does not load ({e}): build it with the CUDA library "
+                               "(python -c 'import __graft_entry__ as g; g.build()')") from e
+        _host = module
+    return _host
 
 
 class TurboQuantError(RuntimeError):

@@ -116,6 +116,10 @@ class _Side:
             a.qjl_bits, a.qjl_gamma = self.qbits.data_ptr() + 4 * at, self.qgamma.data_ptr() + 4 * at
         return x
 
+    def native_job(self, buf, old: int, new, n_new: int) -> tuple:
+        """The same for csrc/host.cpp: the first ``old`` rows of the buffer, then the first ``n_new`` of the new tokens."""
+        return self.q_block, buf, old, new, n_new, self.hi, self.lo, self.norms, self.qbits, self.qgamma
+
     def dequantize_job(self, n: int, at: int, out_ptr: int, out_rows: int, d: int, with_qjl: bool) -> "_lib.DequantizeArgs":
         """Argument block: tokens [at, at + n) as float32 rows, every lane's ``out_rows`` rows from the last one's."""
         a = _lib.DequantizeArgs.from_buffer_copy(self.r_block)
@@ -143,6 +147,9 @@ class _Side:
             return
         cap = _round_up(max(need, 2 * self.capacity(), 256), 16)
         w_hi, w_lo = kernels.packed_widths(d, self.bits_hi, self.bits_lo)
+        if self.hi is None and used == 0:
+            self.hi, self.lo, self.norms, self.qbits, self.qgamma = _lib.host().storage(b, h, cap, w_hi, w_lo if self.fractional else 0, with_qjl, device.index)
+            return
 
         def grow(old, shape, dtype):
             if old is None and used > 0:   # a sketch that a reloaded state did not carry: zero = no correction
@@ -374,7 +381,7 @@ class TurboQuantKVCache:
         632-672).  Tokens that leave at once are quantized where they are - in the buffer or in the caller's tensors - and
         never pass through the buffer: a long prompt costs one read of its rows, not a fill, a copy and a read back."""
         b, h, t_new, d = k_new.shape
-        dev = k_new.device
+        dev, host = k_new.device, _lib.host()
         have = 0 if self.keys is None else self._fp16_len
         length = have + t_new
         cap = self._fp16_capacity
@@ -390,34 +397,47 @@ class TurboQuantKVCache:
         old = min(n, have)                     # of the n, those that sit in the buffer
         if n > 0:
             at = self._compressed_len
-            jobs, alive = (_lib.QuantizeArgs * 4)(), []
-            for side, buf, new in ((self._k, self.keys, k_new), (self._v, self.values, v_new)):
+            for side in (self._k, self._v):
                 side.reserve(b, h, d, at + n, at, dev, self.qjl_correction)
-                if old:
-                    alive.append(side.quantize_job(jobs[len(alive)], buf[:, :, :old], at))
-                if n > old:
-                    alive.append(side.quantize_job(jobs[len(alive)], new[:, :, :n - old] if n - old < t_new else new, at + old))
-            _lib.check(_lib.launch(dev, "tq_quantize_pack_many", jobs, len(alive), _lib.stream_ptr(dev)))
+            rc = host.quantize(at, self._k.native_job(self.keys, old, k_new, n - old), self._v.native_job(self.values, old, v_new, n - old))
+            if rc is None:                     # rows that have to be laid out or converted first, or another device
+                jobs, alive = (_lib.QuantizeArgs * 4)(), []
+                for side, buf, new in ((self._k, self.keys, k_new), (self._v, self.values, v_new)):
+                    if old:
+                        alive.append(side.quantize_job(jobs[len(alive)], buf[:, :, :old], at))
+                    if n > old:
+                        alive.append(side.quantize_job(jobs[len(alive)], new[:, :, :n - old] if n - old < t_new else new, at + old))
+                rc = _lib.launch(dev, "tq_quantize_pack_many", jobs, len(alive), _lib.stream_ptr(dev))
+            _lib.check(rc)
             # A long prefill would leave buffers sized for the whole prompt; they get the size a fresh cache would get for what
             # remains instead (batch 64 x 32K tokens: 17 GB per layer otherwise).
             small = max(length - n, self.residual_window * 2) + 256
             if cap > 4 * small:
                 cap = small
-        kept = have - old
+        kept, start = have - old, n - old      # tokens that stay in the buffer; the first of the new ones that goes there
+        filled = False
         if self.keys is None or cap != self.keys.shape[2]:
-            nk, nv = torch.zeros((2, b, h, cap, d), dtype=k_new.dtype, device=dev) if k_new.dtype == v_new.dtype else (
-                torch.zeros((b, h, cap, d), dtype=t.dtype, device=dev) for t in (k_new, v_new))
-            if kept > 0:
-                self._append(nk, nv, self.keys[:, :, old:have], self.values[:, :, old:have], 0)
-            self.keys, self.values = nk, nv
+            pair = host.buffers(k_new, v_new, start, t_new - start, cap, self.keys, self.values, old, kept)
+            if type(pair) is tuple:
+                self.keys, self.values = pair
+                filled = True
+            elif pair is not None:
+                _lib.check(pair)
+            else:
+                nk, nv = (torch.zeros((b, h, cap, d), dtype=t.dtype, device=dev) for t in (k_new, v_new))
+                if kept > 0:
+                    self._append(nk, nv, self.keys[:, :, old:have], self.values[:, :, old:have], 0)
+                self.keys, self.values = nk, nv
         elif old > 0 and kept > 0:             # the kept tokens move to the front (the kernels above have read the buffer by then)
             for buf in (self.keys, self.values):
                 tail = buf[:, :, old:have]
                 buf[:, :, :kept] = tail.clone() if old < kept else tail
-        if n - old < t_new:
-            if n > old:
-                k_new, v_new = k_new[:, :, n - old:], v_new[:, :, n - old:]
-            self._append(self.keys, self.values, k_new, v_new, kept)
+        if not filled and start < t_new:
+            rc = host.append(self.keys, self.values, k_new, v_new, start, t_new - start, kept)
+            if rc is None:
+                self._append(self.keys, self.values, k_new[:, :, start:], v_new[:, :, start:], kept)
+            else:
+                _lib.check(rc)
         self._fp16_capacity = cap
         self._fp16_len = length - n
         self._compressed_len += n
@@ -435,12 +455,18 @@ class TurboQuantKVCache:
         n_sink = min(self.fp16_sink_size - self.offset, t_new)
         if n_sink <= 0:
             return keys, values
-        if self.sink_keys is None:
-            b, h, _, d = keys.shape
-            new = torch.empty if n_sink == self.fp16_sink_size else torch.zeros        # (rows without a token yet read as zeros)
-            self.sink_keys = new((b, h, self.fp16_sink_size, d), dtype=keys.dtype, device=keys.device)
-            self.sink_values = new((b, h, self.fp16_sink_size, d), dtype=values.dtype, device=values.device)
-        self._append(self.sink_keys, self.sink_values, keys[:, :, :n_sink], values[:, :, :n_sink], self.offset)
+        pair = _lib.host().buffers(keys, values, 0, n_sink, self.fp16_sink_size, None, None, 0, 0) if self.sink_keys is None and self.offset == 0 else None
+        if type(pair) is tuple:
+            self.sink_keys, self.sink_values = pair
+        elif pair is not None:
+            _lib.check(pair)
+        else:
+            if self.sink_keys is None:
+                b, h, _, d = keys.shape
+                new = torch.empty if n_sink == self.fp16_sink_size else torch.zeros        # (rows without a token yet read as zeros)
+                self.sink_keys = new((b, h, self.fp16_sink_size, d), dtype=keys.dtype, device=keys.device)
+                self.sink_values = new((b, h, self.fp16_sink_size, d), dtype=values.dtype, device=values.device)
+            self._append(self.sink_keys, self.sink_values, keys[:, :, :n_sink], values[:, :, :n_sink], self.offset)
         self._sink_len = self.offset + n_sink
         return keys[:, :, n_sink:], values[:, :, n_sink:]
 
@@ -482,19 +508,14 @@ class TurboQuantKVCache:
     def _append_step(self, keys: torch.Tensor, values: torch.Tensor) -> bool:
         """The everyday step: tokens that simply join the recent-token buffer (no sink, no growth, nothing due)."""
         buf = self.keys
-        if (buf is None or self.offset < self.fp16_sink_size or keys.dim() != 4 or keys.shape != values.shape or keys.dtype is not buf.dtype
-                or values.dtype is not buf.dtype or self.values.dtype is not buf.dtype or not keys.is_contiguous() or not values.is_contiguous()):
+        if buf is None or self.offset < self.fp16_sink_size or keys.dim() != 4:
             return False
-        b, h, t, d = keys.shape
+        t = keys.shape[2]
         have, cap = self._fp16_len, self._fp16_capacity
-        if have + t > cap or cap != buf.shape[2] or t == 0 or self._due(have + t) > 0 or buf.shape[0] != b or buf.shape[1] != h or buf.shape[3] != d:
+        if have + t > cap or cap != buf.shape[2] or t == 0 or self._due(have + t) > 0 or keys.shape != values.shape:
             return False
-        stream = _lib.here(keys, values, buf)
-        if stream is None or not buf.is_contiguous() or not self.values.is_contiguous():
-            return False
-        rc = _lib.lib().tq_append_tokens(keys.data_ptr(), values.data_ptr(), buf.data_ptr(), self.values.data_ptr(), b * h, t,
-                                         d * buf.element_size(), t, cap, have, stream)
-        if rc == -2:                          # (layout not supported)
+        rc = _lib.host().append(buf, self.values, keys, values, 0, t, have)
+        if rc is None:
             return False
         _lib.check(rc)
         self._fp16_len = have + t
@@ -560,6 +581,17 @@ class TurboQuantKVCache:
         s_len, c_len, r_len = self._sink_len, self._compressed_len, self._fp16_len
         if (s_len > 0) + (c_len > 0) + (r_len > 0) < 2:
             return None
+        k, v = self._k, self._v
+        kd = vd = None
+        if c_len > 0 and (self.qjl_correction or self.head_dim == 256):
+            self._ensure_dense()
+            kd, vd = self._dense_k, self._dense_v
+        res = _lib.host().fetch(self.sink_keys, self.sink_values, s_len, self.keys, self.values, r_len, c_len, (k.r_block, k.hi, k.lo, k.norms),
+                                (v.r_block, v.hi, v.lo, v.norms), kd, vd)
+        if type(res) is tuple:
+            return res
+        if res is not None:
+            _lib.check(res)
         ref = self.keys if r_len > 0 else self.sink_keys
         b, h, _, d = ref.shape
         dt = torch.float32 if c_len > 0 else ref.dtype

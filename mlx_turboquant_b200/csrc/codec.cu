@@ -300,23 +300,49 @@ extern "C" int tq_quantize_from_rotated(const float* y, int64_t n, int d, const 
     return check_launch("tq_quantize_from_rotated");
 }
 
-// ---- append rows to the uncompressed token buffers ------------------------------------------------------
+// ---- rows of the uncompressed token buffers ------------------------------------------------------
 namespace tq {
-// One launch copies the new rows of keys AND values: thread -> (tensor, lane, row, 16-byte chunk).
-__global__ void append_rows_kernel(const uint4* __restrict__ k_new, const uint4* __restrict__ v_new, uint4* __restrict__ k_buf,
-                                   uint4* __restrict__ v_buf, int64_t lanes, int64_t t_new, int chunks, int64_t src_ls, int64_t dst_ls,
-                                   int64_t dst_row0) {
-    const int64_t total = 2 * lanes * t_new * chunks;
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x) {
-        const int c = int(i % chunks);
-        int64_t r = i / chunks;
-        const int64_t row = r % t_new; r /= t_new;
-        const int64_t lane = r % lanes;
-        const bool is_v = r >= lanes;
-        const uint4* src = (is_v ? v_new : k_new) + (lane * src_ls + row) * chunks + c;
-        uint4* dst = (is_v ? v_buf : k_buf) + (lane * dst_ls + dst_row0 + row) * chunks + c;
-        *dst = __ldg(src);
+// Keys and values of a buffer in one launch: of every lane rows [0, kept) from an older buffer, the next t_new from the caller's rows, zeros
+// behind them (torch.zeros and two copies before: 16 us for 9 MB a side, 8 now).  A block: ROWS_U x its threads 16-byte chunks of a lane; no
+// more threads than a lane has chunks, so that a token of many lanes is one wave.
+constexpr int ROWS_T = 256, ROWS_U = 4;
+struct RowsParams {
+    const uint4 *k_old, *v_old, *k_new, *v_new;
+    uint4 *k_buf, *v_buf;
+    int64_t old_ls, src_ls, dst_ls;                    // rows between lanes
+    uint32_t lanes, kept, t_new, n_rows, chunks, blocks_per_lane;
+};
+__global__ void __launch_bounds__(ROWS_T) rows_kernel(const __grid_constant__ RowsParams p) {
+    const uint32_t lane2 = blockIdx.x / p.blocks_per_lane, blk = blockIdx.x - lane2 * p.blocks_per_lane;
+    const bool is_v = lane2 >= p.lanes;
+    const int64_t lane = is_v ? lane2 - p.lanes : lane2;
+    const uint4* old = (is_v ? p.v_old : p.k_old) + lane * p.old_ls * p.chunks;
+    const uint4* src = (is_v ? p.v_new : p.k_new) + lane * p.src_ls * p.chunks;
+    uint4* dst = (is_v ? p.v_buf : p.k_buf) + lane * p.dst_ls * p.chunks;
+    const uint32_t a = p.kept * p.chunks, b = a + p.t_new * p.chunks, n = p.n_rows * p.chunks;
+    uint4 x[ROWS_U];
+#pragma unroll
+    for (int u = 0; u < ROWS_U; ++u) {
+        const uint32_t i = (blk * ROWS_U + u) * blockDim.x + threadIdx.x;
+        x[u] = make_uint4(0u, 0u, 0u, 0u);
+        if (i < a) x[u] = old[i];
+        else if (i < b) x[u] = src[i - a];
     }
+#pragma unroll
+    for (int u = 0; u < ROWS_U; ++u) {
+        const uint32_t i = (blk * ROWS_U + u) * blockDim.x + threadIdx.x;
+        if (i < n) dst[i] = x[u];
+    }
+}
+
+static int launch_rows(const char* what, RowsParams p, int64_t lanes, int64_t n_rows, int64_t row_bytes, cudaStream_t s) {
+    if (row_bytes % 16 || !aligned(p.k_new, 16) || !aligned(p.v_new, 16) || !aligned(p.k_buf, 16) || !aligned(p.v_buf, 16) || !aligned(p.k_old, 16) || !aligned(p.v_old, 16))
+        return fail(TQ_ERR_UNSUPPORTED, "%s: rows must be multiples of 16 bytes at 16-byte aligned addresses", what);
+    const int64_t chunks = row_bytes / 16, threads = std::min<int64_t>(ROWS_T, (n_rows * chunks + 31) / 32 * 32), per = threads * ROWS_U, blocks = (n_rows * chunks + per - 1) / per;
+    if (n_rows * chunks >= (int64_t(1) << 31) || 2 * lanes * blocks >= (int64_t(1) << 31)) return fail(TQ_ERR_UNSUPPORTED, "%s: too many rows", what);
+    p.lanes = uint32_t(lanes); p.n_rows = uint32_t(n_rows); p.chunks = uint32_t(chunks); p.blocks_per_lane = uint32_t(blocks);
+    rows_kernel<<<unsigned(2 * lanes * blocks), unsigned(threads), 0, s>>>(p);
+    return check_launch(what);
 }
 }  // namespace tq
 
@@ -327,14 +353,31 @@ extern "C" int tq_append_tokens(const void* k_new, const void* v_new, void* k_bu
         return fail(TQ_ERR_INVALID, "tq_append_tokens: bad sizes");
     if (lanes == 0 || t_new == 0) return TQ_OK;
     if (!k_new || !v_new || !k_buf || !v_buf) return fail(TQ_ERR_INVALID, "tq_append_tokens: null pointer");
-    if (row_bytes % 16 || !aligned(k_new, 16) || !aligned(v_new, 16) || !aligned(k_buf, 16) || !aligned(v_buf, 16))
-        return fail(TQ_ERR_UNSUPPORTED, "tq_append_tokens: rows must be multiples of 16 bytes at 16-byte aligned addresses");
-    const int chunks = int(row_bytes / 16);
-    const int64_t total = 2 * lanes * t_new * chunks;
-    const int threads = 256;
-    const unsigned blocks = unsigned(std::min<int64_t>((total + threads - 1) / threads, 148 * 8));
-    append_rows_kernel<<<blocks, threads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint4*>(k_new), static_cast<const uint4*>(v_new), static_cast<uint4*>(k_buf), static_cast<uint4*>(v_buf),
-        lanes, t_new, chunks, src_lane_stride, dst_lane_stride, dst_row0);
-    return check_launch("tq_append_tokens");
+    const int64_t step = std::max<int64_t>(1, (int64_t(1) << 30) / ((row_bytes + 15) / 16));       // (the kernel counts a lane's chunks in 32 bits)
+    for (int64_t at = 0; at < t_new; at += step) {
+        const int64_t n = std::min(step, t_new - at), from = at * row_bytes, to = (dst_row0 + at) * row_bytes;
+        RowsParams p{};
+        p.k_new = reinterpret_cast<const uint4*>(static_cast<const unsigned char*>(k_new) + from);
+        p.v_new = reinterpret_cast<const uint4*>(static_cast<const unsigned char*>(v_new) + from);
+        p.k_buf = reinterpret_cast<uint4*>(static_cast<unsigned char*>(k_buf) + to);
+        p.v_buf = reinterpret_cast<uint4*>(static_cast<unsigned char*>(v_buf) + to);
+        p.src_ls = src_lane_stride; p.dst_ls = dst_lane_stride; p.t_new = uint32_t(n);
+        if (int rc = launch_rows("tq_append_tokens", p, lanes, n, row_bytes, static_cast<cudaStream_t>(stream))) return rc;
+    }
+    return TQ_OK;
+}
+
+extern "C" int tq_fill_tokens(const void* k_old, const void* v_old, int64_t kept, int64_t old_lane_stride, const void* k_new, const void* v_new, int64_t t_new,
+                              int64_t src_lane_stride, void* k_buf, void* v_buf, int64_t lanes, int64_t row_bytes, int64_t capacity, void* stream) {
+    using namespace tq;
+    if (lanes < 0 || t_new < 0 || kept < 0 || row_bytes <= 0 || capacity < kept + t_new || (t_new > 0 && src_lane_stride < t_new) || (kept > 0 && old_lane_stride < kept))
+        return fail(TQ_ERR_INVALID, "tq_fill_tokens: bad sizes");
+    if (lanes == 0 || capacity == 0) return TQ_OK;
+    if (!k_buf || !v_buf || (t_new > 0 && (!k_new || !v_new)) || (kept > 0 && (!k_old || !v_old))) return fail(TQ_ERR_INVALID, "tq_fill_tokens: null pointer");
+    RowsParams p{};
+    if (kept > 0) { p.k_old = static_cast<const uint4*>(k_old); p.v_old = static_cast<const uint4*>(v_old); p.kept = uint32_t(kept); }
+    if (t_new > 0) { p.k_new = static_cast<const uint4*>(k_new); p.v_new = static_cast<const uint4*>(v_new); p.t_new = uint32_t(t_new); }
+    p.k_buf = static_cast<uint4*>(k_buf); p.v_buf = static_cast<uint4*>(v_buf);
+    p.old_ls = old_lane_stride; p.src_ls = src_lane_stride; p.dst_ls = capacity;
+    return launch_rows("tq_fill_tokens", p, lanes, capacity, row_bytes, static_cast<cudaStream_t>(stream));
 }

@@ -100,13 +100,10 @@ def quantize_pack(x: torch.Tensor, rotation: torch.Tensor, boundaries_hi: torch.
     return out_hi, out_lo, out_norms
 
 
-_ROW_DTYPES = {torch.float16: _lib.TQ_F16, torch.bfloat16: _lib.TQ_BF16, torch.float32: _lib.TQ_F32}
-
-
 class RowCodec:
-    """Quantize and dequantize plain contiguous rows with one table set: the argument blocks are filled once, a call copies
-    them (calls may come from several threads) and sets what differs.  Returns None for anything but the plain case, which
-    the caller then hands to ``quantize_pack`` / ``dequantize`` (their checks and conversions cost some 10 us a call)."""
+    """Quantize and dequantize plain contiguous rows with one table set: the argument blocks are filled once, a call (native, csrc/host.cpp)
+    copies them and sets what differs; calls may come from several threads.  Returns None for anything but the plain case, which the
+    caller then hands to ``quantize_pack`` / ``dequantize``."""
 
     def __init__(self, d: int, bits: int, rotation: torch.Tensor, centroids: torch.Tensor, boundaries: torch.Tensor):
         self.of = (rotation, centroids, boundaries)                # kept alive: the blocks hold their addresses
@@ -118,35 +115,16 @@ class RowCodec:
         self._q, self._r = bytes(q), bytes(r)
 
     def quantize(self, x: torch.Tensor):
-        code = _ROW_DTYPES.get(x.dtype)
-        if not self.ok or code is None or not x.is_contiguous() or x.shape[-1] != self.d:
-            return None
-        stream = _lib.here(x, self.of[0])
-        if stream is None:
-            return None
-        lead = x.shape[:-1]
-        packed, norms = x.new_empty((*lead, self.width), dtype=torch.uint8), x.new_empty(lead, dtype=torch.float32)
-        a = _lib.QuantizeArgs.from_buffer_copy(self._q)
-        a.x, a.x_dtype, a.packed_hi, a.norms = x.data_ptr(), code, packed.data_ptr(), norms.data_ptr()
-        a.n_rows = a.out_lane_stride = norms.numel()
-        _lib.check(_lib.lib().tq_quantize_pack(C.byref(a), stream))
-        return packed, norms
+        return self._result(_lib.host().codec_quantize(self._q, self.width, x, self.of[0])) if self.ok else None
 
     def dequantize(self, packed: torch.Tensor, norms: torch.Tensor):
-        if (not self.ok or packed.dtype != torch.uint8 or norms.dtype != torch.float32 or not packed.is_contiguous() or not norms.is_contiguous()
-                or packed.numel() != norms.numel() * self.width):
-            return None
-        stream = _lib.here(packed, norms, self.of[0])
-        if stream is None:
-            return None
-        out = norms.new_empty((*norms.shape, self.d))
-        a = _lib.DequantizeArgs.from_buffer_copy(self._r)
-        a.packed_hi, a.norms, a.out = packed.data_ptr(), norms.data_ptr(), out.data_ptr()
-        n = norms.numel()
-        a.n_rows = a.in_lane_stride = n
-        a.out_lane_stride = n * self.d
-        _lib.check(_lib.lib().tq_dequantize(C.byref(a), stream))
-        return out
+        return self._result(_lib.host().codec_dequantize(self._r, self.width, packed, norms, self.of[0])) if self.ok else None
+
+    @staticmethod
+    def _result(res):
+        if type(res) is int:
+            _lib.check(res)
+        return res
 
 
 def _uniform_lanes(x: torch.Tensor, lanes: int, t: int, d: int) -> torch.Tensor:
