@@ -38,6 +38,7 @@
 // them.  A tile is fetched from memory once and three times from L2.  (524,288 rows at 4 bits: 4602 us in the CUDA-core row kernel before, 244 here; 3.5 bits 4576 / 254, bf16 4595 / 252.)
 // Every mbarrier wait is bounded: on a timeout the kernel raises a status word, drains and frees its TMEM.
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 
 #include <cuda.h>
@@ -961,10 +962,46 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
 
 using namespace tq;
 
+namespace tq {
+static int quantize_sms() {
+    static std::atomic<int> sms[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    int n = sms[dev].load();
+    if (!n) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        sms[dev].store(n);
+    }
+    return n;
+}
+}
+
+// The jobs of one compression side by side: tiles per CTA with which all of them fit the SMs at once, or 0 where that would be above 8.
+// A CTA pays 6 us of set-up (R as operand tiles) before its first tile and 1 to 1.5 us per tile: with a CTA per tile, up to the SMs, each
+// job's set-up waited for the one before it.  us for keys and values of 8 lanes, one after the other / side by side:
+//   tokens                          2048          4096          8192         16384
+//   d = 128 fp16, 4 and 2 bits   15.7 / 12.4   18.6 / 16.5   24.7 / 22.6   36.3 / 36.7
+//   d = 128 bf16, 4 and 2 bits   18.5 / 14.4   21.1 / 20.5   28.8 / 28.6   41.0 / 45.1
+//   d = 128 fp16, 3.5 bits       17.9 / 13.6   20.6 / 16.6   26.7 / 22.6   39.0 / 34.9
+//   d = 64 fp16, 4 bits          14.4 / 11.3   16.8 / 14.4   20.7 / 18.5   30.8 / 28.9
+// The widths cost different times per tile: from 9 tiles on (between the last two columns) the cheaper job's CTAs end early.
+int tq_quantize_tiles_each(const tq_quantize_args* q, int n) {
+    int64_t total = 0, tiles[8];
+    if (n > 8) return 0;
+    for (int i = 0; i < n; ++i) total += tiles[i] = q[i].n_lanes * ((q[i].n_rows + tc::TM - 1) / tc::TM);
+    const int64_t room = q[0].d == 256 ? quantize_sms() / 4 : quantize_sms();
+    for (int64_t each = std::max<int64_t>(1, (total + room - 1) / room); each <= 8; ++each) {
+        int64_t ctas = 0;
+        for (int i = 0; i < n; ++i) ctas += (tiles[i] + each - 1) / each;
+        if (ctas <= room) return int(each);
+    }
+    return 0;
+}
+
 // Takes the call when it fits the tensor-core kernel: fp16 / bf16 rows, d in {64, 96, 128} or 256 without a sketch, 16-byte aligned rows, no
 // rotated-row output, a bit-width pair the epilogue is compiled for.  Otherwise reports "not handled" and the caller uses
 // the general CUDA-core kernel.
-int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled, bool follows) {
+int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled, bool follows, int tiles_each) {
     *handled = false;
     const int d = q->d;
     if ((d != 64 && d != 96 && d != 128 && (d != 256 || q->qjl_bits)) || (q->x_dtype != TQ_F16 && q->x_dtype != TQ_BF16) || q->y_out) return TQ_OK;
@@ -982,7 +1019,6 @@ int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled
     // (one row takes 8 us here and 38 in the row kernel at d = 128, 8 and 116 at d = 256: no size is too small)
     const bool qjl = q->qjl_bits != nullptr;
     static bool attr_set[16] = {false};
-    static int sms[16] = {0};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 16) return TQ_OK;
@@ -993,7 +1029,6 @@ int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled
         if (e == cudaSuccess) e = cudaFuncSetAttribute(tc::quantize_tc_kernel<false, false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(tc::quantize_tc_kernel<true, false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
         if (e != cudaSuccess) return fail(TQ_ERR_LAUNCH, "tq_quantize_pack: shared memory %d B: %s", tc::SMEM_BYTES, cudaGetErrorString(e));
-        if (cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms[dev] <= 0) sms[dev] = 148;
         attr_set[dev] = true;
     }
     static PFN_cuTensorMapEncodeTiled encode = nullptr;
@@ -1030,7 +1065,8 @@ int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled
     p.rot = q->rot; p.bnd_hi = q->bnd_hi; p.bnd_lo = q->bnd_lo; p.bits_hi = q->bits_hi; p.bits_lo = q->bits_lo;
     p.p_hi = q->packed_hi; p.p_lo = q->packed_lo; p.norms = q->norms; p.out_lane_stride = q->out_lane_stride;
     p.qjl_proj_rot = q->qjl_proj_rot; p.cent_hi = q->cent_hi; p.cent_lo = q->cent_lo; p.qjl_bits = q->qjl_bits; p.qjl_gamma = q->qjl_gamma;
-    const unsigned grid = d == 256 ? 4 * unsigned(std::min<int64_t>(p.n_tiles, sms[dev] / 4)) : unsigned(std::min<int64_t>(p.n_tiles, sms[dev]));
+    const int64_t room = d == 256 ? quantize_sms() / 4 : quantize_sms(), ctas = std::min(room, tiles_each > 0 ? (p.n_tiles + tiles_each - 1) / tiles_each : p.n_tiles);
+    const unsigned grid = unsigned(d == 256 ? 4 * ctas : ctas);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;

@@ -308,11 +308,12 @@ extern "C" int tq_rotate(const void* x, int x_dtype, const float* rot, float* ou
     return launch_rowops(a, static_cast<cudaStream_t>(stream), "tq_rotate");
 }
 
-int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled, bool follows);
+int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled, bool follows, int tiles_each);
+int tq_quantize_tiles_each(const tq_quantize_args* q, int n);
 
 // follows: the launch before this one is a quantize of the same call on the tensor cores, and this one does not depend on it;
-// on return whether the next one may follow in turn.
-static int quantize_pack(const tq_quantize_args* q, void* stream, bool& follows) {
+// on return whether the next one may follow in turn.  tiles_each: tiles per CTA (0: as many CTAs as there are SMs).
+static int quantize_pack(const tq_quantize_args* q, void* stream, bool& follows, int tiles_each = 0) {
     const bool after = follows;
     follows = false;
     if (!q) return fail(TQ_ERR_INVALID, "tq_quantize_pack: null args");
@@ -328,7 +329,7 @@ static int quantize_pack(const tq_quantize_args* q, void* stream, bool& follows)
     if (q->qjl_bits && (!q->qjl_proj_rot || !q->qjl_gamma || !q->cent_hi || (q->bits_lo && !q->cent_lo))) return fail(TQ_ERR_INVALID, "tq_quantize_pack: QJL needs proj, gamma and centroids");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     bool handled = false;
-    int rc = tq_quantize_pack_tc(q, s, &handled, after);
+    int rc = tq_quantize_pack_tc(q, s, &handled, after, tiles_each);
     follows = handled;
     if (handled) return rc;
     RowArgs a{};
@@ -351,8 +352,9 @@ extern "C" int tq_quantize_pack_many(const tq_quantize_args* q, int n, void* str
     // keys and values, buffered and new rows: each is a launch of few tiles in a decode loop or a prefill piece; every one but the
     // first may start while the one before it still runs
     bool follows = false;
+    const int tiles_each = n > 1 ? tq_quantize_tiles_each(q, n) : 0;
     for (int i = 0; i < n; ++i)
-        if (int rc = quantize_pack(q + i, stream, follows)) return rc;
+        if (int rc = quantize_pack(q + i, stream, follows, tiles_each)) return rc;
     return TQ_OK;
 }
 
