@@ -12,15 +12,14 @@
 //              one accumulator.
 // Every product is exact in the fp32 accumulator; the normalisation by the row norm is applied afterwards.
 //
-// Warp roles in a persistent CTA (one per SM; 704 threads, 448 with the sketch on).  Epilogue warps come first (E of them),
+// Warp roles in a persistent CTA (one per SM; 704 threads).  Sixteen epilogue warps come first (E of them),
 // then one MMA warp, four norm warps, one TMA warp:
 //   warps 0..E-1 epilogue; thread <-> one row (TMEM lane) and a share of its sixteen-coordinate chunks (tcgen05.ld).
 //                fp16 rows: all sixteen warps work on the same tile in step, a quarter of the row each, reading the
 //                high and the low accumulator and combining them; two accumulator stages, so the MMAs of the next tile
 //                run meanwhile.  bf16 rows: two groups of eight warps take alternate tiles (two stages each), half a row
-//                per thread.  With the QJL sketch on, a thread owns a whole row (E = 8: two groups of four warps, two
-//                stages each): it forms the quantization residual of every coordinate and accumulates its 32
-//                projections (the projection matrix is read from shared memory as warp-wide broadcasts).
+//                per thread.  With the QJL sketch on, two groups as well and three stages: the quantization residual of
+//                every coordinate replaces it in tensor memory, and the MMA warp multiplies the tile by the projections.
 //                Up to 3 bits a binary search over boundaries (times the row's norm) held in registers adds its
 //                outcome bits straight into the packed word; at 4 bits one lookup in a 513-bin table (bin -> nearest
 //                boundary + count below; see build_bins).  Fractional widths: the threads of a row take chunks of
@@ -53,16 +52,8 @@ namespace tc {
 constexpr int DMAX = 128, TM = 128;              // largest head_dim, rows per tile
 constexpr int A_STAGES_MAX = 3, ACC_STAGES = 4;
 constexpr int N_NORM = 128;                      // threads that read the rows back for the norms
-// epilogue warps: 16, or 8 with the QJL sketch on (its 32 running projections per thread need the registers); then the
-// MMA warp, the norm warps, the TMA warp
-// (twelve warps in three groups were measured too: the compiler then has 96 registers per thread, spills 300 bytes, and the
-// launch takes the same time - the sketch variant is bound by its instruction count, some 30-37 per coordinate, not by how
-// many warps issue them)
-#ifndef TQ_QJL_EPI_WARPS
-#define TQ_QJL_EPI_WARPS 8
-#endif
-__host__ __device__ constexpr int epi_warps(bool qjl) { return qjl ? TQ_QJL_EPI_WARPS : 16; }
-__host__ __device__ constexpr int n_threads(bool qjl) { return epi_warps(qjl) * 32 + 32 + N_NORM + 32; }     // 704 / 448
+constexpr int EPI_WARPS = 16, N_EPI = EPI_WARPS * 32;            // epilogue warps; then the MMA warp, the norm warps, the TMA warp
+constexpr int NT = N_EPI + 32 + N_NORM + 32;
 constexpr int BIN_REP = 8;                       // copies of every lookup-table entry (lane & 7 picks one): fewer bank conflicts
 constexpr int KBLK_BYTES = TM * 128;             // one 64-column K-block of a 128-row operand: 16 KB
 constexpr int OPER_BYTES = 2 * KBLK_BYTES;       // 32 KB per operand tile
@@ -76,14 +67,15 @@ constexpr int OFF_R3 = OFF_A + 2 * OPER_BYTES;             // bf16: third term o
 constexpr int OFF_R1 = OFF_A + 3 * OPER_BYTES;             // R_hi / R_1
 constexpr int OFF_R2 = OFF_R1 + OPER_BYTES;                // R_lo / R_2
 constexpr int OFF_BINS = OFF_R2 + OPER_BYTES;              // NBINS x BIN_REP x 8 B: the table of the 4-bit codebook (only bits_hi can be 4)
-constexpr int OFF_PT = OFF_BINS + NBINS * BIN_REP * 8;     // QJL: (S R^T) as fp16 high / low parts in mma B-fragment order: [d / 16][4 n-tiles][hi | lo][32 lanes] x 8 bytes
+constexpr int OFF_PT = (OFF_BINS + NBINS * BIN_REP * 8 + 1023) / 1024 * 1024;     // QJL: (S R^T) as fp16 high and low parts, operand tiles of 32 rows x 64 columns (PT_KBLK bytes): hi 0, hi 1, lo 0, lo 1
+constexpr int PT_KBLK = QM * 128;
 constexpr int OFF_BND = OFF_PT + DMAX * QM * 4;            // 2 x 16 floats raw boundaries, 2 x 16 floats centroids
 constexpr int OFF_NSQ = OFF_BND + 256;                     // A_STAGES_MAX x 2 x 128 floats: partial sums of squares
 constexpr int OFF_BAR = OFF_NSQ + A_STAGES_MAX * 2 * TM * 4;   // mbarriers: 3 full, 3 a_free, 3 norm-ready, 4 acc_full, 4 acc_free
 constexpr int OFF_MISC = OFF_BAR + 24 * 8;                 // tmem base, abort flag
-constexpr int SK_LD = 32;                                  // QJL: bytes per staged row of 16 fp16 residuals; the two 16-byte halves of rows 4-7 (mod 8) swap places, so the eight rows of an 8 x 8 matrix land in distinct banks
-constexpr int OFF_SKETCH = (OFF_MISC + 64 + 127) / 128 * 128;   // QJL: one 32-row staging buffer per epilogue warp
-constexpr int SMEM_BYTES = OFF_SKETCH + TQ_QJL_EPI_WARPS * 32 * SK_LD;
+constexpr int OFF_EE = (OFF_MISC + 64 + 127) / 128 * 128;   // QJL: squares of the residual, the second half of a row's: SK_STAGES x 128 floats
+constexpr int SK_STAGES = 3, SK_COL0 = SK_STAGES * DMAX;    // QJL: accumulator stages; the sketches' 32 TMEM columns a stage lie behind them
+constexpr int SMEM_BYTES = OFF_EE + SK_STAGES * TM * 4;
 static_assert(SMEM_BYTES <= 227 * 1024, "shared-memory plan");
 
 constexpr int SLICE = 64, NSQ_SLOTS = 8;                   // head_dim 256: output columns of a CTA, norm slots
@@ -157,6 +149,13 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint6
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
+// D = A.B (+ D when accumulate != 0), A in tensor memory: row = lane, two fp16 columns a word
+__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
 // D = A.B + 2^-11 D
 __device__ __forceinline__ void umma_f16_scaled11(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
     const uint32_t one = 1;
@@ -186,6 +185,12 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
                    "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
                  : "r"(taddr) : "memory");
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+                   "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // K-major operand tile in shared memory, 128-byte swizzle: row r of K-block b at  b*16 KB + r*128 B, its 16-byte
@@ -328,38 +333,20 @@ __device__ __forceinline__ void store_words(uint8_t* dst, const uint32_t (&words
 }
 
 struct EpiCtx {
-    const Params& p; unsigned char* smem; uint32_t tmem_base, bar_accfull, bar_accfree, bar_afree, bar_nrm;
+    const Params& p; unsigned char* smem; uint32_t tmem_base, bar_accfull, bar_accfree, bar_afree, bar_nrm, bar_res, bar_proj;
     volatile int* abort_flag; int warp, lane;
     uint8_t* dst; int nb; bool write_norms;        // head_dim 256: the slice's first byte, bytes of a packed row, this slice writes the norms
 };
 
-// QJL: the residual of sixteen coordinates (normalised rotated value minus its centroid) enters the 32 projections and
-// the residual's sum of squares.  A thread owns a row, a warp 32 rows: the projections of the warp's rows are a
-// 32 x 16 by 16 x 32 product per call, done with mma.sync (a CUDA-core version cost 32 multiply-adds and 8 shared-memory
-// reads per coordinate and thread: two thirds of the kernel's instructions).  Only the SIGN of a projection is kept, so
-// the residual is scaled by 2^8 (clear of fp16 subnormals) and split into fp16 high and low parts, as is S R^T:
-// acc += hi x hi + lo x hi + hi x lo reproduces the float32 product to about 2^-21.  The operands go through a
-// 32-row staging buffer of the warp (row = lane) and come back as fragments with ldmatrix.
-struct Sketch {
-    float acc[2][4][4];        // [16-row half of the warp][8 projections][mma accumulator]: rows g / g + 8, projections 2t, 2t + 1
-    uint32_t stage;            // shared-window address of the warp's staging buffer
-    const uint2* bfrag;        // B fragments of S R^T (OFF_PT)
-    int lane;
-};
-__device__ __forceinline__ void sk_mma(float (&c)[4], const uint32_t (&a)[4], uint2 b) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y));
-}
-__device__ __forceinline__ void sk_ldsm(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void sk_sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
+// QJL: the residual of sixteen coordinates (normalised rotated value minus its centroid) enters the residual's sum of squares and goes back
+// into tensor memory, into the sixteen columns it came from: it is the A operand of the 32 projections, a product of 128 x d by d x 32 a
+// tile.  Only the SIGN of a projection is kept, so the residual is scaled by 2^8 (clear of fp16 subnormals) and split into fp16 high and low
+// parts (columns 0-7 and 8-15), as is S R^T: hi x hi + lo x hi + hi x lo reproduces the float32 product to about 2^-21.
+// (With mma.sync a thread kept 32 running projections, a warp staged its residuals through shared memory, and the registers allowed eight
+// epilogue warps: keys at 4 bits and values at 2 of 1,048,576 rows of 96 took 196 + 168 us, 161 + 124 now; the signs are the same.)
 template <int BITS>
-__device__ __forceinline__ void sketch16(const uint32_t* v, uint32_t g0, uint32_t g1, float rinv, const float* cent, int col0, Sketch& sk, float& ee) {
-    uint32_t hi[8], lo[8];
+__device__ __forceinline__ void sketch16(const uint32_t* v, uint32_t g0, uint32_t g1, float rinv, const float* cent, uint32_t taddr, float& ee) {
+    uint32_t x[16];
 #pragma unroll
     for (int i = 0; i < 16; i += 2) {
         float e2[2];
@@ -373,60 +360,10 @@ __device__ __forceinline__ void sketch16(const uint32_t* v, uint32_t g0, uint32_
         const __half2 h = __floats2half2_rn(e2[0], e2[1]);
         const float2 hf = __half22float2(h);
         const __half2 l = __floats2half2_rn(e2[0] - hf.x, e2[1] - hf.y);
-        hi[i >> 1] = *reinterpret_cast<const uint32_t*>(&h);
-        lo[i >> 1] = *reinterpret_cast<const uint32_t*>(&l);
+        x[i >> 1] = *reinterpret_cast<const uint32_t*>(&h);
+        x[8 + (i >> 1)] = *reinterpret_cast<const uint32_t*>(&l);
     }
-    const uint32_t swz = uint32_t((sk.lane >> 2) & 1) * 16;                                            // rows 4-7 (mod 8): halves swapped
-    const uint32_t row = sk.stage + uint32_t(sk.lane) * SK_LD;
-    const uint32_t frag = sk.stage + uint32_t(sk.lane & 15) * SK_LD + ((uint32_t(sk.lane >> 4) * 16) ^ swz);   // ldmatrix row of this lane (second half: + 16 rows)
-    uint32_t ah[2][4], al[2][4];
-    sk_sts128(row + swz, hi[0], hi[1], hi[2], hi[3]);
-    sk_sts128(row + (16 ^ swz), hi[4], hi[5], hi[6], hi[7]);
-    __syncwarp();
-    sk_ldsm(ah[0], frag);
-    sk_ldsm(ah[1], frag + 16 * SK_LD);
-    __syncwarp();
-    sk_sts128(row + swz, lo[0], lo[1], lo[2], lo[3]);
-    sk_sts128(row + (16 ^ swz), lo[4], lo[5], lo[6], lo[7]);
-    __syncwarp();
-    sk_ldsm(al[0], frag);
-    sk_ldsm(al[1], frag + 16 * SK_LD);
-    __syncwarp();
-    const uint2* bf = sk.bfrag + (col0 >> 4) * (4 * 2 * 32) + sk.lane;
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-        const uint2 bh = bf[(nt * 2 + 0) * 32], bl = bf[(nt * 2 + 1) * 32];
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-            sk_mma(sk.acc[mt][nt], ah[mt], bh);
-            sk_mma(sk.acc[mt][nt], al[mt], bh);
-            sk_mma(sk.acc[mt][nt], ah[mt], bl);
-        }
-    }
-}
-// The sign word of this thread's row (row = lane) from the warp's accumulators: bit p set iff projection p >= 0.
-__device__ __forceinline__ uint32_t sketch_bits(const Sketch& sk) {
-    const int g = sk.lane >> 2, t = sk.lane & 3;
-    uint32_t w[4];                                         // rows g, g + 8, 16 + g, 24 + g: this lane's two bits per n-tile
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            uint32_t x = 0;
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt)
-                x |= ((sk.acc[mt][nt][2 * h] >= 0.f ? 1u : 0u) | (sk.acc[mt][nt][2 * h + 1] >= 0.f ? 2u : 0u)) << (8 * nt + 2 * t);
-            x |= __shfl_xor_sync(0xffffffffu, x, 1);
-            x |= __shfl_xor_sync(0xffffffffu, x, 2);
-            w[mt * 2 + h] = x;
-        }
-    // row r = lane is held by the lanes of group g = r & 7 as word (r >> 3)
-    const int src = (sk.lane & 7) * 4;
-    const uint32_t w0 = __shfl_sync(0xffffffffu, w[0], src), w1 = __shfl_sync(0xffffffffu, w[1], src);
-    const uint32_t w2 = __shfl_sync(0xffffffffu, w[2], src), w3 = __shfl_sync(0xffffffffu, w[3], src);
-    const int k = sk.lane >> 3;
-    (void)g;
-    return k == 0 ? w0 : k == 1 ? w1 : k == 2 ? w2 : w3;
+    tmem_st16(taddr, x);
 }
 
 // A run of a row's coordinates ([col0, col0 + 16 * nch) at BITS bits) in rolled steps of 32 coordinates; the step's codes
@@ -436,7 +373,7 @@ __device__ __forceinline__ uint32_t sketch_bits(const Sketch& sk) {
 // NCH: the number of chunks when it is known at compile time (1 or 2: a single step whose shape folds), 0 = nch_rt.
 template <int BITS, bool QJL, bool SPLITACC, int NCH, int TERMS = 2>
 __device__ __forceinline__ void quantize_part(uint32_t t_row, int col0, int nch_rt, int lo_off, const RowCtx& rc, const float (&sb)[7], const float* raw,
-                                              const float* cent, uint8_t* dst, bool live, Sketch& sk, float& ee) {
+                                              const float* cent, uint8_t* dst, bool live, float& ee) {
     constexpr int NW = 2 * 16 * BITS / 32;                                          // words of a step: BITS
     const int nch = NCH ? NCH : nch_rt;
 #pragma unroll 1
@@ -454,7 +391,7 @@ __device__ __forceinline__ void quantize_part(uint32_t t_row, int col0, int nch_
             if (c < nc) {
                 uint32_t g0, g1;
                 uint32_t* vc = v + ((SPLITACC || QJL) ? 0 : 16 * c);
-                if (QJL && !SPLITACC) {                                         // (the sketch keeps 32 accumulators: sixteen columns at a time)
+                if (QJL && !SPLITACC) {                                         // (they are replaced in place: sixteen columns at a time)
                     tmem_ld16(t_row + col0 + (c0 + c) * 16, *reinterpret_cast<uint32_t (*)[16]>(v));
                     tmem_ld_wait();
                 }
@@ -478,7 +415,7 @@ __device__ __forceinline__ void quantize_part(uint32_t t_row, int col0, int nch_
                 quantize16<BITS>(vc, rc, sb, raw, g0, g1);
                 put_group<BITS, NW>(w, 2 * c, g0);
                 put_group<BITS, NW>(w, 2 * c + 1, g1);
-                if constexpr (QJL) sketch16<BITS>(vc, g0, g1, rc.rinv * 256.f, cent, col0 + (c0 + c) * 16, sk, ee);
+                if constexpr (QJL) sketch16<BITS>(vc, g0, g1, rc.rinv * 256.f, cent, t_row + col0 + (c0 + c) * 16, ee);
             }
         }
         if (live) store_words<NW>(dst + c0 * 2 * BITS, w, nc * 2 * BITS);
@@ -493,14 +430,13 @@ __device__ __forceinline__ uint32_t sbase_of(const EpiCtx& e) { return static_ca
 //     row and a quarter of its sixteen-coordinate chunks (of either width) - while the MMAs of the next tile run.
 //   bf16 rows: one accumulator per tile, four stages; two groups of eight warps take alternate tiles (two stages each),
 //     a thread owns one row and half of its chunks.
-//   QJL sketch: a thread needs the whole row (32 running projections) and the registers for it: eight epilogue warps,
-//     two groups of four that take alternate tiles, one accumulator per tile, two stages per group.
+//   QJL sketch: as bf16 rows, three stages: a group hands its residuals to the MMA warp, waits for the tile's projections while
+//     the other group works, and signs them; the MMAs of a third tile run meanwhile.
 template <bool QJL, bool SPLITACC> struct EpiShape {
-    static constexpr int EW = epi_warps(QJL), NT = n_threads(QJL), N_EPI = EW * 32;
-    static constexpr int GROUPS = SPLITACC ? 1 : QJL ? epi_warps(true) / 4 : 2;     // groups of warps that take tiles in turn
-    static constexpr int WPG = EW / GROUPS;                                         // warps per group: 4 row quadrants x SPLIT shares of the columns
+    static constexpr int GROUPS = SPLITACC ? 1 : 2;                                 // groups of warps that take tiles in turn
+    static constexpr int WPG = EPI_WARPS / GROUPS;                                  // warps per group: 4 row quadrants x SPLIT shares of the columns
     static constexpr int SPLIT = WPG / 4;
-    static constexpr int STAGES = SPLITACC ? 2 : 4;                                 // accumulator stages
+    static constexpr int STAGES = SPLITACC ? 2 : QJL ? SK_STAGES : 4;               // accumulator stages
     static constexpr int STAGE_COLS = SPLITACC ? 2 * DMAX : DMAX;
 };
 // DC: head_dim when it is known at compile time (the chunk shares, row widths and store shapes then fold), 0 = read it
@@ -521,10 +457,6 @@ __device__ __forceinline__ void epilogue_loop(const EpiCtx& e) {
     const float* raw_l = raw_h + 16;
     const float* cent_h = raw_h + 32;
     const float* cent_l = raw_h + 48;
-    Sketch sk;
-    sk.stage = static_cast<uint32_t>(__cvta_generic_to_shared(e.smem + OFF_SKETCH)) + uint32_t(e.warp) * 32 * SK_LD;
-    sk.bfrag = reinterpret_cast<const uint2*>(e.smem + OFF_PT);
-    sk.lane = e.lane;
     RowCtx rc;
     rc.bins = reinterpret_cast<const float2*>(e.smem + OFF_BINS) + (e.lane & (BIN_REP - 1));      // 4-bit side only
     float bnd_h[7], bnd_l[7];
@@ -571,28 +503,42 @@ __device__ __forceinline__ void epilogue_loop(const EpiCtx& e) {
         if (tl >= tpl) { tl -= tpl; ++lane_o; }
         const uint32_t t_row = e.tmem_base + (uint32_t(quad * 32) << 16) + a * Sh::STAGE_COLS;
         float ee = 0.f;
-        if (QJL) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) (&sk.acc[0][0][0])[i] = 0.f;
-        }
         // with head_dim 128 and quarter shares every thread has two chunks of an integer width, or one of each fractional width
         constexpr int NCH_H = (DC == 128 && Sh::SPLIT == 4) ? (BL ? 1 : 2) : 0, NCH_L = (DC == 128 && Sh::SPLIT == 4) ? 1 : 0;
         if constexpr (DC == 256)
-            quantize_part<BH, QJL, SPLITACC, 1, TERMS>(t_row, h0 * 16, 1, SLICE, rc, sb_h, raw_h, cent_h, e.dst + orow * e.nb + h0 * 2 * BH, live, sk, ee);
+            quantize_part<BH, QJL, SPLITACC, 1, TERMS>(t_row, h0 * 16, 1, SLICE, rc, sb_h, raw_h, cent_h, e.dst + orow * e.nb + h0 * 2 * BH, live, ee);
         else
-        quantize_part<BH, QJL, SPLITACC, NCH_H>(t_row, h0 * 16, h1 - h0, d, rc, sb_h, raw_h, cent_h, p.p_hi + orow * nb_h + h0 * 2 * BH, live, sk, ee);
-        if (BL) quantize_part<(BL ? BL : 1), QJL, SPLITACC, NCH_L>(t_row, half + l0 * 16, l1 - l0, d, rc, sb_l, raw_l, cent_l, p.p_lo + orow * nb_l + l0 * 2 * BL, live, sk, ee);
-        tc_fence_before();
-        mbar_arrive(e.bar_accfree + 8 * a);                     // the accumulator may be overwritten
-        uint32_t zb = 0;
-        if (QJL) zb = sketch_bits(sk);                          // (every lane of the warp takes part)
-        if (live && part == 0 && (DC != 256 || e.write_norms)) {
-            p.norms[orow] = nrm;
-            if (QJL) {
-                if (nrm == 0.f) zb = 0xffffffffu;               // zero row: the reference's residual is exactly 0, and 0 >= 0
-                p.qjl_bits[orow] = zb;
-                p.qjl_gamma[orow] = nrm * sqrtf(ee) * (1.f / 256.f);   // |x - dequant(x)| = |x| |y_n - c| (the rotation is orthogonal); ee sums 2^16 times the squares
+        quantize_part<BH, QJL, SPLITACC, NCH_H>(t_row, h0 * 16, h1 - h0, d, rc, sb_h, raw_h, cent_h, p.p_hi + orow * nb_h + h0 * 2 * BH, live, ee);
+        if (BL) quantize_part<(BL ? BL : 1), QJL, SPLITACC, NCH_L>(t_row, half + l0 * 16, l1 - l0, d, rc, sb_l, raw_l, cent_l, p.p_lo + orow * nb_l + l0 * 2 * BL, live, ee);
+        if constexpr (QJL) {
+            static_assert(Sh::SPLIT == 2, "two threads a row");
+            float* ee_slot = reinterpret_cast<float*>(e.smem + OFF_EE) + a * TM + row_in_tile;
+            if (part == 1) *ee_slot = ee;
+            tmem_st_wait();
+            tc_fence_before();
+            mbar_arrive(e.bar_res + 8 * a);                     // residuals and squares of this share are there
+            const uint32_t ph = uint32_t(it / Sh::STAGES) & 1u;
+            if (!mbar_wait(e.bar_res + 8 * a, ph, e.abort_flag, 4) || !mbar_wait(e.bar_proj + 8 * a, ph, e.abort_flag, 8)) break;
+            tc_fence_after();
+            uint32_t pr[16], zb = 0;                            // this thread's half of the row's projections
+            tmem_ld16(e.tmem_base + (uint32_t(quad * 32) << 16) + SK_COL0 + a * QM + part * 16, pr);
+            tmem_ld_wait();
+            if (part == 0) ee += *ee_slot;
+            tc_fence_before();
+            mbar_arrive(e.bar_accfree + 8 * a);                 // the accumulator may be overwritten
+#pragma unroll
+            for (int i = 0; i < 16; ++i) zb |= __uint_as_float(pr[i]) >= 0.f ? 1u << i : 0u;
+            if (live) {
+                reinterpret_cast<uint16_t*>(p.qjl_bits + orow)[part] = uint16_t(nrm == 0.f ? 0xffffu : zb);     // zero row: the reference's residual is exactly 0, and 0 >= 0
+                if (part == 0) {
+                    p.norms[orow] = nrm;
+                    p.qjl_gamma[orow] = nrm * sqrtf(ee) * (1.f / 256.f);   // |x - dequant(x)| = |x| |y_n - c| (the rotation is orthogonal); ee sums 2^16 times the squares
+                }
             }
+        } else {
+            tc_fence_before();
+            mbar_arrive(e.bar_accfree + 8 * a);                     // the accumulator may be overwritten
+            if (live && part == 0 && (DC != 256 || e.write_norms)) p.norms[orow] = nrm;
         }
     }
 }
@@ -600,9 +546,9 @@ __device__ __forceinline__ void epilogue_loop(const EpiCtx& e) {
 // SPLITACC (fp16 rows without the sketch): high and low products in two accumulators, one MMA of N = 2 d per k-step
 // against [R_hi ; R_lo].  Otherwise one accumulator: fp16 low products first and the scale-input-d trick, bf16 three terms.
 template <bool QJL, bool SPLITACC, int DC>
-__global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p, const __grid_constant__ CUtensorMap tmap) {
+__global__ void __launch_bounds__(NT, 1) quantize_tc_kernel(Params p, const __grid_constant__ CUtensorMap tmap) {
     using Sh = EpiShape<QJL, SPLITACC>;
-    constexpr int ACCS = Sh::STAGES, NT = Sh::NT, EPI_WARPS = Sh::EW, N_EPI = Sh::N_EPI;
+    constexpr int ACCS = Sh::STAGES;
     extern __shared__ __align__(1024) unsigned char smem[];
     const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // (warp: uniform)
@@ -616,6 +562,7 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
     const uint32_t bar_full = sbase + OFF_BAR, bar_afree = bar_full + 8 * A_STAGES_MAX, bar_nrm = bar_afree + 8 * A_STAGES_MAX;
     const uint32_t bar_accfull = bar_nrm + 8 * A_STAGES_MAX, bar_accfree = bar_accfull + 8 * ACC_STAGES;      // (ACCS of the 4 slots are used)
     const uint32_t bar_drain = bar_accfree + 8 * ACC_STAGES;              // products in flight when a wait ran out
+    const uint32_t bar_res = bar_drain + 8, bar_proj = bar_res + 8 * SK_STAGES;       // QJL: residuals of a stage written (epilogue group -> MMA), its projections done (MMA commit -> group)
 
     if (sbase & 1023u) {                  // the swizzled operand tiles need 1024-byte alignment (uniform across the CTA)
         if (tid == 0) atomicCAS(&g_status, 0, 9);
@@ -634,6 +581,7 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
         if (DC == 256)
             for (int q = 0; q < NSQ_SLOTS; ++q) mbar_init(sbase + OFF_NRMBAR256 + 8 * q, N_NORM);
         mbar_init(bar_drain, 1);
+        for (int a = 0; a < SK_STAGES; ++a) { mbar_init(bar_res + 8 * a, N_EPI / Sh::GROUPS); mbar_init(bar_proj + 8 * a, 1); }
         for (int a = 0; a < ACC_STAGES; ++a) { mbar_init(bar_accfull + 8 * a, 1); mbar_init(bar_accfree + 8 * a, N_EPI / Sh::GROUPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -728,30 +676,26 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
             raw[tid] = val;
         }
         if (QJL) {
-            // (S R^T) is (32, d): as mma B fragments (k = coordinate, n = projection), fp16 high and low parts;
-            // lane (g, t) of fragment (k-step ks, n-tile nt): b0 = coordinates 16 ks + 2t, + 1 of projection 8 nt + g, b1 = the same + 8
-            uint2* bf = reinterpret_cast<uint2*>(smem + OFF_PT);
-            for (int idx = tid; idx < (d / 16) * 4 * 32; idx += NT) {
-                const int ks = idx >> 7, nt = (idx >> 5) & 3, ln = idx & 31, g = ln >> 2, t = ln & 3;
-                const float* srow = p.qjl_proj_rot + (8 * nt + g) * d + 16 * ks + 2 * t;
-                uint32_t hw[2], lw[2];
+            // (S R^T) is (32, d): row = projection, K-blocks of 64 coordinates, swizzled like R
+            for (int idx = tid; idx < QM * (d / 8); idx += NT) {
+                const int j = idx / (d / 8), c = idx - j * (d / 8);
+                const float* srow = p.qjl_proj_rot + j * d + c * 8;
+                __align__(16) __half hi[8], lo[8];
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const float x0 = __ldg(srow + 8 * u), x1 = __ldg(srow + 8 * u + 1);
-                    const __half2 h = __floats2half2_rn(x0, x1);
-                    const float2 hf = __half22float2(h);
-                    const __half2 l = __floats2half2_rn(x0 - hf.x, x1 - hf.y);
-                    hw[u] = *reinterpret_cast<const uint32_t*>(&h);
-                    lw[u] = *reinterpret_cast<const uint32_t*>(&l);
+                for (int i = 0; i < 8; ++i) {
+                    const float x = __ldg(srow + i);
+                    hi[i] = __float2half_rn(x);
+                    lo[i] = __float2half_rn(x - __half2float(hi[i]));
                 }
-                bf[((ks * 4 + nt) * 2 + 0) * 32 + ln] = make_uint2(hw[0], hw[1]);
-                bf[((ks * 4 + nt) * 2 + 1) * 32 + ln] = make_uint2(lw[0], lw[1]);
+                unsigned char* dst = smem + OFF_PT + (c >> 3) * PT_KBLK + j * 128 + (((c & 7) ^ (j & 7)) << 4);
+                *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(hi);
+                *reinterpret_cast<uint4*>(dst + 2 * PT_KBLK) = *reinterpret_cast<const uint4*>(lo);
             }
         }
         __syncthreads();
         if ((DC == 256 ? slice_bits : p.bits_hi) == 4) build_bins(reinterpret_cast<float2*>(smem + OFF_BINS), raw, 15, tid, NT);
     }
-    if (warp == EPI_WARPS) {              // one warp owns the TMEM allocation: 4 stages x 128 columns
+    if (warp == EPI_WARPS) {              // one warp owns the TMEM allocation
         tmem_alloc(sbase + OFF_MISC, 512);
         tmem_relinquish();
     }
@@ -764,7 +708,7 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
 
     if (warp < EPI_WARPS) {
         // ======================= epilogue: row = 32 * (warp % 4) + lane; groups and column halves as in EpiShape =======================
-        EpiCtx e{p, smem, tmem_base, bar_accfull, bar_accfree, bar_afree, bar_nrm, abort_flag, warp, lane, nullptr, 0, true};
+        EpiCtx e{p, smem, tmem_base, bar_accfull, bar_accfree, bar_afree, bar_nrm, bar_res, bar_proj, abort_flag, warp, lane, nullptr, 0, true};
         if constexpr (DC == 256) {
             const int coords = p.bits_lo ? 128 : 256;                      // of a packed row of this slice's width
             e.nb = coords * slice_bits / 8;
@@ -827,6 +771,22 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
         {
             const uint32_t idesc = make_idesc(SPLITACC ? 2 * d : d, bf16);
             const int ksteps = d / 16;
+            // QJL: the projections of tile `n` of this CTA, in the order that leaves the next tiles' products in front of them
+            const uint32_t idesc_p = make_idesc(QM, false);
+            auto project = [&](int n) {
+                const int a = n % ACCS;
+                if (!wait_all(bar_res + 8 * a, uint32_t(n / ACCS) & 1u, abort_flag, 4)) return false;
+                tc_fence_after();
+                const uint32_t res = tmem_base + a * Sh::STAGE_COLS, acc = tmem_base + SK_COL0 + a * QM;
+                for (int ks = 0; ks < ksteps; ++ks) {
+                    const uint64_t hi = smem_desc(sbase + OFF_PT + (ks >> 2) * PT_KBLK, 0, ks & 3), lo = smem_desc(sbase + OFF_PT + (2 + (ks >> 2)) * PT_KBLK, 0, ks & 3);
+                    umma_f16_ta(acc, res + 16 * ks, hi, idesc_p, ks ? 1u : 0u);
+                    umma_f16_ta(acc, res + 16 * ks + 8, hi, idesc_p, 1u);
+                    umma_f16_ta(acc, res + 16 * ks, lo, idesc_p, 1u);
+                }
+                umma_commit(bar_proj + 8 * a);
+                return true;
+            };
             int it = 0;
             for (int64_t tile = blockIdx.x; tile < p.n_tiles; tile += gridDim.x, ++it) {
                 const int a = it % ACCS, s = it % a_stages;
@@ -853,7 +813,11 @@ __global__ void __launch_bounds__(n_threads(QJL), 1) quantize_tc_kernel(Params p
                 }
                 umma_commit(bar_afree + 8 * s);      // rows of this stage consumed
                 umma_commit(bar_accfull + 8 * a);    // the accumulator is complete: its epilogue group may read it
+                if (QJL && it >= ACCS - 1 && !project(it - (ACCS - 1))) break;
             }
+            if (QJL)
+                for (int n = max(0, it - (ACCS - 1)); n < it && !__any_sync(0xffffffffu, *abort_flag != 0); ++n)
+                    if (!project(n)) break;
         }
         if (__any_sync(0xffffffffu, *abort_flag != 0)) { umma_commit(bar_drain); mbar_drain(bar_drain, 0); }
         __syncwarp();
@@ -1072,7 +1036,7 @@ int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(unsigned(tc::n_threads(qjl)));
+    cfg.blockDim = dim3(unsigned(tc::NT));
     cfg.dynamicSmemBytes = tc::SMEM_BYTES;
     cfg.stream = s;
     cfg.attrs = attr;
