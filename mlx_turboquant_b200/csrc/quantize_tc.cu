@@ -270,12 +270,18 @@ struct RowCtx {
 
 // Sixteen coordinates (TMEM columns taddr .. + 15) at BITS bits: the codes go into g0 / g1 (eight codes each, BITS bits
 // per code).  sb: boundaries times the row's norm (register search); raw: unscaled boundaries (table path's fallback).
-template <int BITS>
-__device__ __forceinline__ void quantize16(const uint32_t* v, const RowCtx& rc, const float (&sb)[7], const float* raw, uint32_t& g0, uint32_t& g1) {
+// QJL: v[] leaves as 2^8 times the residuals (rbin and the centroids carry the factor); taddr: where v[] came from.
+template <int BITS, bool QJL>
+__device__ __forceinline__ void quantize16(uint32_t* v, const RowCtx& rc, const float (&sb)[7], const float* raw, uint32_t& g0, uint32_t& g1, const float* cent, uint32_t taddr) {
     g0 = g1 = 0;
+    const auto residual = [&](int i, uint32_t code) { v[i] = __float_as_uint(fmaf(__uint_as_float(v[i]), rc.rbin, -cent[code])); };
     if (BITS <= 3) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) add_code<BITS>(i < 8 ? g0 : g1, __uint_as_float(v[i]), sb, BITS * (i & 7));
+        if constexpr (QJL) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) residual(i, ((i < 8 ? g0 : g1) >> (BITS * (i & 7))) & ((1u << BITS) - 1u));
+        }
     } else {
         // table path: count-below times 16^k goes in with one multiply-add, the compare adds its bit in place
         uint32_t seen = 0;
@@ -288,14 +294,27 @@ __device__ __forceinline__ void quantize16(const uint32_t* v, const RowCtx& rc, 
             const float2 en = rc.bins[min(__float_as_uint(tt) & 0x3FFu, uint32_t(NBINS - 1)) * BIN_REP];     // (the clamp only matters for |y| > |x|, i.e. never)
             seen |= __float_as_uint(en.y);
             uint32_t& w = i < 8 ? g0 : g1;
-            w += __float_as_uint(en.y) * (1u << (4 * (i & 7)));
-            if ((yp * rc.rinv) > en.x) w += 1u << (4 * (i & 7));                  // strict >, codebook.py:220-223
+            if constexpr (QJL) {
+                const uint32_t code = __float_as_uint(en.y) + ((yp * rc.rinv) > en.x ? 1u : 0u);
+                w += code * (1u << (4 * (i & 7)));
+                residual(i, code & 15u);                                           // (a marked bin's is formed again below)
+            } else {
+                w += __float_as_uint(en.y) * (1u << (4 * (i & 7)));
+                if ((yp * rc.rinv) > en.x) w += 1u << (4 * (i & 7));               // strict >, codebook.py:220-223
+            }
         }
         if (__any_sync(0xffffffffu, (seen & MARKED) != 0)) {     // a marked bin was hit: redo the group with the counting loop
             g0 = g1 = 0;
+            if constexpr (QJL) {
+                tmem_ld16(taddr, *reinterpret_cast<uint32_t (*)[16]>(v));
+                tmem_ld_wait();
+            }
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-                (i < 8 ? g0 : g1) |= code_slow(__uint_as_float(v[i]) * rc.rinv, raw, 15) << (4 * (i & 7));
+            for (int i = 0; i < 16; ++i) {
+                const uint32_t code = code_slow(__uint_as_float(v[i]) * rc.rinv, raw, 15);
+                (i < 8 ? g0 : g1) |= code << (4 * (i & 7));
+                if constexpr (QJL) residual(i, code);
+            }
         }
     }
 }
@@ -344,19 +363,13 @@ struct EpiCtx {
 // parts (columns 0-7 and 8-15), as is S R^T: hi x hi + lo x hi + hi x lo reproduces the float32 product to about 2^-21.
 // (With mma.sync a thread kept 32 running projections, a warp staged its residuals through shared memory, and the registers allowed eight
 // epilogue warps: keys at 4 bits and values at 2 of 1,048,576 rows of 96 took 196 + 168 us, 161 + 124 now; the signs are the same.)
-template <int BITS>
-__device__ __forceinline__ void sketch16(const uint32_t* v, uint32_t g0, uint32_t g1, float rinv, const float* cent, uint32_t taddr, float& ee) {
+__device__ __forceinline__ void sketch16(const uint32_t* e, uint32_t taddr, float& ee) {
     uint32_t x[16];
 #pragma unroll
     for (int i = 0; i < 16; i += 2) {
-        float e2[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const uint32_t code = (((i + u) < 8 ? g0 : g1) >> (BITS * ((i + u) & 7))) & ((1u << BITS) - 1u);
-            const float e = fmaf(__uint_as_float(v[i + u]), rinv, -cent[code]);       // 2^8 times the residual (rinv and the centroids carry the factor)
-            ee = fmaf(e, e, ee);
-            e2[u] = e;
-        }
+        const float e2[2] = {__uint_as_float(e[i]), __uint_as_float(e[i + 1])};
+        ee = fmaf(e2[0], e2[0], ee);
+        ee = fmaf(e2[1], e2[1], ee);
         const __half2 h = __floats2half2_rn(e2[0], e2[1]);
         const float2 hf = __half22float2(h);
         const __half2 l = __floats2half2_rn(e2[0] - hf.x, e2[1] - hf.y);
@@ -374,20 +387,20 @@ __device__ __forceinline__ void sketch16(const uint32_t* v, uint32_t g0, uint32_
 template <int BITS, bool QJL, bool SPLITACC, int NCH, int TERMS = 2>
 __device__ __forceinline__ void quantize_part(uint32_t t_row, int col0, int nch_rt, int lo_off, const RowCtx& rc, const float (&sb)[7], const float* raw,
                                               const float* cent, uint8_t* dst, bool live, float& ee) {
-    constexpr int NW = 2 * 16 * BITS / 32;                                          // words of a step: BITS
+    constexpr int STEP = QJL ? 1 : 2, NW = (STEP * 16 * BITS + 31) / 32;            // chunks of a step and its words
     const int nch = NCH ? NCH : nch_rt;
 #pragma unroll 1
-    for (int c0 = 0; c0 < nch; c0 += 2) {
+    for (int c0 = 0; c0 < nch; c0 += STEP) {
         uint32_t v[32], w[NW];
 #pragma unroll
         for (int i = 0; i < NW; ++i) w[i] = 0;
-        const int nc = min(2, nch - c0);                                            // a run may end on a half step
+        const int nc = min(STEP, nch - c0);                                         // a run may end on a half step
         if (!SPLITACC && !QJL) {
             tmem_ld32(t_row + col0 + c0 * 16, v);
             tmem_ld_wait();
         }
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < STEP; ++c) {
             if (c < nc) {
                 uint32_t g0, g1;
                 uint32_t* vc = v + ((SPLITACC || QJL) ? 0 : 16 * c);
@@ -412,10 +425,10 @@ __device__ __forceinline__ void quantize_part(uint32_t t_row, int col0, int nch_
                         for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(fmaf(__uint_as_float(v[16 + i]), 1.f / 2048.f, __uint_as_float(v[i])));
                     }
                 }
-                quantize16<BITS>(vc, rc, sb, raw, g0, g1);
+                quantize16<BITS, QJL>(vc, rc, sb, raw, g0, g1, cent, t_row + col0 + (c0 + c) * 16);
                 put_group<BITS, NW>(w, 2 * c, g0);
                 put_group<BITS, NW>(w, 2 * c + 1, g1);
-                if constexpr (QJL) sketch16<BITS>(vc, g0, g1, rc.rinv * 256.f, cent, t_row + col0 + (c0 + c) * 16, ee);
+                if constexpr (QJL) sketch16(vc, t_row + col0 + (c0 + c) * 16, ee);
             }
         }
         if (live) store_words<NW>(dst + c0 * 2 * BITS, w, nc * 2 * BITS);
@@ -875,7 +888,7 @@ __global__ void __launch_bounds__(NT, 1) quantize_tc_kernel(Params p, const __gr
             for (int c = 0; c < 8; ++c) {
                 const uint4 v = *reinterpret_cast<const uint4*>(rowp + ((c ^ (r & 7)) << 4));
                 uint4 w = make_uint4(0, 0, 0, 0);
-                if (d > 64) w = *reinterpret_cast<const uint4*>(rowp + KBLK_BYTES + ((c ^ (r & 7)) << 4));
+                if (d > 64 + 8 * c) w = *reinterpret_cast<const uint4*>(rowp + KBLK_BYTES + ((c ^ (r & 7)) << 4));
                 if (!bf16) {
                     const __half2* h = reinterpret_cast<const __half2*>(&v);
                     const __half2* g = reinterpret_cast<const __half2*>(&w);
