@@ -54,10 +54,10 @@ constexpr int A_STAGES_MAX = 3, ACC_STAGES = 4;
 constexpr int N_NORM = 128;                      // threads that read the rows back for the norms
 constexpr int EPI_WARPS = 16, N_EPI = EPI_WARPS * 32;            // epilogue warps; then the MMA warp, the norm warps, the TMA warp
 constexpr int NT = N_EPI + 32 + N_NORM + 32;
-constexpr int BIN_REP = 8;                       // copies of every lookup-table entry (lane & 7 picks one): fewer bank conflicts
+constexpr int BIN_REP = 16;                      // copies of every lookup-table entry (lane & 15 picks one): the lanes of a half-warp read banks of their own
 constexpr int KBLK_BYTES = TM * 128;             // one 64-column K-block of a 128-row operand: 16 KB
 constexpr int OPER_BYTES = 2 * KBLK_BYTES;       // 32 KB per operand tile
-constexpr int NBINS = 516;                       // 513 used + guard
+constexpr int NBINS = 257, BIN0 = 128;           // the table's bins: 1/256 wide around (k - BIN0) / 256
 constexpr int QM = 32;                           // projections of the QJL sketch
 constexpr uint32_t WAIT_LIMIT = 4u << 20;        // bounded spin: a few hundred milliseconds at most
 
@@ -210,15 +210,18 @@ __device__ __forceinline__ uint32_t make_idesc(int d, bool bf16) {
     return (1u << 4) | (bf16 ? ((1u << 7) | (1u << 10)) : 0u) | (uint32_t(d >> 3) << 17) | (uint32_t(TM >> 4) << 24);
 }
 
-// Lookup table for the boundary search.  Bin k covers normalised values around (k - 256) / 256 (width 1/256);
-// entry = (boundary to test, number of boundaries below the bin's neighbourhood) where the neighbourhood is the
+// Lookup table for the boundary search.  Bin k covers normalised values around (k - BIN0) / 256 (width 1/256), the first and the last also
+// everything beyond; entry = (boundary to test, number of boundaries below the bin's neighbourhood) where the neighbourhood is the
 // bin widened by one bin on each side, so that a bin index that is off by one through rounding still gives the
 // exact count.  A neighbourhood holding two boundaries is marked (a flag bit in the count) and handled by the plain
-// counting loop.
+// counting loop.  (Half the bins that |y| <= 1 could use, for twice the copies: the outermost boundary of a 4-bit codebook lies at 0.3 for
+// d = 64.  With eight copies of 513 a lookup took 6.6 shared-memory cycles a warp instead of two, and the whole launch 68 % of
+// them.  Keys at 4 bits and values at 2, 8 x 65,536 rows of 128, before / now: bf16 122 / 114 us, fp16 108.8 / 104.7; 8 x 4096 rows, where
+// the table's set-up counts, 20.1 / 16.5 and 16.5 / 15.7.)
 constexpr int MARKED = 0x100;
 __device__ void build_bins(float2* bins, const float* bnd, int n_bnd, int tid, int nthreads) {
     for (int k = tid; k < NBINS; k += nthreads) {
-        const float lo = (float(k) - 256.f - 1.5f) / 256.f, hi = (float(k) - 256.f + 1.5f) / 256.f;
+        const float lo = k > 0 ? (float(k - BIN0) - 1.5f) / 256.f : -INFINITY, hi = k < NBINS - 1 ? (float(k - BIN0) + 1.5f) / 256.f : INFINITY;
         int below = 0, inside = 0;
         float b_in = 2.0f;                    // no boundary near this bin: |y| <= 1 never exceeds the sentinel
         for (int i = 0; i < n_bnd; ++i) {
@@ -226,9 +229,10 @@ __device__ void build_bins(float2* bins, const float* bnd, int n_bnd, int tid, i
             if (b < lo) ++below;
             else if (b <= hi) { ++inside; b_in = b; }
         }
-        const float2 e = make_float2(b_in, __int_as_float(inside > 1 ? (below | MARKED) : below));
+        const float e = __int_as_float(inside > 1 ? (below | MARKED) : below);
 #pragma unroll
-        for (int r = 0; r < BIN_REP; ++r) bins[k * BIN_REP + r] = e;
+        for (int r = 0; r < BIN_REP / 2; ++r)                                        // (eight neighbours write eight different 16-byte columns)
+            *reinterpret_cast<float4*>(bins + k * BIN_REP + 2 * ((r + tid) % (BIN_REP / 2))) = make_float4(b_in, e, b_in, e);
     }
 }
 
@@ -288,10 +292,9 @@ __device__ __forceinline__ void quantize16(uint32_t* v, const RowCtx& rc, const 
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const float yp = __uint_as_float(v[i]);
-            // bin index from the mantissa of (y * 256 + 256 + 2^23): exact rounding to nearest, no convert instruction.
-            // |y| <= 1 keeps the index below 513; NaN and infinity give index 0 (ten low mantissa bits are zero).
-            const float tt = fmaf(yp, rc.rbin, 8388608.f + 256.f);
-            const float2 en = rc.bins[min(__float_as_uint(tt) & 0x3FFu, uint32_t(NBINS - 1)) * BIN_REP];     // (the clamp only matters for |y| > |x|, i.e. never)
+            // bin index from the mantissa of (y * 256 + BIN0 + 2^23): exact rounding to nearest, no convert instruction; a NaN takes the last bin
+            const float tt = fmaxf(fminf(fmaf(yp, rc.rbin, 8388608.f + BIN0), 8388608.f + (NBINS - 1)), 8388608.f);
+            const float2 en = rc.bins[(__float_as_uint(tt) - 0x4B000000u) * BIN_REP];
             seen |= __float_as_uint(en.y);
             uint32_t& w = i < 8 ? g0 : g1;
             if constexpr (QJL) {
@@ -362,7 +365,7 @@ struct EpiCtx {
 // tile.  Only the SIGN of a projection is kept, so the residual is scaled by 2^8 (clear of fp16 subnormals) and split into fp16 high and low
 // parts (columns 0-7 and 8-15), as is S R^T: hi x hi + lo x hi + hi x lo reproduces the float32 product to about 2^-21.
 // (With mma.sync a thread kept 32 running projections, a warp staged its residuals through shared memory, and the registers allowed eight
-// epilogue warps: keys at 4 bits and values at 2 of 1,048,576 rows of 96 took 196 + 168 us, 161 + 124 now; the signs are the same.)
+// epilogue warps: keys at 4 bits and values at 2 of 1,048,576 rows of 96 took 196 + 168 us, 146 + 118 now; the signs are the same.)
 __device__ __forceinline__ void sketch16(const uint32_t* e, uint32_t taddr, float& ee) {
     uint32_t x[16];
 #pragma unroll
@@ -379,10 +382,11 @@ __device__ __forceinline__ void sketch16(const uint32_t* e, uint32_t taddr, floa
     tmem_st16(taddr, x);
 }
 
-// A run of a row's coordinates ([col0, col0 + 16 * nch) at BITS bits) in rolled steps of 32 coordinates; the step's codes
-// (32 * BITS bits) are assembled in registers and stored at once.  Keeping the loop rolled keeps its body within the
-// instruction cache.  SPLITACC: the high and low products sit in two accumulators lo_off columns apart and are combined
-// here (y = hi + 2^-11 lo), sixteen coordinates per pair of loads; otherwise one 32-column load per step.
+// A run of a row's coordinates ([col0, col0 + 16 * nch) at BITS bits) in rolled steps of 32 coordinates, 16 with the sketch; the step's codes
+// are assembled in registers and stored at once.  Keeping the loop rolled keeps its body within the instruction cache (with 32 coordinates a
+// step the sketch's warps stood 2.7 of 9.4 cycles an instruction without one, with 16 0.5 of 7.8: keys and values of 8 x 65,536 rows of 96
+// at 4 and 2 bits 147.7 us before, 134.9 now).  SPLITACC: the high and low products sit in two accumulators lo_off columns apart and are combined
+// here (y = hi + 2^-11 lo), sixteen coordinates per pair of loads; otherwise one load per step.
 // NCH: the number of chunks when it is known at compile time (1 or 2: a single step whose shape folds), 0 = nch_rt.
 template <int BITS, bool QJL, bool SPLITACC, int NCH, int TERMS = 2>
 __device__ __forceinline__ void quantize_part(uint32_t t_row, int col0, int nch_rt, int lo_off, const RowCtx& rc, const float (&sb)[7], const float* raw,
