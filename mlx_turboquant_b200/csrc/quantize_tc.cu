@@ -193,6 +193,22 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// Two float32 operations an instruction, and sums of squares that take 16-bit factors as they are: the launch is bound by the instructions
+// its warps issue (18.8 a coordinate at 3 bits of fp16 rows, 2 of them the norms').  Keys at 4 bits and values at 2, 8 x 65,536 rows, one
+// operation an instruction / now: d = 128 fp16 104.7 / 102.1 us, bf16 114.4 / 111.5, d = 64 at 4 and 4 bits 92.3 / 86.0, d = 96 with
+// sketches 134.3 / 127.8, d = 256 (131,072 rows) 106.7 / 101.0.
+using u64 = unsigned long long;
+__device__ __forceinline__ u64 pk(float a, float b) { u64 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void upk(u64 x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x)); }
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) { u64 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) { u64 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ u64 add2(u64 a, u64 b) { u64 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+// a += the squares of a word's two halves (exact products, one rounding each), low half first
+__device__ __forceinline__ void add_squares(float& a, uint32_t x, bool bf16) {
+    if (bf16) asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tfma.rn.f32.bf16 %0, l, l, %0;\n\tfma.rn.f32.bf16 %0, h, h, %0;\n\t}" : "+f"(a) : "r"(x));
+    else asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tfma.rn.f32.f16 %0, l, l, %0;\n\tfma.rn.f32.f16 %0, h, h, %0;\n\t}" : "+f"(a) : "r"(x));
+}
+
 // K-major operand tile in shared memory, 128-byte swizzle: row r of K-block b at  b*16 KB + r*128 B, its 16-byte
 // chunk c stored at chunk position c ^ (r & 7).  Descriptor for the 16-column slab `ks` (0..3) of K-block b.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t tile_addr, int kblk, int ks) {
@@ -289,21 +305,27 @@ __device__ __forceinline__ void quantize16(uint32_t* v, const RowCtx& rc, const 
     } else {
         // table path: count-below times 16^k goes in with one multiply-add, the compare adds its bit in place
         uint32_t seen = 0;
+        const u64 rbin2 = pk(rc.rbin, rc.rbin), rinv2 = pk(rc.rinv, rc.rinv), bias2 = pk(8388608.f + BIN0, 8388608.f + BIN0);
+        float t2[2], yn2[2];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-            const float yp = __uint_as_float(v[i]);
             // bin index from the mantissa of (y * 256 + BIN0 + 2^23): exact rounding to nearest, no convert instruction; a NaN takes the last bin
-            const float tt = fmaxf(fminf(fmaf(yp, rc.rbin, 8388608.f + BIN0), 8388608.f + (NBINS - 1)), 8388608.f);
+            if (!(i & 1)) {
+                const u64 y2 = pk(__uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+                upk(fma2(y2, rbin2, bias2), t2[0], t2[1]);
+                upk(mul2(y2, rinv2), yn2[0], yn2[1]);
+            }
+            const float yn = yn2[i & 1], tt = fmaxf(fminf(t2[i & 1], 8388608.f + (NBINS - 1)), 8388608.f);
             const float2 en = rc.bins[(__float_as_uint(tt) - 0x4B000000u) * BIN_REP];
             seen |= __float_as_uint(en.y);
             uint32_t& w = i < 8 ? g0 : g1;
             if constexpr (QJL) {
-                const uint32_t code = __float_as_uint(en.y) + ((yp * rc.rinv) > en.x ? 1u : 0u);
+                const uint32_t code = __float_as_uint(en.y) + (yn > en.x ? 1u : 0u);
                 w += code * (1u << (4 * (i & 7)));
                 residual(i, code & 15u);                                           // (a marked bin's is formed again below)
             } else {
                 w += __float_as_uint(en.y) * (1u << (4 * (i & 7)));
-                if ((yp * rc.rinv) > en.x) w += 1u << (4 * (i & 7));               // strict >, codebook.py:220-223
+                if (yn > en.x) w += 1u << (4 * (i & 7));               // strict >, codebook.py:220-223
             }
         }
         if (__any_sync(0xffffffffu, (seen & MARKED) != 0)) {     // a marked bin was hit: redo the group with the counting loop
@@ -366,16 +388,18 @@ struct EpiCtx {
 // parts (columns 0-7 and 8-15), as is S R^T: hi x hi + lo x hi + hi x lo reproduces the float32 product to about 2^-21.
 // (With mma.sync a thread kept 32 running projections, a warp staged its residuals through shared memory, and the registers allowed eight
 // epilogue warps: keys at 4 bits and values at 2 of 1,048,576 rows of 96 took 196 + 168 us, 146 + 118 now; the signs are the same.)
-__device__ __forceinline__ void sketch16(const uint32_t* e, uint32_t taddr, float& ee) {
+__device__ __forceinline__ void sketch16(const uint32_t* e, uint32_t taddr, u64& ee) {
     uint32_t x[16];
 #pragma unroll
     for (int i = 0; i < 16; i += 2) {
         const float e2[2] = {__uint_as_float(e[i]), __uint_as_float(e[i + 1])};
-        ee = fmaf(e2[0], e2[0], ee);
-        ee = fmaf(e2[1], e2[1], ee);
+        const u64 ev = pk(e2[0], e2[1]);
+        ee = fma2(ev, ev, ee);
         const __half2 h = __floats2half2_rn(e2[0], e2[1]);
         const float2 hf = __half22float2(h);
-        const __half2 l = __floats2half2_rn(e2[0] - hf.x, e2[1] - hf.y);
+        float l0, l1;
+        upk(add2(ev, pk(-hf.x, -hf.y)), l0, l1);
+        const __half2 l = __floats2half2_rn(l0, l1);
         x[i >> 1] = *reinterpret_cast<const uint32_t*>(&h);
         x[8 + (i >> 1)] = *reinterpret_cast<const uint32_t*>(&l);
     }
@@ -390,7 +414,7 @@ __device__ __forceinline__ void sketch16(const uint32_t* e, uint32_t taddr, floa
 // NCH: the number of chunks when it is known at compile time (1 or 2: a single step whose shape folds), 0 = nch_rt.
 template <int BITS, bool QJL, bool SPLITACC, int NCH, int TERMS = 2>
 __device__ __forceinline__ void quantize_part(uint32_t t_row, int col0, int nch_rt, int lo_off, const RowCtx& rc, const float (&sb)[7], const float* raw,
-                                              const float* cent, uint8_t* dst, bool live, float& ee) {
+                                              const float* cent, uint8_t* dst, bool live, u64& ee) {
     constexpr int STEP = QJL ? 1 : 2, NW = (STEP * 16 * BITS + 31) / 32;            // chunks of a step and its words
     const int nch = NCH ? NCH : nch_rt;
 #pragma unroll 1
@@ -426,7 +450,12 @@ __device__ __forceinline__ void quantize_part(uint32_t t_row, int col0, int nch_
                     } else {
                         tmem_ld_wait();
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(fmaf(__uint_as_float(v[16 + i]), 1.f / 2048.f, __uint_as_float(v[i])));
+                        for (int i = 0; i < 16; i += 2) {
+                            float y0, y1;
+                            upk(fma2(pk(__uint_as_float(v[16 + i]), __uint_as_float(v[17 + i])), pk(1.f / 2048.f, 1.f / 2048.f), pk(__uint_as_float(v[i]), __uint_as_float(v[i + 1]))), y0, y1);
+                            v[i] = __float_as_uint(y0);
+                            v[i + 1] = __float_as_uint(y1);
+                        }
                     }
                 }
                 quantize16<BITS, QJL>(vc, rc, sb, raw, g0, g1, cent, t_row + col0 + (c0 + c) * 16);
@@ -519,17 +548,20 @@ __device__ __forceinline__ void epilogue_loop(const EpiCtx& e) {
         lane_o += step_o; tl += step_t;
         if (tl >= tpl) { tl -= tpl; ++lane_o; }
         const uint32_t t_row = e.tmem_base + (uint32_t(quad * 32) << 16) + a * Sh::STAGE_COLS;
-        float ee = 0.f;
+        u64 ee2 = 0;                                            // squares of the residual: even and odd coordinates
         // with head_dim 128 and quarter shares every thread has two chunks of an integer width, or one of each fractional width
         constexpr int NCH_H = (DC == 128 && Sh::SPLIT == 4) ? (BL ? 1 : 2) : 0, NCH_L = (DC == 128 && Sh::SPLIT == 4) ? 1 : 0;
         if constexpr (DC == 256)
-            quantize_part<BH, QJL, SPLITACC, 1, TERMS>(t_row, h0 * 16, 1, SLICE, rc, sb_h, raw_h, cent_h, e.dst + orow * e.nb + h0 * 2 * BH, live, ee);
+            quantize_part<BH, QJL, SPLITACC, 1, TERMS>(t_row, h0 * 16, 1, SLICE, rc, sb_h, raw_h, cent_h, e.dst + orow * e.nb + h0 * 2 * BH, live, ee2);
         else
-        quantize_part<BH, QJL, SPLITACC, NCH_H>(t_row, h0 * 16, h1 - h0, d, rc, sb_h, raw_h, cent_h, p.p_hi + orow * nb_h + h0 * 2 * BH, live, ee);
-        if (BL) quantize_part<(BL ? BL : 1), QJL, SPLITACC, NCH_L>(t_row, half + l0 * 16, l1 - l0, d, rc, sb_l, raw_l, cent_l, p.p_lo + orow * nb_l + l0 * 2 * BL, live, ee);
+        quantize_part<BH, QJL, SPLITACC, NCH_H>(t_row, h0 * 16, h1 - h0, d, rc, sb_h, raw_h, cent_h, p.p_hi + orow * nb_h + h0 * 2 * BH, live, ee2);
+        if (BL) quantize_part<(BL ? BL : 1), QJL, SPLITACC, NCH_L>(t_row, half + l0 * 16, l1 - l0, d, rc, sb_l, raw_l, cent_l, p.p_lo + orow * nb_l + l0 * 2 * BL, live, ee2);
         if constexpr (QJL) {
             static_assert(Sh::SPLIT == 2, "two threads a row");
             float* ee_slot = reinterpret_cast<float*>(e.smem + OFF_EE) + a * TM + row_in_tile;
+            float ee, ee_odd;
+            upk(ee2, ee, ee_odd);
+            ee += ee_odd;
             if (part == 1) *ee_slot = ee;
             tmem_st_wait();
             tc_fence_before();
@@ -893,24 +925,11 @@ __global__ void __launch_bounds__(NT, 1) quantize_tc_kernel(Params p, const __gr
                 const uint4 v = *reinterpret_cast<const uint4*>(rowp + ((c ^ (r & 7)) << 4));
                 uint4 w = make_uint4(0, 0, 0, 0);
                 if (d > 64 + 8 * c) w = *reinterpret_cast<const uint4*>(rowp + KBLK_BYTES + ((c ^ (r & 7)) << 4));
-                if (!bf16) {
-                    const __half2* h = reinterpret_cast<const __half2*>(&v);
-                    const __half2* g = reinterpret_cast<const __half2*>(&w);
+                const uint32_t vw[4] = {v.x, v.y, v.z, v.w}, ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const float2 f = __half22float2(h[u]), e = __half22float2(g[u]);
-                        a = fmaf(f.x, f.x, a); a = fmaf(f.y, f.y, a);
-                        b = fmaf(e.x, e.x, b); b = fmaf(e.y, e.y, b);
-                    }
-                } else {
-                    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-                    const __nv_bfloat162* g = reinterpret_cast<const __nv_bfloat162*>(&w);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const float2 f = __bfloat1622float2(h[u]), e = __bfloat1622float2(g[u]);
-                        a = fmaf(f.x, f.x, a); a = fmaf(f.y, f.y, a);
-                        b = fmaf(e.x, e.x, b); b = fmaf(e.y, e.y, b);
-                    }
+                for (int u = 0; u < 4; ++u) {
+                    add_squares(a, vw[u], bf16);
+                    add_squares(b, ww[u], bf16);
                 }
             }
             if constexpr (DC == 256) {
