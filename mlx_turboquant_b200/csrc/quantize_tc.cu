@@ -275,6 +275,24 @@ __device__ __forceinline__ void add_code(uint32_t& grp, float y, const float (&b
         if (p3) grp += 1u << sh;
     }
 }
+// The group word as a float (up to 24 bits: exact), for fp16 rows without the sketch: their launch keeps the pipe of compares and selects 68 %
+// busy at 3 bits, and integer adds share it (8 x 65,536 rows of 128 at 3 and 2 bits 97.0 / 93.1 us, at 4 and 2 102.5 / 98.6; bf16 rows, which
+// wait for their 24 dependent products, lose: d = 64 at 3 bits 67.8 / 69.4).
+template <int BITS>
+__device__ __forceinline__ void add_code(float& grp, float y, const float (&b)[7], int sh) {
+    const float one = float(1u << sh);
+    if (BITS == 1) {
+        asm("{\n\t.reg .pred p;\n\tsetp.gt.f32 p, %1, %2;\n\t@p add.rn.f32 %0, %0, %3;\n\t}" : "+f"(grp) : "f"(y), "f"(b[0]), "f"(one));
+    } else if (BITS == 2) {
+        asm("{\n\t.reg .pred p, q;\n\t.reg .f32 t;\n\tsetp.gt.f32 p, %1, %3;\n\tselp.f32 t, %4, %2, p;\n\tsetp.gt.f32 q, %1, t;\n\t"
+            "@p add.rn.f32 %0, %0, %6;\n\t@q add.rn.f32 %0, %0, %5;\n\t}" : "+f"(grp) : "f"(y), "f"(b[0]), "f"(b[1]), "f"(b[2]), "f"(one), "f"(2.f * one));
+    } else {
+        asm("{\n\t.reg .pred p, q, r;\n\t.reg .f32 t, u, v;\n\tsetp.gt.f32 p, %1, %5;\n\tselp.f32 t, %7, %3, p;\n\tsetp.gt.f32 q, %1, t;\n\t"
+            "selp.f32 u, %4, %2, q;\n\tselp.f32 v, %8, %6, q;\n\tselp.f32 t, v, u, p;\n\tsetp.gt.f32 r, %1, t;\n\t"
+            "@p add.rn.f32 %0, %0, %11;\n\t@q add.rn.f32 %0, %0, %10;\n\t@r add.rn.f32 %0, %0, %9;\n\t}"
+            : "+f"(grp) : "f"(y), "f"(b[0]), "f"(b[1]), "f"(b[2]), "f"(b[3]), "f"(b[4]), "f"(b[5]), "f"(b[6]), "f"(one), "f"(2.f * one), "f"(4.f * one));
+    }
+}
 // Plain counting loop, kept out of line: only reached when two boundaries share a bin neighbourhood.
 __device__ __noinline__ uint32_t code_slow(float y, const float* raw_bnd, int n_bnd) {
     uint32_t c = 0;
@@ -291,13 +309,23 @@ struct RowCtx {
 // Sixteen coordinates (TMEM columns taddr .. + 15) at BITS bits: the codes go into g0 / g1 (eight codes each, BITS bits
 // per code).  sb: boundaries times the row's norm (register search); raw: unscaled boundaries (table path's fallback).
 // QJL: v[] leaves as 2^8 times the residuals (rbin and the centroids carry the factor); taddr: where v[] came from.
-template <int BITS, bool QJL>
+template <int BITS, bool QJL, bool FSUM>
 __device__ __forceinline__ void quantize16(uint32_t* v, const RowCtx& rc, const float (&sb)[7], const float* raw, uint32_t& g0, uint32_t& g1, const float* cent, uint32_t taddr) {
     g0 = g1 = 0;
     const auto residual = [&](int i, uint32_t code) { v[i] = __float_as_uint(fmaf(__uint_as_float(v[i]), rc.rbin, -cent[code])); };
     if (BITS <= 3) {
+        if constexpr (FSUM) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) add_code<BITS>(i < 8 ? g0 : g1, __uint_as_float(v[i]), sb, BITS * (i & 7));
+            for (int h = 0; h < 2; ++h) {
+                float grp = 0.f;
+#pragma unroll
+                for (int i = 8 * h; i < 8 * h + 8; ++i) add_code<BITS>(grp, __uint_as_float(v[i]), sb, BITS * (i & 7));
+                (h ? g1 : g0) = __float2uint_rn(grp);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) add_code<BITS>(i < 8 ? g0 : g1, __uint_as_float(v[i]), sb, BITS * (i & 7));
+        }
         if constexpr (QJL) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) residual(i, ((i < 8 ? g0 : g1) >> (BITS * (i & 7))) & ((1u << BITS) - 1u));
@@ -458,7 +486,7 @@ __device__ __forceinline__ void quantize_part(uint32_t t_row, int col0, int nch_
                         }
                     }
                 }
-                quantize16<BITS, QJL>(vc, rc, sb, raw, g0, g1, cent, t_row + col0 + (c0 + c) * 16);
+                quantize16<BITS, QJL, SPLITACC>(vc, rc, sb, raw, g0, g1, cent, t_row + col0 + (c0 + c) * 16);
                 put_group<BITS, NW>(w, 2 * c, g0);
                 put_group<BITS, NW>(w, 2 * c + 1, g1);
                 if constexpr (QJL) sketch16(vc, t_row + col0 + (c0 + c) * 16, ee);
