@@ -12,8 +12,8 @@
 //              one accumulator.
 // Every product is exact in the fp32 accumulator; the normalisation by the row norm is applied afterwards.
 //
-// Warp roles in a persistent CTA (one per SM; 704 threads).  Sixteen epilogue warps come first (E of them),
-// then one MMA warp, four norm warps, one TMA warp:
+// Warp roles in a persistent CTA (one per SM; 640 threads for fp16 rows, 704 for bf16 rows and sketches).  Sixteen epilogue warps come first (E of them),
+// then one MMA warp, two or four norm warps, one TMA warp:
 //   warps 0..E-1 epilogue; thread <-> one row (TMEM lane) and a share of its sixteen-coordinate chunks (tcgen05.ld).
 //                fp16 rows: all sixteen warps work on the same tile in step, a quarter of the row each, reading the
 //                high and the low accumulator and combining them; two accumulator stages, so the MMAs of the next tile
@@ -25,7 +25,7 @@
 //                boundary + count below; see build_bins).  Fractional widths: the threads of a row take chunks of
 //                either width, so they finish together.
 //   warp  E      allocates TMEM, issues the MMAs (in uniform control flow, one elected lane) and commits them to mbarriers
-//   next four    norms: read each tile back from shared memory for the rows' sums of squares
+//   next         norms: read each tile back from shared memory for the rows' sums of squares
 //   last warp    one thread keeps the operand stages full with tiled TMA copies (cp.async.bulk.tensor, 3-D tensor map
 //                (column, row, lane), 128-byte swizzle as the MMA descriptors expect; rows past a lane's end and
 //                columns past d read as zeros)
@@ -39,6 +39,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdlib>
+#include <type_traits>
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -51,9 +52,13 @@ namespace tc {
 
 constexpr int DMAX = 128, TM = 128;              // largest head_dim, rows per tile
 constexpr int A_STAGES_MAX = 3, ACC_STAGES = 4;
-constexpr int N_NORM = 128;                      // threads that read the rows back for the norms
 constexpr int EPI_WARPS = 16, N_EPI = EPI_WARPS * 32;            // epilogue warps; then the MMA warp, the norm warps, the TMA warp
-constexpr int NT = N_EPI + 32 + N_NORM + 32;
+// Threads that read the rows back for the norms.  fp16 rows without the sketch: two rows each, as with 20 warps in all a thread may have 96
+// registers, with 22 only 80, and the epilogue spilled (8 x 65,536 rows: d = 128 at 3 and 2 bits 97.0 / 94.5 us, d = 64 at 4 and 4 bits 88.0 /
+// 82.0, 2 x 65,536 of 256 100.8 / 97.0).  The others have fewer operand stages or longer chains of products and want theirs back soon: a row
+// each (bf16, d = 64 at 3 bits, 8 x 32,768 rows 39.0 us, with two rows a thread 40.9).
+__host__ __device__ constexpr int n_norm(bool splitacc) { return splitacc ? 64 : 128; }
+__host__ __device__ constexpr int n_threads(bool splitacc) { return N_EPI + 32 + n_norm(splitacc) + 32; }     // 640 / 704
 constexpr int BIN_REP = 16;                      // copies of every lookup-table entry (lane & 15 picks one): the lanes of a half-warp read banks of their own
 constexpr int KBLK_BYTES = TM * 128;             // one 64-column K-block of a 128-row operand: 16 KB
 constexpr int OPER_BYTES = 2 * KBLK_BYTES;       // 32 KB per operand tile
@@ -204,8 +209,9 @@ __device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) { u64 r; asm("fma.rn.f3
 __device__ __forceinline__ u64 mul2(u64 a, u64 b) { u64 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __device__ __forceinline__ u64 add2(u64 a, u64 b) { u64 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 // a += the squares of a word's two halves (exact products, one rounding each), low half first
-__device__ __forceinline__ void add_squares(float& a, uint32_t x, bool bf16) {
-    if (bf16) asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tfma.rn.f32.bf16 %0, l, l, %0;\n\tfma.rn.f32.bf16 %0, h, h, %0;\n\t}" : "+f"(a) : "r"(x));
+template <bool BF16>
+__device__ __forceinline__ void add_squares(float& a, uint32_t x) {
+    if (BF16) asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tfma.rn.f32.bf16 %0, l, l, %0;\n\tfma.rn.f32.bf16 %0, h, h, %0;\n\t}" : "+f"(a) : "r"(x));
     else asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tfma.rn.f32.f16 %0, l, l, %0;\n\tfma.rn.f32.f16 %0, h, h, %0;\n\t}" : "+f"(a) : "r"(x));
 }
 
@@ -623,9 +629,9 @@ __device__ __forceinline__ void epilogue_loop(const EpiCtx& e) {
 // SPLITACC (fp16 rows without the sketch): high and low products in two accumulators, one MMA of N = 2 d per k-step
 // against [R_hi ; R_lo].  Otherwise one accumulator: fp16 low products first and the scale-input-d trick, bf16 three terms.
 template <bool QJL, bool SPLITACC, int DC>
-__global__ void __launch_bounds__(NT, 1) quantize_tc_kernel(Params p, const __grid_constant__ CUtensorMap tmap) {
+__global__ void __launch_bounds__(n_threads(SPLITACC), 1) quantize_tc_kernel(Params p, const __grid_constant__ CUtensorMap tmap) {
     using Sh = EpiShape<QJL, SPLITACC>;
-    constexpr int ACCS = Sh::STAGES;
+    constexpr int ACCS = Sh::STAGES, N_NORM = n_norm(SPLITACC), NT = n_threads(SPLITACC);
     extern __shared__ __align__(1024) unsigned char smem[];
     const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;      // (warp: uniform)
@@ -937,38 +943,51 @@ __global__ void __launch_bounds__(NT, 1) quantize_tc_kernel(Params p, const __gr
         __syncwarp();
     } else {
         // ======================= norm warps: sum of squares of every row, read back from the stage =======================
-        // thread -> row 32 nw + lane, both 64-column blocks: eight consecutive rows hit eight different 16-byte columns
+        // thread -> row 32 nw + lane (and the one 64 further), both 64-column blocks: eight consecutive rows hit eight different 16-byte columns
         // of the swizzled tile, so the 128-bit reads are free of bank conflicts
         const int nw = warp - (EPI_WARPS + 1), r = nw * 32 + lane;
-        constexpr int KH = DC == 256 ? 2 : 1;
+        constexpr int KH = DC == 256 ? 2 : 1, RT = TM / N_NORM;
         int it = 0;                                                        // operand stages so far: KH per tile
-        float a = 0.f, b = 0.f;
+        float a[RT], b[RT];
         for (int64_t tile = tile0; tile < p.n_tiles; tile += (KH == 1 || (it & 1)) ? tile_step : 0, ++it) {
             const int s = it % a_stages;
             if (!mbar_wait(bar_full + 8 * s, uint32_t(it / a_stages) & 1u, abort_flag, 7)) break;
             const unsigned char* rowp = smem + OFF_A + s * OPER_BYTES + r * 128;
-            if (KH == 1 || !(it & 1)) a = b = 0.f;
+            if (KH == 1 || !(it & 1)) {
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const uint4 v = *reinterpret_cast<const uint4*>(rowp + ((c ^ (r & 7)) << 4));
-                uint4 w = make_uint4(0, 0, 0, 0);
-                if (d > 64 + 8 * c) w = *reinterpret_cast<const uint4*>(rowp + KBLK_BYTES + ((c ^ (r & 7)) << 4));
-                const uint32_t vw[4] = {v.x, v.y, v.z, v.w}, ww[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    add_squares(a, vw[u], bf16);
-                    add_squares(b, ww[u], bf16);
-                }
+                for (int h = 0; h < RT; ++h) a[h] = b[h] = 0.f;
             }
+            const auto sum = [&](auto type) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+#pragma unroll
+                    for (int h = 0; h < RT; ++h) {
+                        const uint4 v = *reinterpret_cast<const uint4*>(rowp + h * 64 * 128 + ((c ^ (r & 7)) << 4));
+                        const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) add_squares<decltype(type)::value>(a[h], vw[u]);
+                        if (d > 64 + 8 * c) {
+                            const uint4 w = *reinterpret_cast<const uint4*>(rowp + KBLK_BYTES + h * 64 * 128 + ((c ^ (r & 7)) << 4));
+                            const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) add_squares<decltype(type)::value>(b[h], ww[u]);
+                        }
+                    }
+                }
+            };
+            if (bf16) sum(std::true_type{});
+            else sum(std::false_type{});
             if constexpr (DC == 256) {
                 if (it & 1) {
                     const int q = (it >> 1) % NSQ_SLOTS;
-                    reinterpret_cast<float*>(smem + OFF_NSQ256)[q * TM + r] = a + b;
+#pragma unroll
+                    for (int h = 0; h < RT; ++h) reinterpret_cast<float*>(smem + OFF_NSQ256)[q * TM + r + 64 * h] = a[h] + b[h];
                     mbar_arrive(sbase + OFF_NRMBAR256 + 8 * q);
                 }
             } else {
             float* nsq = reinterpret_cast<float*>(smem + OFF_NSQ) + s * 2 * TM;
-            nsq[r] = a; nsq[TM + r] = b;
+#pragma unroll
+            for (int h = 0; h < RT; ++h) { nsq[r + 64 * h] = a[h]; nsq[TM + r + 64 * h] = b[h]; }
             mbar_arrive(bar_nrm + 8 * s);        // release: the epilogue reads the sums after waiting on this barrier
             }
             mbar_arrive(bar_afree + 8 * s);      // this thread is done reading the stage
@@ -1100,7 +1119,7 @@ int tq_quantize_pack_tc(const tq_quantize_args* q, cudaStream_t s, bool* handled
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(unsigned(tc::NT));
+    cfg.blockDim = dim3(unsigned(tc::n_threads(d == 256 || (!qjl && !p.bf16))));
     cfg.dynamicSmemBytes = tc::SMEM_BYTES;
     cfg.stream = s;
     cfg.attrs = attr;
