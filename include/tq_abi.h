@@ -101,7 +101,7 @@ int tq_quantize_pack_many(const tq_quantize_args* a, int n, void* stream);
 
 /* The tensor-core kernels (quantize, dequantize, several-query attention) and the decode kernels wait on
  * mbarriers with an iteration limit; if a wait ever runs out the kernel drains and finishes, and this returns the
- * code of the first such wait on the current device (quantize 1-9, decode 101-103 and 106-110, several-query-token attention 104 and 111, dequantize 105, gather wait 201; 0 = none).  Synchronises the
+ * code of the first such wait on the current device (quantize 1-9, decode 101-103, 106-110, 112 and 113, several-query-token attention 104 and 111, dequantize 105, gather wait 201; 0 = none).  Synchronises the
  * device; no reference counterpart. */
 int tq_device_status(void);
 /* Back to 0 (after the caller has dealt with a reported time-out). */
