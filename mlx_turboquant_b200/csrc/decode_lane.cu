@@ -514,8 +514,8 @@ __global__ void __launch_bounds__(NT, PER_SM) decode_lane_kernel(DecodeParams p)
             const float2 ml = *reinterpret_cast<const float2*>(src + w * (HPG * PS) + QR);
             const float x = ml.x == -INFINITY ? 0.f : ex2(ml.x - M);
             const bool pk = rank * NW + w < n_pw;
-            if (x == 0.f || (!pk && c >= D)) continue;
-            L = fmaf(x, ml.y, L);
+            L = fmaf(x, ml.y, L);                                       // (weight 0 counts too: 0 x NaN is NaN, and a warp without tokens holds zeros)
+            if (!pk && c >= D) continue;                                // (uncompressed tokens have no sketch rows)
             const float4 v = *reinterpret_cast<const float4*>(src + w * (HPG * PS) + c);
             if (pk) { ap.x = fmaf(x, v.x, ap.x); ap.y = fmaf(x, v.y, ap.y); ap.z = fmaf(x, v.z, ap.z); ap.w = fmaf(x, v.w, ap.w); }
             else { ad.x = fmaf(x, v.x, ad.x); ad.y = fmaf(x, v.y, ad.y); ad.z = fmaf(x, v.z, ad.z); ad.w = fmaf(x, v.w, ad.w); }
@@ -580,7 +580,7 @@ __global__ void __launch_bounds__(NT, PER_SM) decode_lane_kernel(DecodeParams p)
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
                     const float w = wt[h * (MAX_C + 4) + min(r0 + r, MAX_C - 1)];       // (a sum that is not there counts 0, whatever its weight)
-                    if (w == 0.f || r0 + r >= n_pc) continue;
+                    if (r0 + r >= n_pc) continue;
                     y.x = fmaf(w, v[r].x, y.x); y.y = fmaf(w, v[r].y, y.y); y.z = fmaf(w, v[r].z, y.z); y.w = fmaf(w, v[r].w, y.w);
                 }
             }
@@ -596,7 +596,7 @@ __global__ void __launch_bounds__(NT, PER_SM) decode_lane_kernel(DecodeParams p)
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
                     const float w = wt[h * (MAX_C + 4) + min(r0 + r, MAX_C - 1)];
-                    if (w != 0.f && r0 + r < C) y = fmaf(w, u[r], y);
+                    if (r0 + r < C) y = fmaf(w, u[r], y);
                 }
             }
             yd[h * D + c] = y;

@@ -27,10 +27,15 @@ def lane():
     set_tuning("decode_lane_ctas", 0)
 
 
+def _taken(c):
+    from mlx_turboquant_b200 import _lib
+    return _lib.lib().tq_decode_one_launch(C.byref(c._dargs))
+
+
 def _run(c, q, ref, ctas=0):
     from mlx_turboquant_b200 import _lib
     out = c.attend(q, out_dtype=torch.float32)
-    got = _lib.lib().tq_decode_one_launch(C.byref(c._dargs))
+    got = _taken(c)
     assert got == ctas if ctas else got > 0
     _check(out, ref)
     assert _lib.lib().tq_device_status() == 0
@@ -137,3 +142,33 @@ def test_lookup_kernel_lanes_and_folds(oracle, off, b, hq, hkv, t):
 @pytest.mark.parametrize("t", (129, 300, 2500))
 def test_the_table_lookup_kernel(oracle, off, t):
     general.test_k4v2_direct_path_lengths(oracle, t)
+
+
+@pytest.mark.parametrize("ctas", (1, 4))
+@pytest.mark.parametrize("d,kb,vb,dtype", ((128, 4, 2, torch.float16), (96, 3.5, 3, torch.bfloat16), (64, 3, 4, torch.bfloat16), (256, 4, 4, torch.float16)))
+@pytest.mark.parametrize("where", ("new key", "packed norms", "value without weight"))
+def test_nan_reaches_the_result(lane, ctas, d, kb, vb, dtype, where):
+    """A warp whose every score is NaN, or whose weight is 0 and a value NaN: float arithmetic gives NaN for the query heads of that KV head
+    (0 x NaN is NaN, in the softmax sum and in the values), as the other decode kernels do, and leaves the other KV head's alone."""
+    from mlx_turboquant_b200 import TurboQuantKVCache
+    g = torch.Generator(device="cuda").manual_seed(d)
+    r = lambda n, h=2: torch.randn(1, h, n, d, device="cuda", generator=g).to(dtype)  # noqa: E731
+    c = TurboQuantKVCache(head_dim=d, num_kv_heads=2, key_bits=kb, value_bits=vb, residual_window=32, fp16_sink_size=16)
+    c.update(r(300), r(300))
+    while (c._sink_len + c._fp16_len) % 16:
+        c.update(r(1), r(1))
+    q, k, v = r(1, 8) / d ** 0.5, r(1), r(1)
+    columns = slice(None)
+    if where == "new key":                  # alone in the last uncompressed tile
+        k[0, 0] = float("nan")
+    elif where == "packed norms":           # a whole packed tile
+        c._k.norms[0, 0, 32:48] = float("nan")
+    else:                                   # scores of 300 and more: exp leaves nothing for the recent tokens
+        c.sink_keys[0, 0, 0] = 300 * d ** 0.5 * q[0, :4, 0].sum(0)
+        c.values[0, 0, 25, 7] = float("nan")
+        columns = 7
+    lane(ctas)
+    out = c.decode_step(q, k, v)[0, :, 0]
+    assert _taken(c) == ctas
+    assert out[:4, columns].isnan().all()
+    assert out[4:].isfinite().all()
