@@ -72,7 +72,7 @@ template <int D> struct Plan {
     static constexpr uint32_t OFF_SC = OFF_V + ST * K_TILE;                  // float [NSC][2][TN]: key norms, value norms
     static constexpr uint32_t OFF_R = D == 64 ? OFF_SC + NSC * 2 * TN * 4 : OFF_K;      // R (see below): through the key ring where it has no room of its own
     static constexpr uint32_t OFF_BAR = OFF_SC + NSC * 2 * TN * 4 + (D == 64 ? 2 * 64 * 128 : 0);
-    static constexpr uint32_t OFF_SLOT = OFF_BAR + 464;                      // [0] tensor-memory base, [1] abort
+    static constexpr uint32_t OFF_SLOT = OFF_BAR + 496;                      // [0] tensor-memory base, [1] abort
     static constexpr uint32_t OFF_ROW = OFF_SLOT + 16;                       // float2 [NQ * 128]: sum and maximum of a row
     static constexpr size_t NEED = OFF_ROW + NQ * TM * 8 + 1024, SMEM = NEED > 116 * 1024 ? NEED : 116 * 1024;      // one CTA per SM: it takes all of the tensor memory
     static constexpr uint32_t COL_O = NQ * SB * TN;                          // scores first, then the accumulators
@@ -87,7 +87,7 @@ template <int D> struct Plan {
     static_assert((R_RING ? 2 * R_HALF <= ST * K_TILE && (PASSES == 1 || PASSES % 2 == 0) : 2 * R_HALF == 2 * 64 * 128 && PASSES == 1) && RBLK % 1024 == 0 && OFF_R % 1024 == 0, "R's place");
     static_assert(SMEM <= 227 * 1024, "shared memory");
 };
-enum Bars { K_FULL = 0, K_FREE = 4, V_FULL = 8, V_FREE = 12, SC_FULL = 16, SC_FREE = 24, S_FULL = 32, P_FULL = 36, O_DONE = 40, ALL_DONE = 42, DRAIN = 44, ROT_IN = 45, ROT_A = 47, ROT_OUT = 49, R_FULL = 51, R_DONE = 53, Q_FULL = 55 };       // (57 of 8 bytes)
+enum Bars { K_FULL = 0, K_FREE = 4, V_FULL = 8, V_FREE = 12, SC_FULL = 16, SC_FREE = 24, S_FULL = 32, P_FULL = 36, O_DONE = 40, ALL_DONE = 42, DRAIN = 44, ROT_IN = 45, ROT_A = 47, ROT_OUT = 49, R_FULL = 51, R_DONE = 53, Q_FULL = 55, TURNED = 57, ROWS = 59 };       // (61 of 8 bytes)
 
 struct Params {
     void* out; int out_dtype;
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(const __grid_constan
         mbar_init(bar(DRAIN), 1);
         for (int i = 0; i < 2; ++i) {
             mbar_init(bar(ROT_IN + i), 1); mbar_init(bar(ROT_A + i), 256); mbar_init(bar(ROT_OUT + i), 1); mbar_init(bar(Q_FULL + i), 1);
-            mbar_init(bar(R_FULL + i), 1); mbar_init(bar(R_DONE + i), 1);
+            mbar_init(bar(R_FULL + i), 1); mbar_init(bar(R_DONE + i), 1); mbar_init(bar(TURNED + i), 256); mbar_init(bar(ROWS + i), 256);
         }
         for (int i = 0; i < NSC; ++i) { mbar_init(bar(SC_FULL + i), 1); mbar_init(bar(SC_FREE + i), NQ * 256); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -509,7 +509,12 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(const __grid_constan
         const int m = q * TM + (warp & 3) * 32 + lane, mf = q * TM + (warp & 3) * 32 + 16 * hh + g;       // this thread's row where a thread has one; first of its two
         const bool valid = row_valid(m);
         const int pos0 = p.q_pos0 + tq0 + q * p.QT;
-        auto sync_q = [&]() { asm volatile("barrier.sync %0, 256;" ::"r"(1 + q) : "memory"); };       // the warps of the query tile
+        // The eight warps of the query tile meet.  (An mbarrier with the bounded wait, each used once: a warp that has left after a wait that ran
+        // out does not arrive, and the abort flag that it leaves behind ends the others' wait.)
+        auto meet = [&](int which) -> bool {
+            mbar_arrive(bar(which + q));
+            return __all_sync(0xffffffffu, wait_bar(which + q, 0));
+        };
         int last[2];                                               // the last token of the region (packed tokens first) that each row sees
 #pragma unroll
         for (int k = 0; k < 2; ++k) last[k] = row_valid(mf + 8 * k) ? limit_p(p.q_pos0 + row_token(mf + 8 * k)) : -1;
@@ -570,7 +575,8 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(const __grid_constan
                     }
                     tmem_st_wait();
                     tc_fence_before();
-                    sync_q();                                      // (the other warp of these lanes has done the other columns)
+                    ok = meet(TURNED);                             // (the other warp of these lanes has done the other columns)
+                    if (!ok) break;
                     tc_fence_after();
                 }
 #pragma unroll
@@ -715,8 +721,8 @@ __global__ void __launch_bounds__(Plan<D>::NT, 1) fa_kernel(const __grid_constan
             for (int off = 1; off < 4; off <<= 1) l0 += __shfl_xor_sync(0xffffffffu, l0, off);
             if ((lane & 3) == 0) s_row[mf + 8 * k] = make_float2(l0, m_ref[k]);
         }
-        sync_q();
-        const float l_sum = s_row[m].x, m_row = s_row[m].y;
+        if (ok) ok = meet(ROWS);
+        const float l_sum = ok ? s_row[m].x : 0.f, m_row = ok ? s_row[m].y : 0.f;
         if (ok && n > n_p) ok = wait_bar(ALL_DONE + q, 0);
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
