@@ -245,11 +245,6 @@ __device__ __forceinline__ void softmax_scores(float (&s)[4], float vn0, float v
     pr[0] = p0 * st.vsc; pr[1] = p1 * st.vsc; pr[2] = p2 * st.vsc; pr[3] = p3 * st.vsc;
 }
 
-__device__ __forceinline__ uint32_t pack_bf2(float lo, float hi) {
-    const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t*>(&b);
-}
-
 // A stage of a warp's ring holds a tile's scalars (n_sc 16-byte chunks), then its key rows (first part, second part) and value rows, back
 // to back (16 rows of w bytes are w chunks).  Array that chunk c comes from, c made relative to the array's tile, bytes of its rows.
 __device__ __forceinline__ const unsigned char* chunk_source(const DecodeParams& p, int& c, int n_sc, int kwh, int kwl, int vwh, int& rb) {

@@ -114,3 +114,16 @@ def test_a_block_of_query_rows_over_many_long_lanes_unpacks_as_it_goes(monkeypat
     want = c.attend(q, out_dtype=torch.float32)
     assert torch.equal(got, want) == unpacks and (got - want).abs().max() < 1e-3 * want.abs().max()
     assert _lib.lib().tq_device_status() == 0
+
+
+@pytest.mark.parametrize("d", (64, 96, 128, 256))
+@pytest.mark.parametrize("dtype", (torch.float16, torch.bfloat16))
+@pytest.mark.parametrize("hq,hkv,tq", ((2, 2, 17), (8, 2, 4), (8, 2, 5), (6, 2, 33), (16, 2, 2), (16, 2, 34), (4, 4, 129)))
+@pytest.mark.parametrize("t", (140, 2000))                                  # one key range; several, merged from float32 partials
+def test_rows_of_16_and_result_types(d, dtype, hq, hkv, tq, t):
+    """Query rows that fill some of the sixteen-row shares of a block: the others take no part.  A 16-bit result is the float32 one, rounded."""
+    c, q, ref = _case(d, 1, hq, hkv, t, tq, dtype)
+    out = c.attend(q, out_dtype=torch.float32)
+    _check(out, ref)
+    for out_dtype in (torch.float16, torch.bfloat16):
+        assert torch.equal(c.attend(q, out_dtype=out_dtype), out.to(out_dtype))
