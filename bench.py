@@ -345,7 +345,8 @@ def bench_c3(torch, dev, steps, warmup, peak):
     names = {0: "decode_attn_kernel<96, qjl> (general kernel: unpack to shared memory, ldmatrix)",
              2: "decode_stream_kernel<96, qjl> (persistent grid over the packed tiles of all lanes; stream_query_kernel before it, "
                 "stream_merge_kernel after it: three launches per layer-step)",
-             3: "decode_lut_kernel<96, qjl> (persistent grid, lookups of code pairs; lut_merge_kernel after it: two launches per layer-step)"}
+             3: "decode_lut_kernel<96, qjl> (persistent grid, lookups of code pairs; lut_merge_kernel after it: two launches per layer-step)",
+             4: "decode_lane_kernel<96, qjl> (a cluster of CTAs per cache lane: one launch per layer-step)"}
     return {"workload": "phi35mini_layer_decode_attn_b16_ctx8192_k4v2_qjl_sink128_rw128", "us_per_layer_step": us,
             "algorithmic_bytes_per_launch": bytes_step, "hbm_gbs": gbs, "frac_of_peak": gbs / peak,
             "kernel": names.get(choice, str(choice))}
@@ -607,7 +608,7 @@ def run_c4(args):
     choice = _lib.lib().tq_decode_kernel_choice(C.byref(c0._dargs))     # 2: streaming kernel = query + persistent grid + merge launches
     launches_per_call = {2: 3, 3: 2}.get(choice, 1)
     attn_kernel = {0: "decode_attn_kernel", 1: "decode_direct_kernel", 2: "stream_query_kernel + decode_stream_kernel + stream_merge_kernel",
-                   3: "decode_lut_kernel + lut_merge_kernel"}.get(choice, str(choice))
+                   3: "decode_lut_kernel + lut_merge_kernel", 4: "decode_lane_kernel"}.get(choice, str(choice))
     weight_bytes = sum(p.numel() * p.element_size() for p in model.parameters()) - model.embed_tokens.weight.numel() * 2
     floor_ms = (attn_bytes * args.layers + weight_bytes) / (peak * 1e9) * 1e3
     line = {

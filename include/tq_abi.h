@@ -356,11 +356,11 @@ int tq_set_tuning(const char* key, int value);
  * 0 = general kernel (any width, d = 64 / 96 / 128 / 256), 1 = table-lookup kernel (4-bit keys / 2-bit values, d = 128: one CTA
  * per (sequence, KV head, split)), 2 = streaming kernel (the same widths at d = 96 / 128, sign sketches allowed: persistent
  * grid, chosen when the packed tokens of all lanes give every warp a long run), 3 = lookup kernel (2 to 4 bits and the splits
- * 4 | 3 and 3 | 2, d = 64 / 96 / 128 / 256, sign sketches allowed).  Negative: the arguments are invalid
- * (tq_last_error has the text). */
+ * 4 | 3 and 3 | 2, d = 64 / 96 / 128 / 256, sign sketches allowed), 4 = the lookup kernel's widths in one launch, a cluster of CTAs per
+ * cache lane merging on chip (small and middling calls; the workspace requirement is that of the kernel in whose place it runs, which
+ * "decode_lane" 0 shows).  Negative: the arguments are invalid (tq_last_error has the text). */
 int tq_decode_kernel_choice(const tq_decode_args* a);
-/* Whether tq_decode_attn would do the call in one launch, a cluster of CTAs per cache lane merging on chip, in the place of the kernel that
- * tq_decode_kernel_choice names (which keeps its workspace requirement): the CTAs per lane, or 0.  Negative: the arguments are invalid. */
+/* The CTAs per cache lane of kernel 4, or 0 where another one runs.  Negative: the arguments are invalid. */
 int tq_decode_one_launch(const tq_decode_args* a);
 
 #ifdef __cplusplus

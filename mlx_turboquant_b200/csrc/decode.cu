@@ -977,7 +977,7 @@ extern "C" int tq_decode_kernel_choice(const tq_decode_args* a) {
     DecodeParams p;
     bool direct = false;
     if (decode_prepare(a, a ? a->workspace : nullptr, a ? a->workspace_bytes : 0, &p, &direct)) return -1;
-    return p.st_grid > 0 ? (p.st_lut ? 3 : 2) : direct ? 1 : 0;
+    return p.ln_c > 0 ? 4 : p.st_grid > 0 ? (p.st_lut ? 3 : 2) : direct ? 1 : 0;
 }
 
 extern "C" int tq_decode_one_launch(const tq_decode_args* a) {

@@ -13,6 +13,15 @@ from gpu_util import cu, host, host_tables, kv_like
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True, params=(1, 0), ids=("kernel of the rule", "not in one launch"))
+def decode_lane(request):
+    """Once as the rule has it, once without the one-launch kernel, which takes most of these small calls."""
+    from mlx_turboquant_b200.kernels import set_tuning
+    set_tuning("decode_lane", request.param)
+    yield
+    set_tuning("decode_lane", 1)
+
+
 def _bf16_round(a):
     """float32 array rounded to the nearest bfloat16 value (still float32: bfloat16 is a subset)."""
     return torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).to(torch.bfloat16).float().numpy()

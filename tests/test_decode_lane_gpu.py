@@ -32,11 +32,17 @@ def _taken(c):
     return _lib.lib().tq_decode_one_launch(C.byref(c._dargs))
 
 
+def _choice(c):
+    from mlx_turboquant_b200 import _lib
+    return _lib.lib().tq_decode_kernel_choice(C.byref(c._dargs))
+
+
 def _run(c, q, ref, ctas=0):
     from mlx_turboquant_b200 import _lib
     out = c.attend(q, out_dtype=torch.float32)
     got = _taken(c)
     assert got == ctas if ctas else got > 0
+    assert _choice(c) == 4
     _check(out, ref)
     assert _lib.lib().tq_device_status() == 0
 
@@ -108,7 +114,7 @@ def test_what_it_leaves_to_the_others(oracle, lane):
     for t, dtype in ((300, np.float32), (20, np.float16)):
         c, q, ref = _case(oracle, np.random.RandomState(t), 2, 8, 2, t, 128, 4, 2, 32, 8, dtype=dtype)
         _check(c.attend(q, out_dtype=torch.float32), ref)
-        assert takes(c) == 0
+        assert takes(c) == 0 and _choice(c) != 4
     set_tuning("decode_lane", 1)
     from mlx_turboquant_b200 import TurboQuantKVCache
     for b, t, want in ((8, 16384, False), (1, 600, True)):
@@ -116,7 +122,7 @@ def test_what_it_leaves_to_the_others(oracle, lane):
         x = torch.randn(b, 8, t, 128, device="cuda").half()
         c.update(x, x)
         c.attend(torch.zeros(b, 32, 1, 128, device="cuda").half())
-        assert (takes(c) > 0) == want
+        assert (takes(c) > 0) == want == (_choice(c) == 4)
 
 
 @pytest.fixture()

@@ -13,10 +13,24 @@ from test_decode_gpu import _case, _check
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def other_kernels_only():
+    """The one-launch kernel (test_decode_lane_gpu.py) would take most of these small calls."""
+    from mlx_turboquant_b200.kernels import set_tuning
+    set_tuning("decode_lane", 0)
+    yield
+    set_tuning("decode_lane", 1)
+
+
+def _choice(c):
+    from mlx_turboquant_b200 import _lib
+    return _lib.lib().tq_decode_kernel_choice(C.byref(c._dargs))
+
+
 def _run(c, q, ref, want=3):
     from mlx_turboquant_b200 import _lib
     out = c.attend(q, out_dtype=torch.float32)
-    assert _lib.lib().tq_decode_kernel_choice(C.byref(c._dargs)) == want
+    assert _choice(c) == want
     _check(out, ref)
     assert _lib.lib().tq_device_status() == 0
     return out
@@ -71,6 +85,7 @@ def test_decode_steps_append_and_attend(dtype):
     for _ in range(5):
         kn, vn, q = r(1), r(1), r(1, 16) / d ** 0.5
         o1 = c1.decode_step(q, kn, vn)
+        assert _choice(c1) == 3
         c2.update(kn, vn)
         assert torch.equal(o1, c2.attend(q))
     assert torch.equal(c1.keys[:, :, :c1._fp16_len], c2.keys[:, :, :c2._fp16_len])

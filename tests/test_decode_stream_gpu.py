@@ -22,9 +22,11 @@ def stream_forced():
     from mlx_turboquant_b200.kernels import set_tuning
     set_tuning("decode_stream_min_run", 1)
     set_tuning("decode_stream_max_parts", 64)
+    set_tuning("decode_lane", 0)
     yield
     set_tuning("decode_stream_min_run", 24)
     set_tuning("decode_stream_max_parts", 40)
+    set_tuning("decode_lane", 1)
 
 
 def _choice(c):
