@@ -347,7 +347,7 @@ float tq_fp16_table_scale(const float* centroids_host, int n);
  *   "decode_stream_min_run" 1.. (fewest packed 16-token tiles per warp of the persistent grid for which it is chosen over the
  *   table-lookup kernel, default 24; over the general kernel a third of that),
  *   "decode_lut" 0/1/2 (the lookup kernel is never chosen, where it is the faster one, default, or whenever it can run),
- *   "decode_lane" 0/1/2 (the one-launch kernel likewise), "decode_lane_ctas" 0 (auto)..16 (its CTAs per cache lane: 1 to 6, 8, 12, 16),
+ *   "decode_lane" 0/1/2 (the one-launch kernel likewise; 1 leaves calls with a "decode_splits" to the kernels that split), "decode_lane_ctas" 0 (auto)..16 (its CTAs per cache lane: 1 to 6, 8, 12, 16),
  *   "decode_stream_max_parts" 1..64 (most partial results per lane with which it is chosen over the table-lookup kernel; default 40).
  * Changing them changes tq_decode_workspace_bytes for the same sizes. */
 int tq_set_tuning(const char* key, int value);

@@ -861,7 +861,7 @@ int decode_prepare(const tq_decode_args* a, void* workspace, size_t workspace_by
     }
     if (lut) stream = false;
     LanePlan ln{};
-    if (g_tune_lane && tab && a->c_len > 0 && a->dense_dtype != TQ_F32 && lut_supported(d, qjl, a->k_bits_hi, a->k_bits_lo, a->v_bits_hi, a->v_bits_lo)) {
+    if (g_tune_lane && (g_tune_lane == 2 || g_tune_splits == 0) && tab && a->c_len > 0 && a->dense_dtype != TQ_F32 && lut_supported(d, qjl, a->k_bits_hi, a->k_bits_lo, a->v_bits_hi, a->v_bits_lo)) {
         ln = lane_plan(r.lanes * ((r.G + HPG - 1) / HPG), d, qjl, a->k_bits_hi, a->k_bits_lo, a->v_bits_hi, a->v_bits_lo, a->c_len, dense_len, g_tune_lane_ctas);
         if (g_tune_lane == 1 && !lane_is_best(r, ln, lut ? &stp : nullptr, stream)) ln.c = 0;
     }

@@ -125,6 +125,19 @@ def test_what_it_leaves_to_the_others(oracle, lane):
         assert (takes(c) > 0) == want == (_choice(c) == 4)
 
 
+def test_a_split_count_that_is_asked_for(oracle):
+    """goes to the kernels that split, whatever the rule says of the call."""
+    from mlx_turboquant_b200.kernels import set_tuning
+    c, q, ref = _case(oracle, np.random.RandomState(7), 1, 8, 2, 700, 128, 4, 2, 32, 16)
+    try:
+        for splits, want in ((0, 4), (3, 1), (0, 4)):
+            set_tuning("decode_splits", splits)
+            _check(c.attend(q, out_dtype=torch.float32), ref)
+            assert _choice(c) == want
+    finally:
+        set_tuning("decode_splits", 0)
+
+
 @pytest.fixture()
 def off():
     from mlx_turboquant_b200.kernels import set_tuning
