@@ -9,6 +9,8 @@ library raises ``RuntimeError`` when the shared object has not been built
 from __future__ import annotations
 
 import ctypes as C
+import importlib
+import warnings
 from pathlib import Path
 
 import torch
@@ -146,21 +148,29 @@ def lib():
     return _lib
 
 
+class _NoHost:
+    """In the place of the native host path where that does not load: takes nothing, so that every caller goes its own way."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
 _host = None
 
 
 def host():
     """The native host path (csrc/host.cpp): checks, allocations and launches of the calls that are mostly host work.  Its functions return
-    None for anything but the plain case (the callers in this package then take their own path) and a negative status as it is."""
+    None for anything but the plain case (the callers in this package then take their own path) and a negative status as it is.  It is built
+    against one torch and one Python; with others the callers' own steps do the same work, slower, and a warning says so once."""
     global _host
     if _host is None:
         lib()                                             # (the module is linked against the library)
         try:
-            from . import _host as module
+            _host = importlib.import_module("._host", __package__)
         except ImportError as e:
-            raise RuntimeError(f"the native host module does not load ({e}): build it with the CUDA library "
-                               "(python -c 'import __graft_entry__ as g; g.build()')") from e
-        _host = module
+            warnings.warn(f"the native host module does not load ({e}); cache updates and codec calls take 20 to 80 us more each. Build it with the CUDA "
+                          "library (python -c 'import __graft_entry__ as g; g.build()')", RuntimeWarning, stacklevel=3)
+            _host = _NoHost()
     return _host
 
 

@@ -148,8 +148,10 @@ class _Side:
         cap = _round_up(max(need, 2 * self.capacity(), 256), 16)
         w_hi, w_lo = kernels.packed_widths(d, self.bits_hi, self.bits_lo)
         if self.hi is None and used == 0:
-            self.hi, self.lo, self.norms, self.qbits, self.qgamma = _lib.host().storage(b, h, cap, w_hi, w_lo if self.fractional else 0, with_qjl, device.index)
-            return
+            new = _lib.host().storage(b, h, cap, w_hi, w_lo if self.fractional else 0, with_qjl, device.index)
+            if new is not None:
+                self.hi, self.lo, self.norms, self.qbits, self.qgamma = new
+                return
 
         def grow(old, shape, dtype):
             if old is None and used > 0:   # a sketch that a reloaded state did not carry: zero = no correction

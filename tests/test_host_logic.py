@@ -297,3 +297,18 @@ def test_fp16_value_tables_have_no_mean_error():
             err = ((get_codebook_host(d, bits)[0] * s).astype(np.float16).astype(np.float64) / np.float64(s)) * sqrt(d) - c
             assert abs((p * err).sum()) < 2.5e-7 and sqrt((p * err * err).sum()) < 1.3e-4, (d, bits)
     assert [_fp16_scale(128, b) for b in (2, 3, 4)] == [1.49676513671875, 1.2477874755859375, 1.447540283203125]      # symmetric tables: as they were
+
+
+def test_without_the_native_host_module(monkeypatch):
+    """Another torch or Python than it was built for: a warning, and a stand-in that hands every call back to the steps in Python."""
+    import sys
+    from mlx_turboquant_b200 import _lib
+    monkeypatch.setattr(_lib, "_host", None)
+    monkeypatch.setitem(sys.modules, "mlx_turboquant_b200._host", None)           # (import fails)
+    with pytest.warns(RuntimeWarning, match="native host module"):
+        host = _lib.host()
+    for name in ("codec_quantize", "codec_dequantize", "append", "buffers", "storage", "quantize", "fetch"):
+        assert getattr(host, name)(1, 2, 3) is None
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        assert _lib.host() is host                                                # (said once)

@@ -63,3 +63,24 @@ def test_prompt_in_any_layout(kb, vb, qjl, d):
     assert a.meta_state == b.meta_state and a.empty() is False
     for x, y in zip(a.state, b.state):
         assert (x is None) == (y is None) and (x is None or torch.equal(x, y))
+
+
+@pytest.mark.parametrize("qjl", (False, True))
+@pytest.mark.parametrize("kb,vb", ((4, 2), (3.5, 3)))
+def test_the_python_steps_do_the_same(monkeypatch, kb, vb, qjl):
+    """Without the native module: the same bytes in every array, the same dense results, the same codec."""
+    from mlx_turboquant_b200 import TurboQuantKVCache, TurboQuantMSE, _lib
+
+    def run():
+        g = torch.Generator(device="cuda").manual_seed(5)
+        c = TurboQuantKVCache(head_dim=96, num_kv_heads=3, key_bits=kb, value_bits=vb, residual_window=32, fp16_sink_size=8, qjl_correction=qjl)
+        out = [c.update_and_fetch(_rows(g, 2, 3, n, 96), _rows(g, 2, 3, n, 96)) for n in (300, 1, 5, 90)]
+        m = TurboQuantMSE(96, 4)
+        z = m.quantize(_rows(g, 50, 96))
+        n = c._compressed_len
+        sides = [x[:, :, :n].clone() for s in (c._k, c._v) for x in (s.hi, s.lo, s.norms, s.qbits, s.qgamma) if x is not None]
+        return [x for kv in out for x in kv] + sides + [z.packed_indices, z.norms, m.dequantize(z)]
+
+    native = run()
+    monkeypatch.setattr(_lib, "_host", _lib._NoHost())
+    assert all(torch.equal(a, b) for a, b in zip(run(), native, strict=True))
