@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes as C
 import importlib
+import sys
 import warnings
 from pathlib import Path
 
@@ -148,6 +149,11 @@ def lib():
     return _lib
 
 
+def host_abi() -> str:
+    """What the native host module is built against and must be loaded with."""
+    return f"torch {torch.__version__}, C++11 ABI {int(torch._C._GLIBCXX_USE_CXX11_ABI)}, Python {sys.version_info[0]}.{sys.version_info[1]}"
+
+
 class _NoHost:
     """In the place of the native host path where that does not load: takes nothing, so that every caller goes its own way."""
 
@@ -166,8 +172,11 @@ def host():
     if _host is None:
         lib()                                             # (the module is linked against the library)
         try:
-            _host = importlib.import_module("._host", __package__)
-        except ImportError as e:
+            module = importlib.import_module("._host", __package__)
+            if module.built_for != host_abi():            # (inline code of torch's headers: another layout would not show at import)
+                raise ImportError(f"built for {module.built_for}, this is {host_abi()}")
+            _host = module
+        except (ImportError, AttributeError) as e:
             warnings.warn(f"the native host module does not load ({e}); cache updates and codec calls take 20 to 80 us more each. Build it with the CUDA "
                           "library (python -c 'import __graft_entry__ as g; g.build()')", RuntimeWarning, stacklevel=3)
             _host = _NoHost()

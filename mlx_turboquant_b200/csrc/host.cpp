@@ -304,4 +304,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Native host path; see csr
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__host() {
+    PyObject* m = PyModule_Create(&module);
+    if (m && PyModule_AddStringConstant(m, "built_for", TQ_BUILT_FOR)) Py_CLEAR(m);       // (the loader compares it with what is running)
+    return m;
+}

@@ -299,12 +299,13 @@ def test_fp16_value_tables_have_no_mean_error():
     assert [_fp16_scale(128, b) for b in (2, 3, 4)] == [1.49676513671875, 1.2477874755859375, 1.447540283203125]      # symmetric tables: as they were
 
 
-def test_without_the_native_host_module(monkeypatch):
-    """Another torch or Python than it was built for: a warning, and a stand-in that hands every call back to the steps in Python."""
+@pytest.mark.parametrize("module", (None, types.SimpleNamespace(built_for="torch 1.0, C++11 ABI 0, Python 3.6"), types.SimpleNamespace()))
+def test_without_the_native_host_module(monkeypatch, module):
+    """It does not import, or was built for another torch or Python: a warning, and a stand-in that hands every call back to the steps in Python."""
     import sys
     from mlx_turboquant_b200 import _lib
     monkeypatch.setattr(_lib, "_host", None)
-    monkeypatch.setitem(sys.modules, "mlx_turboquant_b200._host", None)           # (import fails)
+    monkeypatch.setitem(sys.modules, "mlx_turboquant_b200._host", module)         # (None: import fails)
     with pytest.warns(RuntimeWarning, match="native host module"):
         host = _lib.host()
     for name in ("codec_quantize", "codec_dequantize", "append", "buffers", "storage", "quantize", "fetch"):
@@ -312,3 +313,16 @@ def test_without_the_native_host_module(monkeypatch):
     with warnings.catch_warnings():
         warnings.simplefilter("error")
         assert _lib.host() is host                                                # (said once)
+
+
+def test_the_host_module_is_rebuilt_for_another_torch(tmp_path):
+    """The build keeps what the module was compiled against, not only when."""
+    import __graft_entry__ as entry
+    src, lib, abi_file = tmp_path / "host.cpp", tmp_path / "_host.so", tmp_path / "host_abi.txt"
+    src.write_text("")
+    assert entry._host_stale(lib, [src], abi_file, "torch 2")
+    lib.write_text("")
+    assert entry._host_stale(lib, [src], abi_file, "torch 2")                     # (against what is not known)
+    abi_file.write_text("torch 2")
+    assert not entry._host_stale(lib, [src], abi_file, "torch 2")
+    assert entry._host_stale(lib, [src], abi_file, "torch 3")
