@@ -758,14 +758,14 @@ static bool lut_is_best(const LutRivals& r) {
     return !(fp16 && r.G == 1 && r.d <= 96 && tiles < (r.qjl ? r.d == 64 ? 5000 : 0 : 7000));
 }
 
-// Whether the one-launch kernel of decode_lane.cu takes a call that it can run: its plan's cost against what the other kernel takes, in us
+// The one-launch kernel of decode_lane.cu takes a call that it can run where its plan costs less than this, by what the other kernel takes, in us
 // (both fitted to 965 measured calls, log errors 0.06 to 0.12; other / one launch).  Lookup kernel: 8 lanes x 48 + 16 tiles at d = 96 16.6 /
 // 8.4, 3 x 369 27.9 / 14.3, 160 x 67 40.3 / 28.4, 32 x 737 38.0 / 32.8, 64 x 1108 59.3 / 58.4, 8 x 1825 at d = 256 55.3 / 77.8, 736 x 102 73.6
 // / 109.  Table-lookup kernel: 8 x 38 tiles 11.9 / 8.4, 8 x 2048 17.0 / 33.8; bfloat16 4 x 113 23.2 / 11.3.  General kernel: 8.7 / 8.5,
 // 16.8 / 12.2, 216 x 49 at d = 64 23.4 / 13.6.  Streaming kernel: while its warps' runs are short (256 x 109 tiles at d = 96 36.2 / 26.2, 248
 // x 218 50.3 / 42.1; 448 x 641 at d = 128 157 / 255).  Of those calls 597 go to one launch, five of them more than 3 % slower.
-static bool lane_is_best(const LutRivals& r, const LanePlan& ln, const StreamPlan* lut, bool stream) {
-    if (!lut && stream && r.run >= 2 * g_tune_stream_min_run) return false;
+static double lane_limit(const LutRivals& r, const StreamPlan* lut, bool stream) {
+    if (!lut && stream && r.run >= 2 * g_tune_stream_min_run) return 0.0;
     const int heads = std::min(r.G, HPG);
     const double dd = r.d / 128.0, tiles = double(r.p_tiles + r.d_tiles), lanes = double(r.lanes * ((r.G + HPG - 1) / HPG)), per_sm = lanes * tiles / r.sms;
     const double bf16 = r.dense_dtype == TQ_BF16, many = r.G > 4, qjl = r.qjl, wide = r.wide;
@@ -776,7 +776,7 @@ static bool lane_is_best(const LutRivals& r, const LanePlan& ln, const StreamPla
     else if (r.direct) other = 9.1 + 0.42 * std::min(r.G, 4) + 6.2 * bf16 + 5.0 * many + 0.095 * per_sm + 11.3 * std::max(0.0, 2.0 * lanes / r.sms - 1.0);
     else other = 7.9 + (r.d == 96 ? 4.9 : 0.0) + 3.9 * many + 1.8 * bf16 + 0.25 * std::min(r.G, 4) + 0.063 * per_sm + 0.0055 * tiles + 0.026 * lanes +
                  9.7 * std::max(0.0, lanes / r.sms - 1.0);
-    return ln.cost + 1.2 * many < 0.9 * other;
+    return 0.9 * other - 1.2 * many;
 }
 
 // Validates the arguments, picks the path and the split plan and fills the kernel parameters.
@@ -862,8 +862,8 @@ int decode_prepare(const tq_decode_args* a, void* workspace, size_t workspace_by
     if (lut) stream = false;
     LanePlan ln{};
     if (g_tune_lane && (g_tune_lane == 2 || g_tune_splits == 0) && tab && a->c_len > 0 && a->dense_dtype != TQ_F32 && lut_supported(d, qjl, a->k_bits_hi, a->k_bits_lo, a->v_bits_hi, a->v_bits_lo)) {
-        ln = lane_plan(r.lanes * ((r.G + HPG - 1) / HPG), d, qjl, a->k_bits_hi, a->k_bits_lo, a->v_bits_hi, a->v_bits_lo, a->c_len, dense_len, g_tune_lane_ctas);
-        if (g_tune_lane == 1 && !lane_is_best(r, ln, lut ? &stp : nullptr, stream)) ln.c = 0;
+        ln = lane_plan(r.lanes * ((r.G + HPG - 1) / HPG), d, qjl, a->k_bits_hi, a->k_bits_lo, a->v_bits_hi, a->v_bits_lo, a->c_len, dense_len, g_tune_lane_ctas, r.sms,
+                       g_tune_lane == 1 ? lane_limit(r, lut ? &stp : nullptr, stream) : INFINITY);
     }
     const SplitPlan sp = plan_splits(a->batch, a->n_q_heads, a->n_kv_heads, a->c_len, dense_len, sm_count(), direct);
     const WsLayout wl = ws_layout(a->batch, a->n_q_heads, a->n_kv_heads, d, sp);

@@ -106,7 +106,7 @@ StreamPlan lut_plan(int batch, int n_q_heads, int n_kv_heads, int d, int64_t c_l
 int launch_decode_lut(const DecodeParams& p, cudaStream_t s);
 // decode_lane.cu: the lookup kernel's operands in one launch, a cluster of CTAs per lane.
 struct LanePlan { int c, per_sm, pw, dw, ns; double cost; };       // (c = 0: it does not take the call)
-LanePlan lane_plan(int64_t lanes, int d, bool qjl, int kb_hi, int kb_lo, int vb_hi, int vb_lo, int64_t c_len, int64_t dense_len, int force_c);
+LanePlan lane_plan(int64_t lanes, int d, bool qjl, int kb_hi, int kb_lo, int vb_hi, int vb_lo, int64_t c_len, int64_t dense_len, int force_c, int sms, double below);
 int launch_decode_lane(const DecodeParams& p, cudaStream_t s);
 int launch_gather_wait(const unsigned long long* ll, const unsigned* epochs, int64_t n_words, void* out, int max_polls, cudaStream_t s);
 int* decode_status_ptr();          // device address of the status word on the current device (null on error)

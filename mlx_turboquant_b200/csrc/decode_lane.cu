@@ -756,17 +756,36 @@ template <int D> static int launch(const DecodeParams& p, cudaStream_t s) {
 // call's, whose tables are then no longer filled under this one (64 lanes x 34 tiles, 128 CTAs: 12.9; 8 x 38, 32 CTAs: 8.4), and the tiles
 // of the busiest warp: twice as much each when two CTAs share an SM (32 lanes x 737 tiles at 3.5 bits: 32.8 with 128 CTAs, 33.3 with 256
 // on as many SMs: clusters are packed onto pairs even where SMs are free); an uncompressed tile counts as 1.6.
-LanePlan lane_plan(int64_t lanes, int d, bool qjl, int kb_hi, int kb_lo, int vb_hi, int vb_lo, int64_t c_len, int64_t dense_len, int force_c) {
+// below: only a plan that costs less is of use.  A long context is turned away by a bound that takes no division: every warp has its share of
+// the tiles at least, and so has every SM.  (Host time of a call's checks and choice: 8 lanes x 32,768 tokens 1.35 us with all plans made, 0.71 now, 0.61
+// without this kernel; 8 lanes x 600, which it takes, 0.97 / 0.78 / 0.49.)
+LanePlan lane_plan(int64_t lanes, int d, bool qjl, int kb_hi, int kb_lo, int vb_hi, int vb_lo, int64_t c_len, int64_t dense_len, int force_c, int sms, double below) {
     LanePlan best{};
     const int64_t p_tiles = (c_len + TILE - 1) / TILE, d_tiles = (dense_len + TILE - 1) / TILE;
     const bool any3 = kb_hi == 3 || kb_lo == 3 || vb_hi == 3 || vb_lo == 3;
     const int rows = c_len > 0 ? packed_bytes(kb_lo ? d / 2 : d, kb_hi) + (kb_lo ? packed_bytes(d / 2, kb_lo) : 0) + packed_bytes(vb_lo ? d / 2 : d, vb_hi) +
                                      (vb_lo ? packed_bytes(d / 2, vb_lo) : 0) : 0;
     if (lanes <= 0 || p_tiles + d_tiles == 0 || p_tiles + d_tiles > (int64_t(1) << 24)) return best;
+    const int max_per_sm = d == 256 ? 1 : 2;
+    const double dd = double(d) / 128.0, work = double(p_tiles) + 1.6 * double(d_tiles);       // packed tiles' worth
+    double tile_us[3], least[3];                                       // per tile; per tile of a lane, at least, by the share of a warp and of an SM
+    for (int per_sm = 1; per_sm <= max_per_sm; ++per_sm) {
+        tile_us[per_sm] = 0.15 + (per_sm == 1 ? 0.61 : 1.29) * dd + 0.45 * dd * qjl + 0.09 * dd * (rows * 16 >= d * 13);
+        least[per_sm] = tile_us[per_sm] / dl::NW * std::max(1.0 / dl::MAX_C, double(lanes) / double(sms * per_sm));
+    }
+    if (2.25 + 5.4 * dd + work * std::min(least[1], least[max_per_sm]) >= below) return best;
+    const dl::Room* room[3];
+    int ns[3];
+    for (int per_sm = 1; per_sm <= max_per_sm; ++per_sm) {
+        room[per_sm] = &dl::room(d, qjl, per_sm);
+        ns[per_sm] = dl::stages(d, qjl, per_sm, any3, rows);
+    }
+    best.cost = below;
     for (int i = 0; i < dl::N_SIZES; ++i) {
         const int c = dl::SIZES[i], nw = dl::NW * c;
         if (force_c > 0 ? c != force_c : c > 1 && dl::NW * dl::SIZES[i - 1] >= p_tiles + d_tiles) continue;       // (a tile per warp already)
         if (lanes * c >= (int64_t(1) << 31)) break;
+        if (2.1 + 0.15 * c + 5.4 * dd + work / nw * std::min(tile_us[1], tile_us[max_per_sm]) >= best.cost * 1.000001) continue;
         // packed warps so that both kinds take as long; costs in tenths of a packed tile
         const int64_t dc = d_tiles * 16, w0 = nw * p_tiles * 10 / (p_tiles * 10 + dc);
         const int lo = p_tiles > 0 ? 1 : 0, hi = d_tiles > 0 ? nw - 1 : nw;
@@ -778,16 +797,15 @@ LanePlan lane_plan(int64_t lanes, int d, bool qjl, int kb_hi, int kb_lo, int vb_
             else if (pw - 1 >= lo && load(pw - 1) < load(pw)) --pw;
         }
         const double tiles = 0.1 * double(load(pw));
-        for (int per_sm = 1; per_sm <= (d == 256 ? 1 : 2); ++per_sm) {
+        for (int per_sm = 1; per_sm <= max_per_sm; ++per_sm) {
             // (the last few clusters of pairs do not find their places: 72 lanes x 4 CTAs, of 74 that fit, take two waves)
-            const int fit = dl::room(d, qjl, per_sm).clusters[i], at_once = per_sm == 2 && c > 2 ? fit * 15 / 16 : fit, ns = dl::stages(d, qjl, per_sm, any3, rows);
-            if (at_once == 0 || ns < 2) continue;                      // (two stages at least: 3.5 / 3.5 bits with sketches have an SM to themselves)
+            const int fit = room[per_sm]->clusters[i], at_once = per_sm == 2 && c > 2 ? fit * 15 / 16 : fit;
+            if (at_once == 0 || ns[per_sm] < 2) continue;              // (two stages at least: 3.5 / 3.5 bits with sketches have an SM to themselves)
             const int64_t waves = (lanes + at_once - 1) / at_once;
-            const double dd = double(d) / 128.0, full = std::clamp((double(lanes) / double(at_once) - 0.4) / 0.3, 0.0, 1.0);
-            const double tile_us = 0.15 + (per_sm == 1 ? 0.61 : 1.29) * dd + 0.45 * dd * qjl + 0.09 * dd * (rows * 16 >= d * 13);
-            const double cost = double(waves) * (2.1 + 0.15 * c + 5.4 * dd + full * (1.3 + 2.9 * dd) + tile_us * tiles);
-            if (best.c > 0 && cost >= best.cost) continue;
-            best.c = c; best.per_sm = per_sm; best.ns = ns; best.cost = cost;
+            const double full = std::clamp((double(lanes) / double(at_once) - 0.4) / 0.3, 0.0, 1.0);
+            const double cost = double(waves) * (2.1 + 0.15 * c + 5.4 * dd + full * (1.3 + 2.9 * dd) + tile_us[per_sm] * tiles);
+            if (cost >= best.cost) continue;
+            best.c = c; best.per_sm = per_sm; best.ns = ns[per_sm]; best.cost = cost;
             best.pw = int(std::min<int64_t>(pw, p_tiles)); best.dw = int(std::min<int64_t>(nw - pw, d_tiles));
         }
     }

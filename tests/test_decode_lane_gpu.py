@@ -191,3 +191,26 @@ def test_nan_reaches_the_result(lane, ctas, d, kb, vb, dtype, where):
     assert _taken(c) == ctas
     assert out[:4, columns].isnan().all()
     assert out[4:].isfinite().all()
+
+
+def test_the_rule_and_the_sizes(oracle):
+    """A bound turns calls away before their plans are made: none with a plan that the rule would take.  (With a forced size the rule sees that plan
+    alone, so it takes the call at some forced size exactly when it takes it at the size of its choice.)"""
+    from mlx_turboquant_b200 import _lib
+    from mlx_turboquant_b200.kernels import set_tuning
+    f = _lib.lib().tq_decode_one_launch
+    taken = 0
+    for b, h, t, d in ((1, 8, 600, 128), (1, 2, 3000, 128), (4, 8, 2000, 96), (1, 8, 9000, 64), (16, 8, 700, 128), (2, 4, 6000, 256), (1, 1, 20000, 128), (40, 8, 300, 64)):
+        a = _lib.DecodeArgs(batch=b, n_q_heads=4 * h, n_kv_heads=h, d=d, c_len=t, c_lane_stride=(t + 15) // 16 * 16, k_bits_hi=3, v_bits_hi=3, sink_len=128, sink_lane_stride=128,
+                            res_len=100, res_lane_stride=512, scale=0.1, v_cent_scale_hi=1.0, v_cent_scale_lo=1.0, workspace_bytes=1 << 40)
+        for name in ("q", "rot", "k_hi", "v_hi", "k_norms", "v_norms", "k_cent_hi", "v_cent_hi", "sink_k", "sink_v", "res_k", "res_v", "out", "workspace"):
+            setattr(a, name, 1 << 40)                                    # (aligned; nothing is launched)
+        own = f(C.byref(a))
+        forced = set()
+        for ctas in (1, 2, 3, 4, 5, 6, 8, 12, 16):
+            set_tuning("decode_lane_ctas", ctas)
+            forced.add(f(C.byref(a)))
+        set_tuning("decode_lane_ctas", 0)
+        assert own >= 0 and own in forced and (own > 0) == (max(forced) > 0)
+        taken += own > 0
+    assert 0 < taken < 8
