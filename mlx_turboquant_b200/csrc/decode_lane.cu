@@ -679,9 +679,10 @@ template <int D, bool QJL, int PER_SM> static const Room& room() {
     if (known[dev].load(std::memory_order_acquire)) return rooms[dev];
     Room r{};
     const unsigned sb = dd::probe_smem_base();
+    if (sb == ~0u) return none;                                // (no answer this time, not no room: asked again at the next call)
     int max_optin = 0;
     auto kernel = decode_lane_kernel<D, QJL, PER_SM>;
-    if (sb != ~0u && sb <= LO_BASE && (sb & 15u) == 0 && cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
+    if (sb <= LO_BASE && (sb & 15u) == 0 && cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
         smem_bytes<D, QJL, PER_SM>() <= size_t(max_optin) &&
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes<D, QJL, PER_SM>())) == cudaSuccess) {
         const bool large = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;

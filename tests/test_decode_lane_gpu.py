@@ -214,3 +214,32 @@ def test_the_rule_and_the_sizes(oracle):
         assert own >= 0 and own in forced and (own > 0) == (max(forced) > 0)
         taken += own > 0
     assert 0 < taken < 8
+
+
+FIRST_CALL = """
+import ctypes as C, torch
+from mlx_turboquant_b200 import TurboQuantKVCache, _lib
+g = torch.Generator(device="cuda").manual_seed(1)
+r = lambda h, n: torch.randn(1, h, n, 128, device="cuda", generator=g).half()
+c = TurboQuantKVCache(head_dim=128, num_kv_heads=4, key_bits=3, value_bits=3, residual_window=32, fp16_sink_size=16)
+c.update(r(4, 500), r(4, 500))
+q = r(16, 1) / 11
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    out = c.attend(q)
+assert _lib.lib().tq_decode_kernel_choice(C.byref(c._dargs)) == 4
+out.zero_()
+graph.replay()
+torch.cuda.synchronize()
+assert torch.equal(out, c.attend(q)) and out.abs().max() > 0 and _lib.lib().tq_device_status() == 0
+"""
+
+
+def test_the_first_call_of_a_process_under_capture():
+    """What the kernel asks the device for once (where its shared memory begins, how many clusters fit) must not end the capture."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    run = subprocess.run([sys.executable, "-c", FIRST_CALL], cwd=Path(__file__).resolve().parent.parent, capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr
