@@ -34,7 +34,7 @@
 //     are two key tiles ahead of the softmax;
 //   * between the two regions the softmax warps leave O as high and low fp16 parts where the scores were, the MMA warp multiplies
 //     them with R's parts in place (three products, the small ones first) and the raw queries replace the rotated ones.
-//   512 queries x 32 lanes over 16,384 tokens at d = 128: 610 us = 880 TFLOP/s (350 with the unpacking inside the kernel).
+//   512 queries x 32 lanes over 16,384 tokens at d = 128: 580 us = 930 TFLOP/s (350 with the unpacking inside the kernel).
 //
 // Every mbarrier wait is bounded; a wait that runs out leaves status 111 (tq_device_status) and raises a flag that ends
 // every other wait; copies and products in flight are waited for (bounded), tensor memory is freed on every path.
@@ -1236,9 +1236,9 @@ bool prefill_fa_applicable(const tq_decode_args* a, int t_q) {
 
 // Whether prefill_tc.cu, which unpacks as it goes, is the faster one of two that take the call: with a single block of 128 query rows
 // per lane nothing is unpacked twice there, and the expansion here costs as much as the attention.  Its time goes by waves of CTAs, a
-// lane each, this one's by lanes x tokens; us on 148 SMs, fa / tc, 4-bit keys and 2-bit values at d = 128 (other widths: always fa):
-// 64 lanes x 8192 195 / 292, 112 x 8192 313 / 330, 128 x 8192 387 / 331, 112 x 16384 604 / 521, 128 x 4000 187 / 199, 160 x 8192 499 / 632,
-// 224 x 8192 627 / 640, 256 x 8192 770 / 658.
+// lane each, this one's by lanes x tokens; us on 148 SMs, fa / tc, 32 queries of 4 heads, 4-bit keys and 2-bit values at d = 128 (other widths:
+// always fa): 64 lanes x 8192 175 / 294, 112 x 8192 285 / 332, 128 x 8192 348 / 336, 112 x 16384 541 / 526, 128 x 4000 171 / 199, 160 x 8192 443 /
+// 644, 224 x 8192 568 / 666, 256 x 8192 695 / 676.  (A sweep of 236 calls of 16 to 296 lanes: the rule's choice is never more than 3 % slower than the other.)
 bool prefill_tc_faster(const tq_decode_args* a, int t_q) {
     const int g = a->n_q_heads / a->n_kv_heads, gp = g <= 1 ? 1 : g <= 2 ? 2 : g <= 4 ? 4 : 8;
     if (a->d != 128 || a->k_bits_hi != 4 || a->k_bits_lo || a->v_bits_hi != 2 || a->v_bits_lo || t_q > fa::TM / gp) return false;
